@@ -24,273 +24,12 @@
 #include <unordered_map>
 
 #include "kernels.cuh"
+#include "tcgen05.cuh"
 
 namespace b200 {
 namespace {
 
-constexpr int BM = 128;
-constexpr int BK = 64;  // 64 16-bit elements = one 128-byte swizzle row
 constexpr int kThreads = 352;  // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue (two groups of four), warp 10 stores
-constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
-
-// ---- PTX wrappers ------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok;
-}
-// Same with a suspend-time hint: the thread may sleep in hardware for up to `ns` nanoseconds (it is woken when the
-// phase completes), so a long wait costs few issue slots of the warps that share its scheduler.
-__device__ __forceinline__ uint32_t mbar_try_wait_hint(uint32_t bar, uint32_t parity, uint32_t ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(ns)
-      : "memory");
-  return ok;
-}
-// Bounded wait.  Returns false when the CTA is aborting (this or another role timed out).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait_hint(bar, parity, 20000u)) return true;
-    if ((it & 63) == 0) {
-      if (*abort_flag) return false;
-      if (global_ns() - t0 > kWaitLimitNs) {
-        *abort_flag = code;
-        return false;
-      }
-    }
-  }
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-// 4D tile load (channels, file, rank, position); coordinates may lie outside the tensor, those elements are
-// zero-filled, which is exactly the zero padding of a same-padded convolution on the 8x8 board.
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
-                                            uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
-      : "memory");
-}
-// Brings a tensor map into the descriptor cache ahead of its first use (the first TMA store of a launch otherwise
-// waited about three microseconds for it).
-__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                   reinterpret_cast<uint64_t>(map)),
-               "r"(src), "r"(x), "r"(y)
-               : "memory");
-}
-__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Waits until at most one of this thread's bulk groups still reads its shared-memory source.
-__device__ __forceinline__ void tma_store_wait_read1() {
-  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-}
-__device__ __forceinline__ void tma_store_wait_read0() {
-  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-__device__ __forceinline__ void tma_store_wait_all0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tcgen05_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tcgen05_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tcgen05_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void tcgen05_mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                                uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-
-// ---- CTA-pair (cta_group::2) helpers -------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// shared::cluster address of the same shared-memory offset in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Arrival on a barrier of a CTA of the cluster.  Relaxed: the arrivals of this kernel only hand tensor memory back
-// to the MMA issuer (ordered by tcgen05.fence), no generic-proxy data is published through them; a release at
-// cluster scope here stalled the arriving thread for 2-3 thousand cycles per tile.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// TMA load whose completion is signalled on a barrier that may live in the peer CTA of the pair (no multicast:
-// each CTA of the pair fetches its own half of the operands).
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
-                                                 uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tcgen05_commit_pair(uint32_t cluster_bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar)
-               : "memory");
-}
-__device__ __forceinline__ void tcgen05_mma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                                     uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major operand tile stored as rows of 128 bytes with the 128-byte
-// swizzle (what a TMA box of 64 16-bit elements x R rows with CU_TENSOR_MAP_SWIZZLE_128B produces):
-// start address >> 4 in bits [0,14), stride between 8-row groups (1024 B) >> 4 in bits [32,46),
-// descriptor version 1 in bits [46,48), layout type 2 (SWIZZLE_128B) in bits [61,64).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
-// Activation of a register array with the selection hoisted out of the element loop.
-template <int N>
-__device__ __forceinline__ void apply_activation(float (&v)[N], int act) {
-  switch (act) {
-    case ACT_RELU:
-#pragma unroll
-      for (int j = 0; j < N; ++j) v[j] = fmaxf(v[j], 0.f);
-      break;
-    case ACT_RELU_2:
-#pragma unroll
-      for (int j = 0; j < N; ++j) { const float t = fmaxf(v[j], 0.f); v[j] = t * t; }
-      break;
-    case ACT_MISH:
-#pragma unroll
-      for (int j = 0; j < N; ++j) v[j] = mish_f(v[j]);
-      break;
-    case ACT_SWISH:
-#pragma unroll
-      for (int j = 0; j < N; ++j) v[j] = swish_f(v[j]);
-      break;
-    case ACT_NONE:
-      break;
-    default:
-#pragma unroll
-      for (int j = 0; j < N; ++j) v[j] = activate<true>(v[j], act);
-      break;
-  }
-}
-
-template <typename T> struct FmtCode;
-template <> struct FmtCode<__half> { static constexpr uint32_t v = 0; };
-template <> struct FmtCode<__nv_bfloat16> { static constexpr uint32_t v = 1; };
-
-// Instruction descriptor of tcgen05.mma.kind::f16: D format fp32 (bits 4-5 = 1), A/B format (bits 7-9,
-// 10-12: 0 = f16, 1 = bf16), both operands K-major (bits 15, 16 = 0), N >> 3 in bits 17-22, M >> 4 in bits 24-28.
-template <typename T, int BN>
-__device__ __forceinline__ constexpr uint32_t make_idesc() {
-  return (1u << 4) | (FmtCode<T>::v << 7) | (FmtCode<T>::v << 10) | ((uint32_t)(BN >> 3) << 17) |
-         ((uint32_t)(BM >> 4) << 24);
-}
-
-struct TcParams {
-  const float* bias;
-  void* C;
-  long long ldc;
-  int M, N, K;
-  int act;
-  float scale, alpha;
-  int out_f32;
-  int* status;
-  int tma_store;  // 1: 16-bit output staged in shared memory and written with TMA stores
-  // CTA-pair kernel: the tiles from split_from on are computed as two half-width tiles each (tiles_v virtual tiles in
-  // all), so that a last, less than half filled wave spreads over all pairs; split_from >= tiles_v means no split
-  int split_from, tiles_v;
-  int conv_cblocks;  // > 0: 3x3 convolution, number of 64-channel blocks of the input (k_blocks = 9 * conv_cblocks)
-  // folded LayerNorm (see GemmParams)
-  const double* a_stats; const float* colsum; float a_inv_c, a_eps;
-  int res_mode;  // 0 none, 1 add the residual tile, 2 add the normalised residual tile
-  const double* res_stats; const float* res_gamma; const float* res_beta; float res_inv_c, res_eps;
-  double* out_stats;
-  int n_split;  // > 0: columns from here on are stored through the second output map
-  // Squeeze-excitation unit fused into the epilogue of a convolution whose tile holds two whole boards and every
-  // output channel (se_k > 0; see GemmParams).
-  const float* se_w1; const float* se_b1; const float* se_w2; const float* se_b2; const float* se_bias; int se_k;
-  int batch_rows;  // > 0: stacked products, rows [b * batch_rows, (b + 1) * batch_rows) use W rows [b * N, (b + 1) * N)
-};
-
 // Per-thread (= per output row) state of the folded-LayerNorm epilogue.
 // The sums are kept in double: a row whose mean is a hundred standard deviations from zero loses the variance's
 // leading digits in fp32 (sum of squares minus squared mean), which the two-pass reference does not.
@@ -298,14 +37,6 @@ struct RowCtx {
   float mean_a = 0.f, rstd_a = 1.f, mean_r = 0.f, rstd_r = 1.f;
   double sum = 0.0, sumsq = 0.0;
 };
-__device__ __forceinline__ void mean_rstd(const double* stats, long long m, float inv_c, float eps, float& mean,
-                                          float& rstd) {
-  const double2 st = *reinterpret_cast<const double2*>(stats + 2 * m);
-  const double mu = st.x * (double)inv_c;
-  const double var = fmax(st.y * (double)inv_c - mu * mu, 0.0);
-  mean = (float)mu;
-  rstd = rsqrtf((float)var + eps);
-}
 __device__ __forceinline__ void load_row_ctx(const TcParams& p, int m, RowCtx& rc) {
   rc.sum = 0.0;
   rc.sumsq = 0.0;
@@ -317,18 +48,6 @@ __device__ __forceinline__ void flush_row_ctx(const TcParams& p, int m, const Ro
     atomicAdd(p.out_stats + 2 * (long long)m, rc.sum);
     atomicAdd(p.out_stats + 2 * (long long)m + 1, rc.sumsq);
   }
-}
-
-// Packs two floats into one 32-bit pair of T; fp16 saturates to the largest finite value.
-template <typename T> __device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t pack_pair<__half>(float lo, float hi) {
-  uint32_t r;
-  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));  // first source -> upper half
-  return r;
-}
-template <> __device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float lo, float hi) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 // One 64-column slab of the epilogue fast path, executed by one group of four warps: TMEM -> registers ->
@@ -1639,18 +1358,6 @@ cudaError_t get_map(const void* ptr, long long ld, int rows, int cols, int box_r
   return cudaSuccess;
 }
 
-void fill_folded(TcParams& p, const GemmParams& g) {
-  p.a_stats = g.a_stats; p.colsum = g.colsum; p.a_inv_c = g.a_inv_c; p.a_eps = g.a_eps;
-  p.res_mode = g.res ? (g.res_stats ? 2 : 1) : 0;
-  p.res_stats = g.res_stats; p.res_gamma = g.res_gamma; p.res_beta = g.res_beta;
-  p.res_inv_c = g.res_inv_c; p.res_eps = g.res_eps;
-  p.out_stats = g.out_stats;
-  p.n_split = 0;
-  p.se_w1 = g.se_w1; p.se_b1 = g.se_b1; p.se_w2 = g.se_w2; p.se_b2 = g.se_b2; p.se_bias = g.se_bias;
-  p.se_k = g.se_k;
-  p.batch_rows = g.batch_rows;
-}
-
 // 4D map over a token-major activation [positions][8][8][channels]; box = 64 channels x 8 x 8 x 2 boards
 // (128 GEMM rows).  Not cached: convolution inputs are few and the encode call is a host-side pure function.
 cudaError_t make_board_map(const void* ptr, int channels, int positions, int prec, CUtensorMap* out) {
@@ -1714,13 +1421,9 @@ cudaError_t launch_bn(const GemmParams& g, int* status, int sm_count, cudaStream
     if (e != cudaSuccess) return e;
   }
   TcParams p;
-  fill_folded(p, g);
+  fill_tc_params(p, g, status);
+  p.n_split = 0;
   p.tma_store = tma_store ? 1 : 0;
-  p.split_from = 0x7fffffff; p.tiles_v = 0;
-  p.bias = g.bias; p.C = g.C; p.ldc = g.ldc;
-  p.M = g.M; p.N = g.N; p.K = g.K; p.act = g.act; p.scale = g.scale; p.alpha = g.alpha;
-  p.out_f32 = g.out_f32 ? 1 : 0; p.status = status;
-  p.conv_cblocks = g.conv_cin > 0 ? ceil_div(g.conv_cin, BK) : 0;
   const int tiles = ceil_div(g.M, BM) * ceil_div(g.N, BN);
   const int grid = tiles < sm_count ? tiles : sm_count;
   return launch_dependent(gemm_tc_kernel<T, BN>, dim3(grid), dim3(kThreads), Cfg::kSmemBytes, s, ma, mw, mc, mr, p);
@@ -1762,13 +1465,8 @@ cudaError_t launch_pair(const GemmParams& g, int* status, int sm_count, cudaStre
     if (e != cudaSuccess) return e;
   }
   TcParams p;
-  fill_folded(p, g);
-  p.n_split = g.n_split;
+  fill_tc_params(p, g, status);
   p.tma_store = 1;
-  p.bias = g.bias; p.C = g.C; p.ldc = g.ldc;
-  p.M = g.M; p.N = g.N; p.K = g.K; p.act = g.act; p.scale = g.scale; p.alpha = g.alpha;
-  p.out_f32 = 0; p.status = status;
-  p.conv_cblocks = conv ? ceil_div(g.conv_cin, BK) : 0;
   const int tiles = ceil_div(g.M, 2 * BM) * ceil_div(g.N, Cfg::BN);
   const int max_pairs = sm_count / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
@@ -1827,6 +1525,10 @@ cudaError_t tma_encode_2d(const void* ptr, long long ld, long long rows, int col
   return cudaSuccess;
 }
 
+cudaError_t gemm_tensor_map(const void* ptr, long long ld, int rows, int cols, int box_rows, int prec, CUtensorMap* out) {
+  return get_map(ptr, ld, rows, cols, box_rows, prec, out);
+}
+
 bool gemm_tc_supported(const GemmParams& p) {
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if (p.conv_cin > 0)
@@ -1859,10 +1561,12 @@ bool pair_eligible(const GemmParams& p, int sm_count) {
 }
 }  // namespace
 
-bool gemm_tc_split_supported(const GemmParams& p, int sm_count) {
-  return gemm_tc_supported(p) && pair_eligible(p, sm_count) && p.n_split > 0 && (p.n_split % 256) == 0 &&
-         p.N > p.n_split && p.N - p.n_split <= 256 && p.C2 && (p.ldc2 % 8) == 0 &&
-         (reinterpret_cast<uintptr_t>(p.C2) & 15) == 0 && !p.res && !p.out_stats && !p.skip;
+bool gemm_tc_split_supported(const GemmParams& p) {
+  if (!gemm_tc_supported(p) || p.n_split <= 0 || p.N <= p.n_split || !p.C2 || (p.ldc2 % 8) != 0 ||
+      (reinterpret_cast<uintptr_t>(p.C2) & 15) != 0 || p.res || p.out_stats || p.skip || p.conv_cin > 0)
+    return false;
+  // what the CTA-pair kernel needs (it switches outputs between tiles); the split-K kernel takes any multiple of eight
+  return (p.n_split % 256) == 0 && p.N - p.n_split <= 256 && p.batch_rows == 0 && !p.out_f32;
 }
 
 // ---- tower kernel, host side ----
@@ -1906,13 +1610,8 @@ cudaError_t gemm_tc_tower_build(const GemmParams* g, int n, int* status, void* h
     L.r = L.c;
     if (q.res && (e = get_map(q.res, q.ldres, q.M, q.N, BM, prec, &L.r)) != cudaSuccess) return e;
     TcParams& p = L.p;
-    fill_folded(p, q);
+    fill_tc_params(p, q, status);
     p.tma_store = 1;
-    p.split_from = 0x7fffffff; p.tiles_v = 0;
-    p.bias = q.bias; p.C = q.C; p.ldc = q.ldc;
-    p.M = q.M; p.N = q.N; p.K = q.K; p.act = q.act; p.scale = q.scale; p.alpha = q.alpha;
-    p.out_f32 = 0; p.status = status;
-    p.conv_cblocks = ceil_div(q.conv_cin, BK);
   }
   return cudaSuccess;
 }
@@ -1948,7 +1647,7 @@ template <typename T>
 cudaError_t launch_gemm_tc(const GemmParams& p, int* status, int sm_count, cudaStream_t s) {
   if (p.M <= 0 || p.N <= 0) return cudaSuccess;
   if (!gemm_tc_supported(p) || p.skip) return cudaErrorInvalidValue;  // residuals go through `res`
-  if (p.n_split > 0 && !gemm_tc_split_supported(p, sm_count)) return cudaErrorInvalidValue;
+  if (p.n_split > 0 && !gemm_tc_split_supported(p)) return cudaErrorInvalidValue;
   if (pair_eligible(p, sm_count))
   {
     // Four epilogue groups when a tile has few k-blocks (the epilogue then sets the pace), two otherwise (fewer
@@ -1960,10 +1659,11 @@ cudaError_t launch_gemm_tc(const GemmParams& p, int* status, int sm_count, cudaS
     return four ? launch_pair<T, 4>(p, status, sm_count, s) : launch_pair<T, 2>(p, status, sm_count, s);
   }
   if (p.se_k > 0) return launch_bn<T, 256>(p, status, sm_count, s);  // the tile must hold every channel of two boards
-  // Wide tiles amortise the A-tile loads; narrow problems take the smallest tile that covers N, and skinny
-  // problems (few rows) the widest tile that still yields at least half an SM count of CTAs.
+  if (p.conv_cin == 0 && p.batch_rows == 0) return launch_gemm_split<T>(p, status, sm_count, s);
+  // Convolutions and stacked products: wide tiles amortise the A-tile loads; narrow problems take the smallest tile that
+  // covers N, and skinny problems (few rows) the widest tile that still yields at least half an SM count of CTAs.
   auto tiles = [&](int bn) { return (long long)ceil_div(p.M, BM) * ceil_div(p.N, bn); };
-  if (p.N > 128 && (tiles(256) >= sm_count / 2 || p.N <= 128)) return launch_bn<T, 256>(p, status, sm_count, s);
+  if (p.N > 128 && tiles(256) >= sm_count / 2) return launch_bn<T, 256>(p, status, sm_count, s);
   if (p.N > 64 && (tiles(128) >= sm_count / 2 || p.N <= 64)) return launch_bn<T, 128>(p, status, sm_count, s);
   if (p.N > 128 && tiles(64) < sm_count / 8) return launch_bn<T, 256>(p, status, sm_count, s);
   return launch_bn<T, 64>(p, status, sm_count, s);

@@ -39,9 +39,9 @@ struct GemmParams {
   // Per-row (sum, sum of squares) of the outputs, accumulated in double with atomic adds into out_stats[M][2]
   // (the caller zeroes it), so that the next product can fold the LayerNorm of this output.
   double* out_stats = nullptr;
-  // Second output of the CTA-pair kernel: columns [n_split, N) go to C2 (leading dimension ldc2, column n - n_split)
-  // instead of C.  n_split must be a multiple of 256 and the remainder at most 256 columns wide; the last tile is then
-  // computed with a narrower MMA.  Lets a narrow product share the operand traffic of a wide one (same A, same folded
+  // Second output: columns [n_split, N) go to C2 (leading dimension ldc2, column n - n_split)
+  // instead of C.  n_split must be a multiple of 256 and the remainder at most 256 columns wide; the last tile of the
+  // CTA-pair kernel is then computed with a narrower MMA.  Lets a narrow product share the operand traffic of a wide one (same A, same folded
   // LayerNorm); no residual / statistics in this mode.
   void* C2 = nullptr; long long ldc2 = 0;
   int n_split = 0;
@@ -60,6 +60,9 @@ struct GemmParams {
   // CTA-pair kernel: compute a sparsely filled last wave as whole 256x256 tiles instead of half-width ones
   // (verification switch; the split is on by default).
   bool whole_tiles = false;
+  // Products of few rows: the K range may be cut over several CTAs (gemm_split.cu).  The sums then depend on the number of
+  // rows; off, a row's result is the same whatever else is in the batch.
+  bool split_k = true;
 };
 
 template <typename T> cudaError_t launch_gemm_simt(const GemmParams& p, cudaStream_t s);
@@ -68,8 +71,8 @@ template <typename T> cudaError_t launch_gemm_simt(const GemmParams& p, cudaStre
 template <typename T> cudaError_t launch_gemm_tc(const GemmParams& p, int* status, int sm_count, cudaStream_t s);
 bool gemm_tc_supported(const GemmParams& p);
 bool gemm_tc_se_supported(const GemmParams& p);
-// Whether launch_gemm_tc would run `p` (with C2 / n_split set) on the CTA-pair kernel, the only one that splits.
-bool gemm_tc_split_supported(const GemmParams& p, int sm_count);
+// Whether launch_gemm_tc can run `p` with its second output (C2 / n_split).
+bool gemm_tc_split_supported(const GemmParams& p);
 // Tower kernel (gemm_tc.cu): the 3x3 convolutions of a residual tower (conv_cin > 0, optional fused squeeze-excitation
 // and skip input), all with the same rows and output channels (at most 256), in one launch.  gemm_tc_tower_build fills
 // a host table of n entries of gemm_tc_tower_layer_bytes() bytes, which the caller copies to the device once;

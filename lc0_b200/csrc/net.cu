@@ -414,6 +414,10 @@ struct Net : NetBase {
   // > 0: the tensor-core launches that follow on this thread use at most this many SMs (persistent grids are sized
   // from it), so that two launches on different streams can share the GPU
   static inline thread_local int t_sm_limit = 0;
+  // Whether products of few rows may cut their K range (GemmParams::split_k): below 64 positions, where one tile per CTA
+  // leaves most SMs idle.  From 64 positions on a position's result does not depend on the size of its batch.
+  static inline thread_local bool t_split_k = true;
+  static constexpr int kSplitKPositions = 64;
   struct DependentLaunchScope {
     bool prev;
     explicit DependentLaunchScope(bool on) : prev(t_dependent_launch) { t_dependent_launch = on; }
@@ -1127,6 +1131,7 @@ struct Net : NetBase {
     p.C = out_f32 ? cf32 : (void*)Cout; p.ldc = ldc; p.M = M; p.N = d.out; p.K = d.in; p.act = act;
     p.skip = skip; p.ldskip = ldskip; p.alpha = alpha_; p.out_f32 = out_f32;
     p.whole_tiles = (opt.flags & B200_FLAG_NO_SPLIT_LAST_WAVE) != 0;
+    p.split_k = t_split_k;
     run_gemm(st, p);
   }
   // A LayerNorm output that is either materialised (stats == nullptr) or kept as its un-normalised input `u`
@@ -1162,6 +1167,7 @@ struct Net : NetBase {
       p.out_stats = out_stats;
     }
     p.whole_tiles = (opt.flags & B200_FLAG_NO_SPLIT_LAST_WAVE) != 0;
+    p.split_k = t_split_k;
     run_gemm(st, p);
   }
   // Tag of the launches that follow on this thread (which product of the layer they are), for the tagged profile.
@@ -1170,7 +1176,7 @@ struct Net : NetBase {
     launches++;
     const double flops = 2.0 * p.M * (double)p.N * p.K * p.batch;
     if constexpr (sizeof(T) == 2) {
-      if (use_tc && p.M >= 64 && gemm_tc_supported(p)) {
+      if (use_tc && gemm_tc_supported(p)) {
         const int sp_ = span_begin(st, K_GEMM_TC, flops, t_tag);
         CK(launch_gemm_tc<T>(p, t_status, t_sm_limit > 0 ? t_sm_limit : sm_count, st));
         span_end(st, sp_);
@@ -1402,7 +1408,7 @@ struct Net : NetBase {
       GemmParams probe;
       probe.A = in.u; probe.lda = E; probe.W = e.qkv.w; probe.ldw = E; probe.C = s.qkv; probe.ldc = 3 * E;
       probe.M = R; probe.N = e.qkvc_out; probe.K = E; probe.C2 = s.sg_c; probe.ldc2 = sg_hc; probe.n_split = 3 * E;
-      merged = gemm_tc_split_supported(probe, sm_count);
+      merged = gemm_tc_split_supported(probe);
     }
     t_tag = TAG_QKV;
     if (merged) {
@@ -1463,6 +1469,7 @@ struct Net : NetBase {
     s.stats_parity = 0;
     t_status = d_status + (&s - slots.data());
     t_slot_ptr = &s;
+    t_split_k = n < kSplitKPositions;
     // not with per-launch event pairs: the spans would then time the overlap with the neighbours
     DependentLaunchScope launch_scope(dependent_launch && !profiling);
     CK(cudaMemsetAsync(d_qdm, 0, (size_t)n * 3 * sizeof(float), st));
@@ -2327,9 +2334,9 @@ int b200_op_gemm_ex(const b200_gemm_desc* d, void* stream) {
   int dev = 0, sms = 0;
   B200_CUDA(cudaGetDevice(&dev));
   B200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (p.n_split > 0 && !gemm_tc_split_supported(p, sms)) {
-    set_error("b200_op_gemm_ex: the second output needs a product large enough for the CTA-pair kernel, n_split a "
-              "multiple of 256 and at most 256 columns beyond it");
+  if (p.n_split > 0 && !gemm_tc_split_supported(p)) {
+    set_error("b200_op_gemm_ex: the second output needs n_split a multiple of 256, at most 256 columns beyond it and no "
+              "residual or statistics");
     return B200_ERR_UNSUPPORTED;
   }
   int* status = nullptr;

@@ -323,6 +323,59 @@ def test_second_output_of_the_pair_kernel_with_folded_input(lib, whole_tiles):
     assert np.all(np.abs(got - ref) <= 2.0 ** -10 * np.abs(ref) + 3e-3)
 
 
+@pytest.mark.parametrize("prec", [1, 2])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 256, 2048), (3, 8192, 256), (7, 40, 72), (63, 1024, 1024), (64, 1536, 1024),
+                                   (65, 1024, 1536), (130, 200, 624), (384, 1024, 1024), (1000, 1858, 64),
+                                   (1537, 128, 512)])
+def test_products_of_few_rows(lib, prec, M, N, K):
+    """The split-K kernel at the edges of its tiles (64 / 128 rows, 32 / 64 / 128 columns, K remainders, columns that are no
+    multiple of eight) with every epilogue form: folded LayerNorm of A, activation, residual normalised on the fly,
+    row statistics.  fp32 reference of the same arithmetic on the stored operands."""
+    dt = DT[prec]
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    A = (rnd(M, K) + 0.5).to(dt)
+    W = (rnd(N, K) * K ** -0.5).to(dt)
+    b, cs = rnd(N) * 0.1, W.float().sum(1).contiguous()
+    a64 = A.double()
+    st_a = torch.stack([a64.sum(1), (a64 * a64).sum(1)], 1).contiguous()
+    C = torch.zeros(M, N, dtype=dt, device="cuda")
+    out_st = torch.zeros(M, 2, device="cuda", dtype=torch.float64)
+    kw = dict(A=A, W=W, bias=b, C=C, M=M, N=N, K=K, precision=prec, activation=oracle.ACT_SWISH, out_stats=out_st,
+              a_stats=st_a, colsum=cs, a_inv_c=1.0 / K, a_eps=1e-3, alpha=0.43)
+    mean = a64.mean(1, keepdim=True)
+    rstd = (a64.var(1, unbiased=False, keepdim=True) + 1e-3).rsqrt()
+    v = rstd * (a64 @ W.double().T - mean * cs.double()) + b.double()
+    ref = 0.43 * v * torch.sigmoid(v)
+    if N % 8 == 0:
+        R = (rnd(M, N) * 2 + 1).to(dt)
+        r64 = R.double()
+        st_r = torch.stack([r64.sum(1), (r64 * r64).sum(1)], 1).contiguous()
+        gamma, beta = 1 + rnd(N) * 0.1, rnd(N) * 0.1
+        kw.update(res=R, res_stats=st_r, res_gamma=gamma, res_beta=beta, res_inv_c=1.0 / N, res_eps=1e-3)
+        rn = (r64 - r64.mean(1, keepdim=True)) * (r64.var(1, unbiased=False, keepdim=True) + 1e-3).rsqrt()
+        ref = ref + rn * gamma.double() + beta.double()
+    else:
+        kw.update(alpha=1.0)
+        ref = ref / 0.43
+    if N % 8:  # the folded forms need rows that TMA can describe elsewhere in the schedule; plain epilogue here
+        for k in ("out_stats", "a_stats", "colsum"):
+            kw.pop(k)
+        v = a64 @ W.double().T + b.double()
+        ref = v * torch.sigmoid(v)
+    _lib.check(lib.b200_op_gemm_ex(_desc(**kw), None))
+    torch.cuda.synchronize()
+    # output rounding of the storage type; fp32 accumulation of K products of magnitude rstd * |A| * |W|, of which the
+    # LayerNorm correction cancels the mean's part: a few 1e-5 at most, 2e-4 with the fast exponential of the activation
+    rt = 2.0 ** -10 if prec == 1 else 2.0 ** -7
+    got = C.double()
+    assert torch.all((got - ref).abs() <= rt * ref.abs() + 1e-3), (got - ref).abs().max().item()
+    if "out_stats" in kw:
+        s_ref = torch.stack([ref.sum(1), (ref * ref).sum(1)], 1)
+        mag = torch.stack([ref.abs().sum(1), s_ref[:, 1]], 1)
+        assert torch.all((out_st - s_ref).abs() <= 1e-3 * mag + 1e-3)
+
+
 def test_gemm_ex_rejects_inconsistent_descriptions(lib):
     a = torch.zeros(256, 64, dtype=torch.float16, device="cuda")
     st = torch.zeros(256, 2, device="cuda", dtype=torch.float64)
