@@ -1,0 +1,328 @@
+// FMA matrix kernel: the products and 3x3 convolutions of the fp32 verification mode, and 16-bit products of shapes that
+// the TMA path does not take (leading dimensions that are no multiple of 8, stacked products, products in fp32 storage).
+// (reference: FullyConnectedLayer::Forward1D, backends/blas/fully_connected_layer.cc:50-106;
+// WinogradConvolution3::Forward, backends/blas/winograd_convolution3.cc:47-57, same sums through F(2x2,3x3) transforms)
+//
+// Bound by the FMA pipe (74 TFLOP/s at 1.965 GHz), for few rows by the latency of the K loop.  Operands are staged
+// K-contiguous as they lie in memory (16-byte cp.async, four floats of one row) in three stages; rows are padded by four floats
+// so that eight rows of a quarter warp fall on different banks.  A thread owns TM x TN outputs whose rows are 8 and whose
+// columns 4 apart and reads TM + TN 16-byte pieces per four k for 4 TM TN FMAs.
+// With GemmParams::split_k the K range of a tile that leaves SMs idle is cut over a cluster of up to eight CTAs, whose sums
+// meet through distributed shared memory in a fixed order.
+#include <atomic>
+
+#include "kernels.cuh"
+
+namespace b200 {
+namespace {
+
+constexpr int kStages = 3;
+
+struct FmaParams {
+  const void* A; long long lda, strideA;
+  const void* W; long long ldw, strideW;
+  const float* bias;
+  void* C; long long ldc, strideC;
+  const void* skip; long long ldskip;
+  int M, N, K, act, out_f32, ks, w_const;
+  float scale, alpha;
+  int vec;       // rows start on 16-byte (16-bit storage: 8-byte) boundaries: operands move as pieces of four elements
+  int conv_cin;  // convolution: A is [M][cin] on 8x8 boards, W is [9][N][cin]
+  int conv_kt;   // ... and k runs over nine taps of conv_kt = cin rounded up to pieces of four
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t local, uint32_t rank) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Four elements of one operand row (fewer at the end of the row: zeros) into shared memory as floats.
+template <typename T>
+__device__ __forceinline__ void stage4(float* dst, const T* row, int left, bool vec) {
+  if (!row || left <= 0) {
+    *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+    return;
+  }
+  if constexpr (sizeof(T) == 4) {
+    if (vec) {
+      cp_async16((uint32_t)__cvta_generic_to_shared(dst), row, left >= 4 ? 16 : left * 4);
+      return;
+    }
+  } else {
+    if (vec && left >= 4) {
+      const uint2 u = *reinterpret_cast<const uint2*>(row);
+      const T* e = reinterpret_cast<const T*>(&u);
+      *reinterpret_cast<float4*>(dst) = make_float4(to_f(e[0]), to_f(e[1]), to_f(e[2]), to_f(e[3]));
+      return;
+    }
+  }
+  float v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = i < left ? to_f(row[i]) : 0.f;
+  *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+template <typename T, bool kFast, int BM, int BN, int TM, int TN, int kBK, int kMinCtas, bool kConv>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), kMinCtas)
+gemm_fma_kernel(const FmaParams p) {
+  constexpr int kThreads = (BM / TM) * (BN / TN);
+  constexpr int kWarpM = 8 * TM, kWarpN = 4 * TN;  // outputs of a warp
+  constexpr int kLd = kBK + 4, kLdOut = BN + 4, kPieces = kBK / 4;
+  constexpr int kRowStep = kThreads / kPieces;     // rows staged at a time
+  static_assert(BM % kWarpM == 0 && BN % kWarpN == 0, "whole warps");
+  extern __shared__ __align__(16) float sm[];      // [stages][BM + BN][kLd]; afterwards [BM][kLdOut] sums
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = (int)blockIdx.x % p.ks;
+  const int n0 = (int)blockIdx.x / p.ks * BN, m0 = blockIdx.y * BM;
+  const T* A = reinterpret_cast<const T*>(p.A) + (long long)blockIdx.z * p.strideA;
+  const T* W = reinterpret_cast<const T*>(p.W) + (long long)blockIdx.z * p.strideW;
+  const int k_blocks = (p.K + kBK - 1) / kBK;
+  const int kb0 = (int)((long long)k_blocks * rank / p.ks), kbn = (int)((long long)k_blocks * (rank + 1) / p.ks) - kb0;
+
+  const int lr = tid / kPieces, lk = tid % kPieces * 4;
+  auto stage_w = [&](int i) {
+    if (i >= kbn) return;
+    float* dst = sm + (i % kStages) * (BM + BN) * kLd + BM * kLd + lk;
+    int k = (kb0 + i) * kBK + lk, left = p.K - k;
+    const T* w = W;
+    if constexpr (kConv) {
+      const int tap = k / p.conv_kt;
+      k -= tap * p.conv_kt;
+      left = tap < 9 ? p.conv_cin - k : 0;
+      w += (long long)tap * p.N * p.conv_cin;
+    }
+#pragma unroll
+    for (int r = 0; r < BN; r += kRowStep) {
+      const int n = n0 + r + lr;
+      if (BN % kRowStep == 0 || r + lr < BN)
+        stage4(dst + (r + lr) * kLd, n < p.N ? w + (long long)n * p.ldw + k : nullptr, left, p.vec);
+    }
+  };
+  auto stage_a = [&](int i) {
+    if (i >= kbn) return;
+    float* dst = sm + (i % kStages) * (BM + BN) * kLd + lk;
+    const int k = (kb0 + i) * kBK + lk;
+    int dy = 0, dx = 0, c = k, left = p.K - k;
+    if constexpr (kConv) {
+      const int tap = k / p.conv_kt;
+      c = k - tap * p.conv_kt;
+      left = tap < 9 ? p.conv_cin - c : 0;
+      dy = tap / 3 - 1;
+      dx = tap % 3 - 1;
+    }
+#pragma unroll
+    for (int r = 0; r < BM; r += kRowStep) {
+      if (BM % kRowStep != 0 && r + lr >= BM) break;
+      const int m = m0 + r + lr;
+      const T* row = nullptr;
+      if (m < p.M) {
+        if constexpr (kConv) {
+          const int y = ((m >> 3) & 7) + dy, x = (m & 7) + dx;
+          if ((unsigned)y < 8u && (unsigned)x < 8u) row = A + (long long)(m + dy * 8 + dx) * p.lda + c;
+        } else {
+          row = A + (long long)m * p.lda + c;
+        }
+      }
+      stage4(dst + (r + lr) * kLd, row, left, p.vec);
+    }
+  };
+
+  // weights do not depend on the kernel before this one (w_const): they are requested while it is still running
+  if (p.w_const) {
+    for (int i = 0; i < kStages - 1; ++i) stage_w(i);
+  }
+  grid_dependency_wait();
+  grid_launch_dependents();
+  for (int i = 0; i < kStages - 1; ++i) {
+    if (!p.w_const) stage_w(i);
+    stage_a(i);
+    cp_async_commit();  // the first group also holds the weights requested above
+  }
+
+  constexpr int kWarpsN = BN / kWarpN;
+  const int wm = warp / kWarpsN * kWarpM + (lane & 7), wn = warp % kWarpsN * kWarpN + (lane >> 3);
+  float acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+
+#pragma unroll 1
+  for (int i = 0; i < kbn; ++i) {
+    cp_async_wait<kStages - 2>();
+    __syncthreads();  // stage i has landed; every thread is done with the stage that is filled next
+    stage_w(i + kStages - 1);
+    stage_a(i + kStages - 1);
+    cp_async_commit();
+    const float* as = sm + (i % kStages) * (BM + BN) * kLd + wm * kLd;
+    const float* ws = sm + (i % kStages) * (BM + BN) * kLd + BM * kLd + wn * kLd;
+#pragma unroll
+    for (int k = 0; k < kBK; k += 4) {
+      float4 a[TM];
+#pragma unroll
+      for (int r = 0; r < TM; ++r) a[r] = *reinterpret_cast<const float4*>(as + r * 8 * kLd + k);
+#pragma unroll
+      for (int c0 = 0; c0 < TN; c0 += 4) {
+        float4 w[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) w[c] = *reinterpret_cast<const float4*>(ws + (c0 + c) * 4 * kLd + k);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int r = 0; r < TM; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              acc[r][c0 + c] = fmaf(reinterpret_cast<const float*>(&a[r])[e], reinterpret_cast<const float*>(&w[c])[e], acc[r][c0 + c]);
+      }
+    }
+  }
+
+  const T* skip = reinterpret_cast<const T*>(p.skip);
+  auto finish = [&](int m, int n, float v) {
+    if (m >= p.M || n >= p.N) return;
+    v *= p.scale;
+    if (p.bias) v += __ldg(p.bias + n);
+    v = activate<kFast>(v, p.act);
+    if (skip) v = p.alpha * v + to_f(skip[(long long)m * p.ldskip + n]);
+    const long long o = (long long)blockIdx.z * p.strideC + (long long)m * p.ldc + n;
+    if (p.out_f32) reinterpret_cast<float*>(p.C)[o] = v;
+    else reinterpret_cast<T*>(p.C)[o] = from_f<T>(v);
+  };
+
+  // The sums go through shared memory, so that whole rows are written, and with a cut K range to the other CTAs.
+  cp_async_wait<0>();
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < TM; ++r)
+#pragma unroll
+    for (int c = 0; c < TN; ++c) sm[(wm + r * 8) * kLdOut + wn + c * 4] = acc[r][c];
+  if (p.ks == 1) {
+    __syncthreads();
+    for (int e = tid; e < BM * BN; e += kThreads) finish(m0 + e / BN, n0 + e % BN, sm[e / BN * kLdOut + e % BN]);
+    return;
+  }
+  cluster_sync();
+  const int slice = BM * BN / p.ks;  // a power of two and at least 64
+  for (int e = rank * slice + tid * 4; e < (rank + 1) * slice; e += kThreads * 4) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < p.ks; ++j) {
+      const float4 u = ld_cluster_v4((uint32_t)__cvta_generic_to_shared(sm + e / BN * kLdOut + e % BN), j);
+      v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+    }
+    const int m = m0 + e / BN, n = n0 + e % BN;
+    finish(m, n, v.x);
+    finish(m, n + 1, v.y);
+    finish(m, n + 2, v.z);
+    finish(m, n + 3, v.w);
+  }
+  cluster_sync();  // the others may still be reading this CTA's sums
+}
+
+template <typename T, int BM, int BN, int TM, int TN, int kBK, int kMinCtas, bool kConv>
+cudaError_t launch_tile(const FmaParams& p, int batch, cudaStream_t s) {
+  constexpr int ring = kStages * (BM + BN) * (kBK + 4) * 4, out = BM * (BN + 4) * 4, smem = ring > out ? ring : out;
+  auto kernel = gemm_fma_kernel<T, (sizeof(T) == 2), BM, BN, TM, TN, kBK, kMinCtas, kConv>;
+  static std::atomic<unsigned long long> attr_mask{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (!(attr_mask.load() >> (dev & 63) & 1ull)) {
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+    attr_mask.fetch_or(1ull << (dev & 63));
+  }
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(ceil_div(p.N, BN) * p.ks, ceil_div(p.M, BM), batch);
+  lc.blockDim = dim3((BM / TM) * (BN / TN));
+  lc.dynamicSmemBytes = smem;
+  lc.stream = s;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (p.ks > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = p.ks;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  if (t_dependent_launch) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  lc.attrs = attr;
+  lc.numAttrs = na;
+  return cudaLaunchKernelEx(&lc, kernel, p);
+}
+
+// CTAs per tile: cuts of the K range, down to four k-blocks of 32 each, while they find SMs that have nothing to do.
+int cuts(const FmaParams& p, int bm, int bn, int batch, bool split, int ctas) {
+  const long long tiles = (long long)ceil_div(p.N, bn) * ceil_div(p.M, bm) * batch;
+  const int k_blocks = ceil_div(p.K, 32);
+  int ks = 1;
+  while (split && ks < 8 && tiles * ks * 2 <= ctas && k_blocks / (ks * 2) >= 4) ks *= 2;
+  return ks;
+}
+
+template <typename T, bool kConv>
+cudaError_t launch_fma(FmaParams p, int batch, bool split, cudaStream_t s) {
+  if constexpr (!kConv) {  // a convolution has whole boards of 64 rows
+    if (p.M <= 8) { p.ks = cuts(p, 8, 64, batch, split, 148); return launch_tile<T, 8, 64, 1, 4, 32, 1, false>(p, batch, s); }
+    if (p.M <= 32) { p.ks = cuts(p, 32, 64, batch, split, 512); return launch_tile<T, 32, 64, 4, 4, 32, 1, false>(p, batch, s); }
+  }
+  p.ks = cuts(p, 64, 64, batch, split, 512);
+  return launch_tile<T, 64, 64, 8, 4, 32, 4, kConv>(p, batch, s);
+}
+
+template <typename T> bool aligned4(const void* ptr, long long ld, long long stride) {
+  return (reinterpret_cast<uintptr_t>(ptr) % (4 * sizeof(T))) == 0 && ld % 4 == 0 && stride % 4 == 0;
+}
+
+}  // namespace
+
+template <typename T>
+cudaError_t launch_gemm_fma(const GemmParams& g, cudaStream_t s) {
+  if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return cudaSuccess;
+  FmaParams p = {};
+  p.A = g.A; p.lda = g.lda; p.strideA = g.strideA;
+  p.W = g.W; p.ldw = g.ldw; p.strideW = g.strideW;
+  p.bias = g.bias;
+  p.C = g.C; p.ldc = g.ldc; p.strideC = g.strideC;
+  p.skip = g.skip; p.ldskip = g.ldskip;
+  p.M = g.M; p.N = g.N; p.K = g.K; p.act = g.act; p.out_f32 = g.out_f32;
+  p.scale = g.scale; p.alpha = g.alpha;
+  p.vec = aligned4<T>(g.A, g.lda, g.strideA) && aligned4<T>(g.W, g.ldw, g.strideW);
+  p.w_const = g.batch == 1;  // a product per position (the policy head's Q K^T) has an activation on both sides
+  return launch_fma<T, false>(p, g.batch, g.split_k, s);
+}
+
+template <typename T>
+cudaError_t launch_conv3x3(const T* x, int cin, const T* w, const float* bias, T* y, int cout, int n, int act,
+                           bool split, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  FmaParams p = {};
+  p.A = x; p.lda = cin; p.W = w; p.ldw = cin; p.bias = bias; p.C = y; p.ldc = cout;
+  p.M = n * 64; p.N = cout; p.act = act; p.conv_cin = cin; p.conv_kt = ceil_div(cin, 4) * 4; p.K = 9 * p.conv_kt;
+  p.scale = 1.f; p.alpha = 1.f; p.w_const = 1;
+  p.vec = aligned4<T>(x, cin, 0) && aligned4<T>(w, cin, 0);
+  return launch_fma<T, true>(p, 1, split, s);
+}
+
+#define INSTANTIATE(T)                                                          \
+  template cudaError_t launch_gemm_fma<T>(const GemmParams&, cudaStream_t);     \
+  template cudaError_t launch_conv3x3<T>(const T*, int, const T*, const float*, T*, int, int, int, bool, cudaStream_t);
+INSTANTIATE(float)
+INSTANTIATE(__half)
+INSTANTIATE(__nv_bfloat16)
+
+}  // namespace b200

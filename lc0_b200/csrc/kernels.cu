@@ -1,5 +1,4 @@
-// Memory-bound and small-matrix kernels of the evaluation path, plus the plain FMA matrix kernel
-// used by the fp32 verification mode and for shapes the tensor-core kernel does not take.
+// Memory-bound and small kernels of the evaluation path.
 #include "kernels.cuh"
 
 namespace b200 {
@@ -139,79 +138,6 @@ template <typename T>
 cudaError_t launch_expand_pre12(const uint64_t* masks, const float* values, int n, T* out, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   expand_pre12_kernel<T><<<ceil_div((long long)n * 768, 256), 256, 0, s>>>(masks, values, n, out);
-  return cudaGetLastError();
-}
-
-// ------------------------------------------------------------------------------------------------
-// Plain FMA GEMM: 64x64 tile, 16-deep k-steps, 256 threads x (4x4) outputs, fp32 accumulation.
-// (reference: FullyConnectedLayer::Forward1D, backends/blas/fully_connected_layer.cc:50-106)
-// ------------------------------------------------------------------------------------------------
-template <typename T, bool kFast>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(GemmParams p) {
-  __shared__ float As[16][64 + 4];
-  __shared__ float Ws[16][64 + 4];
-  const int b = blockIdx.z;
-  const T* A = reinterpret_cast<const T*>(p.A) + (long long)b * p.strideA;
-  const T* W = reinterpret_cast<const T*>(p.W) + (long long)b * p.strideW;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-  const int lr = tid >> 2;        // 0..63 tile row
-  const int lc = (tid & 3) * 4;   // 0,4,8,12 k offset
-  for (int k0 = 0; k0 < p.K; k0 += 16) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int k = k0 + lc + i;
-      const int m = m0 + lr, n = n0 + lr;
-      As[lc + i][lr] = (m < p.M && k < p.K) ? to_f(A[(long long)m * p.lda + k]) : 0.f;
-      Ws[lc + i][lr] = (n < p.N && k < p.K) ? to_f(W[(long long)n * p.ldw + k]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      float a[4], w[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = Ws[k][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  const T* skip = reinterpret_cast<const T*>(p.skip);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= p.M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= p.N) continue;
-      float v = acc[i][j] * p.scale;
-      if (p.bias) v += p.bias[n];
-      v = activate<kFast>(v, p.act);
-      if (skip) v = p.alpha * v + to_f(skip[(long long)m * p.ldskip + n]);
-      const long long o = (long long)b * p.strideC + (long long)m * p.ldc + n;
-      if (p.out_f32) reinterpret_cast<float*>(p.C)[o] = v;
-      else reinterpret_cast<T*>(p.C)[o] = from_f<T>(v);
-    }
-  }
-}
-
-template <typename T>
-cudaError_t launch_gemm_simt(const GemmParams& p, cudaStream_t s) {
-  if (p.M <= 0 || p.N <= 0 || p.batch <= 0) return cudaSuccess;
-  dim3 grid(ceil_div(p.N, 64), ceil_div(p.M, 64), p.batch);
-  gemm_simt_kernel<T, (sizeof(T) == 2)><<<grid, 256, 0, s>>>(p);
   return cudaGetLastError();
 }
 
@@ -668,81 +594,6 @@ cudaError_t launch_head_final(const T* h, int k, const float* w, const float* b,
 
 // ------------------------------------------------------------------------------------------------
 // Residual tower on NHWC activations [n*64][C].
-// 3x3 convolution as an implicit GEMM over (tap, cin): same 64x64x16 FMA tiling as gemm_simt_kernel;
-// the A tile gathers the shifted board square (zero outside the board).
-// (reference: WinogradConvolution3::Forward, backends/blas/winograd_convolution3.cc:47-57, computes the
-// same sums through F(2x2,3x3) transforms.)
-// ------------------------------------------------------------------------------------------------
-template <typename T, bool kFast>
-__global__ void __launch_bounds__(256)
-conv3x3_kernel(const T* __restrict__ x, int cin, const T* __restrict__ w, const float* __restrict__ bias,
-               T* __restrict__ y, int cout, int rows, int act) {
-  __shared__ float As[16][64 + 4];
-  __shared__ float Ws[16][64 + 4];
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int lr = tid >> 2, lc = (tid & 3) * 4;
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-  const int m = m0 + lr;  // this thread's A row: (sample, square)
-  const int sq = m & 63, sx = sq & 7, sy = sq >> 3;
-  for (int tap = 0; tap < 9; ++tap) {
-    const int dy = tap / 3 - 1, dx = tap % 3 - 1;
-    const int yy = sy + dy, xx = sx + dx;
-    const bool inside = m < rows && yy >= 0 && yy < 8 && xx >= 0 && xx < 8;
-    const T* arow = x + ((long long)(m - sq) + yy * 8 + xx) * cin;
-    const T* wt = w + (long long)tap * cout * cin;
-    for (int k0 = 0; k0 < cin; k0 += 16) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int k = k0 + lc + i;
-        const int n = n0 + lr;
-        As[lc + i][lr] = (inside && k < cin) ? to_f(arow[k]) : 0.f;
-        Ws[lc + i][lr] = (n < cout && k < cin) ? to_f(wt[(long long)n * cin + k]) : 0.f;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        float a[4], ww[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) ww[j] = Ws[k][tx * 4 + j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], ww[j], acc[i][j]);
-      }
-      __syncthreads();
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int mm = m0 + ty * 4 + i;
-    if (mm >= rows) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= cout) continue;
-      float v = acc[i][j];
-      if (bias) v += bias[n];
-      y[(long long)mm * cout + n] = from_f<T>(activate<kFast>(v, act));
-    }
-  }
-}
-
-template <typename T>
-cudaError_t launch_conv3x3(const T* x, int cin, const T* w, const float* bias, T* y, int cout, int n, int act,
-                           cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  dim3 grid(ceil_div(cout, 64), n);
-  conv3x3_kernel<T, (sizeof(T) == 2)><<<grid, 256, 0, s>>>(x, cin, w, bias, y, cout, n * 64, act);
-  return cudaGetLastError();
-}
-
 // Squeeze-excitation block, one CTA per sample (reference: ApplySEUnit, backends/blas/se_unit.cc:31-91;
 // GPU twin SE_Layer_NHWC, backends/cuda/fp16_kernels.cu:55-136).
 template <typename T, bool kFast>
@@ -964,7 +815,6 @@ cudaError_t launch_legal_softmax(const float* policy, const unsigned short* move
 }
 
 #define INSTANTIATE(T)                                                                                        \
-  template cudaError_t launch_gemm_simt<T>(const GemmParams&, cudaStream_t);                                  \
   template cudaError_t launch_expand_planes<T>(const uint64_t*, const float*, int, T*, cudaStream_t);         \
   template cudaError_t launch_expand_tokens<T>(const uint64_t*, const float*, int, const float*, const T*,    \
                                                int, int, T*, cudaStream_t);                                   \
@@ -979,8 +829,6 @@ cudaError_t launch_legal_softmax(const float* policy, const unsigned short* move
   template cudaError_t launch_policy_gather<T>(const T*, long long, const short*, int, float*, cudaStream_t); \
   template cudaError_t launch_head_final<T>(const T*, int, const float*, const float*, int, int, float*,      \
                                             cudaStream_t);                                                    \
-  template cudaError_t launch_conv3x3<T>(const T*, int, const T*, const float*, T*, int, int, int,            \
-                                         cudaStream_t);                                                       \
   template cudaError_t launch_se<T>(const T*, const float*, const T*, const float*, const float*,             \
                                     const float*, const float*, T*, int, int, int, int, cudaStream_t);        \
   template cudaError_t launch_bias_skip_act<T>(const T*, const float*, const T*, T*, int, int, int,           \

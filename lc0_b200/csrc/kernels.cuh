@@ -65,7 +65,8 @@ struct GemmParams {
   bool split_k = true;
 };
 
-template <typename T> cudaError_t launch_gemm_simt(const GemmParams& p, cudaStream_t s);
+// FMA kernel (gemm_fma.cu): any shape and alignment, batched products; no folded LayerNorm, residual or statistics.
+template <typename T> cudaError_t launch_gemm_fma(const GemmParams& p, cudaStream_t s);
 // tcgen05 / TMEM / TMA kernel (gemm_tc.cu); T is __half or __nv_bfloat16, batch must be 1.
 // `status` is a device int the kernel sets non-zero when a bounded wait gives up.
 template <typename T> cudaError_t launch_gemm_tc(const GemmParams& p, int* status, int sm_count, cudaStream_t s);
@@ -156,10 +157,10 @@ cudaError_t launch_head_final(const T* h, int k, const float* w, const float* b,
                               float* qdm, cudaStream_t s);
 
 // ---- residual tower (NHWC activations [n*64][C]) ----
-// 3x3 same-padded convolution as an implicit GEMM; w: [9][Cout][Cin] (tap-major).
+// 3x3 same-padded convolution as an implicit GEMM (gemm_fma.cu); w: [9][Cout][Cin] (tap-major), split as GemmParams::split_k.
 template <typename T>
 cudaError_t launch_conv3x3(const T* x, int cin, const T* w, const float* bias, T* y, int cout, int n,
-                           int act, cudaStream_t s);
+                           int act, bool split, cudaStream_t s);
 // Squeeze-excitation + skip + activation (se_unit.cc:31-91) on NHWC: y = act(sig(z0)*x + skip + z1 + sig(z0)*b).
 template <typename T>
 cudaError_t launch_se(const T* x, const float* conv_bias, const T* skip, const float* w1, const float* b1,

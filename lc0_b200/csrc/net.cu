@@ -1186,7 +1186,7 @@ struct Net : NetBase {
     if (p.a_stats || p.res || p.out_stats)
       throw Fail{B200_ERR_UNSUPPORTED, "internal: folded LayerNorm product outside the tensor-core kernel"};
     const int sp_ = span_begin(st, K_GEMM_FMA, flops);
-    CK(launch_gemm_simt<T>(p, st));
+    CK(launch_gemm_fma<T>(p, st));
     span_end(st, sp_);
   }
   // Any other kernel: counted, and timed under the class "other" (work = algorithmic bytes).
@@ -1287,7 +1287,7 @@ struct Net : NetBase {
     }
     launches++;
     const int sp_ = span_begin(st, K_GEMM_FMA, 2.0 * n * 64 * (double)c.cout * 9 * c.cin);
-    CK(launch_conv3x3<T>(x, c.cin, c.w, bias, y, c.cout, n, act, st));
+    CK(launch_conv3x3<T>(x, c.cin, c.w, bias, y, c.cout, n, act, t_split_k, st));
     span_end(st, sp_);
   }
   // Second convolution of a residual block with its squeeze-excitation unit, the skip connection and the activation
@@ -1610,7 +1610,7 @@ struct Net : NetBase {
         p.A = s.pq; p.lda = pol_dm; p.strideA = 64LL * pol_dm;
         p.W = s.pk; p.ldw = pol_dm; p.strideW = 64LL * pol_dm;
         p.C = s.logits; p.ldc = 64; p.strideC = 4096; p.out_f32 = true;
-        p.M = 64; p.N = 64; p.K = pol_dm; p.batch = n; p.scale = 1.0f / sqrtf((float)pol_dm);
+        p.M = 64; p.N = 64; p.K = pol_dm; p.batch = n; p.scale = 1.0f / sqrtf((float)pol_dm); p.split_k = t_split_k;
         run_gemm(st, p);
         other(st, (double)n * (4096 + 1858) * 4, [&] {
           return launch_policy_attn_gather<T>(s.logits, s.pk, pol_w4, pol_dm, d_attn_src, n, d_policy, st);
@@ -2298,7 +2298,7 @@ int b200_op_gemm(const void* A, const void* W, const float* bias, void* C, int M
   }
   auto run = [&](auto tag) -> int {
     using T = decltype(tag);
-    B200_CUDA(launch_gemm_simt<T>(p, (cudaStream_t)stream));
+    B200_CUDA(launch_gemm_fma<T>(p, (cudaStream_t)stream));
     return B200_OK;
   };
   return by_precision(precision, [&] { return run(float()); }, [&] { return run(__half()); },
@@ -2461,7 +2461,7 @@ int b200_op_policy_attention(const void* q, const void* k, const float* w4, int 
     p.W = k; p.ldw = dm; p.strideW = 64LL * dm;
     p.C = scratch_logits; p.ldc = 64; p.strideC = 4096; p.out_f32 = true;
     p.M = 64; p.N = 64; p.K = dm; p.batch = n; p.scale = 1.0f / sqrtf((float)dm);
-    B200_CUDA(launch_gemm_simt<T>(p, (cudaStream_t)stream));
+    B200_CUDA(launch_gemm_fma<T>(p, (cudaStream_t)stream));
     B200_CUDA(launch_policy_attn_gather<T>(scratch_logits, (const T*)k, w4, dm, src, n, policy, (cudaStream_t)stream));
     return B200_OK;
   };

@@ -78,7 +78,7 @@ extern "C" int b200_op_policy_attention_static(const void* q, const void* k, con
     p.W = k; p.ldw = dm; p.strideW = 64LL * dm;
     p.C = s->logits; p.ldc = 64; p.strideC = 4096; p.out_f32 = true;
     p.M = 64; p.N = 64; p.K = dm; p.batch = n; p.scale = 1.0f / sqrtf((float)dm);
-    B200_CUDA(launch_gemm_simt<T>(p, st));
+    B200_CUDA(launch_gemm_fma<T>(p, st));
     B200_CUDA(launch_policy_attn_gather<T>(s->logits, static_cast<const T*>(k), w4, dm, s->table, n, policy, st));
     return B200_OK;
   };
