@@ -17,6 +17,7 @@
 // cuBLAS calls and softmax_opt_64_kernel (backends/cuda/layers.cc:1803-1850, common_kernels.cu:775-835).
 #include <cuda.h>
 
+#include <atomic>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -229,17 +230,22 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 
 
 // ------------------------------------------------------------------------------------------------
-// Attention policy head tail on tensor cores, one CTA (4 warps) per position:
-//   logits = Q K^T / sqrt(dm)  (64 x 64, dm streamed through shared memory in 64-wide double-buffered chunks),
-//   promotion offsets from the rank-8 keys, and the gather of the 1858 move logits, written as fp32.
+// Attention policy head tail on tensor cores, one CTA (8 warps) per position:
+//   logits = Q K^T / sqrt(dm)  (64 x 64), promotion offsets from the rank-8 keys, and the gather of the 1858 move logits,
+//   written as fp32.
+// Bound by HBM reads of Q and K for many positions, by the latency of one CTA's loads for few.  dm is streamed through
+// shared memory in stages of two 64-wide chunks, three stages deep; warps 0-3 multiply the even chunks and warps 4-7 the
+// odd ones, and their sums meet in shared memory.  The promotion products (4 x 8 dot products over the rank-8 keys)
+// read the keys from the stages as they pass, eight threads per product.
 // Reference: network_blas.cc:850-914; GPU twins: a batched cuBLAS call, promotion_logits_kernel and
 // policyMap_kernel (backends/cuda/layers.cc:1898-1979, common_kernels.cu:1116-1201, :703-734).
 // ------------------------------------------------------------------------------------------------
 constexpr int kPolRow = 64 * 2 + 16;          // bytes per staged row (64 values + padding)
-constexpr int kPolStage = 2 * 64 * kPolRow;   // Q chunk + K chunk
+constexpr int kPolChunk = 2 * 64 * kPolRow;   // Q chunk + K chunk
+constexpr int kPolStages = 3, kPolBytes = kPolStages * 2 * kPolChunk;
 
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256, 2)
 policy_attn_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const float* __restrict__ w4, int dm,
                       const short* __restrict__ src_slot, float scale, float* __restrict__ policy) {
   extern __shared__ __align__(16) uint8_t sm[];
@@ -247,19 +253,22 @@ policy_attn_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const fl
   const int n = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const T* qn = q + (long long)n * 64 * dm;
   const T* kn = k + (long long)n * 64 * dm;
-  const int chunks = (dm + 63) / 64;
-  auto stage_load = [&](int c, int st) {
-    uint8_t* sq = sm + st * kPolStage;
-    uint8_t* sk = sq + 64 * kPolRow;
-    for (int i = tid; i < 64 * 8; i += 128) {
-      const int r = i >> 3, ch = i & 7;
-      const int col = c * 64 + ch * 8;
-      if (col < dm) {  // dm is a multiple of 8
-        cp_async16(sq + r * kPolRow + ch * 16, qn + (long long)r * dm + col);
-        cp_async16(sk + r * kPolRow + ch * 16, kn + (long long)r * dm + col);
-      } else {
-        *reinterpret_cast<uint4*>(sq + r * kPolRow + ch * 16) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(sk + r * kPolRow + ch * 16) = make_uint4(0, 0, 0, 0);
+  const int steps = (dm + 127) / 128;
+  auto stage_load = [&](int step) {
+    if (step < steps) {
+      uint8_t* st = sm + (step % kPolStages) * 2 * kPolChunk;
+#pragma unroll
+      for (int i = tid; i < 2 * 64 * 8; i += 256) {
+        const int half = i >> 9, r = (i >> 3) & 63, ch = i & 7;
+        const int col = step * 128 + half * 64 + ch * 8;
+        uint8_t* dst = st + half * kPolChunk + r * kPolRow + ch * 16;
+        if (col < dm) {  // dm is a multiple of 8
+          cp_async16(dst, qn + (long long)r * dm + col);
+          cp_async16(dst + 64 * kPolRow, kn + (long long)r * dm + col);
+        } else {
+          *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+          *reinterpret_cast<uint4*>(dst + 64 * kPolRow) = make_uint4(0, 0, 0, 0);
+        }
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -269,17 +278,18 @@ policy_attn_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const fl
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-  stage_load(0, 0);
-  const int m0 = warp * 16;
-  for (int c = 0; c < chunks; ++c) {
-    if (c + 1 < chunks) {
-      stage_load(c + 1, (c + 1) & 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-    const uint8_t* sq = sm + (c & 1) * kPolStage;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  for (int i = 0; i < kPolStages - 1; ++i) stage_load(i);
+  const int group = warp >> 2, m0 = (warp & 3) * 16;
+  const int pi = tid >> 6, pj = (tid >> 3) & 7, part = tid & 7;  // promotion product and this thread's eighth of a chunk
+  float promo = 0.f;
+  for (int c = 0; c < steps; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kPolStages - 2) : "memory");
+    __syncthreads();  // stage c has landed; every thread is done with the stage that is filled next
+    stage_load(c + kPolStages - 1);
+    const uint8_t* st = sm + (c % kPolStages) * 2 * kPolChunk;
+    const uint8_t* sq = st + group * kPolChunk;
     const uint8_t* sk = sq + 64 * kPolRow;
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
@@ -293,29 +303,41 @@ policy_attn_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const fl
         mma16816<T>(s[2 * np + 1], a, b[2], b[3]);
       }
     }
-    __syncthreads();  // the stage may be overwritten by the load issued in the next iteration
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int col = c * 128 + half * 64 + part * 8;
+      if (col >= dm) continue;
+      const uint4 u = *reinterpret_cast<const uint4*>(st + half * kPolChunk + (64 + 56 + pj) * kPolRow + part * 16);
+      const T* key = reinterpret_cast<const T*>(&u);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) promo = fmaf(to_f(key[i]), __ldg(w4 + pi * dm + col + i), promo);
+    }
   }
-  // promotion offsets: 4 x 8 dot products of the rank-8 keys with w4 (4 per warp... 8 per warp over 4 warps)
-  for (int t = warp * 8; t < warp * 8 + 8; ++t) {
-    const int i = t >> 3, j = t & 7;
-    const T* key = kn + (long long)(56 + j) * dm;
-    float a = 0.f;
-    for (int cc = lane; cc < dm; cc += 32) a = fmaf(to_f(key[cc]), w4[i * dm + cc], a);
-    a = warp_sum(a);
-    if (lane == 0) off[i][j] = a;
-  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) promo += __shfl_xor_sync(0xffffffffu, promo, o);
+  if (part == 0) off[pi][pj] = promo;
   // logits to shared memory (fp32 [64][65]), reusing the staging area
   float* lg = reinterpret_cast<float*>(sm);
   const int g = lane >> 2, t4 = lane & 3;
+  __syncthreads();
+  if (group == 1) {
 #pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    lg[(m0 + g) * 65 + nt * 8 + 2 * t4] = s[nt][0] * scale;
-    lg[(m0 + g) * 65 + nt * 8 + 2 * t4 + 1] = s[nt][1] * scale;
-    lg[(m0 + g + 8) * 65 + nt * 8 + 2 * t4] = s[nt][2] * scale;
-    lg[(m0 + g + 8) * 65 + nt * 8 + 2 * t4 + 1] = s[nt][3] * scale;
+    for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) lg[(m0 + g + (j >> 1) * 8) * 65 + nt * 8 + 2 * t4 + (j & 1)] = s[nt][j];
   }
   __syncthreads();
-  for (int j = tid; j < 1858; j += 128) {
+  if (group == 0) {
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float* l = lg + (m0 + g + (j >> 1) * 8) * 65 + nt * 8 + 2 * t4 + (j & 1);
+        *l = (s[nt][j] + *l) * scale;
+      }
+  }
+  __syncthreads();
+  for (int j = tid; j < 1858; j += 256) {
     const int slot = src_slot[j];
     float v;
     if (slot < 4096) {
@@ -402,8 +424,17 @@ template <typename T>
 cudaError_t launch_policy_attn_tc(const T* q, const T* k, const float* w4, int dm, const short* src_slot, int n,
                                   float* policy, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  policy_attn_tc_kernel<T><<<n, 128, 2 * kPolStage, s>>>(q, k, w4, dm, src_slot, 1.0f / sqrtf((float)dm), policy);
-  return cudaGetLastError();
+  static std::atomic<unsigned long long> attr_mask{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (!(attr_mask.load() >> (dev & 63) & 1ull)) {
+    e = cudaFuncSetAttribute(policy_attn_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPolBytes);
+    if (e != cudaSuccess) return e;
+    attr_mask.fetch_or(1ull << (dev & 63));
+  }
+  return launch_dependent(policy_attn_tc_kernel<T>, dim3(n), dim3(256), kPolBytes, s, q, k, w4, dm, src_slot,
+                          1.0f / sqrtf((float)dm), policy);
 }
 template cudaError_t launch_policy_attn_tc<__half>(const __half*, const __half*, const float*, int, const short*, int,
                                                    float*, cudaStream_t);
