@@ -361,115 +361,113 @@ cudaError_t launch_gate(T* x, const float* gate_mult, const float* gate_add, int
 // 64-token attention, one CTA per (sample, head), fp32 arithmetic in shared memory
 // (reference: network_blas.cc:352-439; GPU twins are two batched cuBLAS calls + softmax_opt_64_kernel).
 // ------------------------------------------------------------------------------------------------
+// Bound by the FMA pipe and shared-memory reads.  A thread owns four query rows (16 threads to a row) and four keys
+// 16 apart, later four rows and two channels 16 apart, and reads every operand as 16-byte pieces along the contraction; rows of
+// depth + 4 (68 for the probabilities and the transposed V) floats put eight neighbouring rows on different banks.
+// The fp32 mode uses expf for parity with the CPU oracle.
 template <typename T>
 __global__ void __launch_bounds__(256)
 attention_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long ld,
                  const T* __restrict__ bias, T* __restrict__ out, long long ldo, int heads, int depth,
                  float scale) {
-  extern __shared__ float smem[];
-  const int dp = depth + 1;
-  float* sq = smem;             // [64][dp]
-  float* sk = sq + 64 * dp;     // [64][dp]
-  float* sv = sk + 64 * dp;     // [64][dp]
-  float* sp = sv + 64 * dp;     // [64][65]
+  constexpr bool kFast = sizeof(T) == 2;
+  constexpr int kLdP = 68;
+  extern __shared__ __align__(16) float smem[];
+  const int d4 = (depth + 3) >> 2, dp = d4 * 4 + 4;
+  float* sq = smem;              // [64][dp]
+  float* sk = sq + 64 * dp;      // [64][dp]
+  float* sp = smem;              // [64][kLdP], over Q and K once they have been read
+  float* sv = smem + (2 * dp > kLdP ? 2 * dp : kLdP) * 64;  // [depth][kLdP], transposed
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const int tid = threadIdx.x;
   const int n = blockIdx.x / heads, h = blockIdx.x - n * heads;
   const long long base = (long long)n * 64 * ld + (long long)h * depth;
-  for (int i = threadIdx.x; i < 64 * depth; i += 256) {
-    const int r = i / depth, c = i - r * depth;
-    sq[r * dp + c] = to_f(q[base + r * ld + c]);
-    sk[r * dp + c] = to_f(k[base + r * ld + c]);
-    sv[r * dp + c] = to_f(v[base + r * ld + c]);
+  for (int i = tid; i < 64 * d4; i += 256) {
+    const int r = i / d4, c = (i - r * d4) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const bool in = c + e < depth;
+      sq[r * dp + c + e] = in ? to_f(q[base + r * ld + c + e]) : 0.f;
+      sk[r * dp + c + e] = in ? to_f(k[base + r * ld + c + e]) : 0.f;
+    }
+  }
+  for (int i = tid; i < 64 * d4; i += 256) {
+    const int r = i & 63, c = (i >> 6) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (c + e < depth) sv[(c + e) * kLdP + r] = to_f(v[base + r * ld + c + e]);
   }
   __syncthreads();
-  const int row = threadIdx.x >> 2, part = threadIdx.x & 3;
-  float sc[16];
-  const T* brow = bias ? bias + (((long long)n * heads + h) * 64 + row) * 64 : nullptr;
-  float mx = -3.0e38f;
+  const int tx = tid & 15, row0 = (tid >> 4) * 4;
+  float sc[4][4];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int col = part + 4 * j;  // interleaved so the 4 lanes of a row hit different banks
-    float a = 0.f;
-    for (int c = 0; c < depth; ++c) a = fmaf(sq[row * dp + c], sk[col * dp + c], a);
-    a *= scale;
-    if (brow) a += to_f(brow[col]);
-    sc[j] = a;
-    mx = fmaxf(mx, a);
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sc[i][j] = 0.f;
+#pragma unroll 2
+  for (int c = 0; c < d4 * 4; c += 4) {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(sq + (row0 + i) * dp + c);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(sk + (tx + 16 * j) * dp + c);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        sc[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, sc[i][j]))));
   }
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-  float sum = 0.f;
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    sc[j] = __expf(sc[j] - mx);
-    sum += sc[j];
+  for (int i = 0; i < 4; ++i) {
+    const T* brow = bias ? bias + (((long long)n * heads + h) * 64 + row0 + i) * 64 + tx : nullptr;
+    float mx = -3.0e38f, sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      sc[i][j] *= scale;
+      if (brow) sc[i][j] += to_f(brow[16 * j]);
+      mx = fmaxf(mx, sc[i][j]);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      sc[i][j] = kFast ? __expf(sc[i][j] - mx) : expf(sc[i][j] - mx);
+      sum += sc[i][j];
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sc[i][j] = sc[i][j] / sum;
   }
-  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-  const float inv = 1.0f / sum;
+  __syncthreads();  // Q and K have been read
 #pragma unroll
-  for (int j = 0; j < 16; ++j) sp[row * 65 + part + 4 * j] = sc[j] * inv;
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sp[(row0 + i) * kLdP + tx + 16 * j] = sc[i][j];
   __syncthreads();
-  // O[row][c] for c = part, part+4, ...
-  for (int c = part; c < depth; c += 4) {
-    float a = 0.f;
-#pragma unroll 8
-    for (int j = 0; j < 64; ++j) a = fmaf(sp[row * 65 + j], sv[j * dp + c], a);
-    out[((long long)n * 64 + row) * ldo + (long long)h * depth + c] = from_f<T>(a);
-  }
-}
-
-// fp32 mode uses expf for parity with the CPU oracle.
-template <>
-__global__ void __launch_bounds__(256)
-attention_kernel<float>(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                        long long ld, const float* __restrict__ bias, float* __restrict__ out, long long ldo,
-                        int heads, int depth, float scale) {
-  extern __shared__ float smem[];
-  const int dp = depth + 1;
-  float* sq = smem;
-  float* sk = sq + 64 * dp;
-  float* sv = sk + 64 * dp;
-  float* sp = sv + 64 * dp;
-  const int n = blockIdx.x / heads, h = blockIdx.x - n * heads;
-  const long long base = (long long)n * 64 * ld + (long long)h * depth;
-  for (int i = threadIdx.x; i < 64 * depth; i += 256) {
-    const int r = i / depth, c = i - r * depth;
-    sq[r * dp + c] = q[base + r * ld + c];
-    sk[r * dp + c] = k[base + r * ld + c];
-    sv[r * dp + c] = v[base + r * ld + c];
-  }
-  __syncthreads();
-  const int row = threadIdx.x >> 2, part = threadIdx.x & 3;
-  float sc[16];
-  const float* brow = bias ? bias + (((long long)n * heads + h) * 64 + row) * 64 : nullptr;
-  float mx = -3.0e38f;
+  for (int c0 = tx; c0 < depth; c0 += 32) {
+    const int c1 = c0 + 16 < depth ? c0 + 16 : c0;
+    float o[4][2];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int col = part + 4 * j;
-    float a = 0.f;
-    for (int c = 0; c < depth; ++c) a = fmaf(sq[row * dp + c], sk[col * dp + c], a);
-    a *= scale;
-    if (brow) a += brow[col];
-    sc[j] = a;
-    mx = fmaxf(mx, a);
-  }
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-  float sum = 0.f;
+    for (int i = 0; i < 4; ++i) o[i][0] = o[i][1] = 0.f;
+#pragma unroll 4
+    for (int j = 0; j < 64; j += 4) {
+      const float4 v0 = *reinterpret_cast<const float4*>(sv + c0 * kLdP + j);
+      const float4 v1 = *reinterpret_cast<const float4*>(sv + c1 * kLdP + j);
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    sc[j] = expf(sc[j] - mx);
-    sum += sc[j];
-  }
-  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      for (int i = 0; i < 4; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(sp + (row0 + i) * kLdP + j);
+        o[i][0] = fmaf(a.w, v0.w, fmaf(a.z, v0.z, fmaf(a.y, v0.y, fmaf(a.x, v0.x, o[i][0]))));
+        o[i][1] = fmaf(a.w, v1.w, fmaf(a.z, v1.z, fmaf(a.y, v1.y, fmaf(a.x, v1.x, o[i][1]))));
+      }
+    }
 #pragma unroll
-  for (int j = 0; j < 16; ++j) sp[row * 65 + part + 4 * j] = sc[j] / sum;
-  __syncthreads();
-  for (int c = part; c < depth; c += 4) {
-    float a = 0.f;
-    for (int j = 0; j < 64; ++j) a = fmaf(sp[row * 65 + j], sv[j * dp + c], a);
-    out[((long long)n * 64 + row) * ldo + (long long)h * depth + c] = a;
+    for (int i = 0; i < 4; ++i) {
+      T* dst = out + ((long long)n * 64 + row0 + i) * ldo + (long long)h * depth;
+      dst[c0] = from_f<T>(o[i][0]);
+      if (c0 + 16 < depth) dst[c0 + 16] = from_f<T>(o[i][1]);
+    }
   }
 }
 
@@ -478,13 +476,14 @@ cudaError_t launch_attention(const T* q, const T* k, const T* v, long long ld, c
                              long long ldo, int n, int heads, int depth, float scale, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   if (depth > 128) return cudaErrorInvalidValue;
-  const size_t smem = (size_t)(3 * 64 * (depth + 1) + 64 * 65) * sizeof(float);
+  const int dp = ceil_div(depth, 4) * 4 + 4;
+  const size_t smem = (size_t)(64 * (2 * dp > 68 ? 2 * dp : 68) + depth * 68) * sizeof(float);
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(attention_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  attention_kernel<T><<<n * heads, 256, smem, s>>>(q, k, v, ld, bias, out, ldo, heads, depth, scale);
-  return cudaGetLastError();
+  return launch_dependent(attention_kernel<T>, dim3(n * heads), dim3(256), smem, s, q, k, v, ld, bias, out, ldo, heads, depth,
+                          scale);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -501,14 +500,22 @@ policy_attn_gather_kernel(const float* __restrict__ logits, const T* __restrict_
   __shared__ float off[4][8];
   const int n = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // 32 dot products (4 promotion rows x 8 files), 4 per warp.
-  for (int t = warp * 4; t < warp * 4 + 4; ++t) {
-    const int i = t >> 3, j = t & 7;
-    const T* key = kp + ((long long)n * 64 + 56 + j) * dm;
-    float a = 0.f;
-    for (int c = lane; c < dm; c += 32) a = fmaf(to_f(key[c]), w4[i * dm + c], a);
-    a = warp_sum(a);
-    if (lane == 0) off[i][j] = a;
+  // 32 dot products (4 promotion rows x 8 files), 4 per warp with one row of w4 between them; eight steps of loads in flight
+  {
+    const int i = warp >> 1, j0 = (warp & 1) * 4;
+    const T* key = kp + ((long long)n * 64 + 56 + j0) * dm;
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int c = lane; c < dm; c += 32) {
+      const float w = w4[i * dm + c];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) a[j] = fmaf(to_f(key[(long long)j * dm + c]), w, a[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      a[j] = warp_sum(a[j]);
+      if (lane == 0) off[i][j0 + j] = a[j];
+    }
   }
   __syncthreads();
   const float* lg = logits + (long long)n * 4096;

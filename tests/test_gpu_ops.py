@@ -69,6 +69,26 @@ def test_fma_gemm(lib, prec):
     assert np.abs(C.float().cpu().numpy() - ref).max() <= tol * max(1.0, np.abs(ref).max())
 
 
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (8, 64, 2048), (9, 65, 2047), (32, 4096, 256), (33, 63, 516), (64, 1024, 1024),
+                                   (65, 130, 31), (200, 300, 1000), (1024, 1536, 128)])
+def test_fma_gemm_tiles(lib, prec, M, N, K):
+    """Edges of the FMA kernel's tiles (8 / 32 / 64 rows, 64 columns), K remainders, rows that cannot be read as 16-byte
+    pieces, K ranges cut over a cluster."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = torch.randn(M, K, device="cuda", generator=g).to(DT[prec])
+    W = torch.randn(N, K, device="cuda", generator=g).to(DT[prec])
+    b = torch.randn(N, device="cuda", generator=g)
+    C = torch.zeros(M, N, dtype=DT[prec], device="cuda")
+    _lib.check(lib.b200_op_gemm(A.data_ptr(), W.data_ptr(), b.data_ptr(), C.data_ptr(), M, N, K, oracle.ACT_NONE, prec, 0, None))
+    torch.cuda.synchronize()
+    ref = A.double() @ W.double().T + b.double()
+    mag = A.double().abs() @ W.double().abs().T + b.double().abs()
+    # K + 1 roundings of sums no larger than mag, and the rounding of the storage type
+    bound = (K + 2) * 2.0 ** -24 * mag + (2.0 ** -11 * ref.abs() + 2.0 ** -24 if prec == 1 else 0.0)
+    assert torch.all((C.double() - ref).abs() <= bound), (C.double() - ref).abs().max().item()
+
+
 def test_gemm_tc_rejects_fp32(lib):
     assert lib.b200_op_gemm(None, None, None, None, 128, 128, 64, 3, 0, 1, None) == _lib.ERR_UNSUPPORTED
 
