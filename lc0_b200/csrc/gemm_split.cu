@@ -330,9 +330,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
 }
 
-// Tile width, cluster size and stages of a product: the least of a cost model in cycles.  What it weighs, as measured with
-// chains of dependent launches (M x N x K; us at 1 / 2 / 4 / 8 CTAs per tile of 64 columns): 64x1024x1024 9.5 / 6.7 / 5.6 / 5.9,
-// 1x256x2048 14.8 / 9.5 / 6.7 / 5.5, 256x3104x1024 11.2 / 9.3 / 15.4 / 26.6 (more CTAs than SMs), 32x4096x256 4.3 / 5.0 / 5.8.
+// Tile width, cluster size and stages of a product: the least of a cost model in microseconds, fitted to chains of dependent
+// launches (M x N x K; us measured at columns per tile / CTAs per tile):
+//   1536x1024x1024  32/1 19.5  64/1 11.2  64/2 17.6  128/1 13.9  128/2 12.5    2368x768x256   32/1 10.3  64/1 6.7  128/1 9.2
+//   512x1024x1024   32/1 10.0  32/2 7.9   64/1 11.3  64/4 9.1    128/1 13.6    2368x256x256   32/1 5.3   64/1 6.6  128/1 9.0
+//   512x1024x1536   32/2 9.5   64/2 10.9  64/4 9.8   128/2 12.7                64x1024x1024   32/4 5.9   64/1 9.8  64/4 6.3
+//   1x256x2048      32/1 15.2  32/4 7.1   32/8 5.9   64/4 7.2                  32x4096x256    32/1 4.6   64/1 4.7  128/1 5.5
+// A CTA's time grows with its tile's width and its k-blocks, not with a second CTA beside it on the SM: what is waited for is
+// the latency of loads and of the epilogue.  Beyond two CTAs per SM the rest runs in another round.
 struct SplitPlan { int bn, ks, a_rows, stages; };
 
 SplitPlan split_plan(const GemmParams& g, int sm_count) {
@@ -347,12 +352,9 @@ SplitPlan split_plan(const GemmParams& g, int sm_count) {
       if (ks > k_blocks || (ks > 1 && !g.split_k)) break;
       const int kb = ceil_div(k_blocks, ks);
       const long long ctas = (long long)n_tiles * m_tiles * ks;
-      const double per_sm = (double)ceil_div(ctas, sm_count);
-      // cycles: operand bytes at 64 per cycle and SM, the exchange of the partial tiles, a fixed part per CTA round
-      const double load = (double)kb * (a_rows + bn) * 128 / 64.0;
-      const double exchange = ks > 1 ? 500.0 + a_rows * bn * 4 / 64.0 : 0.0;
-      const double finish = (double)a_rows / ks * bn / 8 / 256.0 * 60.0 + a_rows * bn * 4 / 128.0;
-      const double cost = per_sm * (load + exchange + finish) + 300.0 * (per_sm - 1);
+      const int rounds = ceil_div(ctas, 2 * sm_count);
+      const double tile = 2.5 + a_rows * bn * (1.0 / 3300), exchange = ks == 1 ? 0.0 : (0.25 + 0.2 * ks) * (a_rows == 64 ? 1.0 : 1.6);
+      const double cost = rounds * (tile + 0.39 * kb + exchange + (ctas > sm_count ? 0.5 : 0.0));
       if (cost < best_cost) {
         best_cost = cost;
         best = SplitPlan{bn, ks, a_rows, kb};

@@ -1659,7 +1659,10 @@ cudaError_t launch_gemm_tc(const GemmParams& p, int* status, int sm_count, cudaS
     return four ? launch_pair<T, 4>(p, status, sm_count, s) : launch_pair<T, 2>(p, status, sm_count, s);
   }
   if (p.se_k > 0) return launch_bn<T, 256>(p, status, sm_count, s);  // the tile must hold every channel of two boards
-  if (p.conv_cin == 0 && p.batch_rows == 0) return launch_gemm_split<T>(p, status, sm_count, s);
+  // More 128x128 tiles than two per SM: the persistent kernel's wide tiles (256x32768x768, the dense positional encoding of 256
+  // positions: 24 us, against 30 on gemm_split.cu's kernel).
+  const bool few = (long long)ceil_div(p.M, BM) * ceil_div(p.N, 128) <= 2 * sm_count;
+  if (p.conv_cin == 0 && p.batch_rows == 0 && (few || p.n_split > 0)) return launch_gemm_split<T>(p, status, sm_count, s);
   // Convolutions and stacked products: wide tiles amortise the A-tile loads; narrow problems take the smallest tile that
   // covers N, and skinny problems (few rows) the widest tile that still yields at least half an SM count of CTAs.
   auto tiles = [&](int bn) { return (long long)ceil_div(p.M, BM) * ceil_div(p.N, bn); };
