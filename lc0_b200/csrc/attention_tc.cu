@@ -65,7 +65,7 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(outb + 2 * L::kTile);
   uint64_t* empty_bar = full_bar + NS;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty_bar + NS);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   if (tid == 0) {
     for (int i = 0; i < NS; ++i) {
       mbar_init(smem_u32(&full_bar[i]), 1);
@@ -87,7 +87,7 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 
   if (warp == 4) {
     // ---------------- producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int item = blockIdx.x; item < items; item += gridDim.x, ++it) {
         const int s = it % NS;

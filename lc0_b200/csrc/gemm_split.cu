@@ -87,7 +87,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float4* rowv = reinterpret_cast<float4*>(misc + 256);          // [rows of this CTA's slice] mean_a, rstd_a, mean_r, rstd_r
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int ks = cfg.ks, rank = ks > 1 ? (int)cluster_ctarank() : 0;
   const int n0 = ((int)blockIdx.x / ks) * BN, m0 = (int)blockIdx.y * cfg.a_rows;
   const int k_blocks = (p.K + BK - 1) / BK;
@@ -126,7 +126,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   if (warp == 8) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const int early = kbn < S ? kbn : S;
       for (int i = 0; i < early; ++i) {
         const uint32_t fb = smem_u32(&full_bar[i]);
@@ -134,26 +134,29 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         tma_load_2d(smem_u32(smem + i * stage_bytes) + cfg.a_rows * 128, &tmap_w, (kb0 + i) * BK, n0, fb);
       }
       grid_dependency_wait();
+      int s = 0;
+      uint32_t ph = 0;
       for (int i = 0; i < kbn; ++i) {
-        const int s = i % S;
         const uint32_t fb = smem_u32(&full_bar[s]), sa = smem_u32(smem + s * stage_bytes);
         if (i >= early) {
-          if (!mbar_wait(smem_u32(&empty_bar[s]), ((i / S) & 1) ^ 1, abort_flag, 1)) break;
+          if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, 1)) break;
           mbar_expect_tx(fb, stage_bytes);
           tma_load_2d(sa + cfg.a_rows * 128, &tmap_w, (kb0 + i) * BK, n0, fb);
         }
         tma_load_2d(sa, &tmap_a, (kb0 + i) * BK, m0, fb);
+        if (++s == S) { s = 0; ph ^= 1; }
       }
     }
     __syncwarp();
   } else if (warp == 9) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc<T, BN>();
       bool ok = true;
+      int s = 0;
+      uint32_t ph = 0;
       for (int i = 0; i < kbn; ++i) {
-        const int s = i % S;
-        if (!mbar_wait(smem_u32(&full_bar[s]), (i / S) & 1, abort_flag, 3)) { ok = false; break; }
+        if (!mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag, 3)) { ok = false; break; }
         tcgen05_fence_after();
         const uint32_t sa = smem_u32(smem + s * stage_bytes);
         const uint64_t adesc = make_smem_desc(sa), bdesc = make_smem_desc(sa + cfg.a_rows * 128);
@@ -161,6 +164,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         for (int k = 0; k < BK / 16; ++k)
           tcgen05_mma_f16(tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
         if (i + S < kbn) tcgen05_commit(smem_u32(&empty_bar[s]));
+        if (++s == S) { s = 0; ph ^= 1; }
       }
       if (ok) tcgen05_commit(smem_u32(tfull_bar));
     }

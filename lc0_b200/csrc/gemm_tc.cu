@@ -457,7 +457,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   float* se_gb = reinterpret_cast<float*>(bar_mem + 512 + 8192);    // [2 boards][gate 256 | shift 256]
   float* se_vec = se_gb + 1024;                                     // se_bias [N], se_b1 [se_k], se_b2 [2N]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int m_tiles = (p.M + BM - 1) / BM, n_tiles = (p.N + BN - 1) / BN;
   const int tiles = m_tiles * n_tiles;
   const int k_blocks = p.conv_cblocks > 0 ? 9 * p.conv_cblocks : (p.K + BK - 1) / BK;
@@ -501,7 +501,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
@@ -527,7 +527,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc<T, BN>();
       uint32_t it = 0, tile_it = 0;
       bool ok = true;
@@ -556,7 +556,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
   } else if (warp == 10) {
     // ---------------- store warp: TMA stores of the staged slabs ----------------
-    if (lane == 0 && p.tma_store)
+    if (p.tma_store && elect_one())
       store_warp_loop<2, 2>(p, &tmap_c, &tmap_c, &tmap_r, epi_mem, stg_full, stg_free, res_bar, 0, 2, blockIdx.x, gridDim.x,
                             tiles, n_tiles, BM, 0, BN, 0x7fffffff, abort_flag);
   } else {
@@ -817,7 +817,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
   float* se_gb = reinterpret_cast<float*>(bar_mem + 512 + 8192);    // [2 boards][gate 256 | shift 256]
   float* se_w = se_gb + 1024;                                       // the layer's squeeze-excitation parameters (kSeWBytes)
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 32) {
     for (int l = 0; l < n_layers; ++l) {
       tma_prefetch_map(&layers[l].a);
@@ -861,7 +861,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, nslot[2] = {0, 0};  // nslot: tiles issued per block of the pair
       bool ok = true;
       for (TowerWalk w(n_layers, row_blocks); w.valid() && ok; w.next()) {
@@ -903,7 +903,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc<T, BN>();
       uint32_t it = 0, tile_it = 0;
       bool ok = true;
@@ -931,7 +931,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
     }
   } else if (warp == 10) {
     // ---------------- store warp ----------------
-    if (lane == 0)
+    if (elect_one())
       tower_store_loop(layers, n_layers, row_blocks, epi_mem, stg_full, stg_free, res_bar, done_bar, abort_flag);
   } else {
     // ---------------- epilogue (warps 2..9: two groups of four warps, alternating 64-column slabs) ----------------
@@ -1090,7 +1090,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   float* se_gb = reinterpret_cast<float*>(bar_mem + 512 + 16 * 1024);   // [2 boards][gate 256 | shift 256]
   float* se_vec = se_gb + 1024;                                         // se_bias [N], se_b1 [se_k], se_b2 [2N]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int m_tiles = (p.M + 2 * BM - 1) / (2 * BM), n_tiles = (p.N + BN - 1) / BN;
@@ -1148,17 +1148,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
-    if (lane == 0) {
-      uint32_t it = 0;
+    if (elect_one()) {
+      int s = 0;         // stage and phase of the next k-block
+      uint32_t ph = 0;
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += pairs) {
         const int m0 = (tile_of(t) / n_tiles) * (2 * BM) + (int)rank * BM;
         // a narrower tile is computed with a narrower MMA, of which each CTA supplies half the W rows
         const int n0 = col_of(t) + (int)rank * (mma_n_of(t) / 2) + (p.batch_rows > 0 ? (m0 / p.batch_rows) * p.N : 0);
         const bool half = t >= split_from;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % S;
-          const uint32_t ph = (it / S) & 1;
+        for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, 1)) { ok = false; break; }
           const uint32_t fb_local = smem_u32(&full_bar[s]);
           // both CTAs' bytes land on this barrier; a half-width tile takes 64 W rows per CTA instead of 128
@@ -1175,15 +1174,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             tma_load_2d_pair(sa, &tmap_a, kb * BK, m0, fb);
             tma_load_2d_pair(sa + BM * BK * 2, half ? &tmap_wh : &tmap_w, kb * BK, n0, fb);
           }
+          if (++s == S) { s = 0; ph ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (even CTA only) ----------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc_base = (1u << 4) | (FmtCode<T>::v << 7) | (FmtCode<T>::v << 10) |
                                       ((uint32_t)((2 * BM) >> 4) << 24);
-      uint32_t it = 0, tile_it = 0;
+      int s = 0;         // stage and phase of the next k-block
+      uint32_t ph = 0, tile_it = 0;
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += pairs, ++tile_it) {
         const uint32_t acc = tile_it & 1, aph = (tile_it >> 1) & 1;
@@ -1191,9 +1192,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         const uint32_t idesc = idesc_base | ((uint32_t)(mma_n_of(t) >> 3) << 17);
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % S;
-          const uint32_t ph = (it / S) & 1;
+        for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag, 3)) { ok = false; break; }
           tcgen05_fence_after();
           const uint32_t sa = smem_u32(smem + s * Cfg::kStageBytes);
@@ -1202,20 +1201,15 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
             tcgen05_mma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          const uint32_t eb = smem_u32(&empty_bar[s]);
-          tcgen05_commit_pair(mapa(eb, 0));  // frees the stage in both CTAs once the MMAs have read it
-          tcgen05_commit_pair(mapa(eb, 1));
+          tcgen05_commit_both(smem_u32(&empty_bar[s]));  // frees the stage in both CTAs once the MMAs have read it
+          if (++s == S) { s = 0; ph ^= 1; }
         }
-        if (ok) {
-          const uint32_t tb = smem_u32(&tfull_bar[acc]);
-          tcgen05_commit_pair(mapa(tb, 0));
-          tcgen05_commit_pair(mapa(tb, 1));
-        }
+        if (ok) tcgen05_commit_both(smem_u32(&tfull_bar[acc]));
       }
     }
   } else if (warp == 2 || warp == 3) {
     // ---------------- store warps (both CTAs): TMA stores of the staged slabs, half of the groups each ----------
-    if (lane == 0)
+    if (elect_one())
       store_warp_loop<kGroups, kBufs>(p, &tmap_c, &tmap_c2, &tmap_r, epi_mem, stg_full, stg_free, res_bar,
                                       (warp - 2) * (kGroups / 2), (warp - 1) * (kGroups / 2), pair, pairs, tiles, n_tiles,
                                       2 * BM, (int)rank * BM, BN, split_from, abort_flag);

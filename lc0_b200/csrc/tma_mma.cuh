@@ -63,6 +63,20 @@ template <> __device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t v)
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+// One lane of a converged warp.  The warp that issues TMA or tcgen05 instructions picks its lane with this and not with a lane
+// index: the compiler then knows that a single thread runs the block and keeps the instructions' operands in uniform
+// registers.  (Figures: tcgen05.cuh.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok));
+  return ok != 0;
+}
+// Index of this thread's warp, known to the compiler to be the same in the whole warp.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
