@@ -6,7 +6,8 @@
 // Bound by the FMA pipe (74 TFLOP/s at 1.965 GHz), for few rows by the latency of the K loop.  Operands are staged
 // K-contiguous as they lie in memory (16-byte cp.async, four floats of one row) in three stages; rows are padded by four floats
 // so that eight rows of a quarter warp fall on different banks.  A thread owns TM x TN outputs whose rows are 8 and whose
-// columns 4 apart and reads TM + TN 16-byte pieces per four k for 4 TM TN FMAs.
+// columns 4 apart and reads TM + TN 16-byte pieces per four k for 4 TM TN FMAs.  Two groups of warps take alternate pieces of k, so
+// that a tile that has an SM to itself still has two warps per scheduler; their sums are added at the end.
 // With GemmParams::split_k the K range of a tile that leaves SMs idle is cut over a cluster of up to eight CTAs, whose sums
 // meet through distributed shared memory in a fixed order.
 #include <atomic>
@@ -47,21 +48,17 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Four elements of one operand row (fewer at the end of the row: zeros) into shared memory as floats.
+// Four elements from `src` into shared memory as floats; those from `left` on are zeros (left may be anything).
 template <typename T>
-__device__ __forceinline__ void stage4(float* dst, const T* row, int left, bool vec) {
-  if (!row || left <= 0) {
-    *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-    return;
-  }
+__device__ __forceinline__ void stage4(float* dst, const T* src, int left, bool vec) {
   if constexpr (sizeof(T) == 4) {
     if (vec) {
-      cp_async16((uint32_t)__cvta_generic_to_shared(dst), row, left >= 4 ? 16 : left * 4);
+      cp_async16((uint32_t)__cvta_generic_to_shared(dst), src, min(max(left, 0), 4) * 4);
       return;
     }
   } else {
     if (vec && left >= 4) {
-      const uint2 u = *reinterpret_cast<const uint2*>(row);
+      const uint2 u = *reinterpret_cast<const uint2*>(src);
       const T* e = reinterpret_cast<const T*>(&u);
       *reinterpret_cast<float4*>(dst) = make_float4(to_f(e[0]), to_f(e[1]), to_f(e[2]), to_f(e[3]));
       return;
@@ -69,14 +66,14 @@ __device__ __forceinline__ void stage4(float* dst, const T* row, int left, bool 
   }
   float v[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = i < left ? to_f(row[i]) : 0.f;
+  for (int i = 0; i < 4; ++i) v[i] = i < left ? to_f(src[i]) : 0.f;
   *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
-template <typename T, bool kFast, int BM, int BN, int TM, int TN, int kBK, int kMinCtas, bool kConv>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), kMinCtas)
+template <typename T, bool kFast, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv>
+__global__ void __launch_bounds__(kGroups * (BM / TM) * (BN / TN), kMinCtas)
 gemm_fma_kernel(const FmaParams p) {
-  constexpr int kThreads = (BM / TM) * (BN / TN);
+  constexpr int kGroupThreads = (BM / TM) * (BN / TN), kThreads = kGroups * kGroupThreads;
   constexpr int kWarpM = 8 * TM, kWarpN = 4 * TN;  // outputs of a warp
   constexpr int kLd = kBK + 4, kLdOut = BN + 4, kPieces = kBK / 4;
   constexpr int kRowStep = kThreads / kPieces;     // rows staged at a time
@@ -90,52 +87,67 @@ gemm_fma_kernel(const FmaParams p) {
   const int k_blocks = (p.K + kBK - 1) / kBK;
   const int kb0 = (int)((long long)k_blocks * rank / p.ks), kbn = (int)((long long)k_blocks * (rank + 1) / p.ks) - kb0;
 
+  // This thread stages the four k from lk on of rows lr, lr + kRowStep, ... of both tiles.
+  constexpr int kRowsA = (BM + kRowStep - 1) / kRowStep, kRowsW = (BN + kRowStep - 1) / kRowStep;
   const int lr = tid / kPieces, lk = tid % kPieces * 4;
+  long long off_a[kRowsA], off_w[kRowsW];
+  uint32_t ok_a[kRowsA], ok_w = 0;  // convolution: bit t of ok_a = tap t of that row lies on the board
+#pragma unroll
+  for (int r = 0; r < kRowsA; ++r) {
+    const int m = m0 + lr + r * kRowStep;
+    const bool in = m < p.M && lr + r * kRowStep < BM;
+    off_a[r] = in ? (long long)m * p.lda : 0;
+    ok_a[r] = in ? 1 : 0;
+    if constexpr (kConv) {
+      ok_a[r] = 0;
+      for (int t = 0; t < 9; ++t) {
+        const int y = ((m >> 3) & 7) + t / 3 - 1, x = (m & 7) + t % 3 - 1;
+        if (in && (unsigned)y < 8u && (unsigned)x < 8u) ok_a[r] |= 1u << t;
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kRowsW; ++r) {
+    const int n = n0 + lr + r * kRowStep;
+    const bool in = n < p.N && lr + r * kRowStep < BN;
+    off_w[r] = in ? (long long)n * p.ldw : 0;
+    if (in) ok_w |= 1u << r;
+  }
   auto stage_w = [&](int i) {
     if (i >= kbn) return;
-    float* dst = sm + (i % kStages) * (BM + BN) * kLd + BM * kLd + lk;
+    float* dst = sm + (i % kStages) * (BM + BN) * kLd + (BM + lr) * kLd + lk;
     int k = (kb0 + i) * kBK + lk, left = p.K - k;
     const T* w = W;
     if constexpr (kConv) {
       const int tap = k / p.conv_kt;
       k -= tap * p.conv_kt;
       left = tap < 9 ? p.conv_cin - k : 0;
-      w += (long long)tap * p.N * p.conv_cin;
+      if (tap < 9) w += (long long)tap * p.N * p.conv_cin;
     }
+    if (left > 0) w += k;
 #pragma unroll
-    for (int r = 0; r < BN; r += kRowStep) {
-      const int n = n0 + r + lr;
-      if (BN % kRowStep == 0 || r + lr < BN)
-        stage4(dst + (r + lr) * kLd, n < p.N ? w + (long long)n * p.ldw + k : nullptr, left, p.vec);
-    }
+    for (int r = 0; r < kRowsW; ++r)
+      if (BN % kRowStep == 0 || lr + r * kRowStep < BN)
+        stage4(dst + r * kRowStep * kLd, w + off_w[r], (ok_w >> r) & 1 ? left : 0, p.vec);
   };
   auto stage_a = [&](int i) {
     if (i >= kbn) return;
-    float* dst = sm + (i % kStages) * (BM + BN) * kLd + lk;
+    float* dst = sm + (i % kStages) * (BM + BN) * kLd + lr * kLd + lk;
     const int k = (kb0 + i) * kBK + lk;
-    int dy = 0, dx = 0, c = k, left = p.K - k;
+    int left = p.K - k, tap = 0;
+    long long at = k;
     if constexpr (kConv) {
-      const int tap = k / p.conv_kt;
-      c = k - tap * p.conv_kt;
+      tap = k / p.conv_kt;
+      const int c = k - tap * p.conv_kt;
       left = tap < 9 ? p.conv_cin - c : 0;
-      dy = tap / 3 - 1;
-      dx = tap % 3 - 1;
+      at = ((tap / 3 - 1) * 8 + tap % 3 - 1) * p.conv_cin + c;
     }
 #pragma unroll
-    for (int r = 0; r < BM; r += kRowStep) {
-      if (BM % kRowStep != 0 && r + lr >= BM) break;
-      const int m = m0 + r + lr;
-      const T* row = nullptr;
-      if (m < p.M) {
-        if constexpr (kConv) {
-          const int y = ((m >> 3) & 7) + dy, x = (m & 7) + dx;
-          if ((unsigned)y < 8u && (unsigned)x < 8u) row = A + (long long)(m + dy * 8 + dx) * p.lda + c;
-        } else {
-          row = A + (long long)m * p.lda + c;
-        }
+    for (int r = 0; r < kRowsA; ++r)
+      if (BM % kRowStep == 0 || lr + r * kRowStep < BM) {
+        const bool in = (ok_a[r] >> tap) & 1 && left > 0;
+        stage4(dst + r * kRowStep * kLd, in ? A + off_a[r] + at : A, in ? left : 0, p.vec);
       }
-      stage4(dst + (r + lr) * kLd, row, left, p.vec);
-    }
   };
 
   // weights do not depend on the kernel before this one (w_const): they are requested while it is still running
@@ -151,7 +163,8 @@ gemm_fma_kernel(const FmaParams p) {
   }
 
   constexpr int kWarpsN = BN / kWarpN;
-  const int wm = warp / kWarpsN * kWarpM + (lane & 7), wn = warp % kWarpsN * kWarpN + (lane >> 3);
+  const int group = tid / kGroupThreads, gw = warp - group * (kGroupThreads / 32);
+  const int wm = gw / kWarpsN * kWarpM + (lane & 7), wn = gw % kWarpsN * kWarpN + (lane >> 3);
   float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
@@ -168,7 +181,8 @@ gemm_fma_kernel(const FmaParams p) {
     const float* as = sm + (i % kStages) * (BM + BN) * kLd + wm * kLd;
     const float* ws = sm + (i % kStages) * (BM + BN) * kLd + BM * kLd + wn * kLd;
 #pragma unroll
-    for (int k = 0; k < kBK; k += 4) {
+    for (int kk = 0; kk < kBK; kk += 4 * kGroups) {
+      const int k = kk + group * 4;
       float4 a[TM];
 #pragma unroll
       for (int r = 0; r < TM; ++r) a[r] = *reinterpret_cast<const float4*>(as + r * 8 * kLd + k);
@@ -204,9 +218,18 @@ gemm_fma_kernel(const FmaParams p) {
   cp_async_wait<0>();
   __syncthreads();
 #pragma unroll
-  for (int r = 0; r < TM; ++r)
+  for (int g = kGroups - 1; g >= 0; --g) {
+    if (group == g) {
 #pragma unroll
-    for (int c = 0; c < TN; ++c) sm[(wm + r * 8) * kLdOut + wn + c * 4] = acc[r][c];
+      for (int r = 0; r < TM; ++r)
+#pragma unroll
+        for (int c = 0; c < TN; ++c) {
+          float* o = sm + (wm + r * 8) * kLdOut + wn + c * 4;
+          *o = g == kGroups - 1 ? acc[r][c] : acc[r][c] + *o;
+        }
+    }
+    if (g > 0) __syncthreads();
+  }
   if (p.ks == 1) {
     __syncthreads();
     for (int e = tid; e < BM * BN; e += kThreads) finish(m0 + e / BN, n0 + e % BN, sm[e / BN * kLdOut + e % BN]);
@@ -229,10 +252,10 @@ gemm_fma_kernel(const FmaParams p) {
   cluster_sync();  // the others may still be reading this CTA's sums
 }
 
-template <typename T, int BM, int BN, int TM, int TN, int kBK, int kMinCtas, bool kConv>
+template <typename T, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv>
 cudaError_t launch_tile(const FmaParams& p, int batch, cudaStream_t s) {
   constexpr int ring = kStages * (BM + BN) * (kBK + 4) * 4, out = BM * (BN + 4) * 4, smem = ring > out ? ring : out;
-  auto kernel = gemm_fma_kernel<T, (sizeof(T) == 2), BM, BN, TM, TN, kBK, kMinCtas, kConv>;
+  auto kernel = gemm_fma_kernel<T, (sizeof(T) == 2), BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv>;
   static std::atomic<unsigned long long> attr_mask{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -243,7 +266,7 @@ cudaError_t launch_tile(const FmaParams& p, int batch, cudaStream_t s) {
   }
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(ceil_div(p.N, BN) * p.ks, ceil_div(p.M, BM), batch);
-  lc.blockDim = dim3((BM / TM) * (BN / TN));
+  lc.blockDim = dim3(kGroups * (BM / TM) * (BN / TN));
   lc.dynamicSmemBytes = smem;
   lc.stream = s;
   cudaLaunchAttribute attr[2];
@@ -265,23 +288,26 @@ cudaError_t launch_tile(const FmaParams& p, int batch, cudaStream_t s) {
   return cudaLaunchKernelEx(&lc, kernel, p);
 }
 
-// CTAs per tile: cuts of the K range, down to four k-blocks of 32 each, while they find SMs that have nothing to do.
+// CTAs per tile: cuts of the K range, down to four k-blocks of 32 each, while they find SMs with little to do.  Measured (us at
+// 1 / 2 / 4 / 8 cuts): 64x64 tiles 256x1024x1024 38 / 23 / 21 / 26, 256x3072x1024 67 / 57 / 60 / 73, 1024x1024x1024 67 / 73 /
+// 76 / 94, 64x1024x1024 37 / 22 / 13 / 13, 64x3072x1024 37 / 23 / 21 / 24; 32x64 tiles 16x256x2048 45 / 25 / 15 / 10,
+// 16x8192x256 8 / 9 / 13.
 int cuts(const FmaParams& p, int bm, int bn, int batch, bool split, int ctas) {
   const long long tiles = (long long)ceil_div(p.N, bn) * ceil_div(p.M, bm) * batch;
   const int k_blocks = ceil_div(p.K, 32);
   int ks = 1;
-  while (split && ks < 8 && tiles * ks * 2 <= ctas && k_blocks / (ks * 2) >= 4) ks *= 2;
+  while (split && ks < 8 && tiles * ks * 2 <= (ks == 4 ? 148 : ctas) && k_blocks / (ks * 2) >= 4) ks *= 2;
   return ks;
 }
 
 template <typename T, bool kConv>
 cudaError_t launch_fma(FmaParams p, int batch, bool split, cudaStream_t s) {
   if constexpr (!kConv) {  // a convolution has whole boards of 64 rows
-    if (p.M <= 8) { p.ks = cuts(p, 8, 64, batch, split, 148); return launch_tile<T, 8, 64, 1, 4, 32, 1, false>(p, batch, s); }
-    if (p.M <= 32) { p.ks = cuts(p, 32, 64, batch, split, 512); return launch_tile<T, 32, 64, 4, 4, 32, 1, false>(p, batch, s); }
+    if (p.M <= 8) { p.ks = cuts(p, 8, 64, batch, split, 148); return launch_tile<T, 8, 64, 1, 4, 32, 2, 2, false>(p, batch, s); }
+    if (p.M <= 32) { p.ks = cuts(p, 32, 64, batch, split, 148); return launch_tile<T, 32, 64, 4, 4, 32, 2, 2, false>(p, batch, s); }
   }
-  p.ks = cuts(p, 64, 64, batch, split, 512);
-  return launch_tile<T, 64, 64, 8, 4, 32, 4, kConv>(p, batch, s);
+  p.ks = cuts(p, 64, 64, batch, split, 400);
+  return launch_tile<T, 64, 64, 8, 4, 32, 2, 2, kConv>(p, batch, s);
 }
 
 template <typename T> bool aligned4(const void* ptr, long long ld, long long stride) {
