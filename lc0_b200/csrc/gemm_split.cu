@@ -17,6 +17,11 @@
 // Chains of dependent launches, before (one 128xBN tile per CTA of gemm_tc.cu's kernel, FMA kernel below 64 rows) and now:
 // 64x1024x1024 15 -> 5.9 us, 1x256x2048 135 -> 5.3 us, 1x8192x256 21 -> 4.5 us, 32x4096x256 24 -> 4.2 us; one position of the
 // BT4-class network 4.37 -> 0.97 ms, 24 positions 4.47 -> 2.09 ms.
+// With a LayerNorm in front (GemmParams::ln_gamma; 256-wide rows, smolgen's two inner LayerNorms) warps 0-7 load the 64 rows of
+// A themselves, normalise them in registers and write them to the operand tiles in the swizzle TMA would have used; gamma and
+// beta arrive by bulk copy ahead of the grid dependency.  A LayerNorm vector may span several rows of A (smolgen's
+// second one: 32 heads x 256), as long as a tile holds whole vectors.  Every column tile repeats the LayerNorm: worth it
+// while a launch costs more than that (Net::gemm_with_ln has the line).
 // Every wait is bounded by wall-clock time like those of gemm_tc.cu; the cluster barriers are reached by all threads
 // whatever happened before them.
 #include <atomic>
@@ -33,7 +38,15 @@ struct SplitCfg {
   int stages;  // shared-memory stages
   int a_rows;  // 64 or 128: rows of an A box = rows of the tile that exist
   int ks;      // CTAs per tile (cluster size)
+  // LayerNorm in front of the product (kLN): x [M][256], vectors of `group` consecutive rows
+  const void* x;
+  const float* gamma;
+  const float* beta;
+  int group;
+  float eps;
 };
+constexpr int kLnK = 256;  // row width of A with a LayerNorm: four k-blocks, all of them resident
+constexpr int kLnMaxGroup = 32;
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -68,9 +81,31 @@ template <int BN> struct SplitTile {
     const int ring = stages * stage_bytes(a_rows), part = a_rows * BN * 4;  // the partial tiles reuse the ring
     return (ring > part ? ring : part) + kTail + kMisc;
   }
+  __host__ __device__ static constexpr int ln_bytes(int group) { return group * kLnK * 8; }  // gamma and beta
 };
 
-template <typename T, int BN>
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+               "r"(bytes), "r"(bar)
+               : "memory");
+}
+// Sum over the rows of a LayerNorm vector of each row's `v` (four lanes per row, eight rows per warp, 64 rows per CTA): over
+// lanes by shuffles, over warps (vectors of more than eight rows) through red[8].  All 256 threads call it.
+__device__ __forceinline__ float ln_sum(float v, int group, float* red) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  for (int o = 1; o < group && o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, 4 * o);
+  if (group > 8) {
+    const int warp = threadIdx.x >> 5, span = group >> 3;
+    if ((threadIdx.x & 31) == 0) red[warp] = v;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    v = 0.f;
+    for (int w = warp & ~(span - 1), e = w + span; w < e; ++w) v += red[w];
+  }
+  return v;
+}
+
+template <typename T, int BN, bool kLN>
 __global__ void __launch_bounds__(kSplitThreads)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const TcParams p,
                   const SplitCfg cfg) {
@@ -85,7 +120,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint64_t* tfull_bar = empty_bar + kMaxStages;                  // accumulator complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* gb_bar = reinterpret_cast<uint64_t*>(misc + 216);    // kLN: gamma and beta have landed
+  uint64_t* a_bar = gb_bar + 1;                                  // kLN: the normalised rows are in place
   float4* rowv = reinterpret_cast<float4*>(misc + 256);          // [rows of this CTA's slice] mean_a, rstd_a, mean_r, rstd_r
+  float* ln_gb = reinterpret_cast<float*>(misc + 256 + 128 * 16);  // kLN: gamma [group * 256], beta [group * 256]
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int ks = cfg.ks, rank = ks > 1 ? (int)cluster_ctarank() : 0;
@@ -102,6 +140,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       mbar_init(smem_u32(&empty_bar[i]), 1);
     }
     mbar_init(smem_u32(tfull_bar), 1);
+    if (kLN) {
+      mbar_init(smem_u32(gb_bar), 1);
+      mbar_init(smem_u32(a_bar), 256);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -130,13 +172,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const int early = kbn < S ? kbn : S;
       for (int i = 0; i < early; ++i) {
         const uint32_t fb = smem_u32(&full_bar[i]);
-        mbar_expect_tx(fb, stage_bytes);
+        mbar_expect_tx(fb, kLN ? BN * 128 : stage_bytes);
         tma_load_2d(smem_u32(smem + i * stage_bytes) + cfg.a_rows * 128, &tmap_w, (kb0 + i) * BK, n0, fb);
+      }
+      if constexpr (kLN) {
+        const uint32_t bytes = cfg.group * kLnK * 4, gb = smem_u32(gb_bar);
+        mbar_expect_tx(gb, 2 * bytes);
+        bulk_load(smem_u32(ln_gb), cfg.gamma, bytes, gb);
+        bulk_load(smem_u32(ln_gb) + bytes, cfg.beta, bytes, gb);
       }
       grid_dependency_wait();
       int s = 0;
       uint32_t ph = 0;
-      for (int i = 0; i < kbn; ++i) {
+      for (int i = 0; !kLN && i < kbn; ++i) {
         const uint32_t fb = smem_u32(&full_bar[s]), sa = smem_u32(smem + s * stage_bytes);
         if (i >= early) {
           if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, 1)) break;
@@ -152,10 +200,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
       constexpr uint32_t idesc = make_idesc<T, BN>();
-      bool ok = true;
+      bool ok = !kLN || mbar_wait(smem_u32(a_bar), 0, abort_flag, 5);
       int s = 0;
       uint32_t ph = 0;
-      for (int i = 0; i < kbn; ++i) {
+      for (int i = 0; ok && i < kbn; ++i) {
         if (!mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag, 3)) { ok = false; break; }
         tcgen05_fence_after();
         const uint32_t sa = smem_u32(smem + s * stage_bytes);
@@ -178,6 +226,51 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       load8(p.res_beta, col, p.N, ve);
     }
     grid_dependency_wait();
+    if constexpr (kLN) {
+      // row tid / 4; its 16-byte pieces q, q + 4, ..., q + 28 (piece c is piece c % 8 of k-block c / 8)
+      const int row = tid >> 2, q = tid & 3, m = m0 + row;
+      uint4 u[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        u[i] = m < p.M ? *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(cfg.x) + (long long)m * kLnK + (q + 4 * i) * 8)
+                       : make_uint4(0, 0, 0, 0);
+      float* red = reinterpret_cast<float*>(rowv);  // rowv is not used here: no statistics come with a LayerNorm in front
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum += to_f(reinterpret_cast<const T*>(&u[i])[j]);
+      const float inv = 1.0f / (float)(cfg.group * kLnK);  // a power of two
+      const float mean = ln_sum(sum, cfg.group, red) * inv;
+      float var = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float d = to_f(reinterpret_cast<const T*>(&u[i])[j]) - mean;
+          var = fmaf(d, d, var);
+        }
+      const float rstd = 1.0f / sqrtf(ln_sum(var, cfg.group, red + 8) * inv + cfg.eps);
+      mbar_wait(smem_u32(gb_bar), 0, abort_flag, 6);
+      const float* gamma = ln_gb + (row & (cfg.group - 1)) * kLnK;
+      const float* beta = gamma + cfg.group * kLnK;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int c = q + 4 * i;
+        const T* e = reinterpret_cast<const T*>(&u[i]);
+        float v[8], g[8], b[8];
+        *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(gamma + c * 8);
+        *reinterpret_cast<float4*>(g + 4) = *reinterpret_cast<const float4*>(gamma + c * 8 + 4);
+        *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(beta + c * 8);
+        *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(beta + c * 8 + 4);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = b[j] + g[j] * (to_f(e[j]) - mean) * rstd;
+        st_shared_v4(smem_u32(smem + (c >> 3) * stage_bytes) + row * 128 + (((c & 7) ^ (row & 7)) << 4), pack_pair<T>(v[0], v[1]),
+                     pack_pair<T>(v[2], v[3]), pack_pair<T>(v[4], v[5]), pack_pair<T>(v[6], v[7]));
+      }
+      fence_async_smem();  // the tensor core reads the rows through the asynchronous proxy
+      mbar_arrive(smem_u32(a_bar));
+    }
     if (tid < rp && (p.a_stats || p.res_mode == 2)) {
       const int m = m0 + rank * rp + tid;
       float4 v = make_float4(0.f, 1.f, 0.f, 1.f);
@@ -371,14 +464,15 @@ SplitPlan split_plan(const GemmParams& g, int sm_count) {
   return best;
 }
 
-template <typename T, int BN>
+template <typename T, int BN, bool kLN = false>
 cudaError_t launch_split_bn(const GemmParams& g, const SplitPlan& plan, int* status, cudaStream_t s) {
   static std::atomic<unsigned long long> attr_mask{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (!(attr_mask.load() >> (dev & 63) & 1ull)) {
-    e = cudaFuncSetAttribute(gemm_split_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+    e = cudaFuncSetAttribute(gemm_split_kernel<T, BN, kLN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kLN ? SplitTile<BN>::bytes(64, kLnK / BK) + SplitTile<BN>::ln_bytes(kLnMaxGroup) : 112 * 1024);
     if (e != cudaSuccess) return e;
     attr_mask.fetch_or(1ull << (dev & 63));
   }
@@ -388,11 +482,11 @@ cudaError_t launch_split_bn(const GemmParams& g, const SplitPlan& plan, int* sta
   if ((e = gemm_tensor_map(g.W, g.ldw, g.N, g.K, BN, prec, &mw)) != cudaSuccess) return e;
   TcParams p;
   fill_tc_params(p, g, status);
-  const SplitCfg cfg{plan.stages, plan.a_rows, plan.ks};
+  const SplitCfg cfg{plan.stages, plan.a_rows, plan.ks, g.A, g.ln_gamma, g.ln_beta, g.ln_group, g.ln_eps};
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(ceil_div(g.N, BN) * plan.ks, ceil_div(g.M, plan.a_rows));
   lc.blockDim = dim3(kSplitThreads);
-  lc.dynamicSmemBytes = SplitTile<BN>::bytes(plan.a_rows, plan.stages);
+  lc.dynamicSmemBytes = SplitTile<BN>::bytes(plan.a_rows, plan.stages) + (kLN ? SplitTile<BN>::ln_bytes(g.ln_group) : 0);
   lc.stream = s;
   cudaLaunchAttribute attr[2];
   int na = 0;
@@ -410,10 +504,27 @@ cudaError_t launch_split_bn(const GemmParams& g, const SplitPlan& plan, int* sta
   }
   lc.attrs = attr;
   lc.numAttrs = na;
-  return cudaLaunchKernelEx(&lc, gemm_split_kernel<T, BN>, ma, mw, p, cfg);
+  return cudaLaunchKernelEx(&lc, gemm_split_kernel<T, BN, kLN>, ma, mw, p, cfg);
 }
 
 }  // namespace
+
+bool gemm_ln_supported(const GemmParams& g) {
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  return gemm_tc_supported(g) && !g.skip && g.K == kLnK && g.lda == kLnK && g.ln_group >= 1 && g.ln_group <= kLnMaxGroup &&
+         (g.ln_group & (g.ln_group - 1)) == 0 && g.M % g.ln_group == 0 && g.ln_gamma && g.ln_beta && al16(g.A) &&
+         al16(g.ln_gamma) && al16(g.ln_beta) && !g.a_stats && !g.res && !g.out_stats && g.n_split == 0 && g.conv_cin == 0 &&
+         g.batch_rows == 0;
+}
+
+template <typename T>
+cudaError_t launch_gemm_ln(const GemmParams& g, int* status, cudaStream_t s) {
+  if (g.M <= 0 || g.N <= 0) return cudaSuccess;
+  if (!gemm_ln_supported(g)) return cudaErrorInvalidValue;
+  return launch_split_bn<T, 64, true>(g, SplitPlan{64, 1, 64, kLnK / BK}, status, s);
+}
+template cudaError_t launch_gemm_ln<__half>(const GemmParams&, int*, cudaStream_t);
+template cudaError_t launch_gemm_ln<__nv_bfloat16>(const GemmParams&, int*, cudaStream_t);
 
 template <typename T>
 cudaError_t launch_gemm_split(const GemmParams& g, int* status, int sm_count, cudaStream_t s) {

@@ -63,6 +63,12 @@ struct GemmParams {
   // Products of few rows: the K range may be cut over several CTAs (gemm_split.cu).  The sums then depend on the number of
   // rows; off, a row's result is the same whatever else is in the batch.
   bool split_k = true;
+  // LayerNorm of A inside the product (launch_gemm_ln): every ln_group consecutive rows of A, which are 256 wide and packed,
+  // are one LayerNorm vector with ln_gamma / ln_beta [ln_group * 256].
+  const float* ln_gamma = nullptr;
+  const float* ln_beta = nullptr;
+  int ln_group = 1;
+  float ln_eps = 0.f;
 };
 
 // FMA kernel (gemm_fma.cu): any shape and alignment, batched products; no folded LayerNorm, residual or statistics.
@@ -71,6 +77,9 @@ template <typename T> cudaError_t launch_gemm_fma(const GemmParams& p, cudaStrea
 // `status` is a device int the kernel sets non-zero when a bounded wait gives up.
 template <typename T> cudaError_t launch_gemm_tc(const GemmParams& p, int* status, int sm_count, cudaStream_t s);
 bool gemm_tc_supported(const GemmParams& p);
+// Product with the LayerNorm of its input in front (gemm_split.cu), for few rows.
+bool gemm_ln_supported(const GemmParams& p);
+template <typename T> cudaError_t launch_gemm_ln(const GemmParams& p, int* status, cudaStream_t s);
 bool gemm_tc_se_supported(const GemmParams& p);
 // Whether launch_gemm_tc can run `p` with its second output (C2 / n_split).
 bool gemm_tc_split_supported(const GemmParams& p);

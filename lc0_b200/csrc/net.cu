@@ -1170,6 +1170,27 @@ struct Net : NetBase {
     p.split_k = t_split_k;
     run_gemm(st, p);
   }
+  // d(LayerNorm(x)) in one launch, every `group` rows of x being one LayerNorm vector; false where it does not apply: other
+  // widths, and batches at which the LayerNorm repeated in every column tile costs more than its own launch.
+  bool gemm_with_ln(cudaStream_t st, const T* x, const float* gamma, const float* beta, int group, const Dense<T>& d, T* y,
+                    long long ldc, int M, int act) {
+    if constexpr (sizeof(T) == 2) {
+      GemmParams p;
+      p.A = x; p.lda = d.in; p.W = d.w; p.ldw = d.in; p.bias = d.b; p.C = y; p.ldc = ldc;
+      p.M = M; p.N = d.out; p.K = d.in; p.act = act;
+      p.ln_gamma = gamma; p.ln_beta = beta; p.ln_group = group; p.ln_eps = 1e-3f;
+      if (!use_tc || M > (group > 1 ? kLnInProductRows : 64) || !gemm_ln_supported(p)) return false;
+      launches++;
+      const int sp_ = span_begin(st, K_GEMM_TC, 2.0 * p.M * (double)p.N * p.K, t_tag);
+      CK(launch_gemm_ln<T>(p, t_status, st));
+      span_end(st, sp_);
+      return true;
+    }
+    return false;
+  }
+  // Rows of a generator product up to which its LayerNorm (vectors over several rows) is worth repeating in 64 column tiles: one
+  // position of the BT4-class network 847 -> 820 us; at 768 rows (24 positions) 1730 -> 2163 us, one CTA of 139 KB per SM.
+  static constexpr int kLnInProductRows = 256;
   // Tag of the launches that follow on this thread (which product of the layer they are), for the tagged profile.
   static inline thread_local int t_tag = 0;
   void run_gemm(cudaStream_t st, const GemmParams& p) {
@@ -1422,11 +1443,17 @@ struct Net : NetBase {
       t_tag = TAG_SMOLGEN_DENSE;
       if (!merged) gemm_ln(st, in, E, e.sg_compress, s.sg_c, sg_hc, R, ACT_NONE);
       gemm(st, s.sg_c, 64 * sg_hc, e.sg_d1, s.sg_h1, sg_hid, n, act_smolgen);
-      ln(st, s.sg_h1, s.sg_h1, nullptr, e.sg_ln1g, e.sg_ln1b, n, sg_hid, 1.f, 1e-3f);
-      gemm(st, s.sg_h1, sg_hid, e.sg_d2, s.sg_h2, sg_gen, n, act_smolgen);
-      ln(st, s.sg_h2, s.sg_h2, nullptr, e.sg_ln2g, e.sg_ln2b, n, sg_gen, 1.f, 1e-3f);
+      if (!gemm_with_ln(st, s.sg_h1, e.sg_ln1g, e.sg_ln1b, 1, e.sg_d2, s.sg_h2, sg_gen, n, act_smolgen)) {
+        ln(st, s.sg_h1, s.sg_h1, nullptr, e.sg_ln1g, e.sg_ln1b, n, sg_hid, 1.f, 1e-3f);
+        gemm(st, s.sg_h1, sg_hid, e.sg_d2, s.sg_h2, sg_gen, n, act_smolgen);
+      }
       t_tag = TAG_SMOLGEN_BIAS;
-      gemm(st, s.sg_h2, sg_gen / H, smolgen_w, s.sg_bias, 4096, n * H, ACT_NONE);
+      if (!gemm_with_ln(st, s.sg_h2, e.sg_ln2g, e.sg_ln2b, H, smolgen_w, s.sg_bias, 4096, n * H, ACT_NONE)) {
+        t_tag = TAG_SMOLGEN_DENSE;
+        ln(st, s.sg_h2, s.sg_h2, nullptr, e.sg_ln2g, e.sg_ln2b, n, sg_gen, 1.f, 1e-3f);
+        t_tag = TAG_SMOLGEN_BIAS;
+        gemm(st, s.sg_h2, sg_gen / H, smolgen_w, s.sg_bias, 4096, n * H, ACT_NONE);
+      }
       bias = s.sg_bias;
     }
     run_attention(st, s.qkv, 3 * E, bias, s.att, E, n, H);  // :352-439

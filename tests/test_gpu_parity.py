@@ -151,6 +151,26 @@ def test_fp16_at_the_measured_batch_sizes_against_reference(batch):
     nw.close()
 
 
+@pytest.mark.parametrize("precision", ["fp16", "bf16"])
+@pytest.mark.parametrize("batch", [1, 2, 8, 9, 31, 65])
+def test_bt4_class_layers_at_small_batches_against_reference(batch, precision):
+    """The batches a search sends, in line: K cut over clusters (below 64 positions), smolgen's LayerNorms inside the products
+    that follow them (up to 64 positions, the second one up to 8), tiles of 64 rows and less."""
+    net, pos, n, g = load_compact("cfg4_2layer_b1024")
+    idx = np.arange(batch)
+    nw = network.Network(net, "precision=%s,max_batch=%d,side_stream=0" % (precision, batch))
+    for rep in range(3):
+        out = nw.evaluate(pos["masks"][idx], pos["values"][idx])
+        assert nw.device_status() == 0
+        if precision == "fp16":
+            _assert_half_against_compact(out, g, pos, idx)
+        else:  # bf16 keeps 8 bits of mantissa where fp16 keeps 11
+            worst, _, _ = _compact_errors(out, g, pos, idx)
+            assert worst <= 8 * HALF_ATOL
+            assert np.abs(out["q"] - g["q"][idx]).max() <= 8 * HALF_ATOL
+    nw.close()
+
+
 @pytest.mark.parametrize("batch", [64, 1024])
 def test_fp32_at_the_measured_batch_sizes_against_reference(batch):
     net, pos, n, g = load_compact("cfg4_2layer_b1024")
