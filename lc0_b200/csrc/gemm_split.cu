@@ -15,8 +15,8 @@
 // A tile of at most 64 rows loads 64-row boxes of A; the upper half of the 128-row MMA then reads whatever follows in
 // shared memory and its results are never looked at.
 // Chains of dependent launches, before (one 128xBN tile per CTA of gemm_tc.cu's kernel, FMA kernel below 64 rows) and now:
-// 64x1024x1024 15 -> 5.9 us, 1x256x2048 135 -> 5.3 us, 1x8192x256 21 -> 4.5 us, 32x4096x256 24 -> 4.2 us; one position of the
-// BT4-class network 4.37 -> 0.97 ms, 24 positions 4.47 -> 2.09 ms.
+// 64x1024x1024 15 -> 5.9 us, 1x256x2048 135 -> 5.3 us, 1x8192x256 21 -> 4.5 us, 32x4096x256 24 -> 4.2 us; with everything in this file one
+// position of the BT4-class network 4.37 -> 0.82 ms, 24 positions 4.47 -> 1.73 ms.
 // With a LayerNorm in front (GemmParams::ln_gamma; 256-wide rows, smolgen's two inner LayerNorms) warps 0-7 load the 64 rows of
 // A themselves, normalise them in registers and write them to the operand tiles in the swizzle TMA would have used; gamma and
 // beta arrive by bulk copy ahead of the grid dependency.  A LayerNorm vector may span several rows of A (smolgen's
@@ -428,7 +428,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 }
 
 // Tile width, cluster size and stages of a product: the least of a cost model in microseconds, fitted to chains of dependent
-// launches (M x N x K; us measured at columns per tile / CTAs per tile):
+// launches (M x N x K; us measured at columns per tile / CTAs per tile, 5 - 20 % more than with today's elected issue):
 //   1536x1024x1024  32/1 19.5  64/1 11.2  64/2 17.6  128/1 13.9  128/2 12.5    2368x768x256   32/1 10.3  64/1 6.7  128/1 9.2
 //   512x1024x1024   32/1 10.0  32/2 7.9   64/1 11.3  64/4 9.1    128/1 13.6    2368x256x256   32/1 5.3   64/1 6.6  128/1 9.0
 //   512x1024x1536   32/2 9.5   64/2 10.9  64/4 9.8   128/2 12.7                64x1024x1024   32/4 5.9   64/1 9.8  64/4 6.3
