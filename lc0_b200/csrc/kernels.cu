@@ -87,9 +87,9 @@ expand_tokens_vec_kernel(const uint64_t* __restrict__ masks, const float* __rest
   }
   __syncthreads();
   T* o = out + (long long)n * 64 * cin;
-  const int vec_per_row = cin >> 3;
-  for (int idx = threadIdx.x; idx < 64 * vec_per_row; idx += blockDim.x) {
-    const int sq = idx / vec_per_row, c = (idx - sq * vec_per_row) << 3;
+  const int vec_per_row = cin >> 3, rows = 64 / gridDim.y, sq0 = blockIdx.y * rows;
+  for (int idx = threadIdx.x; idx < rows * vec_per_row; idx += blockDim.x) {
+    const int r0 = idx / vec_per_row, sq = sq0 + r0, c = (idx - r0 * vec_per_row) << 3;
     Vec8<T> r;
     if (c < 112) {
 #pragma unroll
@@ -116,7 +116,9 @@ cudaError_t launch_expand_tokens(const uint64_t* masks, const float* values, int
   if (n <= 0) return cudaSuccess;
   const bool aligned = (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (reinterpret_cast<uintptr_t>(pe_dense) & 15) == 0;
   if ((cin & 7) == 0 && (pe_ch & 7) == 0 && aligned)
-    expand_tokens_vec_kernel<T><<<n, 256, 0, s>>>(masks, values, pe_static, pe_dense, pe_ch, cin, out);
+    // Few positions: eight (four) CTAs to a position, 8 (16) squares each; one CTA took 16 us for one position's 80 KB.
+    expand_tokens_vec_kernel<T><<<dim3(n, n <= 148 ? 8 : n <= 592 ? 4 : 1), 256, 0, s>>>(masks, values, pe_static, pe_dense,
+                                                                                        pe_ch, cin, out);
   else
     expand_tokens_kernel<T><<<n, 256, 0, s>>>(masks, values, pe_static, pe_dense, pe_ch, cin, out);
   return cudaGetLastError();
@@ -338,6 +340,9 @@ cudaError_t launch_layer_norm(T* out, const T* x, const T* skip, const float* ga
 }
 
 // Input gating x * mult + add (reference: network_blas.cc:669-682; gates re-laid out [64][C] at load).
+// Memory-bound.  The vector form gates eight channels of one square in kGateBoards positions per thread, so that the gates
+// (fp32, [64][C]) are read once for all of them; the scalar form takes widths that are no multiple of eight.
+constexpr int kGateBoards = 4;
 template <typename T>
 __global__ void gate_kernel(T* __restrict__ x, const float* __restrict__ mult, const float* __restrict__ add,
                             long long total, int C) {
@@ -348,11 +353,42 @@ __global__ void gate_kernel(T* __restrict__ x, const float* __restrict__ mult, c
   const long long g = (row & 63) * C + c;
   x[idx] = from_f<T>(to_f(x[idx]) * mult[g] + add[g]);
 }
+template <typename T>
+__global__ void __launch_bounds__(256)
+gate_vec_kernel(T* __restrict__ x, const float* __restrict__ mult, const float* __restrict__ add, int boards, int C) {
+  const int piece = blockIdx.x * 256 + threadIdx.x;  // piece of eight channels of a board
+  if (piece >= 8 * C) return;
+  const long long board = 64LL * C;
+  float m[8], a[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    m[i] = __ldg(mult + piece * 8 + i);
+    a[i] = __ldg(add + piece * 8 + i);
+  }
+  grid_dependency_wait();
+  grid_launch_dependents();
+  T* p = x + (long long)piece * 8;
+  const int b0 = blockIdx.y * kGateBoards, b1 = b0 + kGateBoards < boards ? b0 + kGateBoards : boards;
+  Vec8<T> v[kGateBoards];
+#pragma unroll
+  for (int i = 0; i < kGateBoards; ++i)
+    if (b0 + i < b1) v[i] = *reinterpret_cast<const Vec8<T>*>(p + (b0 + i) * board);
+#pragma unroll
+  for (int i = 0; i < kGateBoards; ++i) {
+    if (b0 + i >= b1) break;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[i].v[j] = from_f<T>(to_f(v[i].v[j]) * m[j] + a[j]);
+    *reinterpret_cast<Vec8<T>*>(p + (b0 + i) * board) = v[i];
+  }
+}
 
 template <typename T>
 cudaError_t launch_gate(T* x, const float* gate_mult, const float* gate_add, int rows, int C, cudaStream_t s) {
   const long long total = (long long)rows * C;
   if (total <= 0) return cudaSuccess;
+  if ((C & 7) == 0 && (rows & 63) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0)
+    return launch_dependent(gate_vec_kernel<T>, dim3(ceil_div(8LL * C, 256), ceil_div(rows / 64, kGateBoards)), dim3(256), 0, s,
+                            x, gate_mult, gate_add, rows / 64, C);
   gate_kernel<T><<<ceil_div(total, 256), 256, 0, s>>>(x, gate_mult, gate_add, total, C);
   return cudaGetLastError();
 }
