@@ -1180,7 +1180,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (even CTA only) ----------------
-    if (rank == 0 && elect_one()) {
+    // Products of few k-blocks (four epilogue groups) keep the slower issue, a lane index and one commit per CTA: the 10 x 256
+    // attention network takes 1281 - 1290 us at 512 positions with it and 1316 us with the elected lane and the commit to both CTAs,
+    // presumably because MMAs that arrive in a burst hold up the epilogue warps that set the pace there.  With it, 256
+    // positions of the BT4-class network would take 5967 us instead of 5861, of the 20 x 256 residual network 1338 instead of 1252.
+    constexpr bool kFastIssue = kGroups != 4;
+    auto commit = [](uint32_t bar) {
+      if constexpr (kFastIssue) {
+        tcgen05_commit_both(bar);
+      } else {
+        tcgen05_commit_pair(mapa(bar, 0));
+        tcgen05_commit_pair(mapa(bar, 1));
+      }
+    };
+    bool issuer;
+    if constexpr (kFastIssue) issuer = rank == 0 && elect_one();
+    else issuer = rank == 0 && lane == 0;
+    if (issuer) {
       constexpr uint32_t idesc_base = (1u << 4) | (FmtCode<T>::v << 7) | (FmtCode<T>::v << 10) |
                                       ((uint32_t)((2 * BM) >> 4) << 24);
       int s = 0;         // stage and phase of the next k-block
@@ -1201,10 +1217,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
             tcgen05_mma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          tcgen05_commit_both(smem_u32(&empty_bar[s]));  // frees the stage in both CTAs once the MMAs have read it
+          commit(smem_u32(&empty_bar[s]));  // frees the stage in both CTAs once the MMAs have read it
           if (++s == S) { s = 0; ph ^= 1; }
         }
-        if (ok) tcgen05_commit_both(smem_u32(&tfull_bar[acc]));
+        if (ok) commit(smem_u32(&tfull_bar[acc]));
       }
     }
   } else if (warp == 2 || warp == 3) {
