@@ -28,9 +28,13 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
 // ---- programmatic dependent launch --------------------------------------------------------------------------
 // A kernel launched through launch_dependent() may be made resident, and run its prologue (barrier initialisation,
 // tensor-memory allocation, descriptor prefetch), while the kernel before it in the stream is still running.  Such a
-// kernel calls grid_dependency_wait() in every thread before its first access to global memory: the call returns
-// when the kernels before it have completed and their writes are visible.  grid_launch_dependents() lets the kernel
-// after it do the same in turn.  Both are no-ops in a kernel that was launched the ordinary way.
+// kernel calls grid_dependency_wait() in every thread that touches global memory, before it reads anything a kernel may
+// have written and before it writes at all: the call returns when the kernels before it have completed and their writes
+// are visible.  What may be read ahead of it are loaded weights alone: parameter vectors (bias, LayerNorm and gate
+// parameters, column sums) and, where GemmParams::w_const says so, the matrix W.  Every launch waits in some thread, so a kernel
+// is over only when those before it are.  grid_launch_dependents() lets the kernel after it be made resident; it promises
+// nothing about data and may come before this kernel's own wait.  Both are no-ops in a kernel that was launched the
+// ordinary way.
 #ifdef __CUDACC__
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -328,7 +328,7 @@ cudaError_t launch_gemm_fma(const GemmParams& g, cudaStream_t s) {
   p.M = g.M; p.N = g.N; p.K = g.K; p.act = g.act; p.out_f32 = g.out_f32;
   p.scale = g.scale; p.alpha = g.alpha;
   p.vec = aligned4<T>(g.A, g.lda, g.strideA) && aligned4<T>(g.W, g.ldw, g.strideW);
-  p.w_const = g.batch == 1;  // a product per position (the policy head's Q K^T) has an activation on both sides
+  p.w_const = g.w_const;
   return launch_fma<T, false>(p, g.batch, g.split_k, s);
 }
 

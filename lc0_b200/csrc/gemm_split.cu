@@ -170,6 +170,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // ---------------- TMA producer ----------------
     if (elect_one()) {
       const int early = kbn < S ? kbn : S;
+      if (!p.w_const) grid_dependency_wait();
       for (int i = 0; i < early; ++i) {
         const uint32_t fb = smem_u32(&full_bar[i]);
         mbar_expect_tx(fb, kLN ? BN * 128 : stage_bytes);

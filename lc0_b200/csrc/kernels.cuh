@@ -14,6 +14,9 @@ struct GemmParams {
   const float* bias = nullptr;
   void* C = nullptr; long long ldc = 0, strideC = 0;
   const void* skip = nullptr; long long ldskip = 0;
+  // W is a loaded weight: nothing in flight writes it, so a kernel may request it ahead of grid_dependency_wait().  Off
+  // for an activation on W's side (the policy head's Q K^T, whose keys the launch just before may still be writing).
+  bool w_const = false;
   int M = 0, N = 0, K = 0, batch = 1;
   int act = ACT_NONE;
   float scale = 1.0f, alpha = 1.0f;

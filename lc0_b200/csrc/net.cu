@@ -1127,7 +1127,7 @@ struct Net : NetBase {
             const T* skip = nullptr, long long ldskip = 0, float alpha_ = 1.f, bool out_f32 = false,
             void* cf32 = nullptr) {
     GemmParams p;
-    p.A = A; p.lda = lda; p.W = d.w; p.ldw = d.in; p.bias = d.b;
+    p.A = A; p.lda = lda; p.W = d.w; p.ldw = d.in; p.w_const = true; p.bias = d.b;
     p.C = out_f32 ? cf32 : (void*)Cout; p.ldc = ldc; p.M = M; p.N = d.out; p.K = d.in; p.act = act;
     p.skip = skip; p.ldskip = ldskip; p.alpha = alpha_; p.out_f32 = out_f32;
     p.whole_tiles = (opt.flags & B200_FLAG_NO_SPLIT_LAST_WAVE) != 0;
@@ -1149,7 +1149,7 @@ struct Net : NetBase {
                T* C2 = nullptr, long long ldc2 = 0, int n_split = 0, bool zero_stats = true) {
     GemmParams p;
     p.C2 = C2; p.ldc2 = ldc2; p.n_split = n_split;
-    p.A = in.u; p.lda = lda; p.W = d.w; p.ldw = d.in; p.bias = d.b;
+    p.A = in.u; p.lda = lda; p.W = d.w; p.ldw = d.in; p.w_const = true; p.bias = d.b;
     p.C = Cout; p.ldc = ldc; p.M = M; p.N = d.out; p.K = d.in; p.act = act;
     if (in.stats) {
       if (!d.colsum) throw Fail{B200_ERR_INVALID, "internal: folded input for a layer without folded weights"};
@@ -1176,7 +1176,7 @@ struct Net : NetBase {
                     long long ldc, int M, int act) {
     if constexpr (sizeof(T) == 2) {
       GemmParams p;
-      p.A = x; p.lda = d.in; p.W = d.w; p.ldw = d.in; p.bias = d.b; p.C = y; p.ldc = ldc;
+      p.A = x; p.lda = d.in; p.W = d.w; p.ldw = d.in; p.w_const = true; p.bias = d.b; p.C = y; p.ldc = ldc;
       p.M = M; p.N = d.out; p.K = d.in; p.act = act;
       p.ln_gamma = gamma; p.ln_beta = beta; p.ln_group = group; p.ln_eps = 1e-3f;
       if (!use_tc || M > (group > 1 ? kLnInProductRows : 64) || !gemm_ln_supported(p)) return false;

@@ -292,6 +292,7 @@ struct TcParams {
   const float* se_w1; const float* se_b1; const float* se_w2; const float* se_b2; const float* se_bias; int se_k;
   void* C2; long long ldc2;  // second output of gemm_split.cu (the pair kernel has a tensor map for it)
   int vec_c;                 // gemm_split.cu: C (and C2) may be written in 16-byte pieces
+  int w_const;               // gemm_split.cu: W may be requested ahead of the grid dependency
   int batch_rows;  // > 0: stacked products, rows [b * batch_rows, (b + 1) * batch_rows) use W rows [b * N, (b + 1) * N)
 };
 
@@ -332,6 +333,7 @@ inline void fill_tc_params(TcParams& p, const GemmParams& g, int* status) {
   p.se_w1 = g.se_w1; p.se_b1 = g.se_b1; p.se_w2 = g.se_w2; p.se_b2 = g.se_b2; p.se_bias = g.se_bias;
   p.se_k = g.se_k;
   p.batch_rows = g.batch_rows;
+  p.w_const = g.w_const ? 1 : 0;
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   const int per16 = g.out_f32 ? 4 : 8;
   p.vec_c = al16(g.C) && (g.ldc % per16) == 0 && (g.n_split == 0 || (al16(g.C2) && (g.ldc2 % per16) == 0));

@@ -529,6 +529,34 @@ def test_dependent_launches_match_ordinary_launches(name, batch):
     assert np.abs(outs[0]["m"] - outs[1]["m"]).max() <= 1e-3 * max(1.0, np.abs(outs[1]["m"]).max())
 
 
+@pytest.mark.parametrize("precision", ["fp16", "bf16"])
+@pytest.mark.parametrize("graphs", [0, 1])
+@pytest.mark.parametrize("dm", [100, 101])
+def test_single_positions_with_a_policy_width_off_the_tensor_cores(dm, graphs, precision):
+    """A policy d_model that is no multiple of 8 takes the FMA kernel for Q K^T, whose keys the launch just before writes:
+    they may not be requested ahead of it, and at one position nothing but the caller can tell them from a weight.
+    Different positions in consecutive calls, dependent launches against ordinary ones and against the oracle."""
+    from lc0_b200 import netproto
+    net = netproto.parse_net(netproto.encode("Net", mknet.make_net("cfg4_mini", pol_dmodel=dm)))
+    _, pos, n, g = load_case("cfg4_mini")
+    want = oracle.forward(*weights.flatten(net), pos["masks"][:6], pos["values"][:6])
+    rt = 2.0 ** -10 if precision == "fp16" else 2.0 ** -7  # of activations that pass through some ten roundings
+    outs = []
+    for dep in (1, 0):
+        nw = network.Network(net, "precision=%s,max_batch=1,slots=1,graph_capture=%d,dependent_launch=%d" % (precision, graphs, dep))
+        out = []
+        for rep in range(4):
+            for i in range(6):
+                out.append(nw.evaluate(pos["masks"][i:i + 1], pos["values"][i:i + 1])["policy"][0])
+        assert nw.device_status() == 0
+        nw.close()
+        outs.append(np.array(out))
+    # row statistics are summed by atomics: the two schedules may differ by a rounding of the storage type here and there
+    assert np.abs(outs[0] - outs[1]).max() <= rt * max(1.0, np.abs(outs[1]).max())
+    ref = np.tile(want["policy"], (4, 1))
+    assert np.abs(outs[0] - ref).max() <= 16 * rt * max(1.0, np.abs(ref).max())
+
+
 def test_split_last_wave_matches_whole_tiles():
     """Products whose last wave of 256x256 tiles fills at most half of the CTA pairs compute that wave as half-width
     tiles (out-projection and FFN2 here, both with residual input and row statistics): same results as whole tiles."""
