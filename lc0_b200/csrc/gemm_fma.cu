@@ -8,8 +8,11 @@
 // so that eight rows of a quarter warp fall on different banks.  A thread owns TM x TN outputs whose rows are 8 and whose
 // columns 4 apart and reads TM + TN 16-byte pieces per four k for 4 TM TN FMAs.  Two groups of warps take alternate pieces of k, so
 // that a tile that has an SM to itself still has two warps per scheduler; their sums are added at the end.
-// With GemmParams::split_k the K range of a tile that leaves SMs idle is cut over a cluster of up to eight CTAs, whose sums
-// meet through distributed shared memory in a fixed order.
+// A sum does not depend on the number of rows: the K range is summed in pieces whose number follows from N and K alone
+// (k_pieces), a piece group by group, and the pieces' sums are added one after the other.  A tile that leaves SMs idle has a CTA
+// of a cluster for every piece or pair of pieces, whose sums meet through distributed shared memory; otherwise one CTA takes
+// the pieces in turn and keeps the total in shared memory, which costs 2 - 5 % of a product against one running sum (4096x3072x1024
+// 676 -> 692 us, 1024x1024x1024 69.5 -> 71.8; with totals in registers beside the running sums 740 and 76).
 #include <atomic>
 
 #include "kernels.cuh"
@@ -25,7 +28,8 @@ struct FmaParams {
   const float* bias;
   void* C; long long ldc, strideC;
   const void* skip; long long ldskip;
-  int M, N, K, act, out_f32, ks, w_const;
+  int M, N, K, act, out_f32, w_const;
+  int pieces, ks;  // pieces of the K range that are summed one by one; CTAs per tile: pieces, pieces / 2 or 1
   float scale, alpha;
   int vec;       // rows start on 16-byte (16-bit storage: 8-byte) boundaries: operands move as pieces of four elements
   int conv_cin;  // convolution: A is [M][cin] on 8x8 boards, W is [9][N][cin]
@@ -70,7 +74,7 @@ __device__ __forceinline__ void stage4(float* dst, const T* src, int left, bool 
   *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
-template <typename T, bool kFast, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv>
+template <typename T, bool kFast, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv, bool kTotals>
 __global__ void __launch_bounds__(kGroups * (BM / TM) * (BN / TN), kMinCtas)
 gemm_fma_kernel(const FmaParams p) {
   constexpr int kGroupThreads = (BM / TM) * (BN / TN), kThreads = kGroups * kGroupThreads;
@@ -78,14 +82,16 @@ gemm_fma_kernel(const FmaParams p) {
   constexpr int kLd = kBK + 4, kLdOut = BN + 4, kPieces = kBK / 4;
   constexpr int kRowStep = kThreads / kPieces;     // rows staged at a time
   static_assert(BM % kWarpM == 0 && BN % kWarpN == 0, "whole warps");
-  extern __shared__ __align__(16) float sm[];      // [stages][BM + BN][kLd]; afterwards [BM][kLdOut] sums
+  extern __shared__ __align__(16) float sm[];      // [stages][BM + BN][kLd]; afterwards [1 or 2][BM][kLdOut] sums
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = (int)blockIdx.x % p.ks;
   const int n0 = (int)blockIdx.x / p.ks * BN, m0 = blockIdx.y * BM;
   const T* A = reinterpret_cast<const T*>(p.A) + (long long)blockIdx.z * p.strideA;
   const T* W = reinterpret_cast<const T*>(p.W) + (long long)blockIdx.z * p.strideW;
   const int k_blocks = (p.K + kBK - 1) / kBK;
-  const int kb0 = (int)((long long)k_blocks * rank / p.ks), kbn = (int)((long long)k_blocks * (rank + 1) / p.ks) - kb0;
+  auto piece_start = [&](int j) { return (int)((long long)k_blocks * j / p.pieces); };
+  const int first = kTotals ? rank * (p.pieces / p.ks) : rank, own_pieces = kTotals ? p.pieces / p.ks : 1;  // of this CTA
+  const int kb0 = piece_start(first), kbn = piece_start(first + own_pieces) - kb0;
 
   // This thread stages the four k from lk on of rows lr, lr + kRowStep, ... of both tiles.
   constexpr int kRowsA = (BM + kRowStep - 1) / kRowStep, kRowsW = (BN + kRowStep - 1) / kRowStep;
@@ -166,40 +172,72 @@ gemm_fma_kernel(const FmaParams p) {
   const int group = tid / kGroupThreads, gw = warp - group * (kGroupThreads / 32);
   const int wm = gw / kWarpsN * kWarpM + (lane & 7), wn = gw % kWarpsN * kWarpN + (lane >> 3);
   float acc[TM][TN];
+  auto clear = [&] {
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-
+      for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+  };
+  clear();
+  static_assert(kGroups == 2 && TN == 4, "held_at: one float4 per row of a thread");
+  // kTotals: [TM][threads], of the rows that a thread's group owns the total so far, of the others the last piece
+  auto held_at = [&](int t) { return reinterpret_cast<float4*>(sm + kStages * (BM + BN) * kLd) + t; };
+  int i = 0;
+  for (int piece = 1;; ++piece) {
+    const int end = kTotals ? piece_start(first + piece) - kb0 : kbn;
 #pragma unroll 1
-  for (int i = 0; i < kbn; ++i) {
-    cp_async_wait<kStages - 2>();
-    __syncthreads();  // stage i has landed; every thread is done with the stage that is filled next
-    stage_w(i + kStages - 1);
-    stage_a(i + kStages - 1);
-    cp_async_commit();
-    const float* as = sm + (i % kStages) * (BM + BN) * kLd + wm * kLd;
-    const float* ws = sm + (i % kStages) * (BM + BN) * kLd + BM * kLd + wn * kLd;
+    for (; i < end; ++i) {
+      cp_async_wait<kStages - 2>();
+      __syncthreads();  // stage i has landed; every thread is done with the stage that is filled next
+      stage_w(i + kStages - 1);
+      stage_a(i + kStages - 1);
+      cp_async_commit();
+      const float* as = sm + (i % kStages) * (BM + BN) * kLd + wm * kLd;
+      const float* ws = sm + (i % kStages) * (BM + BN) * kLd + BM * kLd + wn * kLd;
 #pragma unroll
-    for (int kk = 0; kk < kBK; kk += 4 * kGroups) {
-      const int k = kk + group * 4;
-      float4 a[TM];
+      for (int kk = 0; kk < kBK; kk += 4 * kGroups) {
+        const int k = kk + group * 4;
+        float4 a[TM];
 #pragma unroll
-      for (int r = 0; r < TM; ++r) a[r] = *reinterpret_cast<const float4*>(as + r * 8 * kLd + k);
+        for (int r = 0; r < TM; ++r) a[r] = *reinterpret_cast<const float4*>(as + r * 8 * kLd + k);
 #pragma unroll
-      for (int c0 = 0; c0 < TN; c0 += 4) {
-        float4 w[4];
+        for (int c0 = 0; c0 < TN; c0 += 4) {
+          float4 w[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) w[c] = *reinterpret_cast<const float4*>(ws + (c0 + c) * 4 * kLd + k);
+          for (int c = 0; c < 4; ++c) w[c] = *reinterpret_cast<const float4*>(ws + (c0 + c) * 4 * kLd + k);
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+          for (int e = 0; e < 4; ++e)
 #pragma unroll
-          for (int r = 0; r < TM; ++r)
+            for (int r = 0; r < TM; ++r)
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-              acc[r][c0 + c] = fmaf(reinterpret_cast<const float*>(&a[r])[e], reinterpret_cast<const float*>(&w[c])[e], acc[r][c0 + c]);
+              for (int c = 0; c < 4; ++c)
+                acc[r][c0 + c] = fmaf(reinterpret_cast<const float*>(&a[r])[e], reinterpret_cast<const float*>(&w[c])[e], acc[r][c0 + c]);
+        }
       }
     }
+    if (end == kbn) break;
+    // The piece is complete: a row's sums of both groups are added to the total in the group that owns the row.  The
+    // thread's index is read again here: kept through the main loop it cost 1.5 %.
+    uint32_t t0;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t0));
+    const int grp = t0 / kGroupThreads, partner = grp == 0 ? kGroupThreads : -kGroupThreads;
+    float4* held = held_at(t0);
+#pragma unroll
+    for (int r = 0; r < TM; ++r)
+      if (r % 2 != grp) held[r * kThreads] = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < TM; ++r) {
+      if (r % 2 != grp) continue;
+      const float4 o = held[r * kThreads + partner];
+      float4 t = make_float4(acc[r][0] + o.x, acc[r][1] + o.y, acc[r][2] + o.z, acc[r][3] + o.w);
+      if (piece > 1) {
+        const float4 b = held[r * kThreads];
+        t = make_float4(b.x + t.x, b.y + t.y, b.z + t.z, b.w + t.w);
+      }
+      held[r * kThreads] = t;
+    }
+    clear();
   }
 
   const T* skip = reinterpret_cast<const T*>(p.skip);
@@ -221,12 +259,21 @@ gemm_fma_kernel(const FmaParams p) {
   for (int g = kGroups - 1; g >= 0; --g) {
     if (group == g) {
 #pragma unroll
-      for (int r = 0; r < TM; ++r)
+      for (int r = 0; r < TM; ++r) {
+        float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (kTotals && g == 0) total = held_at(tid)[r * kThreads + (r % 2 == 0 ? 0 : kGroupThreads)];
 #pragma unroll
         for (int c = 0; c < TN; ++c) {
           float* o = sm + (wm + r * 8) * kLdOut + wn + c * 4;
-          *o = g == kGroups - 1 ? acc[r][c] : acc[r][c] + *o;
+          float v = g == kGroups - 1 ? acc[r][c] : acc[r][c] + *o;
+          if (kTotals && g == 0) {
+            const float t = reinterpret_cast<const float*>(&total)[c];
+            if (p.ks == 1) v = t + v;
+            else o[BM * kLdOut] = t;  // two pieces of a cut range stay apart: the total is the first one
+          }
+          *o = v;
         }
+      }
     }
     if (g > 0) __syncthreads();
   }
@@ -238,9 +285,14 @@ gemm_fma_kernel(const FmaParams p) {
   cluster_sync();
   const int slice = BM * BN / p.ks;  // a power of two and at least 64
   for (int e = rank * slice + tid * 4; e < (rank + 1) * slice; e += kThreads * 4) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(sm + e / BN * kLdOut + e % BN);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int j = 0; j < p.ks; ++j) {
-      const float4 u = ld_cluster_v4((uint32_t)__cvta_generic_to_shared(sm + e / BN * kLdOut + e % BN), j);
+      if (kTotals) {
+        const float4 u = ld_cluster_v4(at + BM * kLdOut * 4, j);
+        v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+      }
+      const float4 u = ld_cluster_v4(at, j);
       v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
     }
     const int m = m0 + e / BN, n = n0 + e % BN;
@@ -252,10 +304,12 @@ gemm_fma_kernel(const FmaParams p) {
   cluster_sync();  // the others may still be reading this CTA's sums
 }
 
-template <typename T, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv>
-cudaError_t launch_tile(const FmaParams& p, int batch, cudaStream_t s) {
-  constexpr int ring = kStages * (BM + BN) * (kBK + 4) * 4, out = BM * (BN + 4) * 4, smem = ring > out ? ring : out;
-  auto kernel = gemm_fma_kernel<T, (sizeof(T) == 2), BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv>;
+template <typename T, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv, bool kTotals>
+cudaError_t launch_kernel(const FmaParams& p, int batch, cudaStream_t s) {
+  constexpr int ring = kStages * (BM + BN) * (kBK + 4) * 4, out = BM * (BN + 4) * 4;
+  static_assert(ring >= 2 * out, "the sums take the place of the ring");
+  constexpr int smem = ring + (kTotals ? kGroups * BM * BN * 4 : 0);
+  auto kernel = gemm_fma_kernel<T, (sizeof(T) == 2), BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv, kTotals>;
   static std::atomic<unsigned long long> attr_mask{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -288,25 +342,42 @@ cudaError_t launch_tile(const FmaParams& p, int batch, cudaStream_t s) {
   return cudaLaunchKernelEx(&lc, kernel, p);
 }
 
-// CTAs per tile: cuts of the K range, down to four k-blocks of 32 each, while they find SMs with little to do.  Measured (us at
-// 1 / 2 / 4 / 8 cuts): 64x64 tiles 256x1024x1024 38 / 23 / 21 / 26, 256x3072x1024 67 / 57 / 60 / 73, 1024x1024x1024 67 / 73 /
+template <typename T, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv>
+cudaError_t launch_tile(const FmaParams& p, int batch, cudaStream_t s) {
+  if (p.ks == p.pieces) return launch_kernel<T, BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv, false>(p, batch, s);
+  return launch_kernel<T, BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv, true>(p, batch, s);
+}
+
+// Pieces of the K range: from N and K alone, so that every number of rows has the same sums.  As many as give the column tiles of
+// one row block work for 64 CTAs (128 when there are 64 k-blocks of 32 and more), of four k-blocks at least.
+int k_pieces(int N, int K) {
+  const int k_blocks = ceil_div(K, 32), n_tiles = ceil_div(N, 64), want = k_blocks >= 64 ? 128 : 64;
+  int pieces = 1;
+  while (pieces < 8 && pieces * n_tiles < want && k_blocks >= pieces * 8) pieces *= 2;
+  return pieces;
+}
+
+// CTAs per tile: one for each piece or for each pair of pieces, while that finds SMs with little to do.  Measured in us at 1 / 2 / 4 /
+// 8 CTAs per tile (fp32): 64x64 tiles 256x1024x1024 38 / 23 / 21 / 26, 256x3072x1024 67 / 57 / 60 / 73, 1024x1024x1024 67 / 73 /
 // 76 / 94, 64x1024x1024 37 / 22 / 13 / 13, 64x3072x1024 37 / 23 / 21 / 24; 32x64 tiles 16x256x2048 45 / 25 / 15 / 10,
-// 16x8192x256 8 / 9 / 13.
-int cuts(const FmaParams& p, int bm, int bn, int batch, bool split, int ctas) {
-  const long long tiles = (long long)ceil_div(p.N, bn) * ceil_div(p.M, bm) * batch;
-  const int k_blocks = ceil_div(p.K, 32);
-  int ks = 1;
-  while (split && ks < 8 && tiles * ks * 2 <= (ks == 4 ? 148 : ctas) && k_blocks / (ks * 2) >= 4) ks *= 2;
-  return ks;
+// 16x8192x256 8 / 9 / 13.  Uncut, 149 - 200 tiles take two rounds of SMs: 200 tiles of a 3x3 convolution of 128 channels at four CTAs
+// each, ten of them 1.89 instead of 2.17 ms.
+int cuts(const FmaParams& p, int bm, int batch) {
+  const long long tiles = (long long)ceil_div(p.N, 64) * ceil_div(p.M, bm) * batch;
+  auto fits = [&](int ks) { return tiles * ks <= (bm < 64 || ks == 8 ? 148 : 400); };
+  if (fits(p.pieces)) return p.pieces;
+  return p.pieces >= 4 && (fits(p.pieces / 2) || (bm == 64 && tiles > 148 && tiles <= 200)) ? p.pieces / 2 : 1;
 }
 
 template <typename T, bool kConv>
-cudaError_t launch_fma(FmaParams p, int batch, bool split, cudaStream_t s) {
-  if constexpr (!kConv) {  // a convolution has whole boards of 64 rows
-    if (p.M <= 8) { p.ks = cuts(p, 8, 64, batch, split, 148); return launch_tile<T, 8, 64, 1, 4, 32, 2, 2, false>(p, batch, s); }
-    if (p.M <= 32) { p.ks = cuts(p, 32, 64, batch, split, 148); return launch_tile<T, 32, 64, 4, 4, 32, 2, 2, false>(p, batch, s); }
+cudaError_t launch_fma(FmaParams p, int batch, cudaStream_t s) {
+  p.pieces = k_pieces(p.N, p.K);
+  const int bm = kConv || p.M > 32 ? 64 : p.M > 8 ? 32 : 8;  // a convolution has whole boards of 64 rows
+  p.ks = cuts(p, bm, batch);
+  if constexpr (!kConv) {
+    if (bm == 8) return launch_tile<T, 8, 64, 1, 4, 32, 2, 2, false>(p, batch, s);
+    if (bm == 32) return launch_tile<T, 32, 64, 4, 4, 32, 2, 2, false>(p, batch, s);
   }
-  p.ks = cuts(p, 64, 64, batch, split, 400);
   return launch_tile<T, 64, 64, 8, 4, 32, 2, 2, kConv>(p, batch, s);
 }
 
@@ -329,24 +400,24 @@ cudaError_t launch_gemm_fma(const GemmParams& g, cudaStream_t s) {
   p.scale = g.scale; p.alpha = g.alpha;
   p.vec = aligned4<T>(g.A, g.lda, g.strideA) && aligned4<T>(g.W, g.ldw, g.strideW);
   p.w_const = g.w_const;
-  return launch_fma<T, false>(p, g.batch, g.split_k, s);
+  return launch_fma<T, false>(p, g.batch, s);
 }
 
 template <typename T>
 cudaError_t launch_conv3x3(const T* x, int cin, const T* w, const float* bias, T* y, int cout, int n, int act,
-                           bool split, cudaStream_t s) {
+                           cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   FmaParams p = {};
   p.A = x; p.lda = cin; p.W = w; p.ldw = cin; p.bias = bias; p.C = y; p.ldc = cout;
   p.M = n * 64; p.N = cout; p.act = act; p.conv_cin = cin; p.conv_kt = ceil_div(cin, 4) * 4; p.K = 9 * p.conv_kt;
   p.scale = 1.f; p.alpha = 1.f; p.w_const = 1;
   p.vec = aligned4<T>(x, cin, 0) && aligned4<T>(w, cin, 0);
-  return launch_fma<T, true>(p, 1, split, s);
+  return launch_fma<T, true>(p, 1, s);
 }
 
 #define INSTANTIATE(T)                                                          \
   template cudaError_t launch_gemm_fma<T>(const GemmParams&, cudaStream_t);     \
-  template cudaError_t launch_conv3x3<T>(const T*, int, const T*, const float*, T*, int, int, int, bool, cudaStream_t);
+  template cudaError_t launch_conv3x3<T>(const T*, int, const T*, const float*, T*, int, int, int, cudaStream_t);
 INSTANTIATE(float)
 INSTANTIATE(__half)
 INSTANTIATE(__nv_bfloat16)

@@ -63,8 +63,8 @@ struct GemmParams {
   // CTA-pair kernel: compute a sparsely filled last wave as whole 256x256 tiles instead of half-width ones
   // (verification switch; the split is on by default).
   bool whole_tiles = false;
-  // Products of few rows: the K range may be cut over several CTAs (gemm_split.cu).  The sums then depend on the number of
-  // rows; off, a row's result is the same whatever else is in the batch.
+  // Products of few rows on tensor cores: the K range may be cut over several CTAs (gemm_split.cu).  The sums then depend on
+  // the number of rows; off, a row's result is the same whatever else is in the batch.
   bool split_k = true;
   // LayerNorm of A inside the product (launch_gemm_ln): every ln_group consecutive rows of A, which are 256 wide and packed,
   // are one LayerNorm vector with ln_gamma / ln_beta [ln_group * 256].
@@ -74,7 +74,8 @@ struct GemmParams {
   float ln_eps = 0.f;
 };
 
-// FMA kernel (gemm_fma.cu): any shape and alignment, batched products; no folded LayerNorm, residual or statistics.
+// FMA kernel (gemm_fma.cu): any shape and alignment, batched products; no folded LayerNorm, residual or statistics.  A row's
+// result is the same whatever the number of rows.
 template <typename T> cudaError_t launch_gemm_fma(const GemmParams& p, cudaStream_t s);
 // tcgen05 / TMEM / TMA kernel (gemm_tc.cu); T is __half or __nv_bfloat16, batch must be 1.
 // `status` is a device int the kernel sets non-zero when a bounded wait gives up.
@@ -169,10 +170,10 @@ cudaError_t launch_head_final(const T* h, int k, const float* w, const float* b,
                               float* qdm, cudaStream_t s);
 
 // ---- residual tower (NHWC activations [n*64][C]) ----
-// 3x3 same-padded convolution as an implicit GEMM (gemm_fma.cu); w: [9][Cout][Cin] (tap-major), split as GemmParams::split_k.
+// 3x3 same-padded convolution as an implicit GEMM (gemm_fma.cu); w: [9][Cout][Cin] (tap-major).
 template <typename T>
 cudaError_t launch_conv3x3(const T* x, int cin, const T* w, const float* bias, T* y, int cout, int n,
-                           int act, bool split, cudaStream_t s);
+                           int act, cudaStream_t s);
 // Squeeze-excitation + skip + activation (se_unit.cc:31-91) on NHWC: y = act(sig(z0)*x + skip + z1 + sig(z0)*b).
 template <typename T>
 cudaError_t launch_se(const T* x, const float* conv_bias, const T* skip, const float* w1, const float* b1,

@@ -1308,7 +1308,7 @@ struct Net : NetBase {
     }
     launches++;
     const int sp_ = span_begin(st, K_GEMM_FMA, 2.0 * n * 64 * (double)c.cout * 9 * c.cin);
-    CK(launch_conv3x3<T>(x, c.cin, c.w, bias, y, c.cout, n, act, t_split_k, st));
+    CK(launch_conv3x3<T>(x, c.cin, c.w, bias, y, c.cout, n, act, st));
     span_end(st, sp_);
   }
   // Second convolution of a residual block with its squeeze-excitation unit, the skip connection and the activation
@@ -1637,7 +1637,7 @@ struct Net : NetBase {
         p.A = s.pq; p.lda = pol_dm; p.strideA = 64LL * pol_dm;
         p.W = s.pk; p.ldw = pol_dm; p.strideW = 64LL * pol_dm;
         p.C = s.logits; p.ldc = 64; p.strideC = 4096; p.out_f32 = true;
-        p.M = 64; p.N = 64; p.K = pol_dm; p.batch = n; p.scale = 1.0f / sqrtf((float)pol_dm); p.split_k = t_split_k;
+        p.M = 64; p.N = 64; p.K = pol_dm; p.batch = n; p.scale = 1.0f / sqrtf((float)pol_dm);
         run_gemm(st, p);
         other(st, (double)n * (4096 + 1858) * 4, [&] {
           return launch_policy_attn_gather<T>(s.logits, s.pk, pol_w4, pol_dm, d_attn_src, n, d_policy, st);

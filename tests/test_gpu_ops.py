@@ -89,6 +89,26 @@ def test_fma_gemm_tiles(lib, prec, M, N, K):
     assert torch.all((C.double() - ref).abs() <= bound), (C.double() - ref).abs().max().item()
 
 
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("N,K", [(64, 100), (128, 255), (128, 256), (130, 511), (130, 512), (1024, 1024), (32, 1024), (256, 2047),
+                                 (256, 2048), (64, 1022)])
+def test_fma_gemm_rows_do_not_depend_on_their_number(lib, prec, N, K):
+    """One summation order per (N, K): K in one, two, four or eight pieces, each by a CTA of its own (few tiles) or one after the
+    other (many), tiles of 8, 32 and 64 rows."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    rows = 64 * 210 + 5
+    A = torch.randn(rows, K, device="cuda", generator=g).to(DT[prec])
+    W = torch.randn(N, K, device="cuda", generator=g).to(DT[prec])
+    outs = []
+    for M in (rows, 1, 5, 8, 9, 32, 33, 64, 65, 200, 3000):
+        C = torch.zeros(M, N, dtype=DT[prec], device="cuda")
+        _lib.check(lib.b200_op_gemm(A.data_ptr(), W.data_ptr(), None, C.data_ptr(), M, N, K, oracle.ACT_NONE, prec, 0, None))
+        torch.cuda.synchronize()
+        outs.append(C)
+    for C in outs[1:]:
+        assert torch.equal(C, outs[0][:C.shape[0]]), C.shape
+
+
 def test_gemm_tc_rejects_fp32(lib):
     assert lib.b200_op_gemm(None, None, None, None, 128, 128, 64, 3, 0, 1, None) == _lib.ERR_UNSUPPORTED
 

@@ -171,6 +171,21 @@ def test_bt4_class_layers_at_small_batches_against_reference(batch, precision):
     nw.close()
 
 
+@pytest.mark.parametrize("name", ["cfg4_2layer", "cfg1", "cfg2_mini", "cfg3_mini_polenc"])
+def test_fp32_results_do_not_depend_on_the_batch(name):
+    """The verification mode has one summation order at every batch size: a position alone and among others, bit for bit."""
+    net = mknet.make_net(name)
+    _, pos, n, g = load_compact("cfg4_2layer_b1024")
+    masks, values = np.array(pos["masks"][:300]), np.array(pos["values"][:300])
+    nw = network.Network(net, "precision=fp32,max_batch=300")
+    whole = nw.evaluate(masks, values)
+    for batch in (1, 5, 9, 40, 64, 100):
+        out = nw.evaluate(masks[:batch], values[:batch])
+        for k in ("policy", "q", "d", "m"):
+            np.testing.assert_array_equal(out[k], whole[k][:batch])
+    nw.close()
+
+
 @pytest.mark.parametrize("batch", [64, 1024])
 def test_fp32_at_the_measured_batch_sizes_against_reference(batch):
     net, pos, n, g = load_compact("cfg4_2layer_b1024")
