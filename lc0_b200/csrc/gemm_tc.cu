@@ -1421,12 +1421,9 @@ cudaError_t launch_bn(const GemmParams& g, int* status, int sm_count, cudaStream
     e = get_map(g.C, g.ldc, g.M, g.N, BM, prec, &mc);
     if (e != cudaSuccess) return e;
   }
-  const bool folded = g.a_stats || g.res || g.out_stats || g.se_k > 0;
-  if (folded && !tma_store) return cudaErrorInvalidValue;  // the folded-LayerNorm modes live in the TMA-store epilogue
   if (g.se_k > 0 && (BN != 256 || !gemm_tc_se_supported(g))) return cudaErrorInvalidValue;
   CUtensorMap mr = mc;
   if (g.res) {
-    if ((g.ldres % 8) != 0 || (reinterpret_cast<uintptr_t>(g.res) & 15) != 0) return cudaErrorInvalidValue;
     e = get_map(g.res, g.ldres, g.M, g.N, BM, prec, &mr);
     if (e != cudaSuccess) return e;
   }
@@ -1466,7 +1463,6 @@ cudaError_t launch_pair(const GemmParams& g, int* status, int sm_count, cudaStre
   if (e != cudaSuccess) return e;
   CUtensorMap mr = mc, mc2 = mc;
   if (g.res) {
-    if ((g.ldres % 8) != 0 || (reinterpret_cast<uintptr_t>(g.res) & 15) != 0) return cudaErrorInvalidValue;
     e = get_map(g.res, g.ldres, g.M, g.N, BM, prec, &mr);
     if (e != cudaSuccess) return e;
   }
@@ -1573,7 +1569,7 @@ bool pair_eligible(const GemmParams& p, int sm_count) {
 
 bool gemm_tc_split_supported(const GemmParams& p) {
   if (!gemm_tc_supported(p) || p.n_split <= 0 || p.N <= p.n_split || !p.C2 || (p.ldc2 % 8) != 0 ||
-      (reinterpret_cast<uintptr_t>(p.C2) & 15) != 0 || p.res || p.out_stats || p.skip || p.conv_cin > 0)
+      (reinterpret_cast<uintptr_t>(p.C2) & 15) != 0 || p.res || p.out_stats || p.skip || p.conv_cin > 0 || !epilogue_supported(p))
     return false;
   // what the CTA-pair kernel needs (it switches outputs between tiles); the split-K kernel takes any multiple of eight
   return (p.n_split % 256) == 0 && p.N - p.n_split <= 256 && p.batch_rows == 0 && !p.out_f32;
@@ -1658,6 +1654,7 @@ cudaError_t launch_gemm_tc(const GemmParams& p, int* status, int sm_count, cudaS
   if (p.M <= 0 || p.N <= 0) return cudaSuccess;
   if (!gemm_tc_supported(p) || p.skip) return cudaErrorInvalidValue;  // residuals go through `res`
   if (p.n_split > 0 && !gemm_tc_split_supported(p)) return cudaErrorInvalidValue;
+  if (!epilogue_supported(p)) return cudaErrorInvalidValue;
   if (pair_eligible(p, sm_count))
   {
     // Four epilogue groups when a tile has few k-blocks (the epilogue then sets the pace), two otherwise (fewer

@@ -339,6 +339,16 @@ inline void fill_tc_params(TcParams& p, const GemmParams& g, int* status) {
   p.vec_c = al16(g.C) && (g.ldc % per16) == 0 && (g.n_split == 0 || (al16(g.C2) && (g.ldc2 % per16) == 0));
 }
 
+// Whether the epilogues can take the operands of `g`: statistics, a residual and a second output come with 16-bit rows that TMA
+// can write, and the residual with rows that TMA, or a 16-byte load, can read.  The same for every kernel, so that a form is
+// taken or refused whatever the number of rows.
+inline bool epilogue_supported(const GemmParams& g) {
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  const bool folded = g.a_stats || g.res || g.out_stats || g.se_k > 0 || g.n_split > 0;
+  if (folded && (g.out_f32 || (g.ldc % 8) != 0 || !al16(g.C))) return false;
+  return !g.res || ((g.ldres % 8) == 0 && al16(g.res));
+}
+
 }  // namespace
 
 // Tensor map over a row-major 16-bit matrix, box = 64 columns x box_rows, 128-byte swizzle; cached by its arguments.

@@ -416,6 +416,28 @@ def test_products_of_few_rows(lib, prec, M, N, K):
         assert torch.all((out_st - s_ref).abs() <= 1e-3 * mag + 1e-3)
 
 
+@pytest.mark.parametrize("M", [1, 65, 1000, 40000])
+def test_gemm_ex_refuses_rows_its_epilogue_cannot_address(lib, M):
+    """Residuals, statistics and second outputs whose rows do not lie on 16-byte boundaries are refused on the host, whichever
+    kernel the number of rows would have gone to (the split-K kernel's 16-byte loads would be misaligned)."""
+    N, K = 20, 64
+    half = lambda *s: torch.zeros(*s, dtype=torch.float16, device="cuda")
+    A, W, C, R = half(M, K), half(512, K), half(M, 528), half(M * 528 + 8)
+    st = torch.zeros(M, 2, dtype=torch.float64, device="cuda")
+    cs = torch.zeros(512, device="cuda")
+    base = dict(A=A, W=W, C=C, M=M, N=N, K=K, precision=1, activation=oracle.ACT_NONE, ldc=24)
+    good = dict(base, res=R, ldres=24)
+    _lib.check(lib.b200_op_gemm_ex(_desc(**good), None))
+    _lib.check(lib.b200_op_gemm_ex(_desc(**dict(base, ldc=0)), None))  # plain products go through plain stores
+    for bad in (dict(good, ldres=20), dict(good, ldres=0), dict(good, res=R.data_ptr() + 2), dict(good, ldc=20),
+                dict(good, C=C.data_ptr() + 8), dict(base, ldc=20, out_stats=st),
+                dict(base, ldc=20, a_stats=st, colsum=cs, a_inv_c=1.0 / K)):
+        assert lib.b200_op_gemm_ex(_desc(**bad), None) == _lib.ERR_CUDA
+    for bad in (dict(base, N=288, n_split=256, ldc=260, C2=R, ldc2=32), dict(base, N=288, n_split=256, ldc=256, C2=R, ldc2=36)):
+        assert lib.b200_op_gemm_ex(_desc(**bad), None) == _lib.ERR_UNSUPPORTED
+    torch.cuda.synchronize()
+
+
 def test_gemm_ex_rejects_inconsistent_descriptions(lib):
     a = torch.zeros(256, 64, dtype=torch.float16, device="cuda")
     st = torch.zeros(256, 2, device="cuda", dtype=torch.float64)
