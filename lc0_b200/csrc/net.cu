@@ -1179,7 +1179,9 @@ struct Net : NetBase {
       p.A = x; p.lda = d.in; p.W = d.w; p.ldw = d.in; p.w_const = true; p.bias = d.b; p.C = y; p.ldc = ldc;
       p.M = M; p.N = d.out; p.K = d.in; p.act = act;
       p.ln_gamma = gamma; p.ln_beta = beta; p.ln_group = group; p.ln_eps = 1e-3f;
-      if (!use_tc || M > (group > 1 ? kLnInProductRows : 64) || !gemm_ln_supported(p)) return false;
+      // t_split_k: from kSplitKPositions on a position's result is the same in every batch, and the LayerNorm inside the
+      // product adds a row in another order than its own kernel
+      if (!use_tc || !t_split_k || (group > 1 && M > kLnInProductRows) || !gemm_ln_supported(p)) return false;
       launches++;
       const int sp_ = span_begin(st, K_GEMM_TC, 2.0 * p.M * (double)p.N * p.K, t_tag);
       CK(launch_gemm_ln<T>(p, t_status, st));

@@ -186,6 +186,23 @@ def test_fp32_results_do_not_depend_on_the_batch(name):
     nw.close()
 
 
+@pytest.mark.parametrize("precision", ["fp16", "bf16"])
+@pytest.mark.parametrize("side", [0, 1])
+def test_results_do_not_depend_on_the_batch_from_64_positions_on(precision, side):
+    """The line that Net draws (kSplitKPositions): 64 positions are on the same side of it as larger batches, with smolgen's
+    small products in line and on the second stream."""
+    net = mknet.make_net("cfg4_2layer", layers=6)
+    _, pos, n, g = load_compact("cfg4_2layer_b1024")
+    nw = network.Network(net, "precision=%s,max_batch=300,side_stream=%d" % (precision, side))
+    whole = nw.evaluate(pos["masks"][:300], pos["values"][:300])
+    # bit for bit: the atomics that add up a row's statistics add 32 fp32 sums in double, which is exact in any order
+    for batch in (64, 65, 100, 200):
+        out = nw.evaluate(pos["masks"][:batch], pos["values"][:batch])
+        for k in ("policy", "q", "d", "m"):
+            np.testing.assert_array_equal(out[k], whole[k][:batch])
+    nw.close()
+
+
 @pytest.mark.parametrize("batch", [64, 1024])
 def test_fp32_at_the_measured_batch_sizes_against_reference(batch):
     net, pos, n, g = load_compact("cfg4_2layer_b1024")
