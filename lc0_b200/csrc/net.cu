@@ -411,8 +411,8 @@ struct Net : NetBase {
   // Status word of the evaluation being enqueued on this thread (the slot's), handed to every kernel with bounded waits.
   static inline thread_local int* t_status = nullptr;
   static inline thread_local void* t_slot_ptr = nullptr;  // the slot of that evaluation
-  // > 0: the tensor-core launches that follow on this thread use at most this many SMs (persistent grids are sized
-  // from it), so that two launches on different streams can share the GPU
+  // > 0: the persistent grids of the tensor-core launches that follow on this thread have at most this many SMs, so that two
+  // launches on different streams can share the GPU.  The split-K kernel has one tile per CTA and only plans with it.
   static inline thread_local int t_sm_limit = 0;
   // Whether products of few rows may cut their K range (GemmParams::split_k): below 64 positions, where one tile per CTA
   // leaves most SMs idle.  From 64 positions on a position's result does not depend on the size of its batch.
@@ -425,14 +425,16 @@ struct Net : NetBase {
   };
   // smolgen's two small dense layers and their LayerNorms run on a second stream on kSideSms SMs while the QKV product
   // has the rest of the GPU: they are launch- and latency-bound (a quarter of a layer's time at batch 256), not
-  // throughput-bound
+  // throughput-bound.  From kSidePositions on.  Measured, us per evaluation of the BT4-class network beside / in line: 32
+  // positions 2042 / 1750, 64 2410 / 2228, 100 2986 / 2973, 128 3300 / 3367, 256 5915 / 5970.  At fewer positions these products
+  // run on gemm_split.cu's kernel, whose grid does not shrink to kSideSms: there is no GPU left over to put them beside.
   bool side_stream = false;
   bool dependent_launch = false;  // tensor-core products, attention and LayerNorms launched with launch_dependent()
   bool heads_side = false;        // value and moves-left heads on the side stream beside the policy head
   int heads_side_max = 0;         // ... up to this many positions
   bool tower = false;             // residual towers: all 3x3 convolutions in one launch up to tower_max_batch positions
   int tower_max_batch = 0;
-  static constexpr int kSideSms = 8;
+  static constexpr int kSideSms = 8, kSidePositions = 112;
 
   // format
   int network = 0, policy_fmt = 0, value_fmt = 0, emb_fmt = 0;
@@ -1390,7 +1392,7 @@ struct Net : NetBase {
     }
     // With per-launch event pairs on (profiling) the layer runs in line: a span around a launch that shares the GPU
     // with another stream measures the sharing, not the kernel.
-    if (side_stream && !profiling && e.smolgen && R >= 2048) {
+    if (side_stream && !profiling && e.smolgen && n >= kSidePositions) {
       // compression first (it reads the whole layer input: memory-bound, all SMs), then the two small dense layers
       // with their LayerNorms on the side stream while Q, K, V are computed on the other SMs
       cudaStream_t st2 = s.stream2;
@@ -1425,7 +1427,7 @@ struct Net : NetBase {
       finish_layer(s, e, R, x, x1, in, stats2);
       return;
     }
-    // One launch for Q, K, V and the smolgen compression when the CTA-pair kernel takes the product.
+    // One launch for Q, K, V and the smolgen compression where the product may have a second output.
     bool merged = false;
     if (e.smolgen && e.qkvc_out && merge_compress) {
       GemmParams probe;
