@@ -11,9 +11,12 @@
 // A sum does not depend on the number of rows: the K range is summed in pieces whose number follows from N and K alone
 // (k_pieces), a piece group by group, and the pieces' sums are added one after the other.  A tile that leaves SMs idle has a CTA
 // of a cluster for every piece or pair of pieces, whose sums meet through distributed shared memory; otherwise one CTA takes
-// the pieces in turn and keeps the total in shared memory, which costs 2 - 5 % of a product against one running sum (4096x3072x1024
-// 676 -> 692 us, 1024x1024x1024 69.5 -> 71.8; with totals in registers beside the running sums 740 and 76).
+// the pieces in turn and keeps the total in shared memory, which costs up to 4 % against one running sum (4096x3072x1024 in two
+// pieces 676 -> 678 us, 1024x1024x1024 in four 69.4 -> 69.8, 1024x1536x1024 in four 102.5 -> 106.6).
+// Rows that do not start on 16-byte boundaries move in 4-byte cp.async (16-bit storage: plain loads), in a kernel of their own: with
+// both forms of staging in one, the aligned products were 3 - 5 % slower; 4096x1024x1022 336 -> 290 us.
 #include <atomic>
+#include <type_traits>
 
 #include "kernels.cuh"
 
@@ -39,6 +42,9 @@ struct FmaParams {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ float4 ld_cluster_v4(uint32_t local, uint32_t rank) {
@@ -53,20 +59,23 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 // Four elements from `src` into shared memory as floats; those from `left` on are zeros (left may be anything).
-template <typename T>
-__device__ __forceinline__ void stage4(float* dst, const T* src, int left, bool vec) {
+template <bool kVec, typename T>
+__device__ __forceinline__ void stage4(float* dst, const T* src, int left) {
   if constexpr (sizeof(T) == 4) {
-    if (vec) {
-      cp_async16((uint32_t)__cvta_generic_to_shared(dst), src, min(max(left, 0), 4) * 4);
-      return;
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (kVec) {
+      cp_async16(to, src, min(max(left, 0), 4) * 4);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) cp_async4(to + 4 * i, i < left ? src + i : src, i < left ? 4 : 0);
     }
-  } else {
-    if (vec && left >= 4) {
-      const uint2 u = *reinterpret_cast<const uint2*>(src);
-      const T* e = reinterpret_cast<const T*>(&u);
-      *reinterpret_cast<float4*>(dst) = make_float4(to_f(e[0]), to_f(e[1]), to_f(e[2]), to_f(e[3]));
-      return;
-    }
+    return;
+  }
+  if (kVec && left >= 4) {
+    const uint2 u = *reinterpret_cast<const uint2*>(src);
+    const T* e = reinterpret_cast<const T*>(&u);
+    *reinterpret_cast<float4*>(dst) = make_float4(to_f(e[0]), to_f(e[1]), to_f(e[2]), to_f(e[3]));
+    return;
   }
   float v[4];
 #pragma unroll
@@ -74,7 +83,7 @@ __device__ __forceinline__ void stage4(float* dst, const T* src, int left, bool 
   *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
-template <typename T, bool kFast, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv, bool kTotals>
+template <typename T, bool kFast, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv, bool kTotals, bool kVec>
 __global__ void __launch_bounds__(kGroups * (BM / TM) * (BN / TN), kMinCtas)
 gemm_fma_kernel(const FmaParams p) {
   constexpr int kGroupThreads = (BM / TM) * (BN / TN), kThreads = kGroups * kGroupThreads;
@@ -134,7 +143,7 @@ gemm_fma_kernel(const FmaParams p) {
 #pragma unroll
     for (int r = 0; r < kRowsW; ++r)
       if (BN % kRowStep == 0 || lr + r * kRowStep < BN)
-        stage4(dst + r * kRowStep * kLd, w + off_w[r], (ok_w >> r) & 1 ? left : 0, p.vec);
+        stage4<kVec>(dst + r * kRowStep * kLd, w + off_w[r], (ok_w >> r) & 1 ? left : 0);
   };
   auto stage_a = [&](int i) {
     if (i >= kbn) return;
@@ -152,7 +161,7 @@ gemm_fma_kernel(const FmaParams p) {
     for (int r = 0; r < kRowsA; ++r)
       if (BM % kRowStep == 0 || lr + r * kRowStep < BM) {
         const bool in = (ok_a[r] >> tap) & 1 && left > 0;
-        stage4(dst + r * kRowStep * kLd, in ? A + off_a[r] + at : A, in ? left : 0, p.vec);
+        stage4<kVec>(dst + r * kRowStep * kLd, in ? A + off_a[r] + at : A, in ? left : 0);
       }
   };
 
@@ -304,12 +313,12 @@ gemm_fma_kernel(const FmaParams p) {
   cluster_sync();  // the others may still be reading this CTA's sums
 }
 
-template <typename T, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv, bool kTotals>
+template <typename T, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv, bool kTotals, bool kVec>
 cudaError_t launch_kernel(const FmaParams& p, int batch, cudaStream_t s) {
   constexpr int ring = kStages * (BM + BN) * (kBK + 4) * 4, out = BM * (BN + 4) * 4;
   static_assert(ring >= 2 * out, "the sums take the place of the ring");
   constexpr int smem = ring + (kTotals ? kGroups * BM * BN * 4 : 0);
-  auto kernel = gemm_fma_kernel<T, (sizeof(T) == 2), BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv, kTotals>;
+  auto kernel = gemm_fma_kernel<T, (sizeof(T) == 2), BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv, kTotals, kVec>;
   static std::atomic<unsigned long long> attr_mask{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -344,8 +353,13 @@ cudaError_t launch_kernel(const FmaParams& p, int batch, cudaStream_t s) {
 
 template <typename T, int BM, int BN, int TM, int TN, int kBK, int kGroups, int kMinCtas, bool kConv>
 cudaError_t launch_tile(const FmaParams& p, int batch, cudaStream_t s) {
-  if (p.ks == p.pieces) return launch_kernel<T, BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv, false>(p, batch, s);
-  return launch_kernel<T, BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv, true>(p, batch, s);
+  auto launch = [&](auto totals, auto vec) {
+    return launch_kernel<T, BM, BN, TM, TN, kBK, kGroups, kMinCtas, kConv, decltype(totals)::value, decltype(vec)::value>(p, batch, s);
+  };
+  using Yes = std::true_type;
+  using No = std::false_type;
+  if (p.ks == p.pieces) return p.vec ? launch(No(), Yes()) : launch(No(), No());
+  return p.vec ? launch(Yes(), Yes()) : launch(Yes(), No());
 }
 
 // Pieces of the K range: from N and K alone, so that every number of rows has the same sums.  As many as give the column tiles of

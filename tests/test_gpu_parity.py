@@ -186,6 +186,24 @@ def test_fp32_results_do_not_depend_on_the_batch(name):
     nw.close()
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp16"])
+def test_convolutions_whose_rows_are_no_16_byte_pieces(precision):
+    """30 filters: the FMA kernel's convolution stages rows element by element."""
+    from lc0_b200 import netproto
+    net = netproto.parse_net(netproto.encode("Net", mknet.make_net("cfg1_mini", filters=30)))
+    _, pos, n, g = load_case("cfg1_mini")
+    want = oracle.forward(*weights.flatten(net), pos["masks"][:5], pos["values"][:5])
+    nw = network.Network(net, "precision=%s,max_batch=8" % precision)
+    out = nw.evaluate(pos["masks"][:5], pos["values"][:5])
+    nw.close()
+    if precision == "fp32":
+        _assert_fp32_logits(out["policy"], want["policy"])
+        _assert_fp32_scalar(out["q"], want["q"])
+    else:  # storage rounding through five convolutions and two dense layers, each adding its share of a row's norm
+        assert np.abs(out["policy"] - want["policy"]).max() <= 8 * 2.0 ** -11 * np.abs(want["policy"]).max()
+        assert np.abs(out["q"] - want["q"]).max() <= HALF_ATOL
+
+
 @pytest.mark.parametrize("precision", ["fp16", "bf16"])
 @pytest.mark.parametrize("side", [0, 1])
 def test_results_do_not_depend_on_the_batch_from_64_positions_on(precision, side):
