@@ -329,6 +329,12 @@ int b200_op_gemm_ex(const b200_gemm_desc* d, void* stream);
  *   tensor-core kernel (the one the network uses; fp16 / bf16, depth 32 or 64). */
 int b200_op_attention(const void* q, const void* k, const void* v, long long ld, const void* bias, void* out,
                       long long ldo, int n, int heads, int depth, int precision, int variant, void* stream);
+/* b200_op_gemm_ln: C[M][N] = act(LN(x) . W^T + bias) in one launch, as smolgen's dense layers run at few positions
+ *   (LayerNorm2DWithSkipConnection, backends/blas/encoder.h:29-78, before Forward1D): x [M][256], every `group` consecutive rows
+ *   are one LayerNorm vector with gamma / beta [group * 256]; group 1, 2, 4, 8, 16 or 32 and M a multiple of it; W [N][256].
+ *   fp16 / bf16 only; synchronises the stream before returning. */
+int b200_op_gemm_ln(const void* x, const float* gamma, const float* beta, int group, float eps, const void* W,
+                    const float* bias, void* C, int M, int N, int activation, int precision, void* stream);
 /* b200_op_gemm_timed: the tensor-core product of b200_op_gemm queued `launches` times back to back on `stream`
  *   between two CUDA events; *ms_per_launch = elapsed / launches.  With enough launches the host's launch latency
  *   drops out, which is what a launch costs inside a replayed graph (profiling surface only). */

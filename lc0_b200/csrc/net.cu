@@ -2389,6 +2389,35 @@ int b200_op_gemm_ex(const b200_gemm_desc* d, void* stream) {
   return B200_OK;
 }
 
+int b200_op_gemm_ln(const void* x, const float* gamma, const float* beta, int group, float eps, const void* W, const float* bias,
+                    void* C, int M, int N, int activation, int precision, void* stream) {
+  GemmParams p;
+  p.A = x; p.lda = 256; p.W = W; p.ldw = 256; p.bias = bias; p.C = C; p.ldc = N;
+  p.M = M; p.N = N; p.K = 256; p.act = activation;
+  p.ln_gamma = gamma; p.ln_beta = beta; p.ln_group = group; p.ln_eps = eps;
+  if (precision == B200_PREC_FP32 || !gemm_ln_supported(p)) {
+    set_error("b200_op_gemm_ln: 16-bit rows of 256 in whole vectors of 1, 2, 4, 8, 16 or 32 rows, on 16-byte boundaries");
+    return B200_ERR_UNSUPPORTED;
+  }
+  B200_CUDA(gemm_tc_init());
+  int* status = nullptr;
+  B200_CUDA(cudaMalloc(&status, sizeof(int)));
+  cudaStream_t st = (cudaStream_t)stream;
+  cudaError_t err = cudaMemsetAsync(status, 0, sizeof(int), st);
+  if (err == cudaSuccess)
+    err = precision == B200_PREC_FP16 ? launch_gemm_ln<__half>(p, status, st) : launch_gemm_ln<__nv_bfloat16>(p, status, st);
+  if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+  int code = 0;
+  if (err == cudaSuccess) err = cudaMemcpy(&code, status, sizeof(int), cudaMemcpyDeviceToHost);
+  cudaFree(status);
+  B200_CUDA(err);
+  if (code) {
+    set_error("tensor-core GEMM: a bounded device-side wait gave up, status " + std::to_string(code));
+    return B200_ERR_TIMEOUT;
+  }
+  return B200_OK;
+}
+
 int b200_op_gemm_timed(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, int activation,
                        int precision, int launches, float* ms_per_launch, void* stream) {
   GemmParams p;

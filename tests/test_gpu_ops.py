@@ -438,6 +438,87 @@ def test_gemm_ex_refuses_rows_its_epilogue_cannot_address(lib, M):
     torch.cuda.synchronize()
 
 
+@pytest.mark.parametrize("prec", [1, 2])
+@pytest.mark.parametrize("group,M,N", [(1, 1, 256), (1, 63, 8192), (1, 65, 40), (2, 2, 64), (2, 66, 200), (4, 4, 4096), (4, 68, 72),
+                                       (8, 8, 128), (8, 200, 96), (16, 16, 4096), (16, 80, 65), (32, 32, 4096), (32, 96, 100),
+                                       (32, 256, 4096)])
+def test_layer_norm_inside_a_product(lib, prec, group, M, N):
+    """Vectors of 1 to 32 rows (sums over lanes, over one warp, over several), the last tile full or not, columns that are no
+    multiple of the tile or of eight; one vector far from zero mean, one almost constant."""
+    dt = DT[prec]
+    g = torch.Generator(device="cuda").manual_seed(group * 1000 + M + N)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    vec = M // group
+    x = rnd(vec, group * 256)
+    x[0] += 20.0
+    x[-1] *= 1e-2
+    x = x.to(dt)
+    gamma, beta = 1 + 0.2 * rnd(group * 256), 0.2 * rnd(group * 256)
+    W, b = (rnd(N, 256) / 16).to(dt), 0.1 * rnd(N)
+    C = torch.zeros(M, N, dtype=dt, device="cuda")
+    _lib.check(lib.b200_op_gemm_ln(x.data_ptr(), gamma.data_ptr(), beta.data_ptr(), group, 1e-3, W.data_ptr(), b.data_ptr(),
+                                   C.data_ptr(), M, N, oracle.ACT_NONE, prec, None))
+    x64 = x.double()
+    xn = (x64 - x64.mean(1, keepdim=True)) * (x64.var(1, unbiased=False, keepdim=True) + 1e-3).rsqrt()
+    xn = (xn * gamma.double() + beta.double()).reshape(M, 256)
+    ref = xn @ W.double().T + b.double()
+    mag = xn.abs() @ W.double().abs().T
+    # the normalised rows are rounded to the storage type once and so is the result; in fp32, mean and variance of up to 8192
+    # values whose mean is 20 deviations away lose 2^-24 * 20 * (a few) of a deviation
+    u = 2.0 ** -11 if prec == 1 else 2.0 ** -8
+    assert torch.all((C.double() - ref).abs() <= (u + 1e-5) * mag + u * ref.abs() + 1e-4), (C.double() - ref).abs().max().item()
+
+
+def test_layer_norm_inside_a_product_refuses_other_shapes(lib):
+    x = torch.zeros(64, 256, dtype=torch.float16, device="cuda")
+    v = torch.zeros(64 * 256, device="cuda")
+    op = lambda group, M, prec, off=0: lib.b200_op_gemm_ln(x.data_ptr() + off, v.data_ptr(), v.data_ptr(), group, 1e-3, x.data_ptr(),
+                                                           None, x.data_ptr(), M, 64, oracle.ACT_NONE, prec, None)
+    for args in ((1, 4, 0), (3, 6, 1), (64, 64, 1), (0, 4, 1), (8, 12, 1), (1, 4, 1, 8)):
+        assert op(*args) == _lib.ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("prec", [1, 2])
+@pytest.mark.parametrize("M,rest", [(1, 8), (63, 32), (64, 256), (65, 200), (130, 40), (400, 104)])
+def test_second_output_of_products_of_few_rows(lib, prec, M, rest):
+    """Columns beyond n_split go to the second matrix, with the LayerNorm of the input folded in; widths that end inside a tile and
+    row counts that end inside a tile.  Neither matrix is written beyond its columns."""
+    dt, N, K = DT[prec], 512, 320
+    g = torch.Generator(device="cuda").manual_seed(M + rest)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    A, W, b = (rnd(M, K) + 0.5).to(dt), (rnd(N + rest, K) * K ** -0.5).to(dt), 0.1 * rnd(N + rest)
+    a64 = A.double()
+    st = torch.stack([a64.sum(1), (a64 * a64).sum(1)], 1).contiguous()
+    cs = W.float().sum(1).contiguous()
+    C, C2 = torch.full((M, N + 8), 7.0, dtype=dt, device="cuda"), torch.full((M, rest + 8), 7.0, dtype=dt, device="cuda")
+    _lib.check(lib.b200_op_gemm_ex(_desc(A=A, W=W, bias=b, C=C, M=M, N=N + rest, K=K, ldc=N + 8, precision=prec, a_stats=st, colsum=cs,
+                                         activation=oracle.ACT_NONE, a_inv_c=1.0 / K, a_eps=1e-3, C2=C2, ldc2=rest + 8,
+                                         n_split=N), None))
+    rstd = (a64.var(1, unbiased=False, keepdim=True) + 1e-3).rsqrt()
+    ref = rstd * (a64 @ W.double().T - a64.mean(1, keepdim=True) * cs.double()) + b.double()
+    got = torch.cat([C[:, :N], C2[:, :rest]], 1).double()
+    u = 2.0 ** -11 if prec == 1 else 2.0 ** -8
+    # fp32: K products and the mean's correction, each at most rstd * (|A| |W|), a few roundings of it
+    mag = rstd * (a64.abs() @ W.double().abs().T)
+    assert torch.all((got - ref).abs() <= u * ref.abs() + 1e-5 * mag + 1e-6), (got - ref).abs().max().item()
+    assert torch.all(C[:, N:] == 7) and torch.all(C2[:, rest:] == 7)
+
+
+@pytest.mark.parametrize("M,N,ldc", [(1, 8, 9), (65, 129, 131), (200, 1858, 1858), (64, 64, 65)])
+def test_products_of_few_rows_into_unaligned_rows(lib, M, N, ldc):
+    """Output rows that are no 16-byte pieces: element stores, nothing beyond the columns."""
+    K = 136
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    A = torch.randn(M, K, device="cuda", generator=g).half()
+    W = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).half()
+    C = torch.full((M, ldc), 7.0, dtype=torch.float16, device="cuda")
+    _lib.check(lib.b200_op_gemm_ex(_desc(A=A, W=W, C=C, M=M, N=N, K=K, ldc=ldc, precision=1, activation=oracle.ACT_NONE), None))
+    ref = A.double() @ W.double().T
+    mag = A.double().abs() @ W.double().abs().T
+    assert torch.all((C[:, :N].double() - ref).abs() <= 2.0 ** -11 * ref.abs() + (K + 2) * 2.0 ** -24 * mag + 2.0 ** -24)
+    assert torch.all(C[:, N:] == 7)
+
+
 def test_gemm_ex_rejects_inconsistent_descriptions(lib):
     a = torch.zeros(256, 64, dtype=torch.float16, device="cuda")
     st = torch.zeros(256, 2, device="cuda", dtype=torch.float64)
