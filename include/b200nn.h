@@ -67,7 +67,7 @@ void b200_builder_destroy(b200_builder* b);
 typedef struct b200_net_options {
   int gpu;        /* CUDA device ordinal */
   int max_batch;  /* largest batch one computation may hold */
-  int precision;  /* B200_PREC_* */
+  int precision;  /* B200_PREC_*; see "Results and the batch" below */
   int slots;      /* concurrent computations (>= 1) */
   int mlh;        /* 0 disables the moves-left head like the reference's mlh=false */
   int flags;      /* B200_FLAG_* */
@@ -145,6 +145,13 @@ int b200_comp_add_inputs_with_moves(b200_comp* c, const uint64_t* masks, const f
                                     const uint16_t* move_ids, const int* n_moves, int n);
 int b200_comp_set_policy_options(b200_comp* c, float inv_temperature, int compact);
 int b200_comp_legal_policy(const b200_comp* c, int sample, const float** probs, int* n_moves);
+
+/* ---- Results and the batch --------------------------------------------------------------------
+ * fp32: a position's results are the same, bit for bit, whatever else is in its batch and however large the batch is.
+ * fp16 / bf16: they are the same in every batch of fewer than 64 positions, and the same in every batch of 64 and more.  Between
+ *   the two they differ in the last bits of the storage type: below 64 positions the products that see one row per position cut
+ *   their contraction over several SMs.  Requests that b200_mux_* merges and slices that b200_multi_* cuts are batches in this
+ *   sense. */
 
 /* ---- Whole-batch entry points ----------------------------------------------------------------
  * b200_net_eval_host: one call = add n inputs, compute, copy results out.  Host pointers;
@@ -290,7 +297,8 @@ int b200_op_planes_from_training_data(const void* d_records, int n, long long re
  *   `precision` type (BlasComputation::EncodePlanes, network_blas.cc:973-981).
  * b200_op_gemm: C[M][N] = act(A[M][K] . W[N][K]^T + bias) in the given precision, using the
  *   tcgen05 tensor-core kernel when use_tc != 0 (fp16/bf16 only) else the FMA kernel
- *   (FullyConnectedLayer::Forward1D, fully_connected_layer.cc:50-106).
+ *   (FullyConnectedLayer::Forward1D, fully_connected_layer.cc:50-106).  A row of the FMA kernel's result does not depend on
+ *   the number of rows; with tensor cores (here and in _ex) it is one for all numbers of rows below 64 and one from 64 on.
  * b200_op_layer_norm: out = LN(alpha * x + skip) * gamma + beta over rows of width C
  *   (LayerNorm2DWithSkipConnection, backends/blas/encoder.h:29-78). */
 int b200_op_expand_planes(const void* d_masks, const void* d_values, int n, void* d_out,
@@ -306,7 +314,9 @@ int b200_op_gemm(const void* A, const void* W, const float* bias, void* C, int M
  *   - res [M][N] is added after the activation, normalised on the fly with res_stats / res_gamma / res_beta
  *     (res_inv_c = 1/N, res_eps) when those are given;
  *   - out_stats [M][2] (double) accumulates the per-row sum and sum of squares of the outputs (the caller zeroes it);
- *   - columns [n_split, N) go to C2 (leading dimension ldc2) instead of C when n_split > 0.
+ *   - columns [n_split, N) go to C2 (leading dimension ldc2) instead of C when n_split > 0 (a multiple of 256, at most
+ *     256 columns beyond it, no residual or out_stats; any number of rows).
+ *   Rows of C, C2 and res must be 16-byte pieces (base and leading dimension) in every form but the plain product.
  *   Leading dimensions of 0 mean dense.  fp16 / bf16 only; synchronises the stream before returning. */
 typedef struct b200_gemm_desc {
   const void* A; const void* W; const float* bias; void* C;

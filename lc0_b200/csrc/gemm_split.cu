@@ -4,8 +4,8 @@
 // Such a product is bound by latency and by how many SMs pull weights, not by the tensor pipe: with one 128x256 tile per
 // CTA the 1024x1024 projection of one position ran on 4 SMs.  Here a tile is 128 (or 64) rows x BN columns and its K range
 // is cut over the CTAs of a cluster (split-K), so that about one CTA per SM has a few k-blocks each, all of them in
-// flight at once.  The weight tiles do not depend on the kernel before this one: they are requested before
-// griddepcontrol.wait, i.e. while that kernel is still running (two CTAs fit on an SM).
+// flight at once.  Tiles of loaded weights (GemmParams::w_const) do not depend on the kernel before this one: they are requested
+// before griddepcontrol.wait, i.e. while that kernel is still running (two CTAs fit on an SM).
 //   warp 8      TMA producer (W ahead of the grid dependency, then A)
 //   warp 9      tcgen05.mma issuer (cta_group::1, 128xBNx16), accumulator in tensor memory
 //   warps 0-7   accumulator -> fp32 partial tiles in shared memory; with split-K each CTA of the cluster owns a slice of
@@ -16,12 +16,13 @@
 // shared memory and its results are never looked at.
 // Chains of dependent launches, before (one 128xBN tile per CTA of gemm_tc.cu's kernel, FMA kernel below 64 rows) and now:
 // 64x1024x1024 15 -> 5.9 us, 1x256x2048 135 -> 5.3 us, 1x8192x256 21 -> 4.5 us, 32x4096x256 24 -> 4.2 us; with everything in this file one
-// position of the BT4-class network 4.37 -> 0.82 ms, 24 positions 4.47 -> 1.73 ms.
+// position of the BT4-class network 4.37 -> 0.81 ms, 24 positions 4.47 -> 1.71 ms.  (Net does not cut the K range of products with 64
+// rows per position: one position's 1024-wide ones take 7.8 us for 5.9.)
 // With a LayerNorm in front (GemmParams::ln_gamma; 256-wide rows, smolgen's two inner LayerNorms) warps 0-7 load the 64 rows of
 // A themselves, normalise them in registers and write them to the operand tiles in the swizzle TMA would have used; gamma and
 // beta arrive by bulk copy ahead of the grid dependency.  A LayerNorm vector may span several rows of A (smolgen's
 // second one: 32 heads x 256), as long as a tile holds whole vectors.  Every column tile repeats the LayerNorm: worth it
-// while a launch costs more than that (Net::gemm_with_ln has the line).
+// while a launch costs more than that (Net::gemm_with_ln has the line); beyond, ln_rows_kernel does it with the same results.
 // Every wait is bounded by wall-clock time like those of gemm_tc.cu; the cluster barriers are reached by all threads
 // whatever happened before them.
 #include <atomic>
@@ -103,6 +104,69 @@ __device__ __forceinline__ float ln_sum(float v, int group, float* red) {
     for (int w = warp & ~(span - 1), e = w + span; w < e; ++w) v += red[w];
   }
   return v;
+}
+
+// LayerNorm of 64 rows by 256 threads: this thread's 16-byte pieces q, q + 4, ..., q + 28 of row tid / 4 (q = tid % 4), and the
+// mean and reciprocal deviation of the row's vector.  The product and ln_rows_kernel must agree to the last bit, hence the explicit
+// fused multiply-adds.
+template <typename T>
+__device__ __forceinline__ void ln_rows_load(const void* x, int m, int M, int group, float eps, float* red, uint4 (&u)[8], float& mean,
+                                             float& rstd) {
+  const int q = threadIdx.x & 3;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    u[i] = m < M ? *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(x) + (long long)m * kLnK + (q + 4 * i) * 8)
+                 : make_uint4(0, 0, 0, 0);
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sum += to_f(reinterpret_cast<const T*>(&u[i])[j]);
+  const float inv = 1.0f / (float)(group * kLnK);  // a power of two
+  mean = ln_sum(sum, group, red) * inv;
+  float var = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float d = to_f(reinterpret_cast<const T*>(&u[i])[j]) - mean;
+      var = fmaf(d, d, var);
+    }
+  rstd = 1.0f / sqrtf(fmaf(ln_sum(var, group, red + 8), inv, eps));
+}
+// Eight values normalised; gamma and beta point at theirs.
+template <typename T>
+__device__ __forceinline__ uint4 ln_piece(const uint4& u, const float* gamma, const float* beta, float mean, float rstd) {
+  const T* e = reinterpret_cast<const T*>(&u);
+  float v[8], g[8], b[8];
+  *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(gamma);
+  *reinterpret_cast<float4*>(g + 4) = *reinterpret_cast<const float4*>(gamma + 4);
+  *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(beta);
+  *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(beta + 4);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = fmaf(g[j] * (to_f(e[j]) - mean), rstd, b[j]);
+  return make_uint4(pack_pair<T>(v[0], v[1]), pack_pair<T>(v[2], v[3]), pack_pair<T>(v[4], v[5]), pack_pair<T>(v[6], v[7]));
+}
+
+// The same LayerNorm as a launch of its own, where the product has too many column tiles to repeat it in.  Latency-bound: 64 rows of
+// 512 bytes per CTA, all loads of a thread in flight at once.
+template <typename T>
+__global__ void __launch_bounds__(256)
+ln_rows_kernel(const T* x, T* out, const float* __restrict__ gamma, const float* __restrict__ beta, int group, float eps, int M) {
+  __shared__ float red[16];
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const int row = threadIdx.x >> 2, q = threadIdx.x & 3, m = (int)blockIdx.x * 64 + row;
+  uint4 u[8];
+  float mean, rstd;
+  ln_rows_load<T>(x, m, M, group, eps, red, u, mean, rstd);
+  if (m >= M) return;
+  const int at = (row & (group - 1)) * kLnK;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int c = (q + 4 * i) * 8;
+    *reinterpret_cast<uint4*>(out + (long long)m * kLnK + c) = ln_piece<T>(u[i], gamma + at + c, beta + at + c, mean, rstd);
+  }
 }
 
 template <typename T, int BN, bool kLN>
@@ -228,46 +292,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
     grid_dependency_wait();
     if constexpr (kLN) {
-      // row tid / 4; its 16-byte pieces q, q + 4, ..., q + 28 (piece c is piece c % 8 of k-block c / 8)
-      const int row = tid >> 2, q = tid & 3, m = m0 + row;
+      const int row = tid >> 2, q = tid & 3;  // piece c of a row is piece c % 8 of k-block c / 8
       uint4 u[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        u[i] = m < p.M ? *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(cfg.x) + (long long)m * kLnK + (q + 4 * i) * 8)
-                       : make_uint4(0, 0, 0, 0);
-      float* red = reinterpret_cast<float*>(rowv);  // rowv is not used here: no statistics come with a LayerNorm in front
-      float sum = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) sum += to_f(reinterpret_cast<const T*>(&u[i])[j]);
-      const float inv = 1.0f / (float)(cfg.group * kLnK);  // a power of two
-      const float mean = ln_sum(sum, cfg.group, red) * inv;
-      float var = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float d = to_f(reinterpret_cast<const T*>(&u[i])[j]) - mean;
-          var = fmaf(d, d, var);
-        }
-      const float rstd = 1.0f / sqrtf(ln_sum(var, cfg.group, red + 8) * inv + cfg.eps);
+      float mean, rstd;
+      // rowv is not used here: no statistics come with a LayerNorm in front
+      ln_rows_load<T>(cfg.x, m0 + row, p.M, cfg.group, cfg.eps, reinterpret_cast<float*>(rowv), u, mean, rstd);
       mbar_wait(smem_u32(gb_bar), 0, abort_flag, 6);
       const float* gamma = ln_gb + (row & (cfg.group - 1)) * kLnK;
       const float* beta = gamma + cfg.group * kLnK;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int c = q + 4 * i;
-        const T* e = reinterpret_cast<const T*>(&u[i]);
-        float v[8], g[8], b[8];
-        *reinterpret_cast<float4*>(g) = *reinterpret_cast<const float4*>(gamma + c * 8);
-        *reinterpret_cast<float4*>(g + 4) = *reinterpret_cast<const float4*>(gamma + c * 8 + 4);
-        *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(beta + c * 8);
-        *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(beta + c * 8 + 4);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = b[j] + g[j] * (to_f(e[j]) - mean) * rstd;
-        st_shared_v4(smem_u32(smem + (c >> 3) * stage_bytes) + row * 128 + (((c & 7) ^ (row & 7)) << 4), pack_pair<T>(v[0], v[1]),
-                     pack_pair<T>(v[2], v[3]), pack_pair<T>(v[4], v[5]), pack_pair<T>(v[6], v[7]));
+        const uint4 v = ln_piece<T>(u[i], gamma + c * 8, beta + c * 8, mean, rstd);
+        st_shared_v4(smem_u32(smem + (c >> 3) * stage_bytes) + row * 128 + (((c & 7) ^ (row & 7)) << 4), v.x, v.y, v.z, v.w);
       }
       fence_async_smem();  // the tensor core reads the rows through the asynchronous proxy
       mbar_arrive(smem_u32(a_bar));
@@ -429,7 +466,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 }
 
 // Tile width, cluster size and stages of a product: the least of a cost model in microseconds, fitted to chains of dependent
-// launches (M x N x K; us measured at columns per tile / CTAs per tile, 5 - 20 % more than with today's elected issue):
+// launches of this kernel before its issuing lanes were elected (M x N x K; us at columns per tile / CTAs per tile).  A k-block took
+// 731 cycles to issue then, 0.39 us, and takes 495 - 527 now: the model still orders the plans it was fitted to, but weighs a long K
+// range too heavily against the exchange of a cut one, and has not been fitted again.  Tiles of 64 rows also above 64 rows: 10 x 256
+// attention network 2 / 8 / 16 / 37 positions 271 / 283 / 307 / 369 -> 225 / 258 / 271 / 332 us, BT4-class 2 / 8 963 / 1057 -> 842 / 1008.
 //   1536x1024x1024  32/1 19.5  64/1 11.2  64/2 17.6  128/1 13.9  128/2 12.5    2368x768x256   32/1 10.3  64/1 6.7  128/1 9.2
 //   512x1024x1024   32/1 10.0  32/2 7.9   64/1 11.3  64/4 9.1    128/1 13.6    2368x256x256   32/1 5.3   64/1 6.6  128/1 9.0
 //   512x1024x1536   32/2 9.5   64/2 10.9  64/4 9.8   128/2 12.7                64x1024x1024   32/4 5.9   64/1 9.8  64/4 6.3
@@ -442,25 +482,27 @@ SplitPlan split_plan(const GemmParams& g, int sm_count) {
   SplitPlan best{64, 1, 128, 1};
   double best_cost = 1e30;
   const int k_blocks = ceil_div(g.K, BK);
-  const int a_rows = g.M <= 64 ? 64 : 128;
-  const int m_tiles = ceil_div(g.M, a_rows);
-  for (int bn = 32; bn <= 128; bn *= 2) {
-    const int n_tiles = ceil_div(g.N, bn);
-    for (int ks = 1; ks <= 8; ks *= 2) {
-      if (ks > k_blocks || (ks > 1 && !g.split_k)) break;
-      const int kb = ceil_div(k_blocks, ks);
-      const long long ctas = (long long)n_tiles * m_tiles * ks;
-      const int rounds = ceil_div(ctas, 2 * sm_count);
-      const double tile = 2.5 + a_rows * bn * (1.0 / 3300), exchange = ks == 1 ? 0.0 : (0.25 + 0.2 * ks) * (a_rows == 64 ? 1.0 : 1.6);
-      const double cost = rounds * (tile + 0.39 * kb + exchange + (ctas > sm_count ? 0.5 : 0.0));
-      if (cost < best_cost) {
-        best_cost = cost;
-        best = SplitPlan{bn, ks, a_rows, kb};
+  // of plans that cost the same the one with the taller tiles, which fetch W less often
+  for (int a_rows = g.M <= 64 ? 64 : 128; a_rows >= 64; a_rows /= 2) {
+    const int m_tiles = ceil_div(g.M, a_rows);
+    for (int bn = 32; bn <= 128; bn *= 2) {
+      const int n_tiles = ceil_div(g.N, bn);
+      for (int ks = 1; ks <= 8; ks *= 2) {
+        if (ks > k_blocks || (ks > 1 && !g.split_k)) break;
+        const int kb = ceil_div(k_blocks, ks);
+        const long long ctas = (long long)n_tiles * m_tiles * ks;
+        const int rounds = ceil_div(ctas, 2 * sm_count);
+        const double tile = 2.5 + a_rows * bn * (1.0 / 3300), exchange = ks == 1 ? 0.0 : (0.25 + 0.2 * ks) * (a_rows == 64 ? 1.0 : 1.6);
+        const double cost = rounds * (tile + 0.39 * kb + exchange + (ctas > sm_count ? 0.5 : 0.0));
+        if (cost < best_cost) {
+          best_cost = cost;
+          best = SplitPlan{bn, ks, a_rows, kb};
+        }
       }
     }
   }
   // a ring of at most 96 KB leaves room for a second CTA on the SM: the next tile, or the next kernel fetching its weights
-  const int cap = 96 * 1024 / ((a_rows + best.bn) * 128);
+  const int cap = 96 * 1024 / ((best.a_rows + best.bn) * 128);
   if (best.stages > cap) best.stages = cap;
   return best;
 }
@@ -524,6 +566,14 @@ cudaError_t launch_gemm_ln(const GemmParams& g, int* status, cudaStream_t s) {
   if (!gemm_ln_supported(g)) return cudaErrorInvalidValue;
   return launch_split_bn<T, 64, true>(g, SplitPlan{64, 1, 64, kLnK / BK}, status, s);
 }
+template <typename T>
+cudaError_t launch_ln_rows(const T* x, T* out, const float* gamma, const float* beta, int group, float eps, int M, cudaStream_t s) {
+  if (M <= 0) return cudaSuccess;
+  return launch_dependent(ln_rows_kernel<T>, dim3(ceil_div(M, 64)), dim3(256), 0, s, x, out, gamma, beta, group, eps, M);
+}
+template cudaError_t launch_ln_rows<__half>(const __half*, __half*, const float*, const float*, int, float, int, cudaStream_t);
+template cudaError_t launch_ln_rows<__nv_bfloat16>(const __nv_bfloat16*, __nv_bfloat16*, const float*, const float*, int, float, int,
+                                                   cudaStream_t);
 template cudaError_t launch_gemm_ln<__half>(const GemmParams&, int*, cudaStream_t);
 template cudaError_t launch_gemm_ln<__nv_bfloat16>(const GemmParams&, int*, cudaStream_t);
 

@@ -63,9 +63,9 @@ struct GemmParams {
   // CTA-pair kernel: compute a sparsely filled last wave as whole 256x256 tiles instead of half-width ones
   // (verification switch; the split is on by default).
   bool whole_tiles = false;
-  // Products of few rows on tensor cores: the K range may be cut over several CTAs (gemm_split.cu).  The sums then depend on
-  // the number of rows; off, a row's result is the same whatever else is in the batch.
-  bool split_k = true;
+  // Products of few rows on tensor cores: the K range may be cut over several CTAs (gemm_split.cu).  The plan, and with it a row's
+  // sum, is the same for every number of rows up to 64 and follows their number beyond; off, it is the same for all.
+  bool split_k = false;
   // LayerNorm of A inside the product (launch_gemm_ln): every ln_group consecutive rows of A, which are 256 wide and packed,
   // are one LayerNorm vector with ln_gamma / ln_beta [ln_group * 256].
   const float* ln_gamma = nullptr;
@@ -84,6 +84,9 @@ bool gemm_tc_supported(const GemmParams& p);
 // Product with the LayerNorm of its input in front (gemm_split.cu), for few rows.
 bool gemm_ln_supported(const GemmParams& p);
 template <typename T> cudaError_t launch_gemm_ln(const GemmParams& p, int* status, cudaStream_t s);
+// That LayerNorm as a launch of its own (in place or not), with the same results to the last bit.
+template <typename T>
+cudaError_t launch_ln_rows(const T* x, T* out, const float* gamma, const float* beta, int group, float eps, int M, cudaStream_t s);
 bool gemm_tc_se_supported(const GemmParams& p);
 // Whether launch_gemm_tc can run `p` with its second output (C2 / n_split).
 bool gemm_tc_split_supported(const GemmParams& p);

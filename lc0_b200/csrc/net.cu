@@ -414,10 +414,12 @@ struct Net : NetBase {
   // > 0: the persistent grids of the tensor-core launches that follow on this thread have at most this many SMs, so that two
   // launches on different streams can share the GPU.  The split-K kernel has one tile per CTA and only plans with it.
   static inline thread_local int t_sm_limit = 0;
-  // Whether products of few rows may cut their K range (GemmParams::split_k): below 64 positions, where one tile per CTA
-  // leaves most SMs idle.  From 64 positions on a position's result does not depend on the size of its batch.
-  static inline thread_local bool t_split_k = true;
-  static constexpr int kSplitKPositions = 64;
+  // Rows of the products that may cut their K range (GemmParams::split_k); 0: none.  Those with one row per position below 64
+  // positions: one tile of rows, so that the plan is the same for every such batch.  Products with 64 rows per position are not cut:
+  // their plan would follow the batch and with it a position's result (and from two positions on they are no faster for it).
+  // So a position's result is the same in every batch below 64 positions, and in every batch from 64 positions on.
+  static inline thread_local int t_cut_rows = 0;
+  static constexpr int kCutPositions = 64;
   struct DependentLaunchScope {
     bool prev;
     explicit DependentLaunchScope(bool on) : prev(t_dependent_launch) { t_dependent_launch = on; }
@@ -1133,7 +1135,7 @@ struct Net : NetBase {
     p.C = out_f32 ? cf32 : (void*)Cout; p.ldc = ldc; p.M = M; p.N = d.out; p.K = d.in; p.act = act;
     p.skip = skip; p.ldskip = ldskip; p.alpha = alpha_; p.out_f32 = out_f32;
     p.whole_tiles = (opt.flags & B200_FLAG_NO_SPLIT_LAST_WAVE) != 0;
-    p.split_k = t_split_k;
+    p.split_k = M == t_cut_rows;
     run_gemm(st, p);
   }
   // A LayerNorm output that is either materialised (stats == nullptr) or kept as its un-normalised input `u`
@@ -1169,21 +1171,28 @@ struct Net : NetBase {
       p.out_stats = out_stats;
     }
     p.whole_tiles = (opt.flags & B200_FLAG_NO_SPLIT_LAST_WAVE) != 0;
-    p.split_k = t_split_k;
+    p.split_k = M == t_cut_rows;
     run_gemm(st, p);
   }
-  // d(LayerNorm(x)) in one launch, every `group` rows of x being one LayerNorm vector; false where it does not apply: other
-  // widths, and batches at which the LayerNorm repeated in every column tile costs more than its own launch.
-  bool gemm_with_ln(cudaStream_t st, const T* x, const float* gamma, const float* beta, int group, const Dense<T>& d, T* y,
-                    long long ldc, int M, int act) {
+  // d(LayerNorm(x)) below kCutPositions, every `group` rows of x being one LayerNorm vector: in one launch, or in two where the
+  // LayerNorm repeated in every column tile costs more than its own launch, with the same results.  x is overwritten.  False where it
+  // does not apply: other widths, and larger batches, whose LayerNorm kernel adds a vector in another order.
+  bool gemm_with_ln(cudaStream_t st, T* x, const float* gamma, const float* beta, int group, const Dense<T>& d, T* y, long long ldc, int M,
+                    int act) {
     if constexpr (sizeof(T) == 2) {
       GemmParams p;
       p.A = x; p.lda = d.in; p.W = d.w; p.ldw = d.in; p.w_const = true; p.bias = d.b; p.C = y; p.ldc = ldc;
       p.M = M; p.N = d.out; p.K = d.in; p.act = act;
       p.ln_gamma = gamma; p.ln_beta = beta; p.ln_group = group; p.ln_eps = 1e-3f;
-      // t_split_k: from kSplitKPositions on a position's result is the same in every batch, and the LayerNorm inside the
-      // product adds a row in another order than its own kernel
-      if (!use_tc || !t_split_k || (group > 1 && M > kLnInProductRows) || !gemm_ln_supported(p)) return false;
+      if (!use_tc || t_cut_rows == 0 || !gemm_ln_supported(p)) return false;
+      if (M > kLnInProductRows) {
+        launches++;
+        const int sp_ = span_begin(st, K_LAYERNORM, (double)M * d.in * sizeof(T) * 2);
+        CK(launch_ln_rows<T>(x, x, gamma, beta, group, 1e-3f, M, st));
+        span_end(st, sp_);
+        gemm(st, x, d.in, d, y, ldc, M, act);
+        return true;
+      }
       launches++;
       const int sp_ = span_begin(st, K_GEMM_TC, 2.0 * p.M * (double)p.N * p.K, t_tag);
       CK(launch_gemm_ln<T>(p, t_status, st));
@@ -1192,9 +1201,10 @@ struct Net : NetBase {
     }
     return false;
   }
-  // Rows of a generator product up to which its LayerNorm (vectors over several rows) is worth repeating in 64 column tiles: one
-  // position of the BT4-class network 847 -> 820 us; at 768 rows (24 positions) 1730 -> 2163 us, one CTA of 139 KB per SM.
-  static constexpr int kLnInProductRows = 256;
+  // Rows up to which a LayerNorm is worth repeating in the column tiles of its product.  Smolgen's generator (64 column tiles), whole
+  // BT4-class network in us, in a launch of its own / in the product: one position 810 / 788, four 901 / 871, eight 1008 / 1065, 24
+  // 1730 / 2163 (one CTA of 139 KB per SM).
+  static constexpr int kLnInProductRows = 128;
   // Tag of the launches that follow on this thread (which product of the layer they are), for the tagged profile.
   static inline thread_local int t_tag = 0;
   void run_gemm(cudaStream_t st, const GemmParams& p) {
@@ -1500,7 +1510,7 @@ struct Net : NetBase {
     s.stats_parity = 0;
     t_status = d_status + (&s - slots.data());
     t_slot_ptr = &s;
-    t_split_k = n < kSplitKPositions;
+    t_cut_rows = n < kCutPositions ? n : 0;
     // not with per-launch event pairs: the spans would then time the overlap with the neighbours
     DependentLaunchScope launch_scope(dependent_launch && !profiling);
     CK(cudaMemsetAsync(d_qdm, 0, (size_t)n * 3 * sizeof(float), st));
@@ -2301,6 +2311,7 @@ int b200_op_gemm(const void* A, const void* W, const float* bias, void* C, int M
   GemmParams p;
   p.A = A; p.lda = K; p.W = W; p.ldw = K; p.bias = bias; p.C = C; p.ldc = N;
   p.M = M; p.N = N; p.K = K; p.act = activation;
+  p.split_k = M < 64;  // as the network cuts the products with one row per position
   if (use_tc) {
     if (precision == B200_PREC_FP32 || !gemm_tc_supported(p)) {
       set_error("b200_op_gemm: shape or precision not supported by the tensor-core kernel");
@@ -2357,6 +2368,7 @@ int b200_op_gemm_ex(const b200_gemm_desc* d, void* stream) {
   p.out_stats = d->out_stats;
   p.C2 = d->C2; p.ldc2 = d->ldc2; p.n_split = d->n_split;
   p.whole_tiles = d->whole_tiles != 0;
+  p.split_k = d->M < 64;  // as the network cuts the products with one row per position
   if ((p.a_stats && !p.colsum) || (p.res_stats && (!p.res || !p.res_gamma || !p.res_beta)) || !gemm_tc_supported(p)) {
     set_error("b200_op_gemm_ex: inconsistent description or shape not supported by the tensor-core kernel");
     return B200_ERR_UNSUPPORTED;
@@ -2423,6 +2435,7 @@ int b200_op_gemm_timed(const void* A, const void* W, const float* bias, void* C,
   GemmParams p;
   p.A = A; p.lda = K; p.W = W; p.ldw = K; p.bias = bias; p.C = C; p.ldc = N;
   p.M = M; p.N = N; p.K = K; p.act = activation;
+  p.split_k = M < 64;  // as the network cuts the products with one row per position
   if (launches < 1 || !ms_per_launch) {
     set_error("b200_op_gemm_timed: bad argument");
     return B200_ERR_INVALID;

@@ -18,7 +18,7 @@ def _check(gpus):
             masks, values = np.array(pos["masks"][:count]), np.array(pos["values"][:count])
             want = single.evaluate(masks, values)
             got = multi.evaluate(masks, values)
-            # the same kernels on the same rows; tiny batches route some products to the FMA kernel, hence the tolerance
+            # the same rows; batches below and from 64 positions on differ in the last bits, hence the tolerance
             for k in ("policy", "q", "d", "m"):
                 np.testing.assert_allclose(got[k], want[k], atol=2e-3)
         empty = multi.evaluate(np.zeros((0, 112), np.uint64), np.zeros((0, 112), np.float32))

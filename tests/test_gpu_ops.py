@@ -416,6 +416,24 @@ def test_products_of_few_rows(lib, prec, M, N, K):
         assert torch.all((out_st - s_ref).abs() <= 1e-3 * mag + 1e-3)
 
 
+@pytest.mark.parametrize("prec", [1, 2])
+@pytest.mark.parametrize("N,K", [(256, 2048), (1024, 1024), (40, 72), (1858, 2048), (8192, 256)])
+def test_tensor_core_gemm_rows_do_not_depend_on_their_number(lib, prec, N, K):
+    """One result of a row for all numbers of rows below 64 and one from 64 on, whichever kernel and tile they go to."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    A = torch.randn(6000, K, device="cuda", generator=g).to(DT[prec])
+    W = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).to(DT[prec])
+    b = torch.randn(N, device="cuda", generator=g)
+    for sizes in ((63, 1, 2, 8, 33), (6000, 64, 65, 200, 700, 2048)):
+        outs = []
+        for M in sizes:
+            C = torch.zeros(M, N, dtype=DT[prec], device="cuda")
+            _lib.check(lib.b200_op_gemm(A.data_ptr(), W.data_ptr(), b.data_ptr(), C.data_ptr(), M, N, K, oracle.ACT_MISH, prec, 1, None))
+            outs.append(C)
+        for C in outs[1:]:
+            assert torch.equal(C, outs[0][:C.shape[0]]), C.shape
+
+
 @pytest.mark.parametrize("M", [1, 65, 1000, 40000])
 def test_gemm_ex_refuses_rows_its_epilogue_cannot_address(lib, M):
     """Residuals, statistics and second outputs whose rows do not lie on 16-byte boundaries are refused on the host, whichever
@@ -526,5 +544,5 @@ def test_gemm_ex_rejects_inconsistent_descriptions(lib):
     assert lib.b200_op_gemm_ex(_desc(A=a, W=a, C=a, M=256, N=64, K=64, precision=1, a_stats=st), None) == \
         _lib.ERR_UNSUPPORTED  # statistics without column sums
     assert lib.b200_op_gemm_ex(_desc(A=a, W=a, C=a, M=256, N=64, K=64, precision=1, C2=a, ldc2=64, n_split=32),
-                               None) == _lib.ERR_UNSUPPORTED  # too small for the kernel that has a second output
+                               None) == _lib.ERR_UNSUPPORTED  # n_split is no multiple of 256
     assert lib.b200_op_gemm_ex(None, None) == _lib.ERR_INVALID

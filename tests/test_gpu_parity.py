@@ -207,7 +207,7 @@ def test_convolutions_whose_rows_are_no_16_byte_pieces(precision):
 @pytest.mark.parametrize("precision", ["fp16", "bf16"])
 @pytest.mark.parametrize("side", [0, 1])
 def test_results_do_not_depend_on_the_batch_from_64_positions_on(precision, side):
-    """The line that Net draws (kSplitKPositions): 64 positions are on the same side of it as larger batches, with smolgen's
+    """The line that Net draws (kCutPositions): 64 positions are on the same side of it as larger batches, with smolgen's
     small products in line and on the second stream."""
     net = mknet.make_net("cfg4_2layer", layers=6)
     _, pos, n, g = load_compact("cfg4_2layer_b1024")
@@ -215,6 +215,22 @@ def test_results_do_not_depend_on_the_batch_from_64_positions_on(precision, side
     whole = nw.evaluate(pos["masks"][:300], pos["values"][:300])
     # bit for bit: the atomics that add up a row's statistics add 32 fp32 sums in double, which is exact in any order
     for batch in (64, 65, 100, 200):
+        out = nw.evaluate(pos["masks"][:batch], pos["values"][:batch])
+        for k in ("policy", "q", "d", "m"):
+            np.testing.assert_array_equal(out[k], whole[k][:batch])
+    nw.close()
+
+
+@pytest.mark.parametrize("precision", ["fp16", "bf16"])
+@pytest.mark.parametrize("name", ["cfg4_2layer", "cfg3", "cfg2_mini", "cfg4_mini"])
+def test_results_do_not_depend_on_the_batch_below_64_positions(name, precision):
+    """Bit for bit: K ranges are cut by plans that are the same for every such batch, and smolgen's second LayerNorm adds in one
+    order inside its product (few positions) and in its own launch (more)."""
+    net = mknet.make_net(name, **({"layers": 6} if name == "cfg4_2layer" else {}))
+    _, pos, n, g = load_compact("cfg4_2layer_b1024")
+    nw = network.Network(net, "precision=%s,max_batch=63" % precision)
+    whole = nw.evaluate(pos["masks"][:63], pos["values"][:63])
+    for batch in (1, 2, 3, 5, 6, 8, 9, 17, 31, 32, 48):
         out = nw.evaluate(pos["masks"][:batch], pos["values"][:batch])
         for k in ("policy", "q", "d", "m"):
             np.testing.assert_array_equal(out[k], whole[k][:batch])
@@ -454,7 +470,7 @@ def test_graph_replay_matches_plain_launches():
         got = nw.evaluate(pos["masks"][:n], pos["values"][:n])
         np.testing.assert_array_equal(got["policy"], want["policy"])
         np.testing.assert_array_equal(got["q"], want["q"])
-    # a different batch size gets its own graph (tiny batches route some products to the FMA kernel, hence atol)
+    # a different batch size gets its own graph
     for i in range(3):
         other = nw.evaluate(pos["masks"][:5], pos["values"][:5])
         np.testing.assert_allclose(other["policy"], want["policy"][:5], atol=HALF_ATOL)
