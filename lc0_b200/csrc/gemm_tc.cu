@@ -1180,10 +1180,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (even CTA only) ----------------
-    // Products of few k-blocks (four epilogue groups) keep the slower issue, a lane index and one commit per CTA: the 10 x 256
-    // attention network takes 1281 - 1290 us at 512 positions with it and 1316 us with the elected lane and the commit to both CTAs,
-    // presumably because MMAs that arrive in a burst hold up the epilogue warps that set the pace there.  With it, 256
-    // positions of the BT4-class network would take 5967 us instead of 5861, of the 20 x 256 residual network 1338 instead of 1252.
+    // With four epilogue groups the MMAs are issued the slower way, a lane index and one commit per CTA.  That is right for
+    // products of four k-blocks, whose tiles finish faster than the epilogue takes them: in place at 1024 positions, slower issue
+    // / elected lane and one commit for both CTAs, smolgen's projection (256 -> 4096) 107.5 / 129 us, the QKV product of the 10 x
+    // 256 attention network at 512 positions 34.3 / 36.4 us, that network 1290 / 1331 us.  (Why a burst of MMAs costs the epilogue that much
+    // was not found out.)  The form also takes the out-projection of the BT4-class network (16 k-blocks, residual and statistics), which
+    // would be faster the other way: 168 / 157 us at 1024 positions, 51.5 / 49.3 at 256.  With two groups the faster issue took 256
+    // positions of that network from 5967 to 5861 us and of the 20 x 256 residual network from 1338 to 1252.
     constexpr bool kFastIssue = kGroups != 4;
     auto commit = [](uint32_t bar) {
       if constexpr (kFastIssue) {
