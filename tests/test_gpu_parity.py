@@ -154,8 +154,8 @@ def test_fp16_at_the_measured_batch_sizes_against_reference(batch):
 @pytest.mark.parametrize("precision", ["fp16", "bf16"])
 @pytest.mark.parametrize("batch", [1, 2, 8, 9, 31, 65])
 def test_bt4_class_layers_at_small_batches_against_reference(batch, precision):
-    """The batches a search sends, in line: K cut over clusters (below 64 positions), smolgen's LayerNorms inside the products
-    that follow them (up to 64 positions, the second one up to 8), tiles of 64 rows and less."""
+    """The batches a search sends, in line: K cut over clusters and smolgen's LayerNorms inside the products that follow them
+    (below 64 positions, the second one up to 4, then in a launch that adds in the same order), tiles of 64 rows and less."""
     net, pos, n, g = load_compact("cfg4_2layer_b1024")
     idx = np.arange(batch)
     nw = network.Network(net, "precision=%s,max_batch=%d,side_stream=0" % (precision, batch))
