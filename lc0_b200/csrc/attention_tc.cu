@@ -43,6 +43,10 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // global-memory instruction: a version whose compute warps did their own loads and stores was limited by
 // instruction issue (its time followed the SM clock), not by HBM.
 // Every mbarrier wait is bounded; a wait that gives up raises the CTA's abort flag and the status word.
+// `zero0` and `zero1`, when given, are row statistics of the products that follow (two doubles per token), cleared ahead of
+// the first item.  As a memset of its own in every layer this cost a launch and the overlap of the launches around it
+// with their neighbours: one position of the BT4-class network 816 -> 761 us, 24 positions 1722 -> 1667.  (Cleared item by item, by
+// the CTA that has a position's first head, it slowed 4096 positions down by 2 %.)
 // ------------------------------------------------------------------------------------------------
 template <int D, int NS> struct AttnTma {
   static constexpr int kRow = D * 2;              // bytes per Q/K/V/O row = the swizzle span
@@ -57,7 +61,7 @@ __global__ void __launch_bounds__(160, D == 32 ? 4 : 2)
 attention_tma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_b,
                      const __grid_constant__ CUtensorMap map_o, int items, int heads, int has_bias, float scale,
-                     int* status) {
+                     double2* zero0, double2* zero1, int* status) {
   using L = AttnTma<D, NS>;
   extern __shared__ uint8_t sm_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sm_raw) + 1023) & ~uintptr_t(1023));
@@ -104,6 +108,13 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     }
   } else {
     // ---------------- compute: warp w owns query rows 16 w .. 16 w + 15 ----------------
+    if (zero0) {
+      const int rows = items / heads * 64;
+      for (int r = blockIdx.x * 128 + tid; r < rows; r += gridDim.x * 128) {
+        zero0[r] = make_double2(0.0, 0.0);
+        zero1[r] = make_double2(0.0, 0.0);
+      }
+    }
     const int m0 = warp * 16;
     const int g = lane >> 2, t = lane & 3;
     // Per-lane offsets of the ldmatrix rows in a swizzled tile (the same for every item).  Moving 16 rows down adds
@@ -362,8 +373,8 @@ bool attention_tc_supported(long long ld, long long ldo, int depth, const void* 
 
 template <typename T, int D, int NS>
 static cudaError_t launch_attention_tma_cfg(const T* q, const T* k, const T* v, long long ld, const T* bias, T* out,
-                                            long long ldo, int n, int heads, float scale, int* status, int sm_count,
-                                            int ctas_per_sm, cudaStream_t s) {
+                                            long long ldo, int n, int heads, float scale, double* zero0, double* zero1,
+                                            int* status, int sm_count, int ctas_per_sm, cudaStream_t s) {
   using L = AttnTma<D, NS>;
   static bool attr_done[64] = {};
   int dev = 0;
@@ -387,29 +398,30 @@ static cudaError_t launch_attention_tma_cfg(const T* q, const T* k, const T* v, 
   const int max_ctas = sm_count * ctas_per_sm;
   const int grid = items < max_ctas ? items : max_ctas;
   return launch_dependent(attention_tma_kernel<T, D, NS>, dim3(grid), dim3(L::kThreads), L::kBytes, s, mq, mk, mv, mb, mo,
-                          items, heads, bias ? 1 : 0, scale, status);
+                          items, heads, bias ? 1 : 0, scale, reinterpret_cast<double2*>(zero0),
+                          reinterpret_cast<double2*>(zero1), status);
 }
 
 template <typename T>
 cudaError_t launch_attention_tma(const T* q, const T* k, const T* v, long long ld, const T* bias, T* out,
-                                 long long ldo, int n, int heads, int depth, float scale, int* status, int sm_count,
-                                 cudaStream_t s) {
+                                 long long ldo, int n, int heads, int depth, float scale, double* zero0, double* zero1,
+                                 int* status, int sm_count, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   // depth 32: two 20 KB stages and four CTAs per SM (sixteen compute warps) measured best: with three or two CTAs
   // the kernel waits on its compute warps, more stages per CTA buy nothing.
-  if (depth == 32) return launch_attention_tma_cfg<T, 32, 2>(q, k, v, ld, bias, out, ldo, n, heads, scale, status,
-                                                             sm_count, 4, s);
-  if (depth == 64) return launch_attention_tma_cfg<T, 64, 2>(q, k, v, ld, bias, out, ldo, n, heads, scale, status,
-                                                             sm_count, 2, s);
+  if (depth == 32) return launch_attention_tma_cfg<T, 32, 2>(q, k, v, ld, bias, out, ldo, n, heads, scale, zero0, zero1,
+                                                             status, sm_count, 4, s);
+  if (depth == 64) return launch_attention_tma_cfg<T, 64, 2>(q, k, v, ld, bias, out, ldo, n, heads, scale, zero0, zero1,
+                                                             status, sm_count, 2, s);
   return cudaErrorInvalidValue;
 }
 template cudaError_t launch_attention_tma<__half>(const __half*, const __half*, const __half*, long long,
-                                                  const __half*, __half*, long long, int, int, int, float, int*, int,
-                                                  cudaStream_t);
+                                                  const __half*, __half*, long long, int, int, int, float, double*,
+                                                  double*, int*, int, cudaStream_t);
 template cudaError_t launch_attention_tma<__nv_bfloat16>(const __nv_bfloat16*, const __nv_bfloat16*,
                                                          const __nv_bfloat16*, long long, const __nv_bfloat16*,
-                                                         __nv_bfloat16*, long long, int, int, int, float, int*, int,
-                                                         cudaStream_t);
+                                                         __nv_bfloat16*, long long, int, int, int, float, double*,
+                                                         double*, int*, int, cudaStream_t);
 
 }  // namespace b200
 

@@ -44,13 +44,22 @@ cudaError_t launch_expand_planes(const uint64_t* masks, const float* values, int
 // preprocess_for_attention_body_kernel, backends/cuda/common_kernels.cu:1203-1244).
 template <typename T> struct __align__(16) Vec8 { T v[8]; };
 
+// Clears what later launches add to or leave out: a position's row statistics (two doubles per token) and its q, d, m.
+__device__ __forceinline__ void clear_position(int n, double2* stats, float* qdm) {
+  if (stats && threadIdx.x < 64) stats[(long long)n * 64 + threadIdx.x] = make_double2(0.0, 0.0);
+  if (qdm && threadIdx.x < 3) qdm[(long long)n * 3 + threadIdx.x] = 0.f;
+}
+
 template <typename T>
 __global__ void expand_tokens_kernel(const uint64_t* __restrict__ masks, const float* __restrict__ values,
                                      const float* __restrict__ pe_static, const T* __restrict__ pe_dense,
-                                     int pe_ch, int cin, T* __restrict__ out) {
+                                     int pe_ch, int cin, T* __restrict__ out, double2* stats, float* qdm) {
   __shared__ uint64_t sm[112];
   __shared__ float sv[112];
   const int n = blockIdx.x;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  clear_position(n, stats, qdm);
   for (int i = threadIdx.x; i < 112; i += blockDim.x) {
     sm[i] = masks[(long long)n * 112 + i];
     sv[i] = values[(long long)n * 112 + i];
@@ -77,10 +86,13 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 expand_tokens_vec_kernel(const uint64_t* __restrict__ masks, const float* __restrict__ values,
                          const float* __restrict__ pe_static, const T* __restrict__ pe_dense, int pe_ch, int cin,
-                         T* __restrict__ out) {
+                         T* __restrict__ out, double2* stats, float* qdm) {
   __shared__ uint64_t sm[112];
   __shared__ float sv[112];
   const int n = blockIdx.x;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  if (blockIdx.y == 0) clear_position(n, stats, qdm);
   for (int i = threadIdx.x; i < 112; i += blockDim.x) {
     sm[i] = masks[(long long)n * 112 + i];
     sv[i] = values[(long long)n * 112 + i];
@@ -112,16 +124,16 @@ expand_tokens_vec_kernel(const uint64_t* __restrict__ masks, const float* __rest
 
 template <typename T>
 cudaError_t launch_expand_tokens(const uint64_t* masks, const float* values, int n, const float* pe_static,
-                                 const T* pe_dense, int pe_ch, int cin, T* out, cudaStream_t s) {
+                                 const T* pe_dense, int pe_ch, int cin, T* out, double* stats, float* qdm, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
+  double2* st2 = reinterpret_cast<double2*>(stats);
   const bool aligned = (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (reinterpret_cast<uintptr_t>(pe_dense) & 15) == 0;
   if ((cin & 7) == 0 && (pe_ch & 7) == 0 && aligned)
     // Few positions: eight (four) CTAs to a position, 8 (16) squares each; one CTA took 16 us for one position's 80 KB.
-    expand_tokens_vec_kernel<T><<<dim3(n, n <= 148 ? 8 : n <= 592 ? 4 : 1), 256, 0, s>>>(masks, values, pe_static, pe_dense,
-                                                                                        pe_ch, cin, out);
-  else
-    expand_tokens_kernel<T><<<n, 256, 0, s>>>(masks, values, pe_static, pe_dense, pe_ch, cin, out);
-  return cudaGetLastError();
+    return launch_dependent(expand_tokens_vec_kernel<T>, dim3(n, n <= 148 ? 8 : n <= 592 ? 4 : 1), dim3(256), 0, s, masks, values,
+                            pe_static, pe_dense, pe_ch, cin, out, st2, qdm);
+  return launch_dependent(expand_tokens_kernel<T>, dim3(n), dim3(256), 0, s, masks, values, pe_static, pe_dense, pe_ch, cin, out,
+                          st2, qdm);
 }
 
 // First 12 planes, square-major (reference: network_blas.cc:613-621).
@@ -536,6 +548,8 @@ policy_attn_gather_kernel(const float* __restrict__ logits, const T* __restrict_
   __shared__ float off[4][8];
   const int n = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  grid_dependency_wait();
+  grid_launch_dependents();
   // 32 dot products (4 promotion rows x 8 files), 4 per warp with one row of w4 between them; eight steps of loads in flight
   {
     const int i = warp >> 1, j0 = (warp & 1) * 4;
@@ -573,13 +587,14 @@ template <typename T>
 cudaError_t launch_policy_attn_gather(const float* logits, const T* kp, const float* w4, int dm,
                                       const short* src_slot, int n, float* policy, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  policy_attn_gather_kernel<T><<<n, 256, 0, s>>>(logits, kp, w4, dm, src_slot, policy);
-  return cudaGetLastError();
+  return launch_dependent(policy_attn_gather_kernel<T>, dim3(n), dim3(256), 0, s, logits, kp, w4, dm, src_slot, policy);
 }
 
 template <typename T>
 __global__ void policy_gather_kernel(const T* __restrict__ raw, long long ld, const short* __restrict__ src,
                                      float* __restrict__ policy) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int n = blockIdx.x;
   for (int j = threadIdx.x; j < 1858; j += blockDim.x)
     policy[(long long)n * 1858 + j] = to_f(raw[(long long)n * ld + src[j]]);
@@ -589,8 +604,7 @@ template <typename T>
 cudaError_t launch_policy_gather(const T* raw, long long ld, const short* src_slot, int n, float* policy,
                                  cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  policy_gather_kernel<T><<<n, 256, 0, s>>>(raw, ld, src_slot, policy);
-  return cudaGetLastError();
+  return launch_dependent(policy_gather_kernel<T>, dim3(n), dim3(256), 0, s, raw, ld, src_slot, policy);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -600,6 +614,8 @@ cudaError_t launch_policy_gather(const T* raw, long long ld, const short* src_sl
 template <typename T>
 __global__ void head_final_kernel(const T* __restrict__ h, int k, const float* __restrict__ w,
                                   const float* __restrict__ b, int mode, int n, float* __restrict__ qdm) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int sample = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (sample >= n) return;
@@ -631,8 +647,7 @@ template <typename T>
 cudaError_t launch_head_final(const T* h, int k, const float* w, const float* b, int mode, int n, float* qdm,
                               cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  head_final_kernel<T><<<ceil_div(n, 4), 128, 0, s>>>(h, k, w, b, mode, n, qdm);
-  return cudaGetLastError();
+  return launch_dependent(head_final_kernel<T>, dim3(ceil_div(n, 4)), dim3(128), 0, s, h, k, w, b, mode, n, qdm);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -823,6 +838,8 @@ __global__ void __launch_bounds__(128)
 legal_softmax_kernel(const float* __restrict__ policy, const unsigned short* __restrict__ move_ids,
                      const int* __restrict__ n_moves, int n, float inv_t, float* __restrict__ probs) {
   __shared__ float vals[4][kLegalStride];
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sample = blockIdx.x * 4 + w;
   if (sample >= n) return;
@@ -853,14 +870,14 @@ legal_softmax_kernel(const float* __restrict__ policy, const unsigned short* __r
 cudaError_t launch_legal_softmax(const float* policy, const unsigned short* move_ids, const int* n_moves, int n,
                                  float inv_temperature, float* probs, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  legal_softmax_kernel<<<ceil_div(n, 4), 128, 0, s>>>(policy, move_ids, n_moves, n, inv_temperature, probs);
-  return cudaGetLastError();
+  return launch_dependent(legal_softmax_kernel, dim3(ceil_div(n, 4)), dim3(128), 0, s, policy, move_ids, n_moves, n,
+                          inv_temperature, probs);
 }
 
 #define INSTANTIATE(T)                                                                                        \
   template cudaError_t launch_expand_planes<T>(const uint64_t*, const float*, int, T*, cudaStream_t);         \
   template cudaError_t launch_expand_tokens<T>(const uint64_t*, const float*, int, const float*, const T*,    \
-                                               int, int, T*, cudaStream_t);                                   \
+                                               int, int, T*, double*, float*, cudaStream_t);                  \
   template cudaError_t launch_expand_pre12<T>(const uint64_t*, const float*, int, T*, cudaStream_t);          \
   template cudaError_t launch_layer_norm<T>(T*, const T*, const T*, const float*, const float*, const float*, \
                                             const float*, int, int, float, float, cudaStream_t);              \

@@ -110,10 +110,11 @@ cudaError_t tma_encode_2d(const void* ptr, long long ld, long long rows, int col
 template <typename T>
 cudaError_t launch_expand_planes(const uint64_t* masks, const float* values, int n, T* out, cudaStream_t s);
 // tokens[n*64][cin]: columns 0..111 expanded planes (NHWC), columns 112.. positional encoding taken
-// from pe_static [64][pe_ch] (fp32 table) or pe_dense [n][64][pe_ch] (T), zero padded to cin.
+// from pe_static [64][pe_ch] (fp32 table) or pe_dense [n][64][pe_ch] (T), zero padded to cin.  Clears stats [n*64][2] and
+// qdm [n][3] when given.
 template <typename T>
 cudaError_t launch_expand_tokens(const uint64_t* masks, const float* values, int n, const float* pe_static,
-                                 const T* pe_dense, int pe_ch, int cin, T* out, cudaStream_t s);
+                                 const T* pe_dense, int pe_ch, int cin, T* out, double* stats, float* qdm, cudaStream_t s);
 // pre[n][64*12]: first 12 planes, square-major (input of the PE_DENSE preprocessing layer).
 template <typename T>
 cudaError_t launch_expand_pre12(const uint64_t* masks, const float* values, int n, T* out, cudaStream_t s);
@@ -137,11 +138,11 @@ cudaError_t launch_attention(const T* q, const T* k, const T* v, long long ld, c
 bool attention_tc_supported(long long ld, long long ldo, int depth, const void* q, const void* k, const void* v,
                             const void* bias, const void* out);
 // Persistent kernel: TMA loads into a ring of swizzled shared-memory stages, TMA stores of the result; `status`
-// receives 300 + code if a bounded device-side wait gives up.
+// receives 300 + code if a bounded device-side wait gives up.  zero0 and zero1 (both or neither; [n*64][2]) are cleared.
 template <typename T>
 cudaError_t launch_attention_tma(const T* q, const T* k, const T* v, long long ld, const T* bias, T* out,
-                                 long long ldo, int n, int heads, int depth, float scale, int* status, int sm_count,
-                                 cudaStream_t s);
+                                 long long ldo, int n, int heads, int depth, float scale, double* zero0, double* zero1,
+                                 int* status, int sm_count, cudaStream_t s);
 
 // Attention policy: promotion logits + gather to 1858 (network_blas.cc:873-914).
 // logits: fp32 [n][64*64] (already scaled), kp: [n*64][dm] keys, w4: fp32 [4][dm].

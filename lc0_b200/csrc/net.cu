@@ -490,11 +490,9 @@ struct Net : NetBase {
     T *x = nullptr, *x1 = nullptr, *y = nullptr, *qkv = nullptr, *att = nullptr, *ffn = nullptr;
     T *sg_c = nullptr, *sg_h1 = nullptr, *sg_h2 = nullptr, *sg_bias = nullptr;
     T *wino_v = nullptr, *wino_m = nullptr;  // [36][rows_padded][channels]: transformed input / product output
-    // per-row (sum, sum of squares; double) of the folded LayerNorm inputs, laid out [stats2[0] | stats1 | stats2[1]] so that
-    // one memset at the start of a layer clears stats1 and the stats2 buffer that layer writes (layers alternate)
+    // per-row (sum, sum of squares; double) of the folded LayerNorm inputs; layers alternate between the stats2 buffers
     double *stats1 = nullptr, *stats2[2] = {nullptr, nullptr};
     int stats_parity = 0;
-    size_t stats_stride = 0;  // floats between consecutive buffers of that block
     T *pemb = nullptr, *pq = nullptr, *pk = nullptr, *praw = nullptr;
     T *p_qkv = nullptr, *p_att = nullptr, *p_ffn = nullptr, *p_x1 = nullptr, *p_y = nullptr;  // policy-head encoders
     float* logits = nullptr;
@@ -1085,7 +1083,6 @@ struct Net : NetBase {
           s.stats2[0] = blk;
           s.stats1 = blk + R * 2;
           s.stats2[1] = blk + 2 * R * 2;
-          s.stats_stride = (size_t)R * 2;
         }
         s.att = A(R * E);
         s.ffn = A(R * std::max(max_dff, 8));
@@ -1150,7 +1147,7 @@ struct Net : NetBase {
   // alpha * act(...) + LN(res) and optional accumulation of output row statistics.
   void gemm_ln(cudaStream_t st, const LNState& in, long long lda, const Dense<T>& d, T* Cout, long long ldc, int M,
                int act, const LNState* res = nullptr, float alpha_ = 1.f, double* out_stats = nullptr,
-               T* C2 = nullptr, long long ldc2 = 0, int n_split = 0, bool zero_stats = true) {
+               T* C2 = nullptr, long long ldc2 = 0, int n_split = 0) {
     GemmParams p;
     p.C2 = C2; p.ldc2 = ldc2; p.n_split = n_split;
     p.A = in.u; p.lda = lda; p.W = d.w; p.ldw = d.in; p.w_const = true; p.bias = d.b;
@@ -1166,10 +1163,7 @@ struct Net : NetBase {
         p.res_inv_c = 1.0f / d.out; p.res_eps = ln_eps;
       }
     }
-    if (out_stats) {
-      if (zero_stats) CK(cudaMemsetAsync(out_stats, 0, (size_t)M * 2 * sizeof(double), st));
-      p.out_stats = out_stats;
-    }
+    p.out_stats = out_stats;  // cleared by a launch before this one
     p.whole_tiles = (opt.flags & B200_FLAG_NO_SPLIT_LAST_WAVE) != 0;
     p.split_k = M == t_cut_rows;
     run_gemm(st, p);
@@ -1350,7 +1344,9 @@ struct Net : NetBase {
   }
 
   // softmax(Q K^T / sqrt(depth) + bias) V for every (position, head); q, k, v are consecutive column blocks of `qkv`
-  void run_attention(cudaStream_t st, const T* qkv, int ld, const T* bias, T* out, int width, int n, int heads) {
+  // and, when given, the row statistics zero0 and zero1 cleared for the products that follow.
+  void run_attention(cudaStream_t st, const T* qkv, int ld, const T* bias, T* out, int width, int n, int heads,
+                     double* zero0 = nullptr, double* zero1 = nullptr) {
     const int depth = width / heads;
     const float scale = 1.0f / sqrtf((float)depth);
     launches++;
@@ -1361,9 +1357,13 @@ struct Net : NetBase {
     if constexpr (sizeof(T) == 2) {
       if (use_tc && attention_tc_supported(ld, width, depth, qkv, qkv + width, qkv + 2 * width, bias, out)) {
         CK(launch_attention_tma<T>(qkv, qkv + width, qkv + 2 * width, ld, bias, out, width, n, heads, depth, scale,
-                                   t_status, sm_count, st));
+                                   zero0, zero1, t_status, sm_count, st));
         done = true;
       }
+    }
+    if (!done && zero0) {
+      CK(cudaMemsetAsync(zero0, 0, (size_t)n * 64 * 2 * sizeof(double), st));
+      CK(cudaMemsetAsync(zero1, 0, (size_t)n * 64 * 2 * sizeof(double), st));
     }
     if (!done) CK(launch_attention<T>(qkv, qkv + width, qkv + 2 * width, ld, bias, out, width, n, heads, depth, scale, st));
     span_end(st, sp_);
@@ -1391,14 +1391,13 @@ struct Net : NetBase {
     const int R = n * 64;
     const int depth = E / H;
     const T* bias = nullptr;
-    // The statistics this layer accumulates are cleared here, in one memset ahead of all its launches, so that no
-    // memset sits between two products.  The layer input may refer to the other stats2 buffer.
-    double* stats2 = nullptr;
+    // The statistics this layer accumulates are cleared by its attention launch.  The layer input may refer to the other
+    // stats2 buffer.
+    double *stats1 = nullptr, *stats2 = nullptr;
     if (fold_ln) {
-      const int par = s.stats_parity;
+      stats1 = s.stats1;
+      stats2 = s.stats2[s.stats_parity];
       s.stats_parity ^= 1;
-      stats2 = s.stats2[par];
-      CK(cudaMemsetAsync(par == 0 ? s.stats2[0] : s.stats1, 0, (s.stats_stride + (size_t)R * 2) * sizeof(double), st));
     }
     // With per-launch event pairs on (profiling) the layer runs in line: a span around a launch that shares the GPU
     // with another stream measures the sharing, not the kernel.
@@ -1433,7 +1432,7 @@ struct Net : NetBase {
         gemm(st, s.sg_h2, sg_gen / H, smolgen_w, s.sg_bias, 4096, n * H, ACT_NONE);
       }
       bias = s.sg_bias;
-      run_attention(st, s.qkv, 3 * E, bias, s.att, E, n, H);
+      run_attention(st, s.qkv, 3 * E, bias, s.att, E, n, H, stats1, stats2);
       finish_layer(s, e, R, x, x1, in, stats2);
       return;
     }
@@ -1470,7 +1469,7 @@ struct Net : NetBase {
       }
       bias = s.sg_bias;
     }
-    run_attention(st, s.qkv, 3 * E, bias, s.att, E, n, H);  // :352-439
+    run_attention(st, s.qkv, 3 * E, bias, s.att, E, n, H, stats1, stats2);  // :352-439
     finish_layer(s, e, R, x, x1, in, stats2);
   }
   // Output projection, first LayerNorm, FFN, second LayerNorm of an encoder layer (network_blas.cc:441-470).
@@ -1479,12 +1478,12 @@ struct Net : NetBase {
     if (fold_ln) {
       LNState att{s.att, nullptr, nullptr, nullptr}, ffn{s.ffn, nullptr, nullptr, nullptr};
       t_tag = TAG_OUT_PROJ;
-      gemm_ln(st, att, E, e.proj, x1, E, R, ACT_NONE, &in, alpha, s.stats1, nullptr, 0, 0, false);  // u1 = alpha * proj + x
+      gemm_ln(st, att, E, e.proj, x1, E, R, ACT_NONE, &in, alpha, s.stats1);  // u1 = alpha * proj + x
       LNState mid{x1, s.stats1, e.ln1g, e.ln1b};
       t_tag = TAG_FFN1;
       gemm_ln(st, mid, E, e.ffn1, s.ffn, e.ffn1.out, R, act_ffn);                  // relu2(LN1(u1) W1 + b1)
       t_tag = TAG_FFN2;
-      gemm_ln(st, ffn, e.ffn1.out, e.ffn2, x, E, R, ACT_NONE, &mid, alpha, stats2, nullptr, 0, 0, false);  // u2 = alpha * ffn + LN1(u1)
+      gemm_ln(st, ffn, e.ffn1.out, e.ffn2, x, E, R, ACT_NONE, &mid, alpha, stats2);  // u2 = alpha * ffn + LN1(u1)
       t_tag = TAG_NONE;
       in = LNState{x, stats2, e.ln2g, e.ln2b};
       return;
@@ -1501,7 +1500,9 @@ struct Net : NetBase {
     in = LNState{x, nullptr, nullptr, nullptr};
   }
 
-  void forward(Slot& s, const uint64_t* d_masks, const float* d_values, int n, float* d_policy, float* d_qdm) {
+  // policy_mode != 0: followed by the softmax over the slot's legal moves.
+  void forward(Slot& s, const uint64_t* d_masks, const float* d_values, int n, float* d_policy, float* d_qdm, int policy_mode = 0,
+               float inv_t = 1.f) {
     cudaStream_t st = s.stream;
     const int R = n * 64;
     T* flow = nullptr;  // output of the body, [R][body_ch]
@@ -1513,10 +1514,11 @@ struct Net : NetBase {
     t_cut_rows = n < kCutPositions ? n : 0;
     // not with per-launch event pairs: the spans would then time the overlap with the neighbours
     DependentLaunchScope launch_scope(dependent_launch && !profiling);
-    CK(cudaMemsetAsync(d_qdm, 0, (size_t)n * 3 * sizeof(float), st));
+    // The first launch is an ordinary one: what is ahead of it in the stream may be a copy or an event.
     if (!res.empty() || !attn_body) {  // network_blas.cc:564-601
       other(st, (double)R * 112 * sizeof(T), [&] {
-        return launch_expand_tokens<T>(d_masks, d_values, n, nullptr, (const T*)nullptr, 0, 112, s.tokens, st);
+        DependentLaunchScope first(false);
+        return launch_expand_tokens<T>(d_masks, d_values, n, nullptr, (const T*)nullptr, 0, 112, s.tokens, nullptr, d_qdm, st);
       });
       T *cur = s.x, *tmp = s.x1, *tmp2 = s.y;
       bool in_one = false;
@@ -1561,11 +1563,12 @@ struct Net : NetBase {
         other(st, (double)n * 768 * sizeof(T), [&] { return launch_expand_pre12<T>(d_masks, d_values, n, s.pre, st); });
         gemm(st, s.pre, 768, emb_pre, s.pe, 64 * pe_ch, n, ACT_NONE);
         other(st, (double)R * (cin + pe_ch) * sizeof(T), [&] {
-          return launch_expand_tokens<T>(d_masks, d_values, n, nullptr, s.pe, pe_ch, cin, s.tokens, st);
+          return launch_expand_tokens<T>(d_masks, d_values, n, nullptr, s.pe, pe_ch, cin, s.tokens, s.stats2[1], d_qdm, st);
         });
       } else {
         other(st, (double)R * cin * sizeof(T), [&] {
-          return launch_expand_tokens<T>(d_masks, d_values, n, pos_enc, (const T*)nullptr, pe_ch, cin, s.tokens, st);
+          DependentLaunchScope first(false);
+          return launch_expand_tokens<T>(d_masks, d_values, n, pos_enc, (const T*)nullptr, pe_ch, cin, s.tokens, nullptr, d_qdm, st);
         });
       }
       T *x = s.x, *x1 = s.x1;
@@ -1668,6 +1671,11 @@ struct Net : NetBase {
       gemm(st, flow, C, pol_c1x1, s.praw, pol_planes, R, act_default);
       gemm(st, s.praw, 64 * pol_planes, pol_fc, nullptr, 1858, n, ACT_NONE, nullptr, 0, 1.f, true, d_policy);
     }
+    if (policy_mode) {
+      other(st, (double)n * kLegalStride * 6, [&] {
+        return launch_legal_softmax(d_policy, s.d_move_ids, s.d_n_moves, n, inv_t, s.d_probs, st);
+      });
+    }
     if (heads_beside) {
       CK(cudaEventRecord(s.ev_join, hs));
       CK(cudaStreamWaitEvent(st, s.ev_join, 0));
@@ -1716,12 +1724,7 @@ struct Net : NetBase {
     const bool capturing = cap == cudaStreamCaptureStatusActive;
     for (auto& o : slots)
       if (&o != &s) CK(cudaStreamWaitEvent(s.stream, o.compute_done, capturing ? cudaEventWaitExternal : 0));
-    forward(s, s.d_masks, s.d_values, n, s.d_policy, s.d_qdm);
-    if (policy_mode) {
-      other(s.stream, (double)n * kLegalStride * 6, [&] {
-        return launch_legal_softmax(s.d_policy, s.d_move_ids, s.d_n_moves, n, inv_t, s.d_probs, s.stream);
-      });
-    }
+    forward(s, s.d_masks, s.d_values, n, s.d_policy, s.d_qdm, policy_mode, inv_t);
     CK(cudaEventRecordWithFlags(s.compute_done, s.stream, capturing ? cudaEventRecordExternal : 0));
     if (policy_mode) {
       CK(cudaMemcpyAsync(hs.probs, s.d_probs, (size_t)n * kLegalStride * 4, cudaMemcpyDeviceToHost, s.stream));
@@ -2582,7 +2585,7 @@ int b200_op_attention(const void* q, const void* k, const void* v, long long ld,
       B200_CUDA(cudaMalloc(&status, sizeof(int)));
       B200_CUDA(cudaMemset(status, 0, sizeof(int)));
       cudaError_t err = launch_attention_tma<T>((const T*)q, (const T*)k, (const T*)v, ld, (const T*)bias, (T*)out,
-                                                ldo, n, heads, depth, scale, status, sms, st);
+                                                ldo, n, heads, depth, scale, nullptr, nullptr, status, sms, st);
       if (err == cudaSuccess) err = cudaStreamSynchronize(st);
       int code = 0;
       if (err == cudaSuccess) err = cudaMemcpy(&code, status, sizeof(int), cudaMemcpyDeviceToHost);
