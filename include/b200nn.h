@@ -345,6 +345,14 @@ int b200_op_attention(const void* q, const void* k, const void* v, long long ld,
  *   fp16 / bf16 only; synchronises the stream before returning. */
 int b200_op_gemm_ln(const void* x, const float* gamma, const float* beta, int group, float eps, const void* W,
                     const float* bias, void* C, int M, int N, int activation, int precision, void* stream);
+/* b200_op_gemm_f32: C[M][N] = alpha * act(A[M][K] . W[N][K]^T + bias) + skip[M][N] in fp32 on tensor cores, as the network's
+ *   fp32 mode runs its layers with 32 and more rows per position (Forward1D, fully_connected_layer.cc:50-106): operands cut
+ *   into three bf16 pieces, no fewer digits than the FMA kernel.  conv != 0: 3x3 convolution over 8x8 boards, A [M][K] with M a
+ *   multiple of 64, W [9][N][K] (winograd_convolution3.cc:47-57).  Leading dimension of A: lda; bias and skip may be NULL.  K a
+ *   multiple of 8, lda of 4, A on a 16-byte boundary.  A row's sum does not depend on the number of rows.  Allocates and frees the
+ *   weights' pieces and synchronises the stream before returning. */
+int b200_op_gemm_f32(const float* A, long long lda, const float* W, const float* bias, const float* skip, float* C, int M, int N,
+                     int K, int conv, int activation, float alpha, void* stream);
 /* b200_op_gemm_timed: the tensor-core product of b200_op_gemm queued `launches` times back to back on `stream`
  *   between two CUDA events; *ms_per_launch = elapsed / launches.  With enough launches the host's launch latency
  *   drops out, which is what a launch costs inside a replayed graph (profiling surface only). */

@@ -127,6 +127,7 @@ SIGNATURES = {
     "b200_op_scratch_residency_probe": (_I, [_I, _I, _I, _I, ctypes.POINTER(ctypes.c_float)]),
     "b200_op_gemm_ex": (_I, [ctypes.POINTER(GemmDesc), _P]),
     "b200_op_gemm_ln": (_I, [_P, _P, _P, _I, _F, _P, _P, _P, _I, _I, _I, _I, _P]),
+    "b200_op_gemm_f32": (_I, [_P, ctypes.c_longlong, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _P]),
     "b200_op_attention": (_I, [_P, _P, _P, ctypes.c_longlong, _P, _P, ctypes.c_longlong, _I, _I, _I, _I, _I, _P]),
     "b200_op_gemm_timed": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, ctypes.POINTER(ctypes.c_float), _P]),
     "b200_op_policy_attention": (_I, [_P, _P, _P, _I, _I, _P, _P, _I, _P]),

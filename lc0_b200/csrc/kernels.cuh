@@ -11,6 +11,7 @@ struct GemmParams {
   // epilogue(v): v += bias[n]; v = act(v); if (skip) v = alpha * v + skip[m][n]
   const void* A = nullptr; long long lda = 0, strideA = 0;
   const void* W = nullptr; long long ldw = 0, strideW = 0;
+  const void* W3 = nullptr;  // fp32: the three bf16 pieces of W (launch_split_weights), for launch_gemm_f32
   const float* bias = nullptr;
   void* C = nullptr; long long ldc = 0, strideC = 0;
   const void* skip = nullptr; long long ldskip = 0;
@@ -106,6 +107,11 @@ cudaError_t gemm_tc_init();  // resolves the driver entry point used to encode T
 // prec: 1 = fp16, 2 = bf16.  Needs gemm_tc_init().
 cudaError_t tma_encode_2d(const void* ptr, long long ld, long long rows, int cols, int box_cols, int box_rows,
                           int swizzle_bytes, int prec, void* out);
+
+// fp32 products and 3x3 convolutions on tensor cores (gemm_f32.cu), with W cut into pieces [3][...] ahead of time.
+cudaError_t launch_split_weights(const float* w, long long count, void* planes, cudaStream_t s);
+bool gemm_f32_supported(const GemmParams& p);
+cudaError_t launch_gemm_f32(const GemmParams& p, int* status, int sm_count, cudaStream_t s);
 
 template <typename T>
 cudaError_t launch_expand_planes(const uint64_t* masks, const float* values, int n, T* out, cudaStream_t s);

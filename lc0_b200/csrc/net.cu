@@ -167,6 +167,7 @@ template <typename T> struct Dense {
   // Set when the LayerNorm that feeds this layer is folded into it: w holds W * gamma (per input column),
   // b holds b + beta . W^T, and colsum[n] = sum_k (W * gamma)[n][k] of the stored (rounded) weights.
   float* colsum = nullptr;
+  void* w3 = nullptr;    // fp32: w in three bf16 pieces for the tensor-core kernel, or nullptr
 };
 
 template <typename T> struct EncoderW {
@@ -180,6 +181,7 @@ template <typename T> struct EncoderW {
 
 template <typename T> struct ConvW {
   T* w = nullptr;  // [9][Cout][Cin]
+  void* w3 = nullptr;  // fp32: w in three bf16 pieces for the tensor-core kernel, or nullptr
   T* u = nullptr;  // [36][Cout][Cin]: Winograd-transformed filters (only with the winograd option)
   float* b = nullptr;
   int cout = 0, cin = 0;
@@ -401,6 +403,7 @@ struct Net : NetBase {
   DeviceAllocs walloc, salloc;
   int sm_count = 148;
   bool use_tc = false;
+  bool f32_tc = false;  // fp32 storage: layers with 32 and more rows per position on tensor cores (gemm_f32.cu)
   // LayerNorms of the encoder stack folded into the neighbouring tensor-core products (16-bit storage only).
   bool fold_ln = false;
   bool fold_emb_ln = false;  // the embedding block's last LayerNorm is folded into the first encoder layer
@@ -548,6 +551,18 @@ struct Net : NetBase {
     CK(cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
     return d;
   }
+  // The pieces of a layer's weights, on the device, for layers with 32 and more rows per position.  The rule looks at the layer alone, so
+  // that a position's sums are the same in every batch.
+  void* pieces(const T* w, size_t count, int in) {
+    if constexpr (sizeof(T) == 4) {
+      if (!f32_tc || in % 8) return nullptr;
+      void* w3 = walloc.alloc(count * 6);
+      CK(launch_split_weights(w, (long long)count, w3, nullptr));
+      return w3;
+    }
+    return nullptr;
+  }
+  void token_wise(Dense<T>& d) { d.w3 = pieces(d.w, (size_t)d.out * d.in, d.in); }
   Dense<T> dense(const std::string& wname, const std::string& bname, int out, int in) {
     Dense<T> d;
     d.out = out;
@@ -621,6 +636,7 @@ struct Net : NetBase {
       cw.u = up_T(u);
     }
     cw.b = up_f32(prefix + ".biases", cout);
+    cw.w3 = pieces(cw.w, p.size(), cin_);
     return cw;
   }
   Dense<T> conv1(const std::string& prefix, int cout, int cin_) {
@@ -762,6 +778,8 @@ struct Net : NetBase {
     CK(cudaGetDeviceProperties(&prop, opt.gpu));
     sm_count = prop.multiProcessorCount;
     use_tc = sizeof(T) == 2 && !(opt.flags & B200_FLAG_NO_TENSOR_CORES);
+    f32_tc = sizeof(T) == 4 && !(opt.flags & B200_FLAG_NO_TENSOR_CORES) && prop.major == 10;
+    if (f32_tc) CK(gemm_tc_init());
     if (use_tc) {
       if (prop.major != 10)
         throw Fail{B200_ERR_UNSUPPORTED, "the tensor-core path needs an sm_100 device, found sm_" +
@@ -1001,6 +1019,15 @@ struct Net : NetBase {
       add_flops(1, mov_fc1);
     }
 
+    for (auto& e : enc)
+      for (Dense<T>* d : {&e.qkv, &e.proj, &e.ffn1, &e.ffn2, &e.sg_compress})
+        if (d->w) token_wise(*d);
+    for (auto& e : pol_enc)
+      for (Dense<T>* d : {&e.qkv, &e.proj, &e.ffn1, &e.ffn2}) token_wise(*d);
+    for (Dense<T>* d : {&emb, &emb_ffn1, &emb_ffn2, &pol_emb, &pol_q, &pol_k, &pol_c1x1, &val_emb, &mov_emb})
+      if (d->w) token_wise(*d);
+    // smolgen's generator sees one row per head; below 32 of them the FMA kernel has the smaller tiles
+    if (smolgen_w.w && H >= 32) token_wise(smolgen_w);
     alloc_slots();
     build_towers();
     // The uploads above are copies from pageable memory and the slots' streams are non-blocking: everything must have
@@ -1128,7 +1155,7 @@ struct Net : NetBase {
             const T* skip = nullptr, long long ldskip = 0, float alpha_ = 1.f, bool out_f32 = false,
             void* cf32 = nullptr) {
     GemmParams p;
-    p.A = A; p.lda = lda; p.W = d.w; p.ldw = d.in; p.w_const = true; p.bias = d.b;
+    p.A = A; p.lda = lda; p.W = d.w; p.W3 = d.w3; p.ldw = d.in; p.w_const = true; p.bias = d.b;
     p.C = out_f32 ? cf32 : (void*)Cout; p.ldc = ldc; p.M = M; p.N = d.out; p.K = d.in; p.act = act;
     p.skip = skip; p.ldskip = ldskip; p.alpha = alpha_; p.out_f32 = out_f32;
     p.whole_tiles = (opt.flags & B200_FLAG_NO_SPLIT_LAST_WAVE) != 0;
@@ -1150,7 +1177,7 @@ struct Net : NetBase {
                T* C2 = nullptr, long long ldc2 = 0, int n_split = 0) {
     GemmParams p;
     p.C2 = C2; p.ldc2 = ldc2; p.n_split = n_split;
-    p.A = in.u; p.lda = lda; p.W = d.w; p.ldw = d.in; p.w_const = true; p.bias = d.b;
+    p.A = in.u; p.lda = lda; p.W = d.w; p.W3 = d.w3; p.ldw = d.in; p.w_const = true; p.bias = d.b;
     p.C = Cout; p.ldc = ldc; p.M = M; p.N = d.out; p.K = d.in; p.act = act;
     if (in.stats) {
       if (!d.colsum) throw Fail{B200_ERR_INVALID, "internal: folded input for a layer without folded weights"};
@@ -1208,6 +1235,14 @@ struct Net : NetBase {
       if (use_tc && gemm_tc_supported(p)) {
         const int sp_ = span_begin(st, K_GEMM_TC, flops, t_tag);
         CK(launch_gemm_tc<T>(p, t_status, t_sm_limit > 0 ? t_sm_limit : sm_count, st));
+        span_end(st, sp_);
+        return;
+      }
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (gemm_f32_supported(p)) {
+        const int sp_ = span_begin(st, K_GEMM_TC, flops, t_tag);
+        CK(launch_gemm_f32(p, t_status, sm_count, st));
         span_end(st, sp_);
         return;
       }
@@ -1310,6 +1345,16 @@ struct Net : NetBase {
         launches++;
         const int sp_ = span_begin(st, K_GEMM_TC, 2.0 * p.M * (double)p.N * p.K);
         CK(launch_gemm_tc<T>(p, t_status, sm_count, st));
+        span_end(st, sp_);
+        return;
+      }
+    } else {
+      GemmParams p = conv_params(x, c, bias, y, n, act);
+      p.W3 = c.w3;
+      if (gemm_f32_supported(p)) {
+        launches++;
+        const int sp_ = span_begin(st, K_GEMM_TC, 2.0 * p.M * (double)p.N * p.K);
+        CK(launch_gemm_f32(p, t_status, sm_count, st));
         span_end(st, sp_);
         return;
       }
@@ -2428,6 +2473,43 @@ int b200_op_gemm_ln(const void* x, const float* gamma, const float* beta, int gr
   B200_CUDA(err);
   if (code) {
     set_error("tensor-core GEMM: a bounded device-side wait gave up, status " + std::to_string(code));
+    return B200_ERR_TIMEOUT;
+  }
+  return B200_OK;
+}
+
+int b200_op_gemm_f32(const float* A, long long lda, const float* W, const float* bias, const float* skip, float* C, int M, int N,
+                     int K, int conv, int activation, float alpha, void* stream) {
+  if (!A || !W || !C || M < 0 || N <= 0 || K <= 0 || (conv && M % 64)) {
+    set_error("b200_op_gemm_f32: invalid argument");
+    return B200_ERR_INVALID;
+  }
+  GemmParams p;
+  p.A = A; p.lda = lda; p.W = W; p.ldw = K; p.W3 = A; p.bias = bias; p.C = C; p.ldc = N; p.M = M; p.N = N; p.K = conv ? 9 * K : K;
+  p.act = activation; p.skip = skip; p.ldskip = N; p.alpha = alpha; p.conv_cin = conv ? K : 0;
+  if (!gemm_f32_supported(p) || (conv && lda != K)) {
+    set_error("b200_op_gemm_f32: rows of A must be 16-byte pieces and K a multiple of 8");
+    return B200_ERR_UNSUPPORTED;
+  }
+  B200_CUDA(gemm_tc_init());
+  int dev = 0, sms = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  B200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const long long count = (long long)N * p.K;
+  cudaStream_t st = (cudaStream_t)stream;
+  char* scratch = nullptr;  // status word, pieces
+  B200_CUDA(cudaMalloc(&scratch, 256 + count * 6));
+  int code = 0;
+  p.W3 = scratch + 256;
+  cudaError_t err = cudaMemsetAsync(scratch, 0, 256, st);
+  if (err == cudaSuccess) err = launch_split_weights(W, count, scratch + 256, st);
+  if (err == cudaSuccess) err = launch_gemm_f32(p, reinterpret_cast<int*>(scratch), sms, st);
+  if (err == cudaSuccess) err = cudaMemcpyAsync(&code, scratch, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (err == cudaSuccess) err = cudaStreamSynchronize(st);
+  cudaFree(scratch);
+  B200_CUDA(err);
+  if (code) {
+    set_error("fp32 tensor-core product: a bounded device-side wait gave up, status " + std::to_string(code));
     return B200_ERR_TIMEOUT;
   }
   return B200_OK;

@@ -113,6 +113,73 @@ def test_gemm_tc_rejects_fp32(lib):
     assert lib.b200_op_gemm(None, None, None, None, 128, 128, 64, 3, 0, 1, None) == _lib.ERR_UNSUPPORTED
 
 
+def _f32_op(lib, A, W, bias, skip, conv, act=oracle.ACT_NONE, alpha=1.0):
+    M, K, N = A.shape[0], A.shape[1], W.shape[-2]
+    C = torch.full((M, N), 7.0, device="cuda")
+    p = lambda t: None if t is None else t.data_ptr()
+    _lib.check(lib.b200_op_gemm_f32(A.data_ptr(), A.stride(0), W.data_ptr(), p(bias), p(skip), C.data_ptr(), M, N, K, conv, act, alpha, None))
+    return C
+
+
+def _f32_want(A, W, conv):
+    """Sums in 64 bits and the sums of the terms' magnitudes."""
+    if not conv:
+        return A.double() @ W.double().T, A.double().abs() @ W.double().abs().T
+    x = A.double().view(-1, 8, 8, A.shape[1]).permute(0, 3, 1, 2)
+    w = W.double().view(3, 3, W.shape[1], W.shape[2]).permute(2, 3, 0, 1)
+    f = lambda a, b: torch.nn.functional.conv2d(a, b, padding=1).permute(0, 2, 3, 1).reshape(A.shape[0], -1)
+    return f(x, w), f(x.abs(), w.abs())
+
+
+@pytest.mark.parametrize("conv", [0, 1])
+@pytest.mark.parametrize("shape", [(64, 8, 8), (64, 30, 72), (128, 64, 64), (192, 100, 112), (320, 130, 1024), (2048, 3072, 128),
+                                   (64 * 210, 96, 200)])
+def test_fp32_tensor_core_products(lib, conv, shape):
+    """Three bf16 pieces per operand: edges of tiles (32, 64 and 128 columns), of k-blocks and of board rows."""
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = torch.randn(M, K, device="cuda", generator=g)
+    W = torch.randn(*((9, N, K) if conv else (N, K)), device="cuda", generator=g) * K ** -0.5
+    b, skip = torch.randn(N, device="cuda", generator=g), torch.randn(M, N, device="cuda", generator=g)
+    want, size = _f32_want(A, W, conv)
+    got = _f32_op(lib, A, W, None, None, conv)
+    # four truncating additions per 64 k, one rounded addition per 64 k, the pieces left out
+    blocks = (9 if conv else 1) * ((K + 63) // 64)
+    assert ((got.double() - want).abs() <= (8 + blocks + 1) * 2.0 ** -24 * size).all()
+    got = _f32_op(lib, A, W, b, skip, conv, oracle.ACT_RELU, 0.5)
+    want = 0.5 * torch.relu(want + b.double()) + skip.double()
+    assert ((got.double() - want).abs() <= (8 + blocks + 4) * 2.0 ** -24 * (size + b.abs() + skip.abs())).all()
+    whole = _f32_op(lib, A, W, b, None, conv)
+    for rows in {64, M // 128 * 64 or 64}:  # a row's sum is the same among any number of rows
+        assert torch.equal(_f32_op(lib, A[:rows], W, b, None, conv), whole[:rows])
+
+
+@pytest.mark.parametrize("conv", [0, 1])
+def test_fp32_tensor_core_products_of_extreme_values(lib, conv):
+    """Infinities, NaN, values that round to an infinite bf16 and values near the smallest normal: as the FMA kernel has them."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    A, W = torch.randn(128, 64, device="cuda", generator=g), torch.randn(*((9, 40, 64) if conv else (40, 64)), device="cuda", generator=g)
+    A[3, 5], A[17, 6], A[40, 7], A[70, 8] = float("inf"), float("nan"), 3.4e38, -float("inf")
+    A[100] *= 1e-35
+    W[..., 8, :] = torch.tensor([1.0, 0.5] * 32, device="cuda")  # pieces 2 and 3 are zero
+    W *= 0.25
+    want, size = _f32_want(A, W, conv)
+    want32 = want.float()
+    got = _f32_op(lib, A, W, None, None, conv)
+    assert torch.equal(got.isnan(), want32.isnan()) and torch.equal(got.isposinf(), want32.isposinf())
+    assert torch.equal(got.isneginf(), want32.isneginf())
+    ok = want32.isfinite()
+    assert ((got.double() - want).abs()[ok] <= (20 * 2.0 ** -24 * size + 1e-37)[ok]).all()
+
+
+def test_fp32_tensor_core_product_refuses(lib):
+    a = torch.zeros(64 * 72, device="cuda").data_ptr()
+    op = lambda A, lda, M, N, K, conv: lib.b200_op_gemm_f32(A, lda, a, None, None, a, M, N, K, conv, oracle.ACT_NONE, 1.0, None)
+    assert op(a, 12, 8, 8, 12, 0) == _lib.ERR_UNSUPPORTED and op(a, 18, 8, 8, 16, 0) == _lib.ERR_UNSUPPORTED
+    assert op(a + 4, 16, 8, 8, 16, 0) == _lib.ERR_UNSUPPORTED and op(a, 24, 64, 8, 16, 1) == _lib.ERR_UNSUPPORTED
+    assert op(a, 16, 32, 8, 16, 1) == _lib.ERR_INVALID and op(None, 16, 8, 8, 16, 0) == _lib.ERR_INVALID
+
+
 @pytest.mark.parametrize("prec", [0, 1, 2])
 @pytest.mark.parametrize("C", [64, 256, 1024, 8192])
 def test_layer_norm(lib, prec, C):
