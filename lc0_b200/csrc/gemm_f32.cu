@@ -7,21 +7,24 @@
 //   a1 w2 + a2 w1              order 2^-9
 //   a1 w3 + a2 w2 + a3 w1      order 2^-18;  what is left out is below 2^-26 of |a||w|
 // The tensor core adds to its accumulator with truncation, which over a long K range would cost more digits than an FMA chain
-// has to lose.  So the sums of order 1 stay in tensor memory for 64 k only and are then added, rounded, in registers; the
+// has to lose.  So the sums of order 1 stay in tensor memory for 32 k only and are then added, rounded, in registers; the
 // small orders may stay there for the whole range, where truncation at 2^-9 of their size does not count.  A row's sum is taken in the
-// same order at every number of rows, tile width and grid.
+// same order at every number of rows and grid.  Error against sums in 64 bits (relative 2-norm), this kernel / FMA kernel: normal
+// operands 1024x3072x1024 0.95e-7 / 2.9e-7, 4096x256x2304 1.3e-7 / 2.2e-7, 512x4096x256 0.7e-7 / 2.1e-7; non-negative A 1.0e-7 / 2.1e-7;
+// with 64 k per rounded sum the first was 1.04e-7.
 //
-// Measured against sums in 64 bits, relative 2-norm of the error, this kernel / FMA kernel: see DESIGN; the network's outputs too.
-//
-// Bound by the tensor pipe (six MMAs for one: 277 TFLOP/s at the measured bf16 rate; the FMA pipe has 74) with the operand
-// traffic close behind: an A tile of 128 x 64 arrives as 32 KB of fp32 and is cut by the CTA itself, the weights' pieces are
-// made once at load and arrive by TMA (24 KB per k-block at 64 columns, 48 KB at 128).
-//   warps 0-7    fp32 rows of A -> registers (one k-block ahead) -> three bf16 pieces -> swizzled operand tiles
-//   warp 8       TMA of the weights' pieces
-//   warp 9       tcgen05.mma (cta_group::1).  Pieces of W lie one behind the other, so a1 [w2 w3] and a2 [w1 w2] are one MMA each
-//                of twice the width: four MMAs per 16 k instead of six, the narrow ones being bound by the reads of A
-//   warps 10-17  after every k-block: order-1 sums of one of two accumulators -> added in registers; at the end the small
-//                orders, then through shared memory to whole rows: scale, bias, activation, skip
+// The FMA pipe has 74 TFLOP/s and gave half of them; six MMAs for one leave 277 at the measured bf16 rate.  What paces a k-block of
+// 64 columns (0.67 us alone on an SM, its MMAs 0.40, its shared-memory traffic 0.55): waits of the issuing thread, some 150 cycles each, which
+// the queue of MMAs hides only in part.  Hence one wait for A and one for the accumulators per k-block and nothing else.  A's pieces
+// live in tensor memory, where an MMA reads them beside shared memory; in shared memory (48 KB written and 64 KB read more per
+// k-block) it took 0.79 us at 64 columns and 1.25 at 128.  Twice as many converter warps were slower (0.80), waits between the MMAs too.
+// us per launch, FMA kernel / this: 1024x3072x1024 175 / 56, 1024x1024x1024 70 / 19, 64x1024x1024 13 / 13, 4096x3072x1024 678 / 198;
+// 3x3 convolution 128 -> 128 of 64 boards 53 / 16.3.
+//   warp 8       TMA: fp32 tile of A, pieces of W (made once at load); the weights' first stages ahead of the grid dependency
+//   warps 0-7    fp32 rows (a thread has one row, half of 64 k) -> three bf16 pieces -> tensor memory
+//   warp 9       tcgen05.mma (cta_group::1, A from tensor memory)
+//   warps 10-17  after every k-block: order-1 sums of its halves -> added in registers; at the end the small orders, then through
+//                shared memory to whole rows: scale, bias, activation, skip
 // Infinities: inf times a piece that is zero would be NaN, and a value may round to an infinite piece; an output that comes
 // out non-finite is therefore computed again from the fp32 operands, by FMAs.
 // Every wait is bounded like those of gemm_tc.cu.
@@ -33,7 +36,8 @@
 namespace b200 {
 namespace {
 
-constexpr int kF32Threads = 576;
+constexpr int kF32Threads = 18 * 32;
+constexpr int kAStages = 2;
 
 struct F32Params {
   const float* A; long long lda;
@@ -51,13 +55,33 @@ struct F32Params {
 };
 
 template <int BN> struct F32Tile {
-  static constexpr int kA = 3 * 128 * 128, kW = 3 * BN * 128;  // bytes of a k-block's pieces
-  static constexpr int kStage = kA + kW;
-  static constexpr int kStages = BN == 128 ? 2 : 3;
+  static constexpr int kRaw = 128 * 64 * 4, kW = 3 * BN * 128;  // bytes of a k-block: two boxes of 32 fp32 columns, pieces of W
+  static constexpr int kStage = kRaw + kW;
+  static constexpr int kStages = BN == 64 ? 3 : 4;
   static constexpr int kOut = 128 * (BN + 4) * 4;  // the tile's sums, in place of the ring
   static constexpr int kBytes = kStages * kStage + 1024 /*alignment*/ + 256 /*barriers*/;
   static_assert(kStages * kStage >= kOut, "the sums take the place of the ring");
+  // tensor memory: two buffers for the order-1 sums of either half of a k-block, the small orders (BN columns each), stages of A's
+  // pieces (for either half of the k-block 3 x 16 columns)
+  static constexpr int kXCol = 4 * BN, kACol = 5 * BN, kCols = 512;
+  static_assert(kACol + kAStages * 96 <= kCols, "tensor memory");
 };
+
+// D += A W^T with A in tensor memory (one row per lane, two values of k per column).
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t wdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d), "r"(a), "l"(wdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // The three bf16 pieces of two values (the first in the lower half).
 __device__ __forceinline__ void split3(float x, float y, uint32_t& u1, uint32_t& u2, uint32_t& u3) {
@@ -81,10 +105,6 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const float* __restr
   out[2 * count + i] = __ushort_as_bfloat16((unsigned short)u3);
 }
 
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
 // Row m, column n of the product from the fp32 operands, by a whole warp.
 template <bool kConv>
 __device__ __forceinline__ float warp_dot(const F32Params& p, int m, int n) {
@@ -106,14 +126,16 @@ __device__ __forceinline__ float warp_dot(const F32Params& p, int m, int n) {
 
 template <int BN, bool kConv>
 __global__ void __launch_bounds__(kF32Threads, 1)
-gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Params p) {
+gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const F32Params p) {
   using L = F32Tile<BN>;
-  constexpr int S = L::kStages;
+  constexpr int S = L::kStages, AS = kAStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S * L::kStage);  // [S] eight converter warps and the weights
-  uint64_t* empty_bar = full_bar + S;                                      // [S] the k-block's MMAs are done
-  uint64_t* hfull_bar = empty_bar + S;                                     // [2] order-1 sums complete
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S * L::kStage);  // [S] A and W have landed
+  uint64_t* empty_bar = full_bar + S;                                      // [S] read by eight converter warps and the MMAs
+  uint64_t* afull_bar = empty_bar + S;                                     // [AS] pieces of A in place (eight warps)
+  uint64_t* aempty_bar = afull_bar + AS;                                   // [AS] ... and read by the MMAs
+  uint64_t* hfull_bar = aempty_bar + AS;                                   // [2] order-1 sums complete
   uint64_t* hempty_bar = hfull_bar + 2;                                    // [2] ... and read by eight warps
   uint64_t* xfull_bar = hempty_bar + 2;                                    // every MMA done
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xfull_bar + 1);
@@ -125,9 +147,14 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Params p) {
 
   if (tid == 256) {
     tma_prefetch_map(&tmap_w);
+    tma_prefetch_map(&tmap_a);
     for (int i = 0; i < S; ++i) {
-      mbar_init(smem_u32(&full_bar[i]), 9);
-      mbar_init(smem_u32(&empty_bar[i]), 1);
+      mbar_init(smem_u32(&full_bar[i]), 1);
+      mbar_init(smem_u32(&empty_bar[i]), 9);
+    }
+    for (int i = 0; i < AS; ++i) {
+      mbar_init(smem_u32(&afull_bar[i]), 8);
+      mbar_init(smem_u32(&aempty_bar[i]), 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&hfull_bar[i]), 1);
@@ -139,7 +166,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Params p) {
   }
   if (warp == 9) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"((uint32_t)(4 * BN))
+                 "r"((uint32_t)L::kCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -148,83 +175,45 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Params p) {
   tcgen05_fence_after();
   // after the allocation: the next kernel's CTAs must not take the tensor memory that this one still waits for
   grid_launch_dependents();
-  const uint32_t tmem = *tmem_slot;  // order-1 sums of even k-blocks, of odd ones, order 2^-9, order 2^-18: BN columns each
+  const uint32_t tmem = *tmem_slot;
 
   if (warp < 8) {
     // ---------------- A: fp32 rows -> pieces ----------------
-    const int lr = tid >> 3, lp = tid & 7;  // rows lr, lr + 32, ...; eight k from 8 lp on
-    long long off[4];
-    uint32_t ok[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int m = m0 + lr + 32 * r;
-      const bool in = m < p.M;
-      off[r] = in ? (long long)m * p.lda + lp * 8 : 0;
-      ok[r] = in ? 1 : 0;
-      if constexpr (kConv) {
-        ok[r] = 0;
-        for (int t = 0; t < 9; ++t) {
-          const int y = ((m >> 3) & 7) + t / 3 - 1, x = (m & 7) + t % 3 - 1;
-          if (in && (unsigned)y < 8u && (unsigned)x < 8u) ok[r] |= 1u << t;
-        }
-      }
-    }
-    float4 next[4][2];
-    auto load = [&](int i) {
-      int tap = 0, c = i * 64;
-      long long at = c;
-      bool in_k;
-      if constexpr (kConv) {
-        tap = i / p.cblocks;
-        c = (i - tap * p.cblocks) * 64;
-        at = ((tap / 3 - 1) * 8 + tap % 3 - 1) * p.lda + c;
-        in_k = c + lp * 8 < p.conv_cin;
-      } else {
-        in_k = c + lp * 8 < p.K;
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float4* src = reinterpret_cast<const float4*>(p.A + off[r] + at);
-        const bool in = in_k && ((ok[r] >> tap) & 1);
-        next[r][0] = in ? src[0] : make_float4(0.f, 0.f, 0.f, 0.f);
-        next[r][1] = in ? src[1] : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    };
-    grid_dependency_wait();
-    load(0);
-    int s = 0;
-    uint32_t ph = 0;
+    const int quarter = warp & 3, half = warp >> 2, row = quarter * 32 + lane;
+    const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + L::kACol + half * 48;
+    int s = 0, a = 0;
+    uint32_t ph = 0, aph = 0;
     for (int i = 0; i < kbn; ++i) {
-      float4 cur[4][2];
+      if (!mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag, 1)) break;
+      const uint8_t* src = smem + s * L::kStage + half * 16384 + row * 128;
+      float v[32];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) { cur[r][0] = next[r][0]; cur[r][1] = next[r][1]; }
-      if (i + 1 < kbn) load(i + 1);
-      if (i >= S && !mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, 1)) break;
-      const uint32_t st = smem_u32(smem + s * L::kStage) + lr * 128 + ((lp ^ (lr & 7)) << 4);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        uint32_t u[3][4];
-        split3(cur[r][0].x, cur[r][0].y, u[0][0], u[1][0], u[2][0]);
-        split3(cur[r][0].z, cur[r][0].w, u[0][1], u[1][1], u[2][1]);
-        split3(cur[r][1].x, cur[r][1].y, u[0][2], u[1][2], u[2][2]);
-        split3(cur[r][1].z, cur[r][1].w, u[0][3], u[1][3], u[2][3]);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) st_shared_v4(st + j * 16384 + r * 4096, u[j][0], u[j][1], u[j][2], u[j][3]);
-      }
-      fence_async_smem();  // the tensor core reads the pieces through the asynchronous proxy
+      for (int c = 0; c < 8; ++c) *reinterpret_cast<float4*>(v + 4 * c) = *reinterpret_cast<const float4*>(src + ((c ^ (row & 7)) << 4));
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&full_bar[s]));
+      if (lane == 0) mbar_arrive(smem_u32(&empty_bar[s]));
       if (++s == S) { s = 0; ph ^= 1; }
+      if (i >= AS && !mbar_wait(smem_u32(&aempty_bar[a]), aph ^ 1, abort_flag, 2)) break;
+      tcgen05_fence_after();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t u[3][8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) split3(v[16 * h + 2 * c], v[16 * h + 2 * c + 1], u[0][c], u[1][c], u[2][c]);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) tmem_st8(ta + a * 96 + c * 16 + h * 8, u[c]);
+      }
+      tmem_st_wait();
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&afull_bar[a]));
+      if (++a == AS) { a = 0; aph ^= 1; }
     }
   } else if (warp == 8) {
-    // ---------------- weights: loaded once, requested while the kernel before this one is still running ----------------
+    // ---------------- TMA ----------------
     if (elect_one()) {
-      int s = 0;
-      uint32_t ph = 0;
-      for (int i = 0; i < kbn; ++i) {
-        if (i >= S && !mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, 2)) break;
-        const uint32_t fb = smem_u32(&full_bar[s]), dst = smem_u32(smem + s * L::kStage) + L::kA;
-        mbar_expect_tx(fb, L::kW);
+      auto load_w = [&](int i, int s) {
+        const uint32_t fb = smem_u32(&full_bar[s]), dst = smem_u32(smem + s * L::kStage) + L::kRaw;
+        mbar_expect_tx(fb, L::kStage);
         int row = n0, x = i * 64, plane = p.N;
         if constexpr (kConv) {
           const int tap = i / p.cblocks;
@@ -234,6 +223,27 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Params p) {
         }
 #pragma unroll
         for (int j = 0; j < 3; ++j) tma_load_2d(dst + j * BN * 128, &tmap_w, x, row + j * plane, fb);
+      };
+      // loaded weights: requested while the kernel before this one is still running
+      const int early = kbn < S ? kbn : S;
+      for (int i = 0; i < early; ++i) load_w(i, i);
+      grid_dependency_wait();
+      int s = 0;
+      uint32_t ph = 0;
+      for (int i = 0; i < kbn; ++i) {
+        if (i >= early) {
+          if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, 3)) break;
+          load_w(i, s);
+        }
+        const uint32_t fb = smem_u32(&full_bar[s]), dst = smem_u32(smem + s * L::kStage);
+        if constexpr (kConv) {
+          const int tap = i / p.cblocks, x = (i - tap * p.cblocks) * 64;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) tma_load_4d(dst + h * 16384, &tmap_a, x + 32 * h, tap % 3 - 1, tap / 3 - 1, m0 >> 6, fb);
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * 16384, &tmap_a, i * 64 + 32 * h, m0, fb);
+        }
         if (++s == S) { s = 0; ph ^= 1; }
       }
     }
@@ -241,83 +251,82 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Params p) {
   } else if (warp == 9) {
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
-      constexpr uint32_t one = make_idesc<__nv_bfloat16, BN>(), two = make_idesc<__nv_bfloat16, 2 * BN>();
+      constexpr uint32_t one = make_idesc<__nv_bfloat16, BN>();
       bool good = true;
       int s = 0;
-      uint32_t ph = 0;
       for (int i = 0; i < kbn; ++i) {
-        const int b = i & 1;
-        if (i >= 2 && !mbar_wait(smem_u32(&hempty_bar[b]), ((i >> 1) & 1) ^ 1, abort_flag, 3)) { good = false; break; }
-        if (!mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag, 4)) { good = false; break; }
+        // A's pieces are in place; the warps that wrote them have seen the weights land too
+        if (!mbar_wait(smem_u32(&afull_bar[i & 1]), (i >> 1) & 1, abort_flag, 5)) { good = false; break; }
+        if (i > 1 && !mbar_wait(smem_u32(&hempty_bar[i & 1]), ((i >> 1) & 1) ^ 1, abort_flag, 6)) { good = false; break; }
         tcgen05_fence_after();
-        const uint32_t sa = smem_u32(smem + s * L::kStage);
-        const uint64_t a1 = make_smem_desc(sa), a2 = make_smem_desc(sa + 16384), a3 = make_smem_desc(sa + 32768);
-        const uint64_t w1 = make_smem_desc(sa + L::kA), w2 = make_smem_desc(sa + L::kA + BN * 128);
+        const int a = i & 1;
+        const uint32_t sw = smem_u32(smem + s * L::kStage) + L::kRaw, a1 = tmem + L::kACol + a * 96;
+        const uint32_t h = tmem + a * 2 * BN, x = tmem + L::kXCol;
+        const uint64_t w1 = make_smem_desc(sw), w2 = make_smem_desc(sw + BN * 128), w3 = make_smem_desc(sw + 2 * BN * 128);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) tcgen05_mma_f16(tmem + b * BN, a1 + 2 * k, w1 + 2 * k, one, k > 0 ? 1u : 0u);
-        tcgen05_commit(smem_u32(&hfull_bar[b]));
+        for (int k = 0; k < 4; ++k) mma_ts(h + (k >> 1) * BN, a1 + (k >> 1) * 48 + 8 * (k & 1), w1 + 2 * k, one, (k & 1) ? 1u : 0u);
+        tcgen05_commit(smem_u32(&hfull_bar[a]));
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          tcgen05_mma_f16(tmem + 2 * BN, a1 + 2 * k, w2 + 2 * k, two, (i > 0 || k > 0) ? 1u : 0u);
-          tcgen05_mma_f16(tmem + 2 * BN, a2 + 2 * k, w1 + 2 * k, two, 1u);
-          tcgen05_mma_f16(tmem + 3 * BN, a3 + 2 * k, w1 + 2 * k, one, 1u);
+          const uint32_t ak = a1 + (k >> 1) * 48 + 8 * (k & 1);
+          mma_ts(x, ak, w3 + 2 * k, one, (i > 0 || k > 0) ? 1u : 0u);
+          mma_ts(x, ak + 16, w2 + 2 * k, one, 1u);
+          mma_ts(x, ak + 32, w1 + 2 * k, one, 1u);
+          mma_ts(x, ak, w2 + 2 * k, one, 1u);
+          mma_ts(x, ak + 16, w1 + 2 * k, one, 1u);
         }
+        tcgen05_commit(smem_u32(&aempty_bar[a]));
         tcgen05_commit(smem_u32(&empty_bar[s]));
-        if (++s == S) { s = 0; ph ^= 1; }
+        if (++s == S) s = 0;
       }
       if (good) tcgen05_commit(smem_u32(xfull_bar));
     }
     __syncwarp();
   } else {
     // ---------------- sums ----------------
-    constexpr int kCols = BN / 2;  // columns of this warp: its half of the tile, 32 rows
+    // a thread has one row, half of the columns
+    constexpr int kCols = BN / 2;
     const int quarter = warp & 3, half = (warp - 10) >> 2;
     const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + half * kCols;
     float acc[kCols];
 #pragma unroll
     for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
-    auto add = [&](uint32_t at, float* to) {
-#pragma unroll
-      for (int c = 0; c < kCols; c += 16) {
-        uint32_t r[16];
-        tmem_ld16(at + c, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) to[c + j] = __fadd_rn(to[c + j], __uint_as_float(r[j]));
-      }
-    };
     bool good = true;
     for (int i = 0; i < kbn; ++i) {
       const int b = i & 1;
-      if (!mbar_wait(smem_u32(&hfull_bar[b]), (i >> 1) & 1, abort_flag, 5)) { good = false; break; }
+      if (!mbar_wait(smem_u32(&hfull_bar[b]), (i >> 1) & 1, abort_flag, 7)) { good = false; break; }
       tcgen05_fence_after();
-      add(ta + b * BN, acc);
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&hempty_bar[b]));
-    }
-    if (good) good = mbar_wait(smem_u32(xfull_bar), 0, abort_flag, 6);
-    tcgen05_fence_after();
-    // the small orders, smallest first; the ring is free, the sums go through it
-    float* out = reinterpret_cast<float*>(smem);
-    {
-      float* row = out + (quarter * 32 + lane) * (BN + 4) + half * kCols;
 #pragma unroll
       for (int c = 0; c < kCols; c += 16) {
-        uint32_t x1[16], x2[16];
-        tmem_ld16(ta + 2 * BN + c, x1);
-        tmem_ld16(ta + 3 * BN + c, x2);
+        uint32_t r0[16], r1[16];
+        tmem_ld16(ta + 2 * b * BN + c, r0);
+        tmem_ld16(ta + (2 * b + 1) * BN + c, r1);
         tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; j += 4) {
-          float4 v;
-          v.x = __fadd_rn(acc[c + j], __fadd_rn(__uint_as_float(x1[j]), __uint_as_float(x2[j])));
-          v.y = __fadd_rn(acc[c + j + 1], __fadd_rn(__uint_as_float(x1[j + 1]), __uint_as_float(x2[j + 1])));
-          v.z = __fadd_rn(acc[c + j + 2], __fadd_rn(__uint_as_float(x1[j + 2]), __uint_as_float(x2[j + 2])));
-          v.w = __fadd_rn(acc[c + j + 3], __fadd_rn(__uint_as_float(x1[j + 3]), __uint_as_float(x2[j + 3])));
-          *reinterpret_cast<float4*>(row + c + j) = v;
+        if (c + 16 >= kCols) {  // the last columns are in registers: the k-block after the next may overwrite them
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&hempty_bar[b]));
         }
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+          acc[c + k] = __fadd_rn(acc[c + k], __fadd_rn(__uint_as_float(r0[k]), __uint_as_float(r1[k])));
       }
+    }
+    if (good) good = mbar_wait(smem_u32(xfull_bar), 0, abort_flag, 8);
+    tcgen05_fence_after();
+    // the ring is free: the sums go through it, together with the small orders
+    float* out = reinterpret_cast<float*>(smem);
+    float* row = out + (quarter * 32 + lane) * (BN + 4) + half * kCols;
+#pragma unroll
+    for (int c = 0; c < kCols; c += 16) {
+      uint32_t x[16];
+      tmem_ld16(ta + L::kXCol + c, x);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; j += 4)
+        *reinterpret_cast<float4*>(row + c + j) =
+            make_float4(__fadd_rn(acc[c + j], __uint_as_float(x[j])), __fadd_rn(acc[c + j + 1], __uint_as_float(x[j + 1])),
+                        __fadd_rn(acc[c + j + 2], __uint_as_float(x[j + 2])), __fadd_rn(acc[c + j + 3], __uint_as_float(x[j + 3])));
     }
     tcgen05_fence_before();
     asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -378,7 +387,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Params p) {
   __syncthreads();
   if (warp == 9) {
     tcgen05_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(4 * BN)) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)L::kCols) : "memory");
   }
   if (*abort_flag) {
     // Give copies that may still be in flight time to land before the CTA's shared memory is released.
@@ -399,24 +408,24 @@ cudaError_t launch_f32_bn(const F32Params& p, const void* planes, cudaStream_t s
     if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes)) != cudaSuccess) return e;
     attr_mask.fetch_or(1ull << (dev & 63));
   }
-  CUtensorMap mw;
+  CUtensorMap ma, mw;
+  if ((e = gemm_f32_map(p.A, p.lda, p.M, kConv ? p.conv_cin : p.K, kConv, &ma)) != cudaSuccess) return e;
   const int rows = 3 * (kConv ? 9 : 1) * p.N, cols = kConv ? p.conv_cin : p.K;
   if ((e = gemm_tensor_map(planes, cols, rows, cols, BN, TypeTag<__nv_bfloat16>::prec, &mw)) != cudaSuccess) return e;
-  return launch_dependent(kernel, dim3(ceil_div(p.N, BN), ceil_div(p.M, 128)), dim3(kF32Threads), L::kBytes, s, mw, p);
+  return launch_dependent(kernel, dim3(ceil_div(p.N, BN), ceil_div(p.M, 128)), dim3(kF32Threads), L::kBytes, s, ma, mw, p);
 }
 
-// Tile width: the least time of a round of tiles (one per SM) times the rounds.  Cycles of a k-block are those of its MMAs
-// (128 x N x 16: 40 / 48 / 64 / 126 at N = 32 / 64 / 128 / 256); a tile's start and end take what is added.
+// Tile width: rounds of tiles (one per SM) times a tile's time, its k-blocks and its ends in ns.  Measured at 32 / 64 columns, us:
+// 64x1024x1024 13.0 / 16.3, 1024x1024x1024 28.0 / 19.6, 1024x1024x1536 37.1 / 25.4, 1024x3072x1024 82 / 56, 512x4096x256 27.8 / 19.8,
+// convolution of 64 boards 16.3 / 20.7, of 512 111 / 82.
 template <bool kConv>
 cudaError_t launch_f32(const F32Params& p, const void* planes, int sm_count, cudaStream_t s) {
   const long long m_tiles = ceil_div(p.M, 128);
   auto cost = [&](int bn, int block, int ends) {
-    return (long long)ceil_div(m_tiles * ceil_div(p.N, bn), sm_count) * ((long long)p.k_blocks * block + ends);
+    return ceil_div(m_tiles * ceil_div(p.N, bn), sm_count) * ((long long)p.k_blocks * block + ends);
   };
-  const long long c32 = cost(32, 710, 5000), c64 = cost(64, 900, 6000), c128 = cost(128, 1520, 8000);
-  if (c32 < c64 && c32 < c128) return launch_f32_bn<32, kConv>(p, planes, s);
-  if (c64 <= c128) return launch_f32_bn<64, kConv>(p, planes, s);
-  return launch_f32_bn<128, kConv>(p, planes, s);
+  if (cost(32, 525, 4800) < cost(64, 700, 7000)) return launch_f32_bn<32, kConv>(p, planes, s);
+  return launch_f32_bn<64, kConv>(p, planes, s);
 }
 
 bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }

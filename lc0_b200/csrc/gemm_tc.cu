@@ -1534,6 +1534,24 @@ cudaError_t tma_encode_2d(const void* ptr, long long ld, long long rows, int col
   return cudaSuccess;
 }
 
+cudaError_t gemm_f32_map(const float* ptr, long long ld, int rows, int cols, bool board, CUtensorMap* out) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  if (!g_encode) return cudaErrorNotReady;
+  const cuuint64_t row = (cuuint64_t)(board ? cols : ld) * 4;
+  cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)(board ? 8 : rows), 8, (cuuint64_t)rows / 64};
+  cuuint64_t strides[3] = {row, row * 8, row * 64};
+  cuuint32_t box[4] = {32, (cuuint32_t)(board ? 8 : 128), 8, 2};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, board ? 4 : 2, const_cast<float*>(ptr), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled (fp32) failed with CUresult " + std::to_string((int)r));
+    return cudaErrorInvalidValue;
+  }
+  return cudaSuccess;
+}
+
 cudaError_t gemm_tensor_map(const void* ptr, long long ld, int rows, int cols, int box_rows, int prec, CUtensorMap* out) {
   return get_map(ptr, ld, rows, cols, box_rows, prec, out);
 }

@@ -789,8 +789,8 @@ struct Net : NetBase {
     merge_compress = !(opt.flags & B200_FLAG_NO_MERGED_COMPRESS);
     winograd = use_tc && !attn_body && (opt.flags & B200_FLAG_WINOGRAD);
     side_stream = use_tc && attn_body && !(opt.flags & B200_FLAG_NO_SIDE_STREAM) && sm_count >= 4 * kSideSms;
-    dependent_launch = use_tc && !(opt.flags & B200_FLAG_NO_DEPENDENT_LAUNCH);
-    heads_side = use_tc && !(opt.flags & B200_FLAG_NO_SIDE_STREAM) && sm_count >= 4 * kSideSms;
+    dependent_launch = (use_tc || f32_tc) && !(opt.flags & B200_FLAG_NO_DEPENDENT_LAUNCH);
+    heads_side = (use_tc || f32_tc) && !(opt.flags & B200_FLAG_NO_SIDE_STREAM) && sm_count >= 4 * kSideSms;
     // measured: +8 % at batch 64 on a 10 x 128 residual net, +2 % at 256 on a 20 x 256 one, +1.7 % at 64 on the BT4-class net,
     // nothing from 1024 on (the products then fill the GPU on their own)
     heads_side_max = 512;

@@ -362,6 +362,9 @@ inline bool epilogue_supported(const GemmParams& g) {
 
 // Tensor map over a row-major 16-bit matrix, box = 64 columns x box_rows, 128-byte swizzle; cached by its arguments.
 cudaError_t gemm_tensor_map(const void* ptr, long long ld, int rows, int cols, int box_rows, int prec, CUtensorMap* out);
+// Tensor map over fp32 rows, box = 32 columns x 128 rows, 128-byte swizzle; board: over [rows / 64][8][8][cols] (ld ignored), box = 32
+// columns x two boards.
+cudaError_t gemm_f32_map(const float* ptr, long long ld, int rows, int cols, bool board, CUtensorMap* out);
 // Products of few rows (gemm_split.cu).
 template <typename T> cudaError_t launch_gemm_split(const GemmParams& g, int* status, int sm_count, cudaStream_t s);
 
