@@ -144,6 +144,9 @@ int b200_comp_add_input_with_moves(b200_comp* c, const uint64_t* masks, const fl
 int b200_comp_add_inputs_with_moves(b200_comp* c, const uint64_t* masks, const float* values,
                                     const uint16_t* move_ids, const int* n_moves, int n);
 int b200_comp_set_policy_options(b200_comp* c, float inv_temperature, int compact);
+/* The same for the whole batch, after b200_comp_compute: q, d, m of every sample (stride 3) and, with legal moves, their probabilities
+ * (stride 256) and numbers, else NULL.  Valid until the computation is destroyed. */
+int b200_comp_results(const b200_comp* comp, const float** qdm, const float** probs, const int** n_moves);
 int b200_comp_legal_policy(const b200_comp* c, int sample, const float** probs, int* n_moves);
 
 /* ---- Results and the batch --------------------------------------------------------------------

@@ -94,6 +94,7 @@ SIGNATURES = {
     "b200_comp_add_input_with_moves": (_I, [_P, _P, _P, _P, _I]),
     "b200_comp_add_inputs_with_moves": (_I, [_P, _P, _P, _P, _P, _I]),
     "b200_comp_set_policy_options": (_I, [_P, _F, _I]),
+    "b200_comp_results": (_I, [_P, _P, _P, _P]),
     "b200_comp_legal_policy": (_I, [_P, _I, ctypes.POINTER(ctypes.POINTER(_F)), ctypes.POINTER(_I)]),
     "b200_comp_set_encoding": (_I, [_P, _I, _I]),
     "b200_comp_add_position": (_I, [_P, _P, _I, _I, _P, _I]),
