@@ -2200,9 +2200,10 @@ int b200_comp_legal_policy(const b200_comp* c, int sample, const float** probs, 
 }
 int b200_comp_results(const b200_comp* c, const float** qdm, const float** probs, const int** n_moves) {
   if (!c || !qdm || !probs || !n_moves || !c->computed) return B200_ERR_INVALID;
-  *qdm = c->hs->qdm;
-  *probs = c->with_moves ? c->hs->probs : nullptr;
-  *n_moves = c->with_moves ? c->hs->n_moves : nullptr;
+  const bool moves = c->hs && c->with_moves;  // a computation without inputs has no host buffers
+  *qdm = c->hs ? c->hs->qdm : nullptr;
+  *probs = moves ? c->hs->probs : nullptr;
+  *n_moves = moves ? c->hs->n_moves : nullptr;
   return B200_OK;
 }
 void b200_comp_destroy(b200_comp* c) {
