@@ -50,6 +50,37 @@ __device__ __forceinline__ void flush_row_ctx(const TcParams& p, int m, const Ro
   }
 }
 
+// What an epilogue does, known when it is compiled: kAny asks the parameters.  The forms of the encoder's products have kernels of
+// their own: with every question asked at run time an epilogue thread of the four-group form spilled registers.
+enum EpilogueMode { kAny = 0, kPlain = 1 /*bias, activation*/, kNormIn = 2 /*folded LayerNorm of A, bias, activation*/,
+                    kResidual = 3 /*bias, residual (normalised or not), row statistics; no activation*/ };
+template <int kMode> struct Epilogue {
+  static __device__ __forceinline__ bool a_stats(const TcParams& p) { return kMode == kAny ? p.a_stats != nullptr : kMode == kNormIn; }
+  static __device__ __forceinline__ int res_mode(const TcParams& p) { return kMode == kAny || kMode == kResidual ? p.res_mode : 0; }
+  static __device__ __forceinline__ bool out_stats(const TcParams& p) { return kMode == kAny ? p.out_stats != nullptr : kMode == kResidual; }
+};
+inline int epilogue_mode(const GemmParams& g) {
+  if (g.conv_cin > 0 || g.se_k > 0 || g.batch_rows > 0 || g.scale != 1.0f) return kAny;
+  if (g.res) return g.out_stats && !g.a_stats && g.act == ACT_NONE ? kResidual : kAny;
+  if (g.out_stats) return kAny;
+  return g.a_stats ? kNormIn : kPlain;
+}
+
+// Statistics of a row of a later tile, on their way while this one is finished.
+struct RowStats { double2 a = {0.0, 0.0}, r = {0.0, 0.0}; };
+template <int kMode>
+__device__ __forceinline__ void fetch_row_stats(const TcParams& p, int m, RowStats& s) {
+  if (Epilogue<kMode>::a_stats(p) && m < p.M) s.a = *reinterpret_cast<const double2*>(p.a_stats + 2 * (long long)m);
+  if (Epilogue<kMode>::res_mode(p) == 2 && m < p.M) s.r = *reinterpret_cast<const double2*>(p.res_stats + 2 * (long long)m);
+}
+template <int kMode>
+__device__ __forceinline__ void use_row_stats(const TcParams& p, const RowStats& s, RowCtx& rc) {
+  rc.sum = 0.0;
+  rc.sumsq = 0.0;
+  if (Epilogue<kMode>::a_stats(p)) mean_rstd(s.a, p.a_inv_c, p.a_eps, rc.mean_a, rc.rstd_a);
+  if (Epilogue<kMode>::res_mode(p) == 2) mean_rstd(s.r, p.res_inv_c, p.res_eps, rc.mean_r, rc.rstd_r);
+}
+
 // One 64-column slab of the epilogue fast path, executed by one group of four warps: TMEM -> registers ->
 // scale / folded-LayerNorm correction / bias / activation / residual -> 128B-swizzled staging buffer, which the
 // store warp then writes out with a TMA store.  A group alternates between two buffers; `free_bar` completes when
@@ -62,11 +93,12 @@ __device__ __forceinline__ void flush_row_ctx(const TcParams& p, int m, const Ro
 struct ColRegs {
   float bias0 = 0.f, bias1 = 0.f, cs0 = 0.f, cs1 = 0.f, g0 = 0.f, g1 = 0.f, be0 = 0.f, be1 = 0.f;
 };
+template <int kMode = kAny>
 __device__ __forceinline__ void load_col_regs(const TcParams& p, int nb, int lane, ColRegs& c) {
   auto col = [&](const float* src, int i) { return (src && nb + i < p.N) ? __ldg(src + nb + i) : 0.f; };
   if (p.bias) { c.bias0 = col(p.bias, lane); c.bias1 = col(p.bias, 32 + lane); }
-  if (p.a_stats) { c.cs0 = col(p.colsum, lane); c.cs1 = col(p.colsum, 32 + lane); }
-  if (p.res_mode == 2) {
+  if (Epilogue<kMode>::a_stats(p)) { c.cs0 = col(p.colsum, lane); c.cs1 = col(p.colsum, 32 + lane); }
+  if (Epilogue<kMode>::res_mode(p) == 2) {
     c.g0 = col(p.res_gamma, lane); c.g1 = col(p.res_gamma, 32 + lane);
     c.be0 = col(p.res_beta, lane); c.be1 = col(p.res_beta, 32 + lane);
   }
@@ -75,44 +107,46 @@ __device__ __forceinline__ void load_col_regs(const TcParams& p, int nb, int lan
 // kMixed (the tower kernel, whose tiles alternate between layers with and without a residual input): the store thread
 // arrives on `free_bar` after every store and the group always waits for it; a slab with a residual also waits for
 // `res_bar`, whose phase is counted by `res_use` (the number of residual tiles this staging buffer has received).
-template <typename T, bool kSe = false, bool kMixed = false>
+template <typename T, bool kSe = false, bool kMixed = false, int kMode = kAny, int kCols = 32>
 __device__ __forceinline__ void epilogue_slab(const TcParams& p, uint8_t* buf, uint32_t res_bar, uint32_t free_bar,
                                               uint32_t full_bar, uint32_t use, bool leader, uint32_t taddr, int row,
                                               int lane, int nb, int next_nb, ColRegs& cr, float* wvec, RowCtx& rc,
                                               volatile int* abort_flag, const float* se_arg = nullptr,
                                               uint32_t res_use = 0) {
+  using Ep = Epilogue<kMode>;
   const float* se = kSe ? se_arg : nullptr;  // compiled out of the kernels that never fuse squeeze-excitation
   // se != nullptr: gate (se[0..63]) and shift (se[256..319]) of this row's sample for the slab's 64 columns; the
   // activation then follows the residual: act(gate * v + shift + residual)   (se_unit.cc:54-61)
   __syncwarp();  // the previous slab's reads of wvec are done
   if (p.bias) { wvec[lane] = cr.bias0; wvec[32 + lane] = cr.bias1; }
-  if (p.a_stats) { wvec[64 + lane] = cr.cs0; wvec[96 + lane] = cr.cs1; }
-  if (p.res_mode == 2) {
+  if (Ep::a_stats(p)) { wvec[64 + lane] = cr.cs0; wvec[96 + lane] = cr.cs1; }
+  if (Ep::res_mode(p) == 2) {
     wvec[128 + lane] = cr.g0; wvec[160 + lane] = cr.g1;
     wvec[192 + lane] = cr.be0; wvec[224 + lane] = cr.be1;
   }
   __syncwarp();
-  if (next_nb >= 0) load_col_regs(p, next_nb, lane, cr);  // in flight during the arithmetic below
+  if (next_nb >= 0) load_col_regs<kMode>(p, next_nb, lane, cr);  // in flight during the arithmetic below
   uint8_t* srow = buf + row * 128;
-  // The slab is processed as two halves of 32 columns (keeps the register footprint of an epilogue thread small
-  // enough for sixteen epilogue warps per CTA).
+  // kCols = 32: the slab is processed as two halves (keeps the register footprint of an epilogue thread small enough for sixteen
+  // epilogue warps per CTA); 64: in one piece, whose loads and arithmetic overlap.
 #pragma unroll 1
-  for (int h = 0; h < 2; ++h) {
-    uint32_t r[32];
-    tmem_ld32(taddr + 32 * h, r);
-    tmem_ld_wait();
-    float v[32];
-    if (p.scale != 1.0f) {
+  for (int h = 0; h < 64 / kCols; ++h) {
+    uint32_t r[kCols];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.scale;
+    for (int c = 0; c < kCols; c += 32) tmem_ld32(taddr + kCols * h + c, *reinterpret_cast<uint32_t(*)[32]>(r + c));
+    tmem_ld_wait();
+    float v[kCols];
+    if (kMode == kAny && p.scale != 1.0f) {
+#pragma unroll
+      for (int j = 0; j < kCols; ++j) v[j] = __uint_as_float(r[j]) * p.scale;
     } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+      for (int j = 0; j < kCols; ++j) v[j] = __uint_as_float(r[j]);
     }
-    if (p.a_stats) {
+    if (Ep::a_stats(p)) {
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        const float4 cs = *reinterpret_cast<const float4*>(wvec + 64 + 32 * h + j);
+      for (int j = 0; j < kCols; j += 4) {
+        const float4 cs = *reinterpret_cast<const float4*>(wvec + 64 + kCols * h + j);
         v[j] = rc.rstd_a * (v[j] - rc.mean_a * cs.x);
         v[j + 1] = rc.rstd_a * (v[j + 1] - rc.mean_a * cs.y);
         v[j + 2] = rc.rstd_a * (v[j + 2] - rc.mean_a * cs.z);
@@ -121,21 +155,21 @@ __device__ __forceinline__ void epilogue_slab(const TcParams& p, uint8_t* buf, u
     }
     if (se) {
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        const float4 g = *reinterpret_cast<const float4*>(se + 32 * h + j);
-        const float4 b = *reinterpret_cast<const float4*>(se + 256 + 32 * h + j);
+      for (int j = 0; j < kCols; j += 4) {
+        const float4 g = *reinterpret_cast<const float4*>(se + kCols * h + j);
+        const float4 b = *reinterpret_cast<const float4*>(se + 256 + kCols * h + j);
         v[j] = fmaf(g.x, v[j], b.x); v[j + 1] = fmaf(g.y, v[j + 1], b.y);
         v[j + 2] = fmaf(g.z, v[j + 2], b.z); v[j + 3] = fmaf(g.w, v[j + 3], b.w);
       }
     } else {
       if (p.bias) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          const float4 b = *reinterpret_cast<const float4*>(wvec + 32 * h + j);
+        for (int j = 0; j < kCols; j += 4) {
+          const float4 b = *reinterpret_cast<const float4*>(wvec + kCols * h + j);
           v[j] += b.x; v[j + 1] += b.y; v[j + 2] += b.z; v[j + 3] += b.w;
         }
       }
-      apply_activation(v, p.act);
+      if (kMode != kResidual) apply_activation(v, p.act);
     }
     if (h == 0) {
       // Every thread does its own bounded wait (after a failed wait the result is meaningless and the status word
@@ -143,22 +177,22 @@ __device__ __forceinline__ void epilogue_slab(const TcParams& p, uint8_t* buf, u
       // for the buffer itself.
       if (kMixed) {
         mbar_wait(free_bar, (use & 1) ^ 1, abort_flag, 6);
-        if (p.res_mode) mbar_wait(res_bar, res_use & 1, abort_flag, 5);
+        if (Ep::res_mode(p)) mbar_wait(res_bar, res_use & 1, abort_flag, 5);
       } else {
-        if (p.res_mode) mbar_wait(res_bar, use & 1, abort_flag, 5);
+        if (Ep::res_mode(p)) mbar_wait(res_bar, use & 1, abort_flag, 5);
         else mbar_wait(free_bar, (use & 1) ^ 1, abort_flag, 6);
       }
     }
-    if (p.res_mode) {
+    if (Ep::res_mode(p)) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int cc = 4 * h + c;
+      for (int c = 0; c < kCols / 8; ++c) {
+        const int cc = kCols / 8 * h + c;
         const uint4 u = *reinterpret_cast<const uint4*>(srow + ((cc ^ (row & 7)) << 4));
         const T* e = reinterpret_cast<const T*>(&u);
         float s[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) s[i] = to_f(e[i]);
-        if (p.res_mode == 2) {
+        if (Ep::res_mode(p) == 2) {
           const float4 g0 = *reinterpret_cast<const float4*>(wvec + 128 + cc * 8);
           const float4 g1 = *reinterpret_cast<const float4*>(wvec + 132 + cc * 8);
           const float4 b0 = *reinterpret_cast<const float4*>(wvec + 192 + cc * 8);
@@ -174,23 +208,26 @@ __device__ __forceinline__ void epilogue_slab(const TcParams& p, uint8_t* buf, u
       }
     }
     if (se) apply_activation(v, p.act);
-    if (p.out_stats) {
-      float a = 0.f, q = 0.f;
-      const int nh = nb + 32 * h;
-      if (nh + 32 <= p.N) {
+    if (Ep::out_stats(p)) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) { a += v[j]; q = fmaf(v[j], v[j], q); }
-      } else {
+      for (int c = 0; c < kCols; c += 32) {
+        float a = 0.f, q = 0.f;
+        const int nh = nb + kCols * h + c;
+        if (nh + 32 <= p.N) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (nh + j < p.N) { a += v[j]; q = fmaf(v[j], v[j], q); }
+          for (int j = 0; j < 32; ++j) { a += v[c + j]; q = fmaf(v[c + j], v[c + j], q); }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (nh + j < p.N) { a += v[c + j]; q = fmaf(v[c + j], v[c + j], q); }
+        }
+        rc.sum += (double)a;  // 32-column partial sums in fp32, their total in double
+        rc.sumsq += (double)q;
       }
-      rc.sum += (double)a;  // 32-column partial sums in fp32, their total in double
-      rc.sumsq += (double)q;
     }
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int cc = 4 * h + c;
+    for (int c = 0; c < kCols / 8; ++c) {
+      const int cc = kCols / 8 * h + c;
       uint4 o;
       o.x = pack_pair<T>(v[c * 8 + 0], v[c * 8 + 1]);
       o.y = pack_pair<T>(v[c * 8 + 2], v[c * 8 + 3]);
@@ -1044,14 +1081,11 @@ template <int kGroupsT> struct PairCfg {
   static constexpr int kStageBytes = (BM + BN / 2) * BK * 2;  // 32 KB per CTA
   static constexpr int kTmemCols = 512;
   // warp 0 TMA, warp 1 MMA, warps 2 and 3 stores (half of the epilogue groups each), then kGroups epilogue groups of
-  // four warps, each with one staging buffer of 128 rows x 128 bytes: two groups (138 registers per thread; best when
-  // the main loop dominates) or four groups (96 registers; twice the epilogue throughput, for products with few
-  // k-blocks per tile).  The two-group form spends the 32 KB it saves on staging on a fifth pipeline stage: a stage
-  // is refilled only after the MMAs that read it have completed, so with four stages a load has three k-blocks of MMA
-  // time to arrive.  Measured against four stages and two buffers per group, in the network at batch 1024 / 256:
-  // FFN2 (24 k-blocks per tile) 1040 -> 1084 and 872 -> 923 TFLOP/s, out-projection 868 -> 853 and 688 -> 670 (the
-  // residual tile is prefetched one slab ahead instead of two), the whole evaluation +0.9 % and +1.0 %.  Run for
-  // seconds under the power cap the two forms are equal: the clock settles where the power does.
+  // four warps, each with one staging buffer of 128 rows x 128 bytes: two groups (168 registers per thread, whole slabs of 64
+  // columns at a time; best when the main loop dominates) or four groups (96 registers, 32 columns at a time; for products with
+  // few k-blocks per tile, see launch_pair).  The two-group form spends the 32 KB it saves on staging on a fifth pipeline stage: a
+  // stage is refilled only after the MMAs that read it have completed, so with four stages a load has three k-blocks of MMA
+  // time to arrive.
   static constexpr int kGroups = kGroupsT;
   static constexpr int kStages = kGroupsT == 2 ? 5 : 4;
   static constexpr int kBufs = 1;
@@ -1061,7 +1095,7 @@ template <int kGroupsT> struct PairCfg {
                                     4096 /*squeeze-excitation gate and shift*/ + 4096 /*... bias vectors*/;
 };
 
-template <typename T, int kGroups>
+template <typename T, int kGroups, bool kFastIssue, int kMode>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<kGroups>::kThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                     const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_r,
@@ -1180,14 +1214,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (even CTA only) ----------------
-    // With four epilogue groups the MMAs are issued the slower way, a lane index and one commit per CTA.  That is right for
-    // products of four k-blocks, whose tiles finish faster than the epilogue takes them: in place at 1024 positions, slower issue
-    // / elected lane and one commit for both CTAs, smolgen's projection (256 -> 4096) 107.5 / 129 us, the QKV product of the 10 x
-    // 256 attention network at 512 positions 34.3 / 36.4 us, that network 1290 / 1331 us.  (Why a burst of MMAs costs the epilogue that much
-    // was not found out.)  The form also takes the out-projection of the BT4-class network (16 k-blocks, residual and statistics), which
-    // would be faster the other way: 168 / 157 us at 1024 positions, 51.5 / 49.3 at 256.  With two groups the faster issue took 256
-    // positions of that network from 5967 to 5861 us and of the 20 x 256 residual network from 1338 to 1252.
-    constexpr bool kFastIssue = kGroups != 4;
+    // kFastIssue: an elected lane and one commit for both CTAs.  The slower way, a lane index and a commit per CTA, is right for
+    // products of at most eight k-blocks on four epilogue groups, which are paced by their epilogues: the faster MMAs take shared-memory
+    // bandwidth that the epilogue warps then miss.  Slower / faster, us: 32768x768x256 behind a LayerNorm 32.3 / 36.9, 32768x512x256
+    // with Mish 38.3 / 41; the out-projection (16 k-blocks) 41 / 36.4 at 256 positions, 170 / 140 at 1024.
     auto commit = [](uint32_t bar) {
       if constexpr (kFastIssue) {
         tcgen05_commit_both(bar);
@@ -1242,7 +1272,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     ColRegs cr;
     int cr_nb = -1;
     bool se_vec_ok = false;
-    if constexpr (kGroups == 2) {
+    if constexpr (kGroups == 2 && kMode == kAny) {
       if (p.se_k > 0 && 3 * p.N + p.se_k <= 1024) {
         // the squeeze-excitation bias vectors into shared memory while the first tile is computed
         const int eid = (int)threadIdx.x - 128;
@@ -1254,19 +1284,22 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     if (pair < tiles && group * 64 < width_of(pair) && col_of(pair) + group * 64 < p.N) {
       cr_nb = col_of(pair) + group * 64;  // first slab: fetched while the first tile is computed
-      load_col_regs(p, cr_nb, lane, cr);
+      load_col_regs<kMode>(p, cr_nb, lane, cr);
     }
+    auto row_of = [&](int t) { return (tile_of(t) / n_tiles) * (2 * BM) + (int)rank * BM + quarter * 32 + lane; };
+    RowStats row_stats;
+    fetch_row_stats<kMode>(p, row_of(pair), row_stats);
     for (int t = pair; t < tiles; t += pairs, ++tile_it) {
       const uint32_t acc = tile_it & 1, aph = (tile_it >> 1) & 1;
-      const int m0 = (tile_of(t) / n_tiles) * (2 * BM) + (int)rank * BM, n0 = col_of(t), width = width_of(t);
+      const int m = row_of(t), n0 = col_of(t), width = width_of(t);
+      RowCtx rc;
+      use_row_stats<kMode>(p, row_stats, rc);
+      if (t + pairs < tiles) fetch_row_stats<kMode>(p, row_of(t + pairs), row_stats);
       if (!mbar_wait(smem_u32(&tfull_bar[acc]), aph, abort_flag, 4)) break;
       tcgen05_fence_after();
       const uint32_t trow = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
-      const int m = m0 + quarter * 32 + lane;
-      RowCtx rc;
-      load_row_ctx(p, m, rc);
       const float* se_row = nullptr;
-      if constexpr (kGroups == 2) {
+      if constexpr (kGroups == 2 && kMode == kAny) {
         if (p.se_k > 0) {  // this CTA's 128 rows are two boards with all their channels
           se_prepare<BN>(p, trow, quarter, group, lane, (int)threadIdx.x - 128, wvec_all, se_gb, smem_u32(se_bar),
                          se_phase, abort_flag, nullptr, se_vec_ok ? se_vec : nullptr);
@@ -1277,7 +1310,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       for (int c0 = group * 64; c0 < width; c0 += 64 * kGroups) {
         if (n0 + c0 >= p.N) break;  // uniform over the group
         const int idx = group * kBufs + (int)(slab_it % kBufs);
-        if (cr_nb != n0 + c0) load_col_regs(p, n0 + c0, lane, cr);
+        if (cr_nb != n0 + c0) load_col_regs<kMode>(p, n0 + c0, lane, cr);
         // the slab this group handles next: further right in this tile, else the first one of its next tile
         int next_nb = -1;
         if (c0 + 64 * kGroups < width && n0 + c0 + 64 * kGroups < p.N) {
@@ -1287,13 +1320,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           if (nn < p.N) next_nb = nn;
         }
         cr_nb = next_nb;
-        epilogue_slab<T, kGroups == 2>(p, epi_mem + idx * (BM * 128), smem_u32(&res_bar[idx]), smem_u32(&stg_free[idx]),
+        epilogue_slab<T, kGroups == 2 && kMode == kAny, false, kMode, kGroups == 2 && kMode != kAny ? 64 : 32>(p, epi_mem + idx * (BM * 128), smem_u32(&res_bar[idx]), smem_u32(&stg_free[idx]),
                                        smem_u32(&stg_full[idx]), slab_it / kBufs, leader, trow + c0, quarter * 32 + lane,
                                        lane, n0 + c0, next_nb, cr, wvec, rc, abort_flag,
                                        se_row ? se_row + c0 : nullptr);
         ++slab_it;
       }
-      flush_row_ctx(p, m, rc);
+      if (Epilogue<kMode>::out_stats(p)) flush_row_ctx(p, m, rc);
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa(smem_u32(&tempty_bar[acc]), 0));
@@ -1440,15 +1473,15 @@ cudaError_t launch_bn(const GemmParams& g, int* status, int sm_count, cudaStream
 }
 
 
-template <typename T, int kGroups>
-cudaError_t launch_pair(const GemmParams& g, int* status, int sm_count, cudaStream_t s) {
+template <typename T, int kGroups, bool kFastIssue, int kMode>
+cudaError_t launch_pair_mode(const GemmParams& g, int* status, int sm_count, cudaStream_t s) {
   using Cfg = PairCfg<kGroups>;
   static std::atomic<unsigned long long> attr_mask{0};
   int dev = 0;
   cudaError_t de = cudaGetDevice(&dev);
   if (de != cudaSuccess) return de;
   if (!(attr_mask.load() >> (dev & 63) & 1ull)) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<T, kGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<T, kGroups, kFastIssue, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_mask.fetch_or(1ull << (dev & 63));
@@ -1495,8 +1528,31 @@ cudaError_t launch_pair(const GemmParams& g, int* status, int sm_count, cudaStre
     e = get_map(g.W, g.ldw, w_rows, g.K, Cfg::BN / 4, prec, &mwh);
     if (e != cudaSuccess) return e;
   }
-  return launch_dependent(gemm_tc_pair_kernel<T, kGroups>, dim3(2 * pairs), dim3(Cfg::kThreads), Cfg::kSmemBytes, s, ma,
+  return launch_dependent(gemm_tc_pair_kernel<T, kGroups, kFastIssue, kMode>, dim3(2 * pairs), dim3(Cfg::kThreads), Cfg::kSmemBytes, s, ma,
                           mw, mc, mr, mc2, mwh, p);
+}
+
+// Groups of epilogue warps, form of issue and epilogue, from the product's form and k-blocks.  us at two groups / four, slower issue /
+// four, faster issue (M = 64 rows per position):
+//   folded LayerNorm of A  16384x3072x1024 78 / 93 / 85   16384x1536x1024 43 / 51 / 46   32768x768x256 36 / 32 / 37   32768x512x256 43 / 38 / 41
+//   residual, statistics   16384x1024x1024 39 / 41 / 36   16384x1024x1536 48 / 54 / 49   32768x256x256 24 / 22 / 22   32768x256x512 27 / 25 / 25
+//   neither                8192x4096x256 19.5 / 21.7 / 19.6   32768x4096x256 84 / 95 / 87
+// (one kernel that asked for everything at run time: 87, 48.6, 37.5, 41.5; 42, 50.6, 22.9, 25.8; 24.8, 104).
+template <typename T>
+cudaError_t launch_pair(const GemmParams& g, int* status, int sm_count, cudaStream_t s) {
+  const bool few = g.K <= 8 * BK && g.conv_cin == 0 && g.se_k == 0;
+  switch (epilogue_mode(g)) {
+    case kPlain:
+      return launch_pair_mode<T, 2, true, kPlain>(g, status, sm_count, s);
+    case kNormIn:
+      return few ? launch_pair_mode<T, 4, false, kNormIn>(g, status, sm_count, s) : launch_pair_mode<T, 2, true, kNormIn>(g, status, sm_count, s);
+    case kResidual:
+      if (few) return launch_pair_mode<T, 4, false, kResidual>(g, status, sm_count, s);
+      return g.K <= 16 * BK ? launch_pair_mode<T, 4, true, kResidual>(g, status, sm_count, s)
+                            : launch_pair_mode<T, 2, true, kResidual>(g, status, sm_count, s);
+    default:
+      return few ? launch_pair_mode<T, 4, false, kAny>(g, status, sm_count, s) : launch_pair_mode<T, 2, true, kAny>(g, status, sm_count, s);
+  }
 }
 
 }  // namespace
@@ -1676,16 +1732,7 @@ cudaError_t launch_gemm_tc(const GemmParams& p, int* status, int sm_count, cudaS
   if (!gemm_tc_supported(p) || p.skip) return cudaErrorInvalidValue;  // residuals go through `res`
   if (p.n_split > 0 && !gemm_tc_split_supported(p)) return cudaErrorInvalidValue;
   if (!epilogue_supported(p)) return cudaErrorInvalidValue;
-  if (pair_eligible(p, sm_count))
-  {
-    // Four epilogue groups when a tile has few k-blocks (the epilogue then sets the pace), two otherwise (fewer
-    // warps compete with the MMA issuer and the producer).  With a residual input or row statistics a slab costs a
-    // residual fetch, the epilogue and a store in a row, which two groups only hide behind more than 16 k-blocks: the
-    // out-projection (16 k-blocks) went from 838 to 873 TFLOP/s at batch 1024 and from 668 to 723 at batch 256 on four.
-    const bool heavy = p.res != nullptr || p.out_stats != nullptr;
-    const bool four = p.conv_cin == 0 && p.se_k == 0 && (p.K <= 8 * BK || (heavy && p.K <= 16 * BK));
-    return four ? launch_pair<T, 4>(p, status, sm_count, s) : launch_pair<T, 2>(p, status, sm_count, s);
-  }
+  if (pair_eligible(p, sm_count)) return launch_pair<T>(p, status, sm_count, s);
   if (p.se_k > 0) return launch_bn<T, 256>(p, status, sm_count, s);  // the tile must hold every channel of two boards
   // More 128x128 tiles than two per SM: the persistent kernel's wide tiles (256x32768x768, the dense positional encoding of 256
   // positions: 24 us, against 30 on gemm_split.cu's kernel).

@@ -305,13 +305,14 @@ struct TcParams {
   int batch_rows;  // > 0: stacked products, rows [b * batch_rows, (b + 1) * batch_rows) use W rows [b * N, (b + 1) * N)
 };
 
-__device__ __forceinline__ void mean_rstd(const double* stats, long long m, float inv_c, float eps, float& mean,
-                                          float& rstd) {
-  const double2 st = *reinterpret_cast<const double2*>(stats + 2 * m);
+__device__ __forceinline__ void mean_rstd(const double2 st, float inv_c, float eps, float& mean, float& rstd) {
   const double mu = st.x * (double)inv_c;
   const double var = fmax(st.y * (double)inv_c - mu * mu, 0.0);
   mean = (float)mu;
   rstd = rsqrtf((float)var + eps);
+}
+__device__ __forceinline__ void mean_rstd(const double* stats, long long m, float inv_c, float eps, float& mean, float& rstd) {
+  mean_rstd(*reinterpret_cast<const double2*>(stats + 2 * m), inv_c, eps, mean, rstd);
 }
 // Packs two floats into one 32-bit pair of T; fp16 saturates to the largest finite value.
 template <typename T> __device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
