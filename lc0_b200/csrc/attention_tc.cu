@@ -296,6 +296,15 @@ policy_attn_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const fl
   const int pi = tid >> 6, pj = (tid >> 3) & 7, part = tid & 7;  // promotion product and this thread's eighth of a chunk
   float promo = 0.f;
   for (int c = 0; c < steps; ++c) {
+    // this thread's weights of the promotion products, asked for ahead of the wait: behind it each step waited for them too
+    float4 pw[2][2];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int col = c * 128 + half * 64 + part * 8;
+      const float4* w = reinterpret_cast<const float4*>(w4 + pi * dm + (col < dm ? col : 0));
+      pw[half][0] = __ldg(w);
+      pw[half][1] = __ldg(w + 1);
+    }
     asm volatile("cp.async.wait_group %0;" ::"n"(kPolStages - 2) : "memory");
     __syncthreads();  // stage c has landed; every thread is done with the stage that is filled next
     stage_load(c + kPolStages - 1);
@@ -321,7 +330,7 @@ policy_attn_tc_kernel(const T* __restrict__ q, const T* __restrict__ k, const fl
       const uint4 u = *reinterpret_cast<const uint4*>(st + half * kPolChunk + (64 + 56 + pj) * kPolRow + part * 16);
       const T* key = reinterpret_cast<const T*>(&u);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) promo = fmaf(to_f(key[i]), __ldg(w4 + pi * dm + col + i), promo);
+      for (int i = 0; i < 8; ++i) promo = fmaf(to_f(key[i]), reinterpret_cast<const float*>(pw[half])[i], promo);
     }
   }
 #pragma unroll
