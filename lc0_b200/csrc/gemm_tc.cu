@@ -53,14 +53,16 @@ __device__ __forceinline__ void flush_row_ctx(const TcParams& p, int m, const Ro
 // What an epilogue does, known when it is compiled: kAny asks the parameters.  The forms of the encoder's products have kernels of
 // their own: with every question asked at run time an epilogue thread of the four-group form spilled registers.
 enum EpilogueMode { kAny = 0, kPlain = 1 /*bias, activation*/, kNormIn = 2 /*folded LayerNorm of A, bias, activation*/,
-                    kResidual = 3 /*bias, residual (normalised or not), row statistics; no activation*/ };
+                    kResidual = 3 /*bias, residual (normalised or not), row statistics; no activation*/,
+                    kConv = 4 /*convolution: bias, activation; or squeeze-excitation, residual, activation*/ };
 template <int kMode> struct Epilogue {
   static __device__ __forceinline__ bool a_stats(const TcParams& p) { return kMode == kAny ? p.a_stats != nullptr : kMode == kNormIn; }
-  static __device__ __forceinline__ int res_mode(const TcParams& p) { return kMode == kAny || kMode == kResidual ? p.res_mode : 0; }
+  static __device__ __forceinline__ int res_mode(const TcParams& p) { return kMode == kAny || kMode == kResidual || kMode == kConv ? p.res_mode : 0; }
   static __device__ __forceinline__ bool out_stats(const TcParams& p) { return kMode == kAny ? p.out_stats != nullptr : kMode == kResidual; }
 };
 inline int epilogue_mode(const GemmParams& g) {
-  if (g.conv_cin > 0 || g.se_k > 0 || g.batch_rows > 0 || g.scale != 1.0f) return kAny;
+  if (g.batch_rows > 0 || g.scale != 1.0f) return kAny;
+  if (g.conv_cin > 0) return g.a_stats || g.out_stats || g.res_stats || (g.res && g.se_k == 0) ? kAny : kConv;
   if (g.res) return g.out_stats && !g.a_stats && g.act == ACT_NONE ? kResidual : kAny;
   if (g.out_stats) return kAny;
   return g.a_stats ? kNormIn : kPlain;
@@ -268,7 +270,7 @@ __device__ __forceinline__ void epilogue_barrier(uint32_t bar, uint32_t& phase, 
 // gate = sigmoid(z[:C]), shift = z[C:] + gate * conv bias.  Runs on the eight epilogue warps while the accumulator
 // stays in tensor memory; `gb` receives [2 boards][gate 256 | shift 256].  `tmp` is the per-warp scratch area of the
 // slabs (2048 floats), free between two tiles.
-template <int BN>
+template <int BN, int kGroups = 2>
 __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int quarter, int group, int lane, int eid,
                                            float* tmp, float* gb, uint32_t bar, uint32_t& phase,
                                            volatile int* abort_flag, const float* w_smem = nullptr,
@@ -289,7 +291,7 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
   const int C = p.N;
   epilogue_barrier(bar, phase, abort_flag);  // nobody still reads the previous tile's per-warp vectors in `tmp`
 #pragma unroll 1
-  for (int c0 = group * 64; c0 < BN; c0 += 128) {
+  for (int c0 = group * 64; c0 < BN; c0 += 64 * kGroups) {
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
       uint32_t r[32];
@@ -303,8 +305,8 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
     }
   }
   epilogue_barrier(bar, phase, abort_flag);
-  {
-    const int c = eid;  // 256 threads, one channel each
+  if (kGroups == 2 || eid < 256) {
+    const int c = eid;  // one channel per thread
     const float b = c < C ? ld(g_bias + c) : 0.f;
     pool[c] = (part[c] + part[256 + c]) * (1.0f / 64.0f) + b;
     pool[256 + c] = (part[512 + c] + part[768 + c]) * (1.0f / 64.0f) + b;
@@ -313,7 +315,7 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
   // hid[s][k]: four threads per output, a quarter of the channels each (C is a multiple of 16 and se_k of 4, so the
   // quads of a warp run the same trip count).  The weights come from L2: 16-byte loads, several in flight, so that
   // the whole dot product costs about one round trip.
-  for (int o = eid >> 2; o < 2 * p.se_k; o += 64) {
+  for (int o = eid >> 2; o < 2 * p.se_k; o += 32 * kGroups) {
     const int sidx = o / p.se_k, k = o - sidx * p.se_k;
     // the four threads of an output take every fourth 16-byte piece of the row: consecutive addresses (no bank
     // conflicts in shared memory, whole lines per quad in global memory)
@@ -352,7 +354,7 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
     const float ga = 1.0f / (1.0f + expf(-z0a)), gbb = 1.0f / (1.0f + expf(-z0b));
     gb[c] = ga; gb[256 + c] = z1a + ga * cb;
     gb[512 + c] = gbb; gb[768 + c] = z1b + gbb * cb;
-  } else {
+  } else if (kGroups == 2 || eid < 256) {
     gb[eid] = 0.f; gb[256 + eid] = 0.f; gb[512 + eid] = 0.f; gb[768 + eid] = 0.f;
   }
   epilogue_barrier(bar, phase, abort_flag);
@@ -762,24 +764,27 @@ struct TowerCfg {
                                     kSeWBytes;
 };
 
-// The tiles of one CTA in the order it computes them.  With more row blocks than CTAs (gridDim.x * 2 <= row blocks
-// + 1) a CTA takes its blocks two at a time and, for such a pair, goes layer by layer, alternating between the two
-// blocks: a tile then depends on the tile before the previous one, so the wait for a block's stores and for the next
-// layer's first loads falls under the other block's main loop (9.3 us per tile against 13.8; measured on a tower of 128
-// filters).  With fewer blocks each CTA has one: all layers of a block take 21 x 13.8 us, of a pair 21 x 18.5 us.
+// The tiles of one CTA in the order it computes them.  A CTA takes its row blocks up to eight at a time and goes layer by layer
+// over them: a tile then depends on a tile several before it, so the wait for a block's stores, for the next layer's first
+// loads and the epilogue fall under the other blocks' main loops.  Of a tower of 10 x 128 a tile takes 10 us when it is alone, 6.5
+// among two blocks and 5.9 among five or six (two at a time, with the table read from global memory: 10.6, 7.0 and 6.7): what is
+// left is the main loop's operand traffic (32 KB per k-block, 460 cycles).  Towers of 64 / 700 / 1500 positions 222 / 509 / 838 -> 200 / 378 / 746 us.
+constexpr int kTowerBlocks = 8;
 struct TowerWalk {
   int n_layers, first, step, nb;  // nb: row blocks of this CTA
-  int i0 = 0, l = 0, j = 0;       // index of the pair's first block among the CTA's blocks, layer, block of the pair
+  int i0 = 0, l = 0, j = 0;       // index of the group's first block among the CTA's blocks, layer, block of the group
   __device__ TowerWalk(int n_layers_, int row_blocks) : n_layers(n_layers_), first(blockIdx.x), step(gridDim.x) {
     nb = first < row_blocks ? (row_blocks - first + step - 1) / step : 0;
   }
   __device__ bool valid() const { return i0 < nb; }
   __device__ int rb() const { return first + (i0 + j) * step; }
-  __device__ int cnt() const { return nb - i0 >= 2 ? 2 : 1; }  // a CTA with one block (grid = row blocks) never pairs
+  __device__ int cnt() const { return nb - i0 < kTowerBlocks ? nb - i0 : kTowerBlocks; }
+  // tiles of the j-th block of its group (this one and the groups before, which are full) ahead of this tile
+  __device__ uint32_t before() const { return (uint32_t)(i0 / kTowerBlocks * n_layers + l); }
   __device__ void next() {
     if (++j >= cnt()) {
       j = 0;
-      if (++l >= n_layers) { l = 0; i0 += 2; }
+      if (++l >= n_layers) { l = 0; i0 += kTowerBlocks; }
     }
   }
 };
@@ -848,7 +853,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
   uint64_t* stg_full = reinterpret_cast<uint64_t*>(bar_mem + 256);  // [2 groups][2 buffers] slab staged (4 warps)
   uint64_t* stg_free = stg_full + 4;                                // [2 groups][2 buffers] store has read the buffer
   uint64_t* se_bar = reinterpret_cast<uint64_t*>(bar_mem + 384);    // barrier of the 256 epilogue threads
-  uint64_t* done_bar = se_bar + 1;                                  // [2] the latest tile of block 0 / 1 of the pair is in memory
+  uint64_t* done_bar = se_bar + 1;                                  // [kTowerBlocks] the latest tile of a group's block is in memory
   float* wvec_all = reinterpret_cast<float*>(bar_mem + 512);        // 8 warps x 256 floats
   float* wvec = wvec_all + ((threadIdx.x >> 5) & 7) * 256;
   float* se_gb = reinterpret_cast<float*>(bar_mem + 512 + 8192);    // [2 boards][gate 256 | shift 256]
@@ -878,8 +883,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
       mbar_init(smem_u32(&stg_free[i]), 1);
     }
     mbar_init(smem_u32(se_bar), 256);
-    mbar_init(smem_u32(&done_bar[0]), 1);
-    mbar_init(smem_u32(&done_bar[1]), 1);
+    for (int i = 0; i < kTowerBlocks; ++i) mbar_init(smem_u32(&done_bar[i]), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -899,15 +903,16 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (elect_one()) {
-      uint32_t it = 0, nslot[2] = {0, 0};  // nslot: tiles issued per block of the pair
+      uint32_t it = 0;
       bool ok = true;
       for (TowerWalk w(n_layers, row_blocks); w.valid() && ok; w.next()) {
         const TowerLayer& L = layers[w.l];
         const int rb = w.rb();
         const int cblocks = L.p.conv_cblocks, k_blocks = 9 * cblocks, N = L.p.N;
-        // The filters do not depend on this CTA's earlier output: those of the first stages are requested before
-        // the wait for it.
-        const int early = k_blocks < S ? k_blocks : S;
+        // The filters do not depend on this CTA's earlier output: where that is still on its way (the first layer reads what was
+        // complete before the launch), those of the first stages are requested before the wait for it.
+        const bool ready = w.l == 0 || mbar_try_wait(smem_u32(&done_bar[w.j]), (w.before() - 1) & 1);
+        const int early = ready ? 0 : k_blocks < S ? k_blocks : S;
         for (int kb = 0; kb < early && ok; ++kb) {
           const int s = (it + kb) % S;
           const uint32_t ph = ((it + kb) / S) & 1;
@@ -918,9 +923,8 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
           tma_load_2d(smem_u32(smem + s * Cfg::kStageBytes) + BM * BK * 2, &L.w, cb * BK, tap * N, fb);
         }
         if (!ok) break;
-        const uint32_t nth = nslot[w.j]++;
-        if (w.l > 0) {  // the block's previous layer (the first layer reads what was complete before the launch)
-          if (!mbar_wait(smem_u32(&done_bar[w.j]), (nth - 1) & 1, abort_flag, 9)) break;
+        if (w.l > 0) {  // the block's previous layer
+          if (!ready && !mbar_wait(smem_u32(&done_bar[w.j]), (w.before() - 1) & 1, abort_flag, 9)) break;
           fence_proxy_async_all();
         }
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
@@ -982,7 +986,12 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
     int se_layer = -1;  // layer whose squeeze-excitation parameters sit in shared memory
     {
       for (TowerWalk w(n_layers, row_blocks); w.valid(); w.next(), ++tile_it) {
-        const TcParams& P = layers[w.l].p;
+        // what a tower's layers have, in registers: the table lies in global memory
+        const TcParams& table = layers[w.l].p;
+        TcParams P = {};
+        P.bias = table.bias; P.M = table.M; P.N = table.N; P.act = table.act; P.scale = 1.0f; P.alpha = table.alpha;
+        P.res_mode = table.res_mode; P.se_k = table.se_k;
+        P.se_w1 = table.se_w1; P.se_b1 = table.se_b1; P.se_w2 = table.se_w2; P.se_b2 = table.se_b2; P.se_bias = table.se_bias;
         const int rb = w.rb();
         const uint32_t acc = tile_it & 1, aph = (tile_it >> 1) & 1;
         if (group * 64 < P.N) load_col_regs(P, group * 64, lane, cr);  // in flight while the tile is computed
@@ -1014,10 +1023,8 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
         }
         if (!mbar_wait(smem_u32(&tfull_bar[acc]), aph, abort_flag, 4)) break;
         tcgen05_fence_after();
-        const int m = rb * BM + quarter * 32 + lane;
         const uint32_t trow = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
         RowCtx rc;
-        load_row_ctx(P, m, rc);
         const float* se_row = nullptr;
         if (P.se_k > 0) {
           se_prepare<BN>(P, trow, quarter, group, lane, (int)threadIdx.x - 64, wvec_all, se_gb, smem_u32(se_bar), se_phase,
@@ -1030,7 +1037,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
           const int b = (int)(slab_it % kBufs);
           const int idx = group * kBufs + b;
           const int next_nb = (c0 + 128 < BN && c0 + 128 < P.N) ? c0 + 128 : -1;
-          epilogue_slab<T, true, true>(P, gbuf + b * (BM * 128), smem_u32(&res_bar[idx]), smem_u32(&stg_free[idx]),
+          epilogue_slab<T, true, true, kAny, 64>(P, gbuf + b * (BM * 128), smem_u32(&res_bar[idx]), smem_u32(&stg_free[idx]),
                                        smem_u32(&stg_full[idx]), slab_it / kBufs, leader, trow + c0, quarter * 32 + lane, lane,
                                        c0, next_nb, cr, wvec, rc, abort_flag, se_row ? se_row + c0 : nullptr,
                                        b ? res_use1 : res_use0);
@@ -1039,7 +1046,6 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
           }
           ++slab_it;
         }
-        flush_row_ctx(P, m, rc);
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
@@ -1272,13 +1278,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     ColRegs cr;
     int cr_nb = -1;
     bool se_vec_ok = false;
-    if constexpr (kGroups == 2 && kMode == kAny) {
+    if constexpr ((kGroups == 2 && kMode == kAny) || kMode == kConv) {
       if (p.se_k > 0 && 3 * p.N + p.se_k <= 1024) {
         // the squeeze-excitation bias vectors into shared memory while the first tile is computed
         const int eid = (int)threadIdx.x - 128;
-        for (int i = eid; i < p.N; i += 256) se_vec[i] = __ldg(p.se_bias + i);
-        for (int i = eid; i < p.se_k; i += 256) se_vec[p.N + i] = __ldg(p.se_b1 + i);
-        for (int i = eid; i < 2 * p.N; i += 256) se_vec[p.N + p.se_k + i] = __ldg(p.se_b2 + i);
+        for (int i = eid; i < p.N; i += 128 * kGroups) se_vec[i] = __ldg(p.se_bias + i);
+        for (int i = eid; i < p.se_k; i += 128 * kGroups) se_vec[p.N + i] = __ldg(p.se_b1 + i);
+        for (int i = eid; i < 2 * p.N; i += 128 * kGroups) se_vec[p.N + p.se_k + i] = __ldg(p.se_b2 + i);
         se_vec_ok = true;
       }
     }
@@ -1299,9 +1305,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       tcgen05_fence_after();
       const uint32_t trow = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
       const float* se_row = nullptr;
-      if constexpr (kGroups == 2 && kMode == kAny) {
+      if constexpr ((kGroups == 2 && kMode == kAny) || kMode == kConv) {
         if (p.se_k > 0) {  // this CTA's 128 rows are two boards with all their channels
-          se_prepare<BN>(p, trow, quarter, group, lane, (int)threadIdx.x - 128, wvec_all, se_gb, smem_u32(se_bar),
+          se_prepare<BN, kGroups>(p, trow, quarter, group, lane, (int)threadIdx.x - 128, wvec_all, se_gb, smem_u32(se_bar),
                          se_phase, abort_flag, nullptr, se_vec_ok ? se_vec : nullptr);
           se_row = se_gb + (quarter >> 1) * 512;
         }
@@ -1320,7 +1326,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           if (nn < p.N) next_nb = nn;
         }
         cr_nb = next_nb;
-        epilogue_slab<T, kGroups == 2 && kMode == kAny, false, kMode, kGroups == 2 && kMode != kAny ? 64 : 32>(p, epi_mem + idx * (BM * 128), smem_u32(&res_bar[idx]), smem_u32(&stg_free[idx]),
+        epilogue_slab<T, (kGroups == 2 && kMode == kAny) || kMode == kConv, false, kMode,
+                      kGroups == 2 && kMode != kAny && kMode != kConv ? 64 : 32>(p, epi_mem + idx * (BM * 128), smem_u32(&res_bar[idx]), smem_u32(&stg_free[idx]),
                                        smem_u32(&stg_full[idx]), slab_it / kBufs, leader, trow + c0, quarter * 32 + lane,
                                        lane, n0 + c0, next_nb, cr, wvec, rc, abort_flag,
                                        se_row ? se_row + c0 : nullptr);
@@ -1494,7 +1501,7 @@ cudaError_t launch_pair_mode(const GemmParams& g, int* status, int sm_count, cud
   const int w_rows = conv ? 9 * g.N : (g.batch_rows > 0 ? g.N * (g.M / g.batch_rows) : g.N);
   e = get_map(g.W, conv ? g.conv_cin : g.ldw, w_rows, conv ? g.conv_cin : g.K, Cfg::BN / 2, prec, &mw);
   if (e != cudaSuccess) return e;
-  if (g.se_k > 0 && (kGroups != 2 || !gemm_tc_se_supported(g))) return cudaErrorInvalidValue;
+  if (g.se_k > 0 && ((kGroups != 2 && kMode != kConv) || !gemm_tc_se_supported(g))) return cudaErrorInvalidValue;
   e = get_map(g.C, g.ldc, g.M, g.n_split > 0 ? g.n_split : g.N, BM, prec, &mc);
   if (e != cudaSuccess) return e;
   CUtensorMap mr = mc, mc2 = mc;
@@ -1550,6 +1557,8 @@ cudaError_t launch_pair(const GemmParams& g, int* status, int sm_count, cudaStre
       if (few) return launch_pair_mode<T, 4, false, kResidual>(g, status, sm_count, s);
       return g.K <= 16 * BK ? launch_pair_mode<T, 4, true, kResidual>(g, status, sm_count, s)
                             : launch_pair_mode<T, 2, true, kResidual>(g, status, sm_count, s);
+    case kConv:
+      return launch_pair_mode<T, 2, true, kConv>(g, status, sm_count, s);
     default:
       return few ? launch_pair_mode<T, 4, false, kAny>(g, status, sm_count, s) : launch_pair_mode<T, 2, true, kAny>(g, status, sm_count, s);
   }
@@ -1709,7 +1718,7 @@ cudaError_t launch_gemm_tower(const void* d_layers, int n_layers, int channels, 
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  // one row block per CTA while there are SMs for that, two at a time beyond (see TowerWalk)
+  // one row block per CTA while there are SMs for that, several at a time beyond (see TowerWalk)
   const int want = row_blocks <= sm_count ? row_blocks : (row_blocks + 1) / 2;
   const int grid = want < sm_count ? want : sm_count;
   const TowerLayer* layers = static_cast<const TowerLayer*>(d_layers);

@@ -221,6 +221,22 @@ def test_results_do_not_depend_on_the_batch_from_64_positions_on(precision, side
     nw.close()
 
 
+@pytest.mark.parametrize("batch", [295, 297, 600, 1189, 2368])
+def test_tower_with_several_row_blocks_per_cta(batch):
+    """One block of two boards per CTA, two, three, up to eight at a time and a ragged last group: the same bits per position."""
+    net = mknet.make_net("cfg1", blocks=3)
+    _, pos, n, g = load_compact("cfg4_2layer_b1024")
+    idx = np.arange(batch) % 1000
+    masks, values = np.array(pos["masks"]), np.array(pos["values"])
+    nw = network.Network(net, "precision=fp16,max_batch=2368")
+    few, out = nw.evaluate(masks[:200], values[:200]), nw.evaluate(masks[idx], values[idx])
+    assert nw.device_status() == 0
+    nw.close()
+    for k in ("policy", "q", "d"):
+        np.testing.assert_array_equal(out[k][idx < 200], few[k][idx[idx < 200]])
+        np.testing.assert_array_equal(out[k], out[k][np.minimum(idx, batch - 1)])
+
+
 @pytest.mark.parametrize("precision", ["fp16", "bf16"])
 @pytest.mark.parametrize("name", ["cfg4_2layer", "cfg3", "cfg2_mini", "cfg4_mini"])
 def test_results_do_not_depend_on_the_batch_below_64_positions(name, precision):
