@@ -773,7 +773,8 @@ constexpr int kTowerBlocks = 8;
 struct TowerWalk {
   int n_layers, first, step, nb;  // nb: row blocks of this CTA
   int i0 = 0, l = 0, j = 0;       // index of the group's first block among the CTA's blocks, layer, block of the group
-  __device__ TowerWalk(int n_layers_, int row_blocks) : n_layers(n_layers_), first(blockIdx.x), step(gridDim.x) {
+  __device__ TowerWalk(int n_layers_, int row_blocks, int first_ = blockIdx.x, int step_ = gridDim.x)
+      : n_layers(n_layers_), first(first_), step(step_) {
     nb = first < row_blocks ? (row_blocks - first + step - 1) / step : 0;
   }
   __device__ bool valid() const { return i0 < nb; }
@@ -1357,6 +1358,251 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// The tower kernel for 192 and 256 channels, on CTA pairs: a pair owns four boards, a CTA two of them, and a layer is one
+// 256 x N tile of cta_group::2 MMAs.  A CTA reads as A only rows it stored itself and supplies half of the filters, so the two meet in
+// the operand barriers alone.  Against one launch per convolution (pair kernel, one tile per pair: no main loop to hide
+// launch, first loads, epilogue and stores under) the whole evaluation of the 20 x 256 network
+// takes, us, launch per convolution / tower: 16 boards 1022 / 907, 256 1245 / 1169, 592 2059 / 1879, 1024 3590 / 3524, 1500
+// 5299 / 5384, 2048 6833 / 6742 (a layer of 256 boards: 20.8 us).  The squeeze-excitation matrices
+// (96 KB at 256 channels and 32 hidden units) do not fit beside the pipeline and come from L2, its vectors are copied per layer.
+// ------------------------------------------------------------------------------------------------
+template <typename T>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<2>::kThreads, 1)
+gemm_tc_pair_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int row_blocks, int* status) {
+  using Cfg = PairCfg<2>;
+  constexpr int S = Cfg::kStages, BN = Cfg::BN;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* epi_mem = smem + S * Cfg::kStageBytes;
+  uint8_t* bar_mem = epi_mem + Cfg::kEpiBytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(bar_mem);  // [S]  waited on by the even CTA only
+  uint64_t* empty_bar = full_bar + S;                          // [S]  per CTA
+  uint64_t* tfull_bar = empty_bar + S;                         // [2]  per CTA
+  uint64_t* tempty_bar = tfull_bar + 2;                        // [2]  even CTA: one arrival per epilogue warp of both CTAs
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* res_bar = reinterpret_cast<uint64_t*>(bar_mem + 192);   // [2] skip slab landed
+  uint64_t* stg_full = reinterpret_cast<uint64_t*>(bar_mem + 256);  // [2] slab staged (4 warps)
+  uint64_t* stg_free = stg_full + 2;                                // [2] store has read the buffer
+  uint64_t* se_bar = reinterpret_cast<uint64_t*>(bar_mem + 384);
+  uint64_t* done_bar = se_bar + 1;                                  // [kTowerBlocks] the latest tile of a group's block is in memory
+  float* wvec_all = reinterpret_cast<float*>(bar_mem + 512);
+  float* wvec = wvec_all + ((threadIdx.x >> 5) & 15) * 256;
+  float* se_gb = reinterpret_cast<float*>(bar_mem + 512 + 16 * 1024);
+  float* se_vec = se_gb + 1024;
+
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  if (threadIdx.x == 64) {
+    for (int l = 0; l < n_layers; ++l) {
+      tma_prefetch_map(&layers[l].a);
+      tma_prefetch_map(&layers[l].w);
+      tma_prefetch_map(&layers[l].c);
+      if (layers[l].p.res_mode) tma_prefetch_map(&layers[l].r);
+    }
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S; ++i) {
+      mbar_init(smem_u32(&full_bar[i]), 1);
+      mbar_init(smem_u32(&empty_bar[i]), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&tfull_bar[i]), 1);
+      mbar_init(smem_u32(&tempty_bar[i]), 16);
+      mbar_init(smem_u32(&res_bar[i]), 1);
+      mbar_init(smem_u32(&stg_full[i]), 4);
+      mbar_init(smem_u32(&stg_free[i]), 1);
+    }
+    mbar_init(smem_u32(se_bar), 256);
+    for (int i = 0; i < kTowerBlocks; ++i) mbar_init(smem_u32(&done_bar[i]), 2);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"((uint32_t)Cfg::kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the peer's barriers are initialised before anything arrives on them
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_wait();
+  grid_launch_dependents();
+
+  if (warp == 0) {
+    // ---------------- TMA producer (both CTAs) ----------------
+    if (elect_one()) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (TowerWalk w(n_layers, row_blocks, pair, pairs); w.valid() && ok; w.next()) {
+        const TowerLayer& L = layers[w.l];
+        const int board = w.rb() * 4 + (int)rank * 2;
+        const int cblocks = L.p.conv_cblocks, k_blocks = 9 * cblocks, N = L.p.N, n0 = (int)rank * (N / 2);
+        const bool ready = w.l == 0 || mbar_try_wait(smem_u32(&done_bar[w.j]), (w.before() - 1) & 1);
+        const int early = ready ? 0 : k_blocks < S ? k_blocks : S;  // filters ahead of rows that are still on their way
+        auto load_w = [&](int kb, int s) {
+          if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * Cfg::kStageBytes);  // both CTAs' bytes land there
+          const int tap = kb / cblocks, cb = kb - tap * cblocks;
+          tma_load_2d_pair(smem_u32(smem + s * Cfg::kStageBytes) + BM * BK * 2, &L.w, cb * BK, tap * N + n0,
+                           mapa(smem_u32(&full_bar[s]), 0));
+        };
+        for (int kb = 0; kb < early && ok; ++kb) {
+          const int s = (it + kb) % S;
+          if (!mbar_wait(smem_u32(&empty_bar[s]), (((it + kb) / S) & 1) ^ 1, abort_flag, 1)) { ok = false; break; }
+          load_w(kb, s);
+        }
+        if (!ok) break;
+        if (w.l > 0) {  // the block's previous layer
+          if (!ready && !mbar_wait(smem_u32(&done_bar[w.j]), (w.before() - 1) & 1, abort_flag, 9)) break;
+          fence_proxy_async_all();
+        }
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          const int s = it % S;
+          if (kb >= early) {
+            if (!mbar_wait(smem_u32(&empty_bar[s]), ((it / S) & 1) ^ 1, abort_flag, 1)) { ok = false; break; }
+            load_w(kb, s);
+          }
+          const int tap = kb / cblocks, cb = kb - tap * cblocks;
+          tma_load_4d_pair(smem_u32(smem + s * Cfg::kStageBytes), &L.a, cb * BK, tap % 3 - 1, tap / 3 - 1, board,
+                           mapa(smem_u32(&full_bar[s]), 0));
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (even CTA only) ----------------
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc_base = (1u << 4) | (FmtCode<T>::v << 7) | (FmtCode<T>::v << 10) | ((uint32_t)((2 * BM) >> 4) << 24);
+      uint32_t it = 0, tile_it = 0;
+      bool ok = true;
+      for (TowerWalk w(n_layers, row_blocks, pair, pairs); w.valid() && ok; w.next(), ++tile_it) {
+        const int k_blocks = 9 * layers[w.l].p.conv_cblocks;
+        const uint32_t idesc = idesc_base | ((uint32_t)(layers[w.l].p.N >> 3) << 17);
+        const uint32_t acc = tile_it & 1, aph = (tile_it >> 1) & 1;
+        if (!mbar_wait(smem_u32(&tempty_bar[acc]), aph ^ 1, abort_flag, 2)) break;
+        tcgen05_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * BN;
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          const int s = it % S;
+          if (!mbar_wait(smem_u32(&full_bar[s]), (it / S) & 1, abort_flag, 3)) { ok = false; break; }
+          tcgen05_fence_after();
+          const uint32_t sa = smem_u32(smem + s * Cfg::kStageBytes);
+          const uint64_t adesc = make_smem_desc(sa), bdesc = make_smem_desc(sa + BM * BK * 2);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            tcgen05_mma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          tcgen05_commit_both(smem_u32(&empty_bar[s]));
+        }
+        if (ok) tcgen05_commit_both(smem_u32(&tfull_bar[acc]));
+      }
+    }
+  } else if (warp == 2 || warp == 3) {
+    // ---------------- store warps (both CTAs): the slabs of one epilogue group each ----------------
+    if (elect_one()) {
+      const int g = warp - 2;
+      const uint32_t buf = smem_u32(epi_mem + g * (BM * 128));
+      uint32_t count = 0;
+      bool ok = true;
+      // The skip input of a slab goes into the staging buffer that the slab will use, once the store before it has read that.
+      // Its source is the block's output of two layers ago, columns that this thread stored itself.
+      auto fetch = [&](const TowerLayer& L, int c0, int row) {
+        const uint32_t bar = smem_u32(&res_bar[g]);
+        mbar_expect_tx(bar, BM * 128);
+        tma_load_2d(buf, &L.r, c0, row, bar);
+      };
+      for (TowerWalk w(n_layers, row_blocks, pair, pairs); w.valid() && ok; w.next()) {
+        const TowerLayer& L = layers[w.l];
+        const int N = L.p.N, row = w.rb() * (2 * BM) + (int)rank * BM;
+        for (int c0 = g * 64; c0 < N; c0 += 128, ++count) {
+          if (!mbar_wait(smem_u32(&stg_full[g]), count & 1, abort_flag, 7)) { ok = false; break; }
+          tma_store_2d(&L.c, c0, row, buf);
+          tma_store_commit();
+          tma_store_wait_read0();
+          if (c0 + 128 < N) {
+            if (L.p.res_mode) fetch(L, c0 + 128, row);
+            mbar_arrive(smem_u32(&stg_free[g]));
+          }
+        }
+        if (!ok) break;
+        tma_store_wait_all0();    // this group's columns of the tile are in memory
+        fence_proxy_async_all();  // ... before the loads of the block's next layer, which the producer issues after the arrival
+        mbar_arrive(smem_u32(&done_bar[w.j]));
+        TowerWalk nx = w;
+        nx.next();
+        if (nx.valid() && layers[nx.l].p.res_mode) fetch(layers[nx.l], g * 64, nx.rb() * (2 * BM) + (int)rank * BM);
+        mbar_arrive(smem_u32(&stg_free[g]));
+      }
+      tma_store_wait_read0();
+    }
+  } else {
+    // ---------------- epilogue (warps 4..11 of both CTAs: two groups of four warps, alternating 64-column slabs) ----------------
+    const int quarter = warp & 3, group = (warp - 4) >> 2, eid = (int)threadIdx.x - 128;
+    const bool leader = ((warp - 4) & 3) == 0 && lane == 0;
+    uint32_t tile_it = 0, slab_it = 0, se_phase = 0, res_use = 0;
+    ColRegs cr;
+    int se_layer = -1;
+    for (TowerWalk w(n_layers, row_blocks, pair, pairs); w.valid(); w.next(), ++tile_it) {
+      // what a tower's layers have, in registers: the table lies in global memory
+      const TcParams& table = layers[w.l].p;
+      TcParams P = {};
+      P.bias = table.bias; P.M = table.M; P.N = table.N; P.act = table.act; P.scale = 1.0f; P.alpha = table.alpha;
+      P.res_mode = table.res_mode; P.se_k = table.se_k;
+      P.se_w1 = table.se_w1; P.se_b1 = table.se_b1; P.se_w2 = table.se_w2; P.se_b2 = table.se_b2; P.se_bias = table.se_bias;
+      const uint32_t acc = tile_it & 1, aph = (tile_it >> 1) & 1;
+      load_col_regs(P, group * 64, lane, cr);  // in flight while the tile is computed
+      const bool vec = P.se_k > 0 && 3 * P.N + P.se_k <= 1024;
+      if (vec && se_layer != w.l) {
+        // The previous user of the region finished behind the last barrier of its se_prepare; the first barrier of this one
+        // orders the stores below before the reads.
+        for (int i = eid; i < P.N; i += 256) se_vec[i] = __ldg(P.se_bias + i);
+        for (int i = eid; i < P.se_k; i += 256) se_vec[P.N + i] = __ldg(P.se_b1 + i);
+        for (int i = eid; i < 2 * P.N; i += 256) se_vec[P.N + P.se_k + i] = __ldg(P.se_b2 + i);
+        se_layer = w.l;
+      }
+      if (!mbar_wait(smem_u32(&tfull_bar[acc]), aph, abort_flag, 4)) break;
+      tcgen05_fence_after();
+      const uint32_t trow = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
+      RowCtx rc;
+      const float* se_row = nullptr;
+      if (P.se_k > 0) {
+        se_prepare<BN>(P, trow, quarter, group, lane, eid, wvec_all, se_gb, smem_u32(se_bar), se_phase, abort_flag, nullptr,
+                       vec ? se_vec : nullptr);
+        se_row = se_gb + (quarter >> 1) * 512;
+      }
+#pragma unroll 1
+      for (int c0 = group * 64; c0 < P.N; c0 += 128) {
+        epilogue_slab<T, true, true, kAny, 32>(P, epi_mem + group * (BM * 128), smem_u32(&res_bar[group]), smem_u32(&stg_free[group]),
+                                               smem_u32(&stg_full[group]), slab_it, leader, trow + c0, quarter * 32 + lane, lane, c0,
+                                               c0 + 128 < P.N ? c0 + 128 : -1, cr, wvec, rc, abort_flag, se_row ? se_row + c0 : nullptr,
+                                               res_use);
+        if (P.res_mode) ++res_use;
+        ++slab_it;
+      }
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(mapa(smem_u32(&tempty_bar[acc]), 0));
+    }
+  }
+
+  __syncwarp();
+  tcgen05_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    if (threadIdx.x == 0 && status) atomicCAS(status, 0, 700 + *abort_flag);
+    __syncthreads();
+  }
+  cluster_sync_all();  // neither CTA releases tensor or shared memory while its peer may still touch it
+  if (warp == 1) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)Cfg::kTmemCols) : "memory");
+  }
+}
+
 // ---- host side ------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1672,7 +1918,7 @@ bool gemm_tc_tower_supported(const GemmParams* g, int n) {
     if (p.conv_cin <= 0 || !gemm_tc_supported(p) || !tma_ok || p.skip || p.n_split > 0 || p.batch_rows > 0 || p.a_stats ||
         p.out_stats || p.res_stats)
       return false;
-    if (p.M != g[0].M || p.N != g[0].N || p.N > TowerCfg::BN || (p.N % 64) != 0) return false;
+    if (p.M != g[0].M || p.N != g[0].N || p.N > 2 * TowerCfg::BN || (p.N % 64) != 0) return false;
     if (p.se_k > 0 && !gemm_tc_se_supported(p)) return false;
     if (p.res && ((p.ldres % 8) != 0 || (reinterpret_cast<uintptr_t>(p.res) & 15) != 0)) return false;
     // a layer reads what an earlier layer of the same CTA wrote, or something complete before the launch; the skip
@@ -1718,11 +1964,22 @@ cudaError_t launch_gemm_tower(const void* d_layers, int n_layers, int channels, 
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
+  const TowerLayer* layers = static_cast<const TowerLayer*>(d_layers);
+  if (channels > 2 * TowerCfg::BN) return cudaErrorInvalidValue;
+  if (channels > TowerCfg::BN) {
+    static std::atomic<unsigned long long> pair_mask{0};
+    if (!(pair_mask.load() >> (dev & 63) & 1ull)) {
+      e = cudaFuncSetAttribute(gemm_tc_pair_tower_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<2>::kSmemBytes);
+      if (e != cudaSuccess) return e;
+      pair_mask.fetch_or(1ull << (dev & 63));
+    }
+    const int blocks = (row_blocks + 1) / 2, pairs = blocks < sm_count / 2 ? blocks : sm_count / 2;
+    return launch_dependent(gemm_tc_pair_tower_kernel<T>, dim3(2 * pairs), dim3(PairCfg<2>::kThreads), PairCfg<2>::kSmemBytes, s, layers,
+                            n_layers, blocks, status);
+  }
   // one row block per CTA while there are SMs for that, several at a time beyond (see TowerWalk)
   const int want = row_blocks <= sm_count ? row_blocks : (row_blocks + 1) / 2;
   const int grid = want < sm_count ? want : sm_count;
-  const TowerLayer* layers = static_cast<const TowerLayer*>(d_layers);
-  if (channels > TowerCfg::BN) return cudaErrorInvalidValue;
   static std::atomic<unsigned long long> mask{0};
   if (!(mask.load() >> (dev & 63) & 1ull)) {
     e = cudaFuncSetAttribute(gemm_tc_tower_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, TowerCfg::kSmemBytes);

@@ -1308,9 +1308,9 @@ struct Net : NetBase {
   void build_towers() {
     if constexpr (sizeof(T) == 2) {
       // Measured (evaluations per second, tower / per-layer launches): 10 blocks of 128 filters 176 100 / 161 400 at
-      // batch 64 and 670 800 / 589 000 at batch 256; 20 blocks of 256 filters 57 100 / 55 300 at batch 64 and 210 100 /
-      // 212 300 at batch 256: the wide tower stays on one launch per convolution (CTA pairs from 150 positions on).
-      if (!tower || res.empty() || C > 128) { tower = false; return; }
+      // batch 64 and 670 800 / 589 000 at batch 256; 20 blocks of 256 filters, whose tower kernel works on CTA pairs,
+      // 68 300 / 59 400 at batch 64, 219 000 / 205 300 at 256, 304 000 / 300 000 at 2048.
+      if (!tower || res.empty() || C > 256) { tower = false; return; }
       for (const auto& r : res)
         if (!r.se) { tower = false; return; }
       const int nb = opt.max_batch;
@@ -1331,7 +1331,8 @@ struct Net : NetBase {
         CK(cudaMemcpy(s.tower_layers, host.data(), host.size(), cudaMemcpyHostToDevice));
         s.tower_n = (int)g.size();
       }
-      // one CTA per two boards walks all layers: worth it while the launches it replaces are latency-bound
+      // one CTA (wide towers: a pair) walks all layers for up to eight row blocks: ahead of the launches it replaces over
+      // that range
       tower_max_batch = 16 * sm_count;
     } else {
       tower = false;

@@ -221,20 +221,23 @@ def test_results_do_not_depend_on_the_batch_from_64_positions_on(precision, side
     nw.close()
 
 
-@pytest.mark.parametrize("batch", [295, 297, 600, 1189, 2368])
-def test_tower_with_several_row_blocks_per_cta(batch):
-    """One block of two boards per CTA, two, three, up to eight at a time and a ragged last group: the same bits per position."""
-    net = mknet.make_net("cfg1", blocks=3)
+@pytest.mark.parametrize("filters", [128, 192, 256])
+@pytest.mark.parametrize("batch", [1, 5, 295, 297, 600, 1189, 2368])
+def test_tower_with_several_row_blocks_per_cta(filters, batch):
+    """One block of boards per CTA or pair, two, three, up to eight at a time and a ragged last group: the bits of one launch per
+    convolution."""
+    net = mknet.make_net("cfg2", blocks=3, filters=filters)
     _, pos, n, g = load_compact("cfg4_2layer_b1024")
     idx = np.arange(batch) % 1000
-    masks, values = np.array(pos["masks"]), np.array(pos["values"])
-    nw = network.Network(net, "precision=fp16,max_batch=2368")
-    few, out = nw.evaluate(masks[:200], values[:200]), nw.evaluate(masks[idx], values[idx])
-    assert nw.device_status() == 0
-    nw.close()
-    for k in ("policy", "q", "d"):
-        np.testing.assert_array_equal(out[k][idx < 200], few[k][idx[idx < 200]])
-        np.testing.assert_array_equal(out[k], out[k][np.minimum(idx, batch - 1)])
+    masks, values = np.array(pos["masks"])[idx], np.array(pos["values"])[idx]
+    outs = []
+    for tower in (1, 0):
+        nw = network.Network(net, "precision=fp16,max_batch=%d,tower=%d" % (batch, tower))
+        outs.append(nw.evaluate(masks, values))
+        assert nw.device_status() == 0
+        nw.close()
+    for k in ("policy", "q", "d", "m"):
+        np.testing.assert_array_equal(outs[0][k], outs[1][k])
 
 
 @pytest.mark.parametrize("precision", ["fp16", "bf16"])
