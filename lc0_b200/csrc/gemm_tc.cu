@@ -275,7 +275,7 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
                                            float* tmp, float* gb, uint32_t bar, uint32_t& phase,
                                            volatile int* abort_flag, const float* w_smem = nullptr,
                                            const float* v_smem = nullptr) {
-  // w_smem: se_w1 [se_k][C] and se_w2 [2C][se_k]; v_smem: se_bias [C], se_b1 [se_k], se_b2 [2C]: copies in shared
+  // w_smem: se_w1 [se_k][C] and se_w2 [se_k / 4][2C][4]; v_smem: se_bias [C], se_b1 [se_k], se_b2 [2C]: copies in shared
   // memory, made while the tile was computed.  What is not there is read from global memory, and each of the five
   // is then one more round trip in a chain of dependent ones.
   const float* g_w1 = w_smem ? w_smem : p.se_w1;
@@ -335,16 +335,15 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
   if (eid < C) {
     const int c = eid;
     float z0a = ld(g_b2 + c), z1a = ld(g_b2 + C + c), z0b = z0a, z1b = z1a;
-    const float4* w0 = reinterpret_cast<const float4*>(g_w2 + (long long)c * p.se_k);
-    const float4* w1 = reinterpret_cast<const float4*>(g_w2 + (long long)(C + c) * p.se_k);
-    // in shared memory the 16-byte pieces of row r sit at position k ^ (r & 7) (eight or more pieces per row): thread c
-    // reads row c, and without the swizzle every lane of a warp would hit the same banks
-    const int swz = (w_smem && p.se_k >= 32) ? (c & 7) : 0;  // (C + c) & 7 == c & 7: C is a multiple of 16
+    // 16 bytes per output and four hidden units: a warp's loads are consecutive in both memories.  (A row of se_k weights per
+    // thread made every 16-byte load of a warp touch 32 lines: this stage took 7.4 k cycles of a tile's 13.2 k at 256 channels and
+    // 32 hidden units, now 2.8 k.)
+    const float4* w0 = reinterpret_cast<const float4*>(g_w2) + c;
     const float4* ha = reinterpret_cast<const float4*>(hid);
     const float4* hb = reinterpret_cast<const float4*>(hid + 64);
 #pragma unroll 8
     for (int k = 0; k < (p.se_k >> 2); ++k) {
-      const float4 a = ld4(w0 + (k ^ swz)), b = ld4(w1 + (k ^ swz)), xa = ha[k], xb = hb[k];
+      const float4 a = ld4(w0 + k * 2 * C), b = ld4(w0 + (2 * k + 1) * C), xa = ha[k], xb = hb[k];
       z0a = fmaf(a.x, xa.x, fmaf(a.y, xa.y, fmaf(a.z, xa.z, fmaf(a.w, xa.w, z0a))));
       z1a = fmaf(b.x, xa.x, fmaf(b.y, xa.y, fmaf(b.z, xa.z, fmaf(b.w, xa.w, z1a))));
       z0b = fmaf(a.x, xb.x, fmaf(a.y, xb.y, fmaf(a.z, xb.z, fmaf(a.w, xb.w, z0b))));
@@ -1011,12 +1010,8 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
           float4* s2 = s1 + n1;
           float* sv = se_w + 12 * n1;  // se_bias [N], se_b1 [se_k], se_b2 [2N]
           for (int i = eid; i < n1; i += 256) s1[i] = __ldg(g1 + i);
-          const int L = P.se_k >> 2;  // 16-byte pieces per row of se_w2; swizzled within the row (see se_prepare)
 #pragma unroll 4
-          for (int i = eid; i < n2; i += 256) {
-            const int r = i / L, k = i - r * L;
-            s2[r * L + (P.se_k >= 32 ? (k ^ (r & 7)) : k)] = __ldg(g2 + i);
-          }
+          for (int i = eid; i < n2; i += 256) s2[i] = __ldg(g2 + i);
           for (int i = eid; i < P.N; i += 256) sv[i] = __ldg(P.se_bias + i);
           for (int i = eid; i < P.se_k; i += 256) sv[P.N + i] = __ldg(P.se_b1 + i);
           for (int i = eid; i < 2 * P.N; i += 256) sv[P.N + P.se_k + i] = __ldg(P.se_b2 + i);
@@ -1364,7 +1359,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 // the operand barriers alone.  Against one launch per convolution (pair kernel, one tile per pair: no main loop to hide
 // launch, first loads, epilogue and stores under) the whole evaluation of the 20 x 256 network
 // takes, us, launch per convolution / tower: 16 boards 1022 / 907, 256 1245 / 1169, 592 2059 / 1879, 1024 3590 / 3524, 1500
-// 5299 / 5384, 2048 6833 / 6742 (a layer of 256 boards: 20.8 us).  The squeeze-excitation matrices
+// 5299 / 5384, 2048 6833 / 6742 (a layer of 256 boards: 20.8 us, 19.9 since se_prepare reads its second matrix in order).  The squeeze-excitation matrices
 // (96 KB at 256 channels and 32 hidden units) do not fit beside the pipeline and come from L2, its vectors are copied per layer.
 // ------------------------------------------------------------------------------------------------
 template <typename T>
@@ -1443,10 +1438,11 @@ gemm_tc_pair_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, i
         const TowerLayer& L = layers[w.l];
         const int board = w.rb() * 4 + (int)rank * 2;
         const int cblocks = L.p.conv_cblocks, k_blocks = 9 * cblocks, N = L.p.N, n0 = (int)rank * (N / 2);
+        const uint32_t bytes = 2 * (BM + N / 2) * BK * 2;  // of both CTAs: two boards' rows and half of the filters each
         const bool ready = w.l == 0 || mbar_try_wait(smem_u32(&done_bar[w.j]), (w.before() - 1) & 1);
         const int early = ready ? 0 : k_blocks < S ? k_blocks : S;  // filters ahead of rows that are still on their way
         auto load_w = [&](int kb, int s) {
-          if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * Cfg::kStageBytes);  // both CTAs' bytes land there
+          if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), bytes);  // both CTAs' bytes land there
           const int tap = kb / cblocks, cb = kb - tap * cblocks;
           tma_load_2d_pair(smem_u32(smem + s * Cfg::kStageBytes) + BM * BK * 2, &L.w, cb * BK, tap * N + n0,
                            mapa(smem_u32(&full_bar[s]), 0));
@@ -1943,7 +1939,7 @@ cudaError_t gemm_tc_tower_build(const GemmParams* g, int n, int* status, void* h
     memset(&L, 0, sizeof(L));
     cudaError_t e = make_board_map(q.A, q.conv_cin, q.M / 64, prec, &L.a);
     if (e != cudaSuccess) return e;
-    if ((e = get_map(q.W, q.conv_cin, 9 * q.N, q.conv_cin, bn, prec, &L.w)) != cudaSuccess) return e;
+    if ((e = get_map(q.W, q.conv_cin, 9 * q.N, q.conv_cin, q.N > bn ? q.N / 2 : bn, prec, &L.w)) != cudaSuccess) return e;
     if ((e = get_map(q.C, q.ldc, q.M, q.N, BM, prec, &L.c)) != cudaSuccess) return e;
     L.r = L.c;
     if (q.res && (e = get_map(q.res, q.ldres, q.M, q.N, BM, prec, &L.r)) != cudaSuccess) return e;

@@ -51,7 +51,8 @@ struct GemmParams {
   int n_split = 0;
   // Squeeze-excitation unit fused into a convolution (tensor-core kernel, convolution mode, at most 256 output
   // channels): out = act(gate * conv + shift + res) with gate / shift from the board's pooled conv output
-  // (ApplySEUnit, backends/blas/se_unit.cc:31-91).  se_w1 [se_k][N], se_b1 [se_k], se_w2 [2N][se_k], se_b2 [2N],
+  // (ApplySEUnit, backends/blas/se_unit.cc:31-91).  se_w1 [se_k][N], se_b1 [se_k], se_w2 [se_k / 4][2N][4]
+  // (four hidden units of an output together, outputs side by side), se_b2 [2N],
   // se_bias [N] = the convolution's own bias (it enters through the pooled mean and the shift); `bias` stays null and
   // `act` is applied after the residual.  See gemm_tc_se_supported.
   const float* se_w1 = nullptr; const float* se_b1 = nullptr; const float* se_w2 = nullptr;

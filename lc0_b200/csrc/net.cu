@@ -191,6 +191,7 @@ template <typename T> struct ResidualW {
   ConvW<T> c1, c2;
   bool se = false;
   float *se_w1 = nullptr, *se_b1 = nullptr, *se_w2 = nullptr, *se_b2 = nullptr;
+  float* se_w2q = nullptr;  // se_w2 as [se_k / 4][2 C][4], for the convolution's epilogue
   int se_k = 0;
 };
 
@@ -841,6 +842,13 @@ struct Net : NetBase {
           r.se_b1 = up_f32(p + ".se.b1", r.se_k);
           r.se_w2 = up_f32(p + ".se.w2", (size_t)2 * C * r.se_k);
           r.se_b2 = up_f32(p + ".se.b2", 2 * C);
+          if (r.se_k % 4 == 0) {
+            const std::vector<float>& w2 = need(p + ".se.w2", (size_t)2 * C * r.se_k);
+            std::vector<float> q(w2.size());
+            for (size_t o = 0; o < (size_t)2 * C; ++o)
+              for (size_t k = 0; k < (size_t)r.se_k; ++k) q[((k / 4) * 2 * C + o) * 4 + k % 4] = w2[o * r.se_k + k];
+            r.se_w2q = up_f32(q);
+          }
         }
         res.push_back(r);
       }
@@ -1299,7 +1307,7 @@ struct Net : NetBase {
     const ConvW<T>& c = r.c2;
     GemmParams p = conv_params(x, c, nullptr, y, n, act_default);
     p.res = skip; p.ldres = c.cout;
-    p.se_w1 = r.se_w1; p.se_b1 = r.se_b1; p.se_w2 = r.se_w2; p.se_b2 = r.se_b2; p.se_bias = c.b; p.se_k = r.se_k;
+    p.se_w1 = r.se_w1; p.se_b1 = r.se_b1; p.se_w2 = r.se_w2q; p.se_b2 = r.se_b2; p.se_bias = c.b; p.se_k = r.se_k;
     return p;
   }
   // Residual towers whose blocks all carry a squeeze-excitation unit: the table of the tower kernel, once per slot
