@@ -772,11 +772,133 @@ se_vec_kernel(const T* __restrict__ x, const float* __restrict__ conv_bias, cons
   }
 }
 
+// The same with everything that the chain reads in shared memory: w2 comes as [se_k / 4][2C][4] (a row per thread makes every
+// load of a warp touch 32 lines), the matrices are asked for ahead of the wait for the convolution, the tile and (`stage_skip`:
+// where it fits) the skip input in one piece behind it.  A block's work is a chain of short sums, bound by its round trips to L2:
+// with 128 channels, 32 hidden units, fp32 and 64 boards it adds 6.3 us behind the convolution, se_vec_kernel 12.5 us; the
+// 10 x 128 network takes, us, se_vec_kernel / this one: 1 board 499 / 422, 64 602 / 537, 512 2691 / 2595.
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+template <typename T, bool kFast>
+__global__ void __launch_bounds__(256)
+se_staged_kernel(const T* __restrict__ x, const float* __restrict__ conv_bias, const T* __restrict__ skip,
+                 const float* __restrict__ w1, const float* __restrict__ b1, const float* __restrict__ w2q,
+                 const float* __restrict__ b2, T* __restrict__ y, int C, int se_k, int act, int stage_skip) {
+  extern __shared__ __align__(16) uint8_t se_sm[];
+  float* w1s = reinterpret_cast<float*>(se_sm);                 // [se_k][C]
+  float* w2s = w1s + se_k * C;                                  // [se_k / 4][2C][4]
+  T* xs = reinterpret_cast<T*>(w2s + 2 * se_k * C);             // [64][C]
+  T* ss = xs + 64 * C;                                          // [64][C] if stage_skip
+  float* partial = reinterpret_cast<float*>(stage_skip ? ss + 64 * C : ss);  // [nsqg][C]  (nsqg * C == 2048)
+  float* z = partial + 2048;                                    // [2C]
+  float* pool = z + 2 * C;                                      // [C]
+  float* hid = pool + C;                                        // [se_k]
+  float* cb = hid + se_k;                                       // conv_bias [C], b1 [se_k], b2 [2C]
+  float* b1s = cb + C;
+  float* b2s = b1s + se_k;
+  const int n = blockIdx.x, tid = threadIdx.x;
+  const int cgs = C / 8, nsqg = 256 / cgs, cg = tid % cgs, sqg = tid / cgs;
+  for (int i = tid; i < se_k * C / 4; i += 256) copy_async16(w1s + 4 * i, w1 + 4 * i);
+  for (int i = tid; i < se_k * C / 2; i += 256) copy_async16(w2s + 4 * i, w2q + 4 * i);
+  for (int i = tid; i < C; i += 256) cb[i] = conv_bias[i];
+  for (int i = tid; i < se_k; i += 256) b1s[i] = b1[i];
+  for (int i = tid; i < 2 * C; i += 256) b2s[i] = b2[i];
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const T* xg = x + (long long)n * 64 * C;
+  const T* sg = skip + (long long)n * 64 * C;
+  constexpr int kPiece = 16 / sizeof(T);
+  for (int i = tid; i < 64 * C / kPiece; i += 256) copy_async16(xs + kPiece * i, xg + kPiece * i);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  if (stage_skip)
+    for (int i = tid; i < 64 * C / kPiece; i += 256) copy_async16(ss + kPiece * i, sg + kPiece * i);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncthreads();
+  {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int sq = sqg; sq < 64; sq += nsqg) {
+      const Vec8<T> v = *reinterpret_cast<const Vec8<T>*>(xs + sq * C + cg * 8);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += to_f(v.v[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) partial[sqg * C + cg * 8 + j] = acc[j];
+  }
+  __syncthreads();
+  for (int c = tid; c < C; c += 256) {
+    float a = 0.f;
+    for (int g = 0; g < nsqg; ++g) a += partial[g * C + c];
+    pool[c] = a / 64.0f + cb[c];
+  }
+  __syncthreads();
+  const int warp = tid >> 5, lane = tid & 31;
+  for (int o = warp; o < se_k; o += 8) {
+    float a = 0.f;
+    for (int c = lane; c < C; c += 32) a = fmaf(pool[c], w1s[o * C + c], a);
+    a = warp_sum(a);
+    if (lane == 0) hid[o] = activate<false>(a + b1s[o], act);
+  }
+  __syncthreads();
+  for (int o = tid; o < 2 * C; o += 256) {
+    float a = b2s[o];
+    for (int c = 0; c < se_k / 4; ++c) {
+      const float4 w = *reinterpret_cast<const float4*>(w2s + ((long long)c * 2 * C + o) * 4);
+      a = fmaf(hid[4 * c], w.x, a);
+      a = fmaf(hid[4 * c + 1], w.y, a);
+      a = fmaf(hid[4 * c + 2], w.z, a);
+      a = fmaf(hid[4 * c + 3], w.w, a);
+    }
+    z[o] = a;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  for (int c = tid; c < C; c += 256) {  // the gate, and the shift with the gate times the convolution's bias folded in
+    const float g = 1.0f / (1.0f + expf(-z[c]));
+    z[C + c] += g * cb[c];
+    z[c] = g;
+  }
+  __syncthreads();
+  T* yg = y + (long long)n * 64 * C;
+  const T* sr = stage_skip ? ss : sg;
+  float g[8], sh[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    g[j] = z[cg * 8 + j];
+    sh[j] = z[C + cg * 8 + j];
+  }
+#pragma unroll 4
+  for (int sq = sqg; sq < 64; sq += nsqg) {
+    const Vec8<T> v = *reinterpret_cast<const Vec8<T>*>(xs + sq * C + cg * 8);
+    const Vec8<T> r = *reinterpret_cast<const Vec8<T>*>(sr + sq * C + cg * 8);
+    Vec8<T> o;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o.v[j] = from_f<T>(activate<kFast>(g[j] * to_f(v.v[j]) + to_f(r.v[j]) + sh[j], act));
+    *reinterpret_cast<Vec8<T>*>(yg + sq * C + cg * 8) = o;
+  }
+}
+
 template <typename T>
 cudaError_t launch_se(const T* x, const float* conv_bias, const T* skip, const float* w1, const float* b1,
-                      const float* w2, const float* b2, T* y, int C, int se_k, int n, int act, cudaStream_t s) {
+                      const float* w2, const float* w2q, const float* b2, T* y, int C, int se_k, int n, int act, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const int cgs = C / 8;
+  // w2q and se_k % 4: every piece of the copies is 16 aligned bytes (C % 8 == 0 here)
+  if (w2q && se_k % 4 == 0 && C % 8 == 0 && cgs >= 1 && cgs <= 256 && 256 % cgs == 0) {
+    const size_t tile = (size_t)64 * C * sizeof(T), rest = (size_t)(3 * se_k * C + 2048 + 6 * C + 2 * se_k) * sizeof(float);
+    const int stage_skip = rest + 2 * tile <= 200 * 1024;
+    const size_t smem = rest + (stage_skip ? 2 : 1) * tile;
+    if (smem <= 200 * 1024) {
+      const auto kernel = se_staged_kernel<T, (sizeof(T) == 2)>;
+      if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+      }
+      return launch_dependent(kernel, dim3(n), dim3(256), smem, s, x, conv_bias, skip, w1, b1, w2q, b2, y, C, se_k, act,
+                              stage_skip);
+    }
+  }
   if (C % 8 == 0 && cgs <= 256 && 256 % cgs == 0) {
     const size_t smem = (size_t)64 * C * sizeof(T) + (size_t)(2048 + 3 * C + se_k) * sizeof(float);
     if (smem <= 200 * 1024) {
@@ -889,7 +1011,7 @@ cudaError_t launch_legal_softmax(const float* policy, const unsigned short* move
   template cudaError_t launch_policy_gather<T>(const T*, long long, const short*, int, float*, cudaStream_t); \
   template cudaError_t launch_head_final<T>(const T*, int, const float*, const float*, int, int, float*,      \
                                             cudaStream_t);                                                    \
-  template cudaError_t launch_se<T>(const T*, const float*, const T*, const float*, const float*,             \
+  template cudaError_t launch_se<T>(const T*, const float*, const T*, const float*, const float*, const float*, \
                                     const float*, const float*, T*, int, int, int, int, cudaStream_t);        \
   template cudaError_t launch_bias_skip_act<T>(const T*, const float*, const T*, T*, int, int, int,           \
                                                cudaStream_t);

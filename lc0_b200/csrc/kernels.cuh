@@ -188,7 +188,7 @@ cudaError_t launch_conv3x3(const T* x, int cin, const T* w, const float* bias, T
 // Squeeze-excitation + skip + activation (se_unit.cc:31-91) on NHWC: y = act(sig(z0)*x + skip + z1 + sig(z0)*b).
 template <typename T>
 cudaError_t launch_se(const T* x, const float* conv_bias, const T* skip, const float* w1, const float* b1,
-                      const float* w2, const float* b2, T* y, int C, int se_k, int n, int act, cudaStream_t s);
+                      const float* w2, const float* w2q, const float* b2, T* y, int C, int se_k, int n, int act, cudaStream_t s);
 template <typename T>
 cudaError_t launch_bias_skip_act(const T* x, const float* bias, const T* skip, T* y, int C, int rows, int act,
                                  cudaStream_t s);

@@ -1603,7 +1603,7 @@ struct Net : NetBase {
         }
         conv3(st, tmp, r.c2, nullptr, tmp2, n, ACT_NONE);
         other(st, 3.0 * R * C * sizeof(T), [&] {
-          return r.se ? launch_se<T>(tmp2, r.c2.b, cur, r.se_w1, r.se_b1, r.se_w2, r.se_b2, tmp, C, r.se_k, n,
+          return r.se ? launch_se<T>(tmp2, r.c2.b, cur, r.se_w1, r.se_b1, r.se_w2, r.se_w2q, r.se_b2, tmp, C, r.se_k, n,
                                      act_default, st)
                       : launch_bias_skip_act<T>(tmp2, r.c2.b, cur, tmp, C, R, act_default, st);
         });

@@ -204,6 +204,22 @@ def test_convolutions_whose_rows_are_no_16_byte_pieces(precision):
         assert np.abs(out["q"] - want["q"]).max() <= HALF_ATOL
 
 
+@pytest.mark.parametrize("filters,se", [(32, 4), (64, 6), (128, 32), (256, 32), (256, 64), (96, 8)])
+def test_squeeze_excitation_after_the_convolution(filters, se):
+    """Everything in shared memory; hidden units that are no whole 16-byte pieces; the skip input too large to stage; the matrices
+    too large; channels that do not divide the threads.  Same bounds as the configurations' own fp32 results."""
+    from lc0_b200 import netproto
+    net = netproto.parse_net(netproto.encode("Net", mknet.make_net("cfg1_mini", blocks=2, filters=filters, se=se)))
+    _, pos, n, g = load_case("cfg1_mini")
+    want = oracle.forward(*weights.flatten(net), pos["masks"][:3], pos["values"][:3])
+    nw = network.Network(net, "precision=fp32,max_batch=3")
+    out = nw.evaluate(pos["masks"][:3], pos["values"][:3])
+    assert nw.device_status() == 0
+    nw.close()
+    _assert_fp32_logits(out["policy"], want["policy"])
+    _assert_fp32_scalar(out["q"], want["q"])
+
+
 @pytest.mark.parametrize("precision", ["fp16", "bf16"])
 @pytest.mark.parametrize("side", [0, 1])
 def test_results_do_not_depend_on_the_batch_from_64_positions_on(precision, side):
