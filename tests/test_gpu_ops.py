@@ -264,6 +264,34 @@ def test_attention_op(lib, variant, prec, n, heads, depth, with_bias):
     assert (out.float() - want).abs().max().item() <= tol * max(1.0, want.abs().max().item())
 
 
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("heads,depth,pad,shift", [(3, 32, 0, 0), (3, 32, 4, 4), (3, 32, 1, 0), (3, 32, 4, 1), (2, 30, 0, 0),
+                                                   (2, 4, 0, 0), (1, 2, 0, 0), (1, 128, 0, 0)])
+def test_attention_op_rows_in_pieces_of_four(lib, prec, heads, depth, pad, shift):
+    """Rows that start on four-number boundaries and rows that do not (odd leading dimension, shifted base, odd head width).
+    fp32 bound: each score carries (depth + 3) roundings of at most the sum of |q||k|, doubled by the normalisation, the weighted
+    sum 64 more and the exponential a few."""
+    torch.manual_seed(depth + pad)
+    n, e = 2, heads * depth
+    dt = torch.float32 if prec == 0 else DT[prec]
+    ld = 3 * e + pad
+    store = torch.randn(n * 64 * ld + shift, device="cuda").to(dt)
+    qkv = store[shift:].reshape(n * 64, ld)[:, :3 * e]
+    bias = torch.randn(n, heads, 64, 64, device="cuda").to(dt)
+    out = torch.zeros(n * 64, e, device="cuda", dtype=dt)
+    esz = out.element_size()
+    base = store.data_ptr() + shift * esz
+    _lib.check(lib.b200_op_attention(base, base + e * esz, base + 2 * e * esz, ld, bias.data_ptr(), out.data_ptr(), e, n, heads,
+                                     depth, prec, 0, None))
+    torch.cuda.synchronize()
+    q, k, v = (t.permute(0, 2, 1, 3) for t in qkv.double().reshape(n, 64, 3, heads, depth).unbind(2))
+    s = torch.matmul(q, k.transpose(-1, -2)) / depth ** 0.5 + bias.double()
+    want = torch.matmul(torch.softmax(s, -1), v).permute(0, 2, 1, 3).reshape(n * 64, e)
+    size = (torch.matmul(q.abs(), k.abs().transpose(-1, -2)) / depth ** 0.5 + bias.double().abs()).max().item()
+    tol = (2 * (depth + 3) * size + 64 + 16) * 2.0 ** -24 * v.abs().max().item() if prec == 0 else 4e-3 * max(1.0, want.abs().max().item())
+    assert (out.double() - want).abs().max().item() <= tol
+
+
 def test_attention_op_variants_agree(lib):
     """The FMA kernel and the persistent TMA kernel on the same 16-bit inputs."""
     torch.manual_seed(5)
