@@ -74,7 +74,7 @@ typedef struct b200_net_options {
 } b200_net_options;
 
 enum {
-  B200_FLAG_NO_TENSOR_CORES = 1, /* force the plain FMA matrix kernels in fp16/bf16 mode */
+  B200_FLAG_NO_TENSOR_CORES = 1, /* force the plain FMA matrix kernels, in every precision */
   B200_FLAG_NO_GRAPHS = 2,       /* launch kernels one by one instead of replaying captured CUDA graphs */
   /* Verification switches: each turns one fusion of the 16-bit tensor-core schedule off, so that a test can compare
    * the fused schedule with the plain one on the same network (results agree to rounding). */
