@@ -385,15 +385,8 @@ static cudaError_t launch_attention_tma_cfg(const T* q, const T* k, const T* v, 
                                             long long ldo, int n, int heads, float scale, double* zero0, double* zero1,
                                             int* status, int sm_count, int ctas_per_sm, cudaStream_t s) {
   using L = AttnTma<D, NS>;
-  static bool attr_done[64] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  cudaError_t e = raise_smem_limit<&attention_tma_kernel<T, D, NS>>(L::kBytes);
   if (e != cudaSuccess) return e;
-  if (!attr_done[dev & 63]) {
-    e = cudaFuncSetAttribute(attention_tma_kernel<T, D, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
-    if (e != cudaSuccess) return e;
-    attr_done[dev & 63] = true;
-  }
   const int prec = sizeof(T) == 2 && std::is_same<T, __half>::value ? 1 : 2;
   const long long rows = (long long)n * 64;
   CUtensorMap mq, mk, mv, mb, mo;

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <string>
 
 namespace b200 {
@@ -39,6 +40,20 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
+
+// Raises a kernel's limit of dynamic shared memory to the most that any launch of it asks for, once per device.  The limit
+// belongs to the function: set launch by launch to what that launch needs, another thread with a narrower network can
+// lower it between this thread's call and its launch, which is then refused.
+template <auto kKernel>
+cudaError_t raise_smem_limit(int bytes) {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (done.load() >> (dev & 63) & 1ull)) return e;
+  if ((e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) == cudaSuccess)
+    done.fetch_or(1ull << (dev & 63));
+  return e;
+}
 
 // Whether launch_dependent() asks for the overlap (off: an ordinary launch).  Set by the host schedule per thread.
 extern thread_local bool t_dependent_launch;

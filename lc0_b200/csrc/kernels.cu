@@ -552,11 +552,15 @@ template <typename T>
 cudaError_t launch_attention(const T* q, const T* k, const T* v, long long ld, const T* bias, T* out,
                              long long ldo, int n, int heads, int depth, float scale, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  if (depth > 128) return cudaErrorInvalidValue;
-  const int dp = ceil_div(depth, 4) * 4 + 4;
-  const size_t smem = (size_t)(64 * (2 * dp > 68 ? 2 * dp : 68) + depth * 68) * sizeof(float);
+  constexpr int kMaxDepth = 128;
+  if (depth > kMaxDepth) return cudaErrorInvalidValue;
+  auto bytes = [](int d) {
+    const int dp = ceil_div(d, 4) * 4 + 4;
+    return (size_t)(64 * (2 * dp > 68 ? 2 * dp : 68) + d * 68) * sizeof(float);
+  };
+  const size_t smem = bytes(depth);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(attention_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = raise_smem_limit<&attention_kernel<T>>((int)bytes(kMaxDepth));
     if (e != cudaSuccess) return e;
   }
   return launch_dependent(attention_kernel<T>, dim3(n * heads), dim3(256), smem, s, q, k, v, ld, bias, out, ldo, heads, depth,
@@ -912,16 +916,17 @@ template <typename T>
 cudaError_t launch_se(const T* x, const float* conv_bias, const T* skip, const float* w1, const float* b1,
                       const float* w2, const float* w2q, const float* b2, T* y, int C, int se_k, int n, int act, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
+  constexpr size_t kMaxSmem = 200 * 1024;
   const int cgs = C / 8;
   // w2q and se_k % 4: every piece of the copies is 16 aligned bytes (C % 8 == 0 here)
   if (w2q && se_k % 4 == 0 && C % 8 == 0 && cgs >= 1 && cgs <= 256 && 256 % cgs == 0) {
     const size_t tile = (size_t)64 * C * sizeof(T), rest = (size_t)(3 * se_k * C + 2048 + 6 * C + 2 * se_k) * sizeof(float);
-    const int stage_skip = rest + 2 * tile <= 200 * 1024;
+    const int stage_skip = rest + 2 * tile <= kMaxSmem;
     const size_t smem = rest + (stage_skip ? 2 : 1) * tile;
-    if (smem <= 200 * 1024) {
+    if (smem <= kMaxSmem) {
       const auto kernel = se_staged_kernel<T, (sizeof(T) == 2)>;
       if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = raise_smem_limit<&se_staged_kernel<T, (sizeof(T) == 2)>>((int)kMaxSmem);
         if (e != cudaSuccess) return e;
       }
       return launch_dependent(kernel, dim3(n), dim3(256), smem, s, x, conv_bias, skip, w1, b1, w2q, b2, y, C, se_k, act,
@@ -930,10 +935,9 @@ cudaError_t launch_se(const T* x, const float* conv_bias, const T* skip, const f
   }
   if (C % 8 == 0 && cgs <= 256 && 256 % cgs == 0) {
     const size_t smem = (size_t)64 * C * sizeof(T) + (size_t)(2048 + 3 * C + se_k) * sizeof(float);
-    if (smem <= 200 * 1024) {
+    if (smem <= kMaxSmem) {
       if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(se_vec_kernel<T, (sizeof(T) == 2)>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = raise_smem_limit<&se_vec_kernel<T, (sizeof(T) == 2)>>((int)kMaxSmem);
         if (e != cudaSuccess) return e;
       }
       se_vec_kernel<T, (sizeof(T) == 2)><<<n, 256, smem, s>>>(x, conv_bias, skip, w1, b1, w2, b2, y, C, se_k, act);

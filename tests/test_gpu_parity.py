@@ -1,4 +1,6 @@
 """Parity of the CUDA path (through the C ABI) with the CPU oracle and the recorded reference outputs."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -218,6 +220,41 @@ def test_squeeze_excitation_after_the_convolution(filters, se):
     nw.close()
     _assert_fp32_logits(out["policy"], want["policy"])
     _assert_fp32_scalar(out["q"], want["q"])
+
+
+def _mini(kind, width):
+    if kind == "attention":  # heads of depth `width`
+        return mknet.make_net("cfg3_mini", emb=256, heads=256 // width, layers=8)
+    return mknet.make_net("cfg1_mini", blocks=4, filters=width, se=32 if kind == "se" else 6)
+
+
+@pytest.mark.parametrize("kind,widths", [("se", (128, 64)), ("se_odd", (512, 256)), ("attention", (128, 64))])
+def test_networks_of_different_widths_on_different_threads(kind, widths):
+    """Kernels whose shared memory depends on the layer: a network launched on one thread must not lower the limit that another
+    thread's launch of the same kernel needs."""
+    _, pos, n, g = load_case("cfg1_mini")
+    masks, values = pos["masks"][:2], pos["values"][:2]
+    nets = [network.Network(_mini(kind, w), "precision=fp32,max_batch=2,graph_capture=0") for w in widths for _ in range(2)]
+    want = [nw.evaluate(masks, values) for nw in nets]
+    errors = []
+
+    def work(nw, ref):
+        try:
+            for _ in range(300):
+                out = nw.evaluate(masks, values)
+                if not np.array_equal(out["policy"], ref["policy"]):
+                    raise AssertionError("another result")
+        except Exception as e:  # noqa: BLE001 - reported by the test
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in zip(nets, want)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for nw in nets:
+        nw.close()
+    assert not errors, errors[0]
 
 
 @pytest.mark.parametrize("precision", ["fp16", "bf16"])
