@@ -459,6 +459,46 @@ def test_second_output_of_the_pair_kernel_with_folded_input(lib, whole_tiles):
 
 
 @pytest.mark.parametrize("prec", [1, 2])
+@pytest.mark.parametrize("form", ["res act", "stats act", "norm res", "norm res stats"])
+@pytest.mark.parametrize("M,N,K", [(8192, 1024, 512), (8200, 1000, 520), (8200, 1000, 1024), (8192, 1024, 1032)])
+def test_forms_of_the_pair_kernel_that_no_layer_has(lib, prec, form, M, N, K):
+    """Residual or statistics beside an activation or a folded LayerNorm of A: both sides of the lines between two and four
+    groups of epilogue warps (8 and 16 k-blocks), ragged rows, columns and k-blocks."""
+    dt = DT[prec]
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    A, W = (rnd(M, K) + 0.5).to(dt), (rnd(N, K) * K ** -0.5).to(dt)
+    b, cs = rnd(N) * 0.1, W.float().sum(1).contiguous()
+    a64 = A.double()
+    C, out_st = torch.zeros(M, N, dtype=dt, device="cuda"), torch.zeros(M, 2, device="cuda", dtype=torch.float64)
+    kw = dict(A=A, W=W, bias=b, C=C, M=M, N=N, K=K, precision=prec, activation=oracle.ACT_NONE)
+    ref = a64 @ W.double().T
+    if "norm" in form:
+        st_a = torch.stack([a64.sum(1), (a64 * a64).sum(1)], 1).contiguous()
+        kw.update(a_stats=st_a, colsum=cs, a_inv_c=1.0 / K, a_eps=1e-3)
+        ref = (ref - a64.mean(1, keepdim=True) * cs.double()) * (a64.var(1, unbiased=False, keepdim=True) + 1e-3).rsqrt()
+    ref = ref + b.double()
+    if "act" in form:
+        kw.update(activation=oracle.ACT_SWISH)
+        ref = ref * torch.sigmoid(ref)
+    if "res" in form:
+        R = rnd(M, N).to(dt)
+        kw.update(res=R, alpha=0.43)
+        ref = 0.43 * ref + R.double()
+    if "stats" in form:
+        kw.update(out_stats=out_st)
+    _lib.check(lib.b200_op_gemm_ex(_desc(**kw), None))
+    torch.cuda.synchronize()
+    # as in test_products_of_few_rows: rounding of the storage type, fp32 sums, the fast exponential
+    rt = 2.0 ** -10 if prec == 1 else 2.0 ** -7
+    assert torch.all((C.double() - ref).abs() <= rt * ref.abs() + 1e-3), (C.double() - ref).abs().max().item()
+    if "stats" in form:
+        s_ref = torch.stack([ref.sum(1), (ref * ref).sum(1)], 1)
+        mag = torch.stack([ref.abs().sum(1), s_ref[:, 1]], 1)
+        assert torch.all((out_st - s_ref).abs() <= 1e-3 * mag + 1e-3)
+
+
+@pytest.mark.parametrize("prec", [1, 2])
 @pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 256, 2048), (3, 8192, 256), (7, 40, 72), (63, 1024, 1024), (64, 1536, 1024),
                                    (65, 1024, 1536), (130, 200, 624), (384, 1024, 1024), (1000, 1858, 64),
                                    (1537, 128, 512)])
