@@ -763,29 +763,23 @@ struct TowerCfg {
                                     kSeWBytes;
 };
 
-// The tiles of one CTA in the order it computes them.  A CTA takes its row blocks up to eight at a time and goes layer by layer
-// over them: a tile then depends on a tile several before it, so the wait for a block's stores, for the next layer's first
-// loads and the epilogue fall under the other blocks' main loops.  Of a tower of 10 x 128 a tile takes 10 us when it is alone, 6.5
-// among two blocks and 5.9 among five or six (two at a time, with the table read from global memory: 10.6, 7.0 and 6.7): what is
-// left is the main loop's operand traffic (32 KB per k-block, 460 cycles).  Towers of 64 / 700 / 1500 positions 222 / 509 / 838 -> 200 / 378 / 746 us.
+// The tiles of one CTA in the order it computes them: layer by layer over its row blocks (at most eight).  A tile then depends on
+// a tile several before it, so the wait for a block's stores, for the next layer's first loads and the epilogue fall under the
+// other blocks' main loops.  Of a tower of 10 x 128 a tile takes 10 us when it is alone, 6.5 among two blocks and 5.9 among five
+// or six (two at a time, with the table read from global memory: 10.6, 7.0 and 6.7): what is left is the main loop's operand
+// traffic (32 KB per k-block, 460 cycles).  Towers of 64 / 700 / 1500 positions 222 / 509 / 838 -> 200 / 378 / 746 us.
 constexpr int kTowerBlocks = 8;
 struct TowerWalk {
   int n_layers, first, step, nb;  // nb: row blocks of this CTA
-  int i0 = 0, l = 0, j = 0;       // index of the group's first block among the CTA's blocks, layer, block of the group
+  int l = 0, j = 0;               // layer (= tiles of the block ahead of this one), block
   __device__ TowerWalk(int n_layers_, int row_blocks, int first_ = blockIdx.x, int step_ = gridDim.x)
       : n_layers(n_layers_), first(first_), step(step_) {
     nb = first < row_blocks ? (row_blocks - first + step - 1) / step : 0;
   }
-  __device__ bool valid() const { return i0 < nb; }
-  __device__ int rb() const { return first + (i0 + j) * step; }
-  __device__ int cnt() const { return nb - i0 < kTowerBlocks ? nb - i0 : kTowerBlocks; }
-  // tiles of the j-th block of its group (this one and the groups before, which are full) ahead of this tile
-  __device__ uint32_t before() const { return (uint32_t)(i0 / kTowerBlocks * n_layers + l); }
+  __device__ bool valid() const { return l < n_layers && nb > 0; }
+  __device__ int rb() const { return first + j * step; }
   __device__ void next() {
-    if (++j >= cnt()) {
-      j = 0;
-      if (++l >= n_layers) { l = 0; i0 += kTowerBlocks; }
-    }
+    if (++j >= nb) { j = 0; ++l; }
   }
 };
 
@@ -853,7 +847,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
   uint64_t* stg_full = reinterpret_cast<uint64_t*>(bar_mem + 256);  // [2 groups][2 buffers] slab staged (4 warps)
   uint64_t* stg_free = stg_full + 4;                                // [2 groups][2 buffers] store has read the buffer
   uint64_t* se_bar = reinterpret_cast<uint64_t*>(bar_mem + 384);    // barrier of the 256 epilogue threads
-  uint64_t* done_bar = se_bar + 1;                                  // [kTowerBlocks] the latest tile of a group's block is in memory
+  uint64_t* done_bar = se_bar + 1;                                  // [kTowerBlocks] the latest tile of a block is in memory
   float* wvec_all = reinterpret_cast<float*>(bar_mem + 512);        // 8 warps x 256 floats
   float* wvec = wvec_all + ((threadIdx.x >> 5) & 7) * 256;
   float* se_gb = reinterpret_cast<float*>(bar_mem + 512 + 8192);    // [2 boards][gate 256 | shift 256]
@@ -911,7 +905,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
         const int cblocks = L.p.conv_cblocks, k_blocks = 9 * cblocks, N = L.p.N;
         // The filters do not depend on this CTA's earlier output: where that is still on its way (the first layer reads what was
         // complete before the launch), those of the first stages are requested before the wait for it.
-        const bool ready = w.l == 0 || mbar_try_wait(smem_u32(&done_bar[w.j]), (w.before() - 1) & 1);
+        const bool ready = w.l == 0 || mbar_try_wait(smem_u32(&done_bar[w.j]), (uint32_t)(w.l - 1) & 1);
         const int early = ready ? 0 : k_blocks < S ? k_blocks : S;
         for (int kb = 0; kb < early && ok; ++kb) {
           const int s = (it + kb) % S;
@@ -924,7 +918,7 @@ gemm_tc_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, int ro
         }
         if (!ok) break;
         if (w.l > 0) {  // the block's previous layer
-          if (!ready && !mbar_wait(smem_u32(&done_bar[w.j]), (w.before() - 1) & 1, abort_flag, 9)) break;
+          if (!ready && !mbar_wait(smem_u32(&done_bar[w.j]), (uint32_t)(w.l - 1) & 1, abort_flag, 9)) break;
           fence_proxy_async_all();
         }
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
@@ -1381,7 +1375,7 @@ gemm_tc_pair_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, i
   uint64_t* stg_full = reinterpret_cast<uint64_t*>(bar_mem + 256);  // [2] slab staged (4 warps)
   uint64_t* stg_free = stg_full + 2;                                // [2] store has read the buffer
   uint64_t* se_bar = reinterpret_cast<uint64_t*>(bar_mem + 384);
-  uint64_t* done_bar = se_bar + 1;                                  // [kTowerBlocks] the latest tile of a group's block is in memory
+  uint64_t* done_bar = se_bar + 1;                                  // [kTowerBlocks] the latest tile of a block is in memory
   float* wvec_all = reinterpret_cast<float*>(bar_mem + 512);
   float* wvec = wvec_all + ((threadIdx.x >> 5) & 15) * 256;
   float* se_gb = reinterpret_cast<float*>(bar_mem + 512 + 16 * 1024);
@@ -1439,7 +1433,7 @@ gemm_tc_pair_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, i
         const int board = w.rb() * 4 + (int)rank * 2;
         const int cblocks = L.p.conv_cblocks, k_blocks = 9 * cblocks, N = L.p.N, n0 = (int)rank * (N / 2);
         const uint32_t bytes = 2 * (BM + N / 2) * BK * 2;  // of both CTAs: two boards' rows and half of the filters each
-        const bool ready = w.l == 0 || mbar_try_wait(smem_u32(&done_bar[w.j]), (w.before() - 1) & 1);
+        const bool ready = w.l == 0 || mbar_try_wait(smem_u32(&done_bar[w.j]), (uint32_t)(w.l - 1) & 1);
         const int early = ready ? 0 : k_blocks < S ? k_blocks : S;  // filters ahead of rows that are still on their way
         auto load_w = [&](int kb, int s) {
           if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), bytes);  // both CTAs' bytes land there
@@ -1454,7 +1448,7 @@ gemm_tc_pair_tower_kernel(const TowerLayer* __restrict__ layers, int n_layers, i
         }
         if (!ok) break;
         if (w.l > 0) {  // the block's previous layer
-          if (!ready && !mbar_wait(smem_u32(&done_bar[w.j]), (w.before() - 1) & 1, abort_flag, 9)) break;
+          if (!ready && !mbar_wait(smem_u32(&done_bar[w.j]), (uint32_t)(w.l - 1) & 1, abort_flag, 9)) break;
           fence_proxy_async_all();
         }
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
@@ -1959,6 +1953,29 @@ cudaError_t gemm_tc_tower_build(const GemmParams* g, int n, int* status, void* h
 template cudaError_t gemm_tc_tower_build<__half>(const GemmParams*, int, int*, void*);
 template cudaError_t gemm_tc_tower_build<__nv_bfloat16>(const GemmParams*, int, int*, void*);
 
+namespace {
+// Row blocks (two boards) that the tower kernel takes at most: eight per CTA, of wide towers eight pairs of them per pair.
+int tower_row_blocks(int channels, int sm_count) {
+  return channels > TowerCfg::BN ? 2 * kTowerBlocks * (sm_count / 2) : kTowerBlocks * sm_count;
+}
+}  // namespace
+
+// Narrow towers are ahead of one launch per convolution at every size they take (10 x 128, us: 64 boards 234 / 311, 889 578 / 790, 2368
+// 1279 / 1737; 10 x 64 1.36 to 1.65 times).  Wide ones come in whole rounds of four boards per pair, of which the last may be
+// nearly empty, and lose more to that the more rounds precede it.  20 x 256, tower / launches: 593 boards 1955 / 1966, 888 2264 / 2572;
+// 889 2745 / 2674, 920 2780 / 2806, 1184 3130 / 3290; 1185 3606 / 3440, 1340 3829 / 3783, 1420 3939 / 3949, 1480 3996 / 4085; 1481
+// 4489 / 4248, 1776 4946 / 4836, 2368 6544 / 6380.  20 x 192: 1185 2484 / 2486, 1777 3656 / 3646, 2072 3951 / 4101; 2073 4283 / 4217,
+// 2140 4339 / 4398, 2368 4572 / 4664.  So the last round has to be filled to 0.7 of a round per whole round before it less two rounds (from
+// four rounds on a tenth, of five four fifths, six never), at 192 channels to 0.2 less 1.2 (of eight rounds a fifth).
+bool gemm_tc_tower_pays(int channels, int boards, int sm_count) {
+  const int row_blocks = (boards + 1) / 2;
+  if (row_blocks > tower_row_blocks(channels, sm_count)) return false;
+  if (channels <= TowerCfg::BN) return true;
+  const int pairs = sm_count / 2, blocks = (row_blocks + 1) / 2;
+  const int full = (blocks - 1) / pairs, last = blocks - full * pairs;
+  return 10 * last >= pairs * (channels > 192 ? 7 * full - 20 : 2 * full - 12);
+}
+
 // One launch for `n_layers` convolutions over the first `row_blocks` blocks of 128 rows (two boards).
 template <typename T>
 cudaError_t launch_gemm_tower(const void* d_layers, int n_layers, int channels, int row_blocks, int* status, int sm_count,
@@ -1969,6 +1986,7 @@ cudaError_t launch_gemm_tower(const void* d_layers, int n_layers, int channels, 
   if (e != cudaSuccess) return e;
   const TowerLayer* layers = static_cast<const TowerLayer*>(d_layers);
   if (channels > 2 * TowerCfg::BN) return cudaErrorInvalidValue;
+  if (row_blocks > tower_row_blocks(channels, sm_count)) return cudaErrorInvalidValue;
   if (channels > TowerCfg::BN) {
     static std::atomic<unsigned long long> pair_mask{0};
     if (!(pair_mask.load() >> (dev & 63) & 1ull)) {

@@ -95,9 +95,11 @@ bool gemm_tc_split_supported(const GemmParams& p);
 // Tower kernel (gemm_tc.cu): the 3x3 convolutions of a residual tower (conv_cin > 0, optional fused squeeze-excitation
 // and skip input), all with the same rows and output channels (at most 256), in one launch.  gemm_tc_tower_build fills
 // a host table of n entries of gemm_tc_tower_layer_bytes() bytes, which the caller copies to the device once;
-// launch_gemm_tower runs the first `row_blocks` blocks of 128 rows (two boards) through all layers.
+// launch_gemm_tower runs the first `row_blocks` blocks of 128 rows (two boards) through all layers; gemm_tc_tower_pays says for how
+// many boards that is possible and ahead of one launch per convolution.
 bool gemm_tc_tower_supported(const GemmParams* g, int n);
 size_t gemm_tc_tower_layer_bytes();
+bool gemm_tc_tower_pays(int channels, int boards, int sm_count);
 template <typename T> cudaError_t gemm_tc_tower_build(const GemmParams* g, int n, int* status, void* host_layers);
 template <typename T>
 cudaError_t launch_gemm_tower(const void* d_layers, int n_layers, int channels, int row_blocks, int* status, int sm_count,

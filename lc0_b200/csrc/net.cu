@@ -438,8 +438,7 @@ struct Net : NetBase {
   bool dependent_launch = false;  // tensor-core products, attention and LayerNorms launched with launch_dependent()
   bool heads_side = false;        // value and moves-left heads on the side stream beside the policy head
   int heads_side_max = 0;         // ... up to this many positions
-  bool tower = false;             // residual towers: all 3x3 convolutions in one launch up to tower_max_batch positions
-  int tower_max_batch = 0;
+  bool tower = false;             // residual towers: all 3x3 convolutions in one launch where that is ahead (gemm_tc_tower_pays)
   static constexpr int kSideSms = 8, kSidePositions = 112;
 
   // format
@@ -1339,9 +1338,6 @@ struct Net : NetBase {
         CK(cudaMemcpy(s.tower_layers, host.data(), host.size(), cudaMemcpyHostToDevice));
         s.tower_n = (int)g.size();
       }
-      // one CTA (wide towers: a pair) walks all layers for up to eight row blocks: ahead of the launches it replaces over
-      // that range
-      tower_max_batch = 16 * sm_count;
     } else {
       tower = false;
     }
@@ -1577,7 +1573,7 @@ struct Net : NetBase {
       T *cur = s.x, *tmp = s.x1, *tmp2 = s.y;
       bool in_one = false;
       if constexpr (sizeof(T) == 2) {
-        if (tower && s.tower_layers && n <= tower_max_batch) {
+        if (tower && s.tower_layers && gemm_tc_tower_pays(C, n, sm_count)) {
           // input convolution and every block of the tower in one launch (gemm_tc.cu, tower kernel)
           launches++;
           double flops = 2.0 * R * (double)C * 9 * 112;

@@ -293,6 +293,33 @@ def test_tower_with_several_row_blocks_per_cta(filters, batch):
         np.testing.assert_array_equal(outs[0][k], outs[1][k])
 
 
+@pytest.mark.parametrize("filters,batches", [
+    (128, {1: 1, 2368: 1, 2369: 0}), (192, {1776: 1, 1777: 1, 2073: 0, 2368: 1, 2369: 0}),
+    (256, {1: 1, 888: 1, 889: 0, 1000: 1, 1184: 1, 1185: 0, 1400: 0, 1480: 1, 1481: 0, 1776: 0, 2368: 0})])
+def test_tower_runs_where_it_is_ahead(filters, batches):
+    """Wide towers come in rounds of four boards per pair of CTAs: a last round with too few of them goes to one launch per
+    convolution, and so does what is more than eight blocks per CTA or pair.  The launches counted, the bits the same."""
+    net = mknet.make_net("cfg2", blocks=2, filters=filters)
+    _, pos, n, g = load_compact("cfg4_2layer_b1024")
+    idx = np.arange(max(batches)) % 1000
+    masks, values = np.array(pos["masks"])[idx], np.array(pos["values"])[idx]
+    nets = [network.Network(net, "precision=fp16,max_batch=%d,tower=%d" % (max(batches), tower)) for tower in (1, 0)]
+    if nets[0].info.sm_count != 148:
+        pytest.skip("sizes of a GPU with 148 SMs")
+    for batch, one_launch in batches.items():
+        outs, launches = [], []
+        for nw in nets:
+            before = nw.launch_count()
+            outs.append(nw.evaluate(masks[:batch], values[:batch]))
+            launches.append(nw.launch_count() - before)
+            assert nw.device_status() == 0
+        assert launches[1] - launches[0] == (4 if one_launch else 0), (batch, launches)
+        for k in ("policy", "q", "d", "m"):
+            np.testing.assert_array_equal(outs[0][k], outs[1][k])
+    for nw in nets:
+        nw.close()
+
+
 @pytest.mark.parametrize("precision", ["fp16", "bf16"])
 @pytest.mark.parametrize("name", ["cfg4_2layer", "cfg3", "cfg2_mini", "cfg4_mini"])
 def test_results_do_not_depend_on_the_batch_below_64_positions(name, precision):
