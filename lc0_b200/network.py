@@ -67,11 +67,12 @@ class NetworkComputation:
         h = ctypes.c_void_p()
         _lib.check(self._lib.b200_comp_create(network._handle, ctypes.byref(h)))
         self._h = h
-        self._results = None  # copies of the computed batch's results: (q, d, m one after the other, probabilities, move counts)
+        self._results = None  # what _read() returned since the last change to the batch
+        self._computed = False
 
     def add_input(self, masks, values):
         """AddInput: 112 plane masks (uint64) and 112 plane values (float32)."""
-        self._results = None
+        self._changed()
         m = np.ascontiguousarray(masks, np.uint64).reshape(-1)
         v = np.ascontiguousarray(values, np.float32).reshape(-1)
         if m.size != 112 or v.size != 112:
@@ -81,7 +82,7 @@ class NetworkComputation:
     def add_input_with_moves(self, masks, values, move_ids):
         """AddInput plus the policy indices of the position's legal moves (MoveToNNIndex of each move); the
         legal-move softmax then runs on the device (see `legal_policy`)."""
-        self._results = None
+        self._changed()
         m = np.ascontiguousarray(masks, np.uint64).reshape(-1)
         v = np.ascontiguousarray(values, np.float32).reshape(-1)
         ids = np.ascontiguousarray(move_ids, np.uint16).reshape(-1)
@@ -92,7 +93,7 @@ class NetworkComputation:
 
     def add_inputs_with_moves(self, masks, values, move_ids, n_moves):
         """Batch form: move_ids [n][256] (rows padded), n_moves [n]."""
-        self._results = None
+        self._changed()
         m = np.ascontiguousarray(masks, np.uint64).reshape(-1, 112)
         v = np.ascontiguousarray(values, np.float32).reshape(-1, 112)
         ids = np.ascontiguousarray(move_ids, np.uint16).reshape(-1, 256)
@@ -109,7 +110,7 @@ class NetworkComputation:
     def add_position(self, history, from_start, move_ids=None):
         """One position by its game history (records of _lib.BOARD_DTYPE, oldest first, the position itself last)
         instead of its planes: EncodePositionForNN (src/neural/encoder.cc:134) runs on the device."""
-        self._results = None
+        self._changed()
         h = np.ascontiguousarray(history, _lib.BOARD_DTYPE).reshape(-1)
         if move_ids is None:
             _lib.check(self._lib.b200_comp_add_position(self._h, h.ctypes.data, h.size, 1 if from_start else 0, None, -1))
@@ -120,7 +121,7 @@ class NetworkComputation:
 
     def add_positions(self, boards, offsets, from_start, move_ids=None, n_moves=None):
         """Batch form of add_position: concatenated histories with n + 1 offsets; move_ids [n][256], n_moves [n]."""
-        self._results = None
+        self._changed()
         b = np.ascontiguousarray(boards, _lib.BOARD_DTYPE).reshape(-1)
         o = np.ascontiguousarray(offsets, np.int32).reshape(-1)
         f = np.ascontiguousarray(from_start, np.uint8).reshape(-1)
@@ -141,16 +142,16 @@ class NetworkComputation:
 
     def legal_policy(self, sample):
         """Probabilities of the sample's legal moves, in the order the moves were given."""
-        r = self._results
-        if r is not None and r[1] is not None and 0 <= sample < len(r[2]):
-            return r[1][sample, :r[2][sample]].copy()
+        r = self._results or self._read()
+        if r and r[3] is not None and 0 <= sample < r[0]:
+            return r[2][sample, :r[3][sample]].copy()
         p = ctypes.POINTER(ctypes.c_float)()
         n = ctypes.c_int()
         _lib.check(self._lib.b200_comp_legal_policy(self._h, sample, ctypes.byref(p), ctypes.byref(n)))
         return np.ctypeslib.as_array(p, shape=(n.value,)).copy() if n.value else np.zeros(0, np.float32)
 
     def add_inputs(self, masks, values):
-        self._results = None
+        self._changed()
         m = np.ascontiguousarray(masks, np.uint64).reshape(-1, 112)
         v = np.ascontiguousarray(values, np.float32).reshape(-1, 112)
         if m.shape != v.shape:
@@ -158,17 +159,27 @@ class NetworkComputation:
         _lib.check(self._lib.b200_comp_add_inputs(self._h, m.ctypes.data, v.ctypes.data, m.shape[0]))
 
     def compute_blocking(self):
-        self._results = None
+        self._changed()
         _lib.check(self._lib.b200_comp_compute(self._h))
-        # The accessors below are called once per position and value: they read copies taken here (37 positions of a search:
-        # 155 -> 45 us of accessors).
-        n = self.get_batch_size()
+        self._computed = True
+
+    def _changed(self):
+        self._results, self._computed = None, False
+
+    def _read(self):
+        """(number of samples; q, d, m one after the other; probabilities or None; move counts or None) of the computed batch, else
+        None: views of the computation's host buffers, made at the first accessor.  The accessors are called once per position
+        and value, and a C call each made 155 us of the 580 that a search's batch of 37 took, against 45."""
+        n = self.get_batch_size() if self._computed else 0
+        if n == 0:
+            return None
         qdm, probs, moves = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
         _lib.check(self._lib.b200_comp_results(self._h, ctypes.byref(qdm), ctypes.byref(probs), ctypes.byref(moves)))
-        copy = lambda p, kind, count: np.frombuffer(ctypes.string_at(p, 4 * count), kind) if count else np.zeros(0, kind)
-        self._results = (copy(qdm.value, np.float32, 3 * n).tolist(),
-                         copy(probs.value, np.float32, 256 * n).reshape(n, 256) if probs else None,
-                         copy(moves.value, np.int32, n).tolist() if moves else None)
+        view = lambda p, kind, count: memoryview((kind * count).from_address(p.value)).cast("B").cast(kind._type_)
+        self._results = (n, view(qdm, ctypes.c_float, 3 * n),
+                         np.frombuffer(view(probs, ctypes.c_float, 256 * n), np.float32).reshape(n, 256) if probs else None,
+                         view(moves, ctypes.c_int, n) if moves else None)
+        return self._results
 
     def get_batch_size(self):
         return self._lib.b200_comp_batch_size(self._h)
@@ -178,23 +189,23 @@ class NetworkComputation:
             raise IndexError("sample %d out of range" % sample)
 
     def get_q_val(self, sample):
-        r = self._results
-        if r is not None and 0 <= sample and 3 * sample < len(r[0]):
-            return r[0][3 * sample]
+        r = self._results or self._read()
+        if r and 0 <= sample < r[0]:
+            return r[1][3 * sample]
         self._chk(sample)
         return self._lib.b200_comp_q(self._h, sample)
 
     def get_d_val(self, sample):
-        r = self._results
-        if r is not None and 0 <= sample and 3 * sample < len(r[0]):
-            return r[0][3 * sample + 1]
+        r = self._results or self._read()
+        if r and 0 <= sample < r[0]:
+            return r[1][3 * sample + 1]
         self._chk(sample)
         return self._lib.b200_comp_d(self._h, sample)
 
     def get_m_val(self, sample):
-        r = self._results
-        if r is not None and 0 <= sample and 3 * sample < len(r[0]):
-            return r[0][3 * sample + 2]
+        r = self._results or self._read()
+        if r and 0 <= sample < r[0]:
+            return r[1][3 * sample + 2]
         self._chk(sample)
         return self._lib.b200_comp_m(self._h, sample)
 
@@ -211,7 +222,7 @@ class NetworkComputation:
         return np.ctypeslib.as_array(p, shape=(_lib.POLICY_SIZE,)).copy()
 
     def close(self):
-        self._results = None
+        self._changed()
         if self._h:
             self._lib.b200_comp_destroy(self._h)
             self._h = None
