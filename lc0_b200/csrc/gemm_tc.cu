@@ -270,7 +270,7 @@ __device__ __forceinline__ void epilogue_barrier(uint32_t bar, uint32_t& phase, 
 // gate = sigmoid(z[:C]), shift = z[C:] + gate * conv bias.  Runs on the eight epilogue warps while the accumulator
 // stays in tensor memory; `gb` receives [2 boards][gate 256 | shift 256].  `tmp` is the per-warp scratch area of the
 // slabs (2048 floats), free between two tiles.
-template <int BN, int kGroups = 2>
+template <int BN>
 __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int quarter, int group, int lane, int eid,
                                            float* tmp, float* gb, uint32_t bar, uint32_t& phase,
                                            volatile int* abort_flag, const float* w_smem = nullptr,
@@ -291,7 +291,7 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
   const int C = p.N;
   epilogue_barrier(bar, phase, abort_flag);  // nobody still reads the previous tile's per-warp vectors in `tmp`
 #pragma unroll 1
-  for (int c0 = group * 64; c0 < BN; c0 += 64 * kGroups) {
+  for (int c0 = group * 64; c0 < BN; c0 += 128) {
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
       uint32_t r[32];
@@ -305,8 +305,8 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
     }
   }
   epilogue_barrier(bar, phase, abort_flag);
-  if (kGroups == 2 || eid < 256) {
-    const int c = eid;  // one channel per thread
+  {
+    const int c = eid;  // 256 threads, one channel each
     const float b = c < C ? ld(g_bias + c) : 0.f;
     pool[c] = (part[c] + part[256 + c]) * (1.0f / 64.0f) + b;
     pool[256 + c] = (part[512 + c] + part[768 + c]) * (1.0f / 64.0f) + b;
@@ -315,7 +315,7 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
   // hid[s][k]: four threads per output, a quarter of the channels each (C is a multiple of 16 and se_k of 4, so the
   // quads of a warp run the same trip count).  The weights come from L2: 16-byte loads, several in flight, so that
   // the whole dot product costs about one round trip.
-  for (int o = eid >> 2; o < 2 * p.se_k; o += 32 * kGroups) {
+  for (int o = eid >> 2; o < 2 * p.se_k; o += 64) {
     const int sidx = o / p.se_k, k = o - sidx * p.se_k;
     // the four threads of an output take every fourth 16-byte piece of the row: consecutive addresses (no bank
     // conflicts in shared memory, whole lines per quad in global memory)
@@ -353,7 +353,7 @@ __device__ __forceinline__ void se_prepare(const TcParams& p, uint32_t trow, int
     const float ga = 1.0f / (1.0f + expf(-z0a)), gbb = 1.0f / (1.0f + expf(-z0b));
     gb[c] = ga; gb[256 + c] = z1a + ga * cb;
     gb[512 + c] = gbb; gb[768 + c] = z1b + gbb * cb;
-  } else if (kGroups == 2 || eid < 256) {
+  } else {
     gb[eid] = 0.f; gb[256 + eid] = 0.f; gb[512 + eid] = 0.f; gb[768 + eid] = 0.f;
   }
   epilogue_barrier(bar, phase, abort_flag);
@@ -1097,6 +1097,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_r,
                     const __grid_constant__ CUtensorMap tmap_c2, const __grid_constant__ CUtensorMap tmap_wh,
                     const TcParams p) {
+  static_assert(kMode != kConv || kGroups == 2, "se_prepare runs on two epilogue groups");
   using Cfg = PairCfg<kGroups>;
   constexpr int kBufs = Cfg::kBufs;
   constexpr int S = Cfg::kStages;
@@ -1153,7 +1154,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       mbar_init(smem_u32(&tfull_bar[i]), 1);
       mbar_init(smem_u32(&tempty_bar[i]), 8 * kGroups);
     }
-    mbar_init(smem_u32(se_bar), 128 * kGroups);
+    mbar_init(smem_u32(se_bar), 256);
     for (int i = 0; i < 4; ++i) {
       mbar_init(smem_u32(&res_bar[i]), 1);
       mbar_init(smem_u32(&stg_full[i]), 4);
@@ -1268,13 +1269,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     ColRegs cr;
     int cr_nb = -1;
     bool se_vec_ok = false;
-    if constexpr ((kGroups == 2 && kMode == kAny) || kMode == kConv) {
+    if constexpr (kMode == kConv) {
       if (p.se_k > 0 && 3 * p.N + p.se_k <= 1024) {
         // the squeeze-excitation bias vectors into shared memory while the first tile is computed
         const int eid = (int)threadIdx.x - 128;
-        for (int i = eid; i < p.N; i += 128 * kGroups) se_vec[i] = __ldg(p.se_bias + i);
-        for (int i = eid; i < p.se_k; i += 128 * kGroups) se_vec[p.N + i] = __ldg(p.se_b1 + i);
-        for (int i = eid; i < 2 * p.N; i += 128 * kGroups) se_vec[p.N + p.se_k + i] = __ldg(p.se_b2 + i);
+        for (int i = eid; i < p.N; i += 256) se_vec[i] = __ldg(p.se_bias + i);
+        for (int i = eid; i < p.se_k; i += 256) se_vec[p.N + i] = __ldg(p.se_b1 + i);
+        for (int i = eid; i < 2 * p.N; i += 256) se_vec[p.N + p.se_k + i] = __ldg(p.se_b2 + i);
         se_vec_ok = true;
       }
     }
@@ -1295,10 +1296,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       tcgen05_fence_after();
       const uint32_t trow = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
       const float* se_row = nullptr;
-      if constexpr ((kGroups == 2 && kMode == kAny) || kMode == kConv) {
+      if constexpr (kMode == kConv) {
         if (p.se_k > 0) {  // this CTA's 128 rows are two boards with all their channels
-          se_prepare<BN, kGroups>(p, trow, quarter, group, lane, (int)threadIdx.x - 128, wvec_all, se_gb, smem_u32(se_bar),
-                         se_phase, abort_flag, nullptr, se_vec_ok ? se_vec : nullptr);
+          se_prepare<BN>(p, trow, quarter, group, lane, (int)threadIdx.x - 128, wvec_all, se_gb, smem_u32(se_bar), se_phase,
+                         abort_flag, nullptr, se_vec_ok ? se_vec : nullptr);
           se_row = se_gb + (quarter >> 1) * 512;
         }
       }
@@ -1316,11 +1317,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           if (nn < p.N) next_nb = nn;
         }
         cr_nb = next_nb;
-        epilogue_slab<T, (kGroups == 2 && kMode == kAny) || kMode == kConv, false, kMode,
-                      kGroups == 2 && kMode != kAny && kMode != kConv ? 64 : 32>(p, epi_mem + idx * (BM * 128), smem_u32(&res_bar[idx]), smem_u32(&stg_free[idx]),
-                                       smem_u32(&stg_full[idx]), slab_it / kBufs, leader, trow + c0, quarter * 32 + lane,
-                                       lane, n0 + c0, next_nb, cr, wvec, rc, abort_flag,
-                                       se_row ? se_row + c0 : nullptr);
+        epilogue_slab<T, kMode == kConv, false, kMode, kGroups == 2 && kMode != kAny && kMode != kConv ? 64 : 32>(
+            p, epi_mem + idx * (BM * 128), smem_u32(&res_bar[idx]), smem_u32(&stg_free[idx]), smem_u32(&stg_full[idx]),
+            slab_it / kBufs, leader, trow + c0, quarter * 32 + lane, lane, n0 + c0, next_nb, cr, wvec, rc, abort_flag,
+            se_row ? se_row + c0 : nullptr);
         ++slab_it;
       }
       if (Epilogue<kMode>::out_stats(p)) flush_row_ctx(p, m, rc);
@@ -1737,7 +1737,7 @@ cudaError_t launch_pair_mode(const GemmParams& g, int* status, int sm_count, cud
   const int w_rows = conv ? 9 * g.N : (g.batch_rows > 0 ? g.N * (g.M / g.batch_rows) : g.N);
   e = get_map(g.W, conv ? g.conv_cin : g.ldw, w_rows, conv ? g.conv_cin : g.K, Cfg::BN / 2, prec, &mw);
   if (e != cudaSuccess) return e;
-  if (g.se_k > 0 && ((kGroups != 2 && kMode != kConv) || !gemm_tc_se_supported(g))) return cudaErrorInvalidValue;
+  if (g.se_k > 0 && (kMode != kConv || !gemm_tc_se_supported(g))) return cudaErrorInvalidValue;
   e = get_map(g.C, g.ldc, g.M, g.n_split > 0 ? g.n_split : g.N, BM, prec, &mc);
   if (e != cudaSuccess) return e;
   CUtensorMap mr = mc, mc2 = mc;
