@@ -350,8 +350,9 @@ int b200_op_gemm_ln(const void* x, const float* gamma, const float* beta, int gr
                     const float* bias, void* C, int M, int N, int activation, int precision, void* stream);
 /* b200_op_gemm_f32: C[M][N] = alpha * act(A[M][K] . W[N][K]^T + bias) + skip[M][N] in fp32 on tensor cores, as the network's
  *   fp32 mode runs its layers with 32 and more rows per position (Forward1D, fully_connected_layer.cc:50-106): operands cut
- *   into three bf16 pieces, no fewer digits than the FMA kernel.  conv != 0: 3x3 convolution over 8x8 boards, A [M][K] with M a
- *   multiple of 64, W [9][N][K] (winograd_convolution3.cc:47-57).  Leading dimension of A: lda; bias and skip may be NULL.  K a
+ *   into three bf16 pieces (24 bits from 2^-110 up, down to 2^-133 below).  Error at most (7 + 1.34 ceil(K / 64)) 2^-24 sum |a||w| (conv:
+ *   9 ceil(K / 64)); with weights of both signs smaller than the FMA kernel's.  conv != 0: 3x3 convolution over 8x8 boards, A [M][K]
+ *   with M a multiple of 64, W [9][N][K] (winograd_convolution3.cc:47-57).  Leading dimension of A: lda; bias and skip may be NULL.  K a
  *   multiple of 8, lda of 4, A on a 16-byte boundary.  A row's sum does not depend on the number of rows.  Allocates and frees the
  *   weights' pieces and synchronises the stream before returning. */
 int b200_op_gemm_f32(const float* A, long long lda, const float* W, const float* bias, const float* skip, float* C, int M, int N,

@@ -154,6 +154,37 @@ def test_fp32_tensor_core_products(lib, conv, shape):
         assert torch.equal(_f32_op(lib, A[:rows], W, b, None, conv), whole[:rows])
 
 
+def _taps(A):
+    """The rows of A that a 3x3 convolution reads, side by side: [M][9 * K]."""
+    x = torch.nn.functional.pad(A.view(-1, 8, 8, A.shape[1]), (0, 0, 1, 1, 1, 1))
+    return torch.cat([x[:, i:i + 8, j:j + 8] for i in range(3) for j in range(3)], 3).reshape(A.shape[0], -1).contiguous()
+
+
+@pytest.mark.parametrize("conv,M,N,K", [(0, 256, 256, 64), (0, 1024, 1024, 256), (0, 512, 3072, 1024), (0, 512, 1024, 1536),
+                                        (0, 128, 512, 4096), (1, 512, 128, 112), (1, 512, 128, 128), (1, 512, 256, 256)])
+def test_fp32_tensor_core_products_against_the_fma_kernel(lib, conv, M, N, K):
+    """Operands as the networks have them (weights of both signs; A of both or, behind a ReLU, of one): no further from sums in 64
+    bits than the FMA kernel.  Operands that favour it (one sign, many decades, pieces that leave out the most): inside the
+    bound of the header."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    wide = lambda *s: rnd(*s) * torch.exp(4 * rnd(*s))
+    most = lambda *s: torch.full(s, 1 + 2.0 ** -8 - 2.0 ** -17 + 2.0 ** -23, device="cuda")
+    blocks = (9 if conv else 1) * ((K + 63) // 64)
+    shape = (9, N, K) if conv else (N, K)
+    for of_a, of_w, network_like in ((rnd, rnd, True), (lambda *s: rnd(*s).relu(), rnd, True), (lambda *s: rnd(*s).abs(), lambda *s: rnd(*s).abs(), False),
+                                     (wide, wide, False), (most, most, False)):
+        A, W = of_a(M, K), of_w(*shape)
+        a2, w2 = (_taps(A), W.permute(1, 0, 2).reshape(N, -1).contiguous()) if conv else (A, W)
+        want, size = a2.double() @ w2.double().T, a2.double().abs() @ w2.double().abs().T
+        got, fma = _f32_op(lib, A, W, None, None, conv).double(), torch.empty(M, N, device="cuda")
+        assert ((got - want).abs() <= (7 + 1.34 * blocks) * 2.0 ** -24 * size).all()
+        if network_like:
+            _lib.check(lib.b200_op_gemm(a2.data_ptr(), w2.data_ptr(), None, fma.data_ptr(), M, N, a2.shape[1], oracle.ACT_NONE, 0, 0, None))
+            torch.cuda.synchronize()
+            assert (got - want).norm() <= (fma.double() - want).norm()
+
+
 @pytest.mark.parametrize("conv", [0, 1])
 def test_fp32_tensor_core_products_of_extreme_values(lib, conv):
     """Infinities, NaN, values that round to an infinite bf16 and values near the smallest normal: as the FMA kernel has them."""
