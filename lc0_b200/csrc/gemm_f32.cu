@@ -6,27 +6,32 @@
 // pieces is exact in fp32, and of the nine six are summed:
 //   a1 w1                      order 1
 //   a1 w2 + a2 w1              order 2^-8
-//   a1 w3 + a2 w2 + a3 w1      order 2^-16;  what is left out (a2 w3 + a3 w2 + a3 w3) is below 2^-23.99 of |a||w|, and comes to 2^-24.04
+//   a1 w3 + a2 w2 + a3 w1      order 2^-16
+// What is left out (a2 w3 + a3 w2 + a3 w3) is below 2^-23.99 of |a||w|, and comes to 2^-24.04.
 // The tensor core adds to its accumulator with truncation, which over a long K range would cost more digits than an FMA chain
 // has to lose.  So the sums of order 1 stay in tensor memory for 32 k only and are then added, rounded, in registers.  The small
-// orders stay there for the whole range: 20 truncations per 64 k, each below 2^-23 of a sum that is below 2^-6.9 of sum |a||w|, i.e. at most
-// 2^-25.6 of sum |a||w| per 64 k where all terms have one sign.  A row's sum is taken in the same order at every number of rows and grid.
+// orders stay there for the whole range: 20 truncations per 64 k, each below 2^-23 of a sum that is below 2^-6.9 of sum |a||w|,
+// i.e. at most 2^-25.6 of sum |a||w| per 64 k where all terms have one sign.  A row's sum is taken in the same order at every
+// number of rows and grid.
 // Error against sums in 64 bits (relative 2-norm), this kernel / FMA kernel (convolutions: the FMA kernel on the gathered taps), of
 // operands as the networks have them (weights of both signs):
 //   normal operands    1024x1024x256 0.68e-7 / 1.5e-7   1024x3072x1024 0.95e-7 / 2.9e-7   512x1024x1536 1.1e-7 / 2.5e-7
 //                      128x512x4096 1.7e-7 / 2.9e-7   convolutions 112 -> 128 0.94e-7 / 1.5e-7   256 -> 256 1.2e-7 / 2.2e-7
 //   non-negative A     the same within 5 %
-// Where one sign or one term prevails the rounded sums of the FMA kernel are the better ones: both operands non-negative, 1024x3072x1024
-// 0.81e-7 / 1.3e-7, 512x1024x1536 0.80e-7 / 0.77e-7, 128x512x4096 1.3e-7 / 0.80e-7, convolution 256 -> 256 0.99e-7 / 0.68e-7; operands over
-// eight decades 0.4e-7 .. 1.3e-7 / 0.1e-7 .. 1.2e-7; every operand 1 + 2^-8 - 2^-17 + 2^-23 (the most that can be left out), 4096 k 5.3e-7 / 0.6e-7.
+// Where one sign or one term prevails the FMA kernel can be the better one: both operands non-negative, 1024x3072x1024
+// 0.81e-7 / 1.3e-7, 512x1024x1536 0.80e-7 / 0.77e-7, 128x512x4096 1.3e-7 / 0.80e-7, convolution 256 -> 256 0.99e-7 / 0.68e-7;
+// operands over eight decades 0.1e-7 .. 1.3e-7 / 0.1e-7 .. 1.2e-7; every operand 1 + 2^-8 - 2^-17 + 2^-23 (the most that can be
+// left out), 4096 k 5.3e-7 / 0.6e-7.
 // With 64 k per rounded sum 1024x3072x1024 had 1.04e-7.
 //
-// The FMA pipe has 74 TFLOP/s and gave half of them; six MMAs for one leave 277 at the measured bf16 rate.  What paces a k-block of
-// 64 columns (0.67 us alone on an SM, its MMAs 0.40, its shared-memory traffic 0.55): waits of the issuing thread, some 150 cycles each, which
-// the queue of MMAs hides only in part.  Hence one wait for A and one for the accumulators per k-block and nothing else.  A's pieces
-// live in tensor memory, where an MMA reads them beside shared memory; in shared memory (48 KB written and 64 KB read more per
-// k-block) it took 0.79 us at 64 columns and 1.25 at 128.  Twice as many converter warps were slower (0.80), waits between the MMAs too.
-// us per launch, FMA kernel / this: 1024x3072x1024 175 / 56, 1024x1024x1024 70 / 19, 64x1024x1024 13 / 13, 4096x3072x1024 678 / 198;
+// The FMA pipe has 74 TFLOP/s and gave half of them; six MMAs for one leave 277 at the measured bf16 rate.  What paces a
+// k-block of 64 columns (0.67 us alone on an SM, its MMAs 0.40, its shared-memory traffic 0.55): waits of the issuing thread,
+// some 150 cycles each, which the queue of MMAs hides only in part; and what a tile has beside its k-blocks, about 7 us of
+// prologue, first loads and epilogue (4.8 at 32 columns), which nothing covers, since a CTA has one tile: 38 % of it at K =
+// 1024.  Hence one wait for A and one for the accumulators per k-block and nothing else.  A's pieces live in tensor memory,
+// where an MMA reads them beside shared memory; in shared memory (48 KB written and 64 KB read more per k-block) it took 0.79
+// us at 64 columns and 1.25 at 128.  Twice as many converter warps were slower (0.80), waits between the MMAs too. us per
+// launch, FMA kernel / this: 1024x3072x1024 175 / 56, 1024x1024x1024 70 / 19, 64x1024x1024 13 / 13, 4096x3072x1024 678 / 198;
 // 3x3 convolution 128 -> 128 of 64 boards 53 / 16.3.
 //   warp 8       TMA: fp32 tile of A, pieces of W (made once at load); the weights' first stages ahead of the grid dependency
 //   warps 0-7    fp32 rows (a thread has one row, half of 64 k) -> three bf16 pieces -> tensor memory

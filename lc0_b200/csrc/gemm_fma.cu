@@ -1,5 +1,6 @@
 // FMA matrix kernel: the fp32 verification mode's products with fewer than 32 rows per position, its layers of shapes that
-// gemm_f32.cu does not take (and all of it with the tensor cores switched off), and 16-bit products of shapes that the TMA path does not take (leading dimensions that are no multiple of 8, stacked products, products in fp32 storage).
+// gemm_f32.cu does not take (and all of it with the tensor cores switched off), and 16-bit products of shapes that the TMA path
+// does not take (leading dimensions that are no multiple of 8, stacked products, products in fp32 storage).
 // (reference: FullyConnectedLayer::Forward1D, backends/blas/fully_connected_layer.cc:50-106;
 // WinogradConvolution3::Forward, backends/blas/winograd_convolution3.cc:47-57, same sums through F(2x2,3x3) transforms)
 //

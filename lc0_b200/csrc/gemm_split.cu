@@ -457,10 +457,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 }
 
 // Tile width, cluster size and stages of a product: the least of a cost model in microseconds, fitted to chains of dependent
-// launches of this kernel before its issuing lanes were elected (M x N x K; us at columns per tile / CTAs per tile).  A k-block took
-// 731 cycles to issue then, 0.39 us, and takes 495 - 527 now: the model still orders the plans it was fitted to, but weighs a long K
-// range too heavily against the exchange of a cut one, and has not been fitted again.  Tiles of 64 rows also above 64 rows: 10 x 256
-// attention network 2 / 8 / 16 / 37 positions 271 / 283 / 307 / 369 -> 225 / 258 / 271 / 332 us, BT4-class 2 / 8 963 / 1057 -> 842 / 1008.
+// launches of this kernel before its issuing lanes were elected (M x N x K; us at columns per tile / CTAs per tile).  A k-block
+// took 731 cycles to issue then, 0.39 us, and takes 495 - 527 now: the model still orders the plans it was fitted to, but
+// weighs a long K range too heavily against the exchange of a cut one, and has not been fitted again (another plan may cut K
+// elsewhere, and results would change).  Tiles of 64 rows also above 64 rows: 10 x 256 attention network 2 / 8 / 16 / 37
+// positions 271 / 283 / 307 / 369 -> 225 / 258 / 271 / 332 us, BT4-class 2 / 8 963 / 1057 -> 842 / 1008.
 //   1536x1024x1024  32/1 19.5  64/1 11.2  64/2 17.6  128/1 13.9  128/2 12.5    2368x768x256   32/1 10.3  64/1 6.7  128/1 9.2
 //   512x1024x1024   32/1 10.0  32/2 7.9   64/1 11.3  64/4 9.1    128/1 13.6    2368x256x256   32/1 5.3   64/1 6.6  128/1 9.0
 //   512x1024x1536   32/2 9.5   64/2 10.9  64/4 9.8   128/2 12.7                64x1024x1024   32/4 5.9   64/1 9.8  64/4 6.3

@@ -1351,10 +1351,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 // The tower kernel for 192 and 256 channels, on CTA pairs: a pair owns four boards, a CTA two of them, and a layer is one
 // 256 x N tile of cta_group::2 MMAs.  A CTA reads as A only rows it stored itself and supplies half of the filters, so the two meet in
 // the operand barriers alone.  Against one launch per convolution (pair kernel, one tile per pair: no main loop to hide
-// launch, first loads, epilogue and stores under) the whole evaluation of the 20 x 256 network
-// takes, us, launch per convolution / tower: 16 boards 1022 / 907, 256 1245 / 1169, 592 2059 / 1879, 1024 3590 / 3524, 1500
-// 5299 / 5384, 2048 6833 / 6742 (a layer of 256 boards: 20.8 us, 19.9 since se_prepare reads its second matrix in order).  The squeeze-excitation matrices
-// (96 KB at 256 channels and 32 hidden units) do not fit beside the pipeline and come from L2, its vectors are copied per layer.
+// launch, first loads, epilogue and stores under) the whole evaluation of the 20 x 256 network on the device takes, us, launch per
+// convolution / tower: 4 boards 973 / 811, 256 959 / 897, 592 1808 / 1467, 1000 2935 / 2899; further sizes, and those that it does
+// not take, at gemm_tc_tower_pays.  A layer of 256 boards: 20.8 us, 19.9 since se_prepare reads its second matrix in order.  The
+// squeeze-excitation matrices (96 KB at 256 channels and 32 hidden units) do not fit beside the pipeline and come from L2, its
+// vectors are copied per layer.
 // ------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<2>::kThreads, 1)
@@ -1960,13 +1961,14 @@ int tower_row_blocks(int channels, int sm_count) {
 }
 }  // namespace
 
-// Narrow towers are ahead of one launch per convolution at every size they take (10 x 128, us: 64 boards 234 / 311, 889 578 / 790, 2368
-// 1279 / 1737; 10 x 64 1.36 to 1.65 times).  Wide ones come in whole rounds of four boards per pair, of which the last may be
-// nearly empty, and lose more to that the more rounds precede it.  20 x 256, tower / launches: 593 boards 1955 / 1966, 888 2264 / 2572;
-// 889 2745 / 2674, 920 2780 / 2806, 1184 3130 / 3290; 1185 3606 / 3440, 1340 3829 / 3783, 1420 3939 / 3949, 1480 3996 / 4085; 1481
-// 4489 / 4248, 1776 4946 / 4836, 2368 6544 / 6380.  20 x 192: 1185 2484 / 2486, 1777 3656 / 3646, 2072 3951 / 4101; 2073 4283 / 4217,
-// 2140 4339 / 4398, 2368 4572 / 4664.  So the last round has to be filled to 0.7 of a round per whole round before it less two rounds (from
-// four rounds on a tenth, of five four fifths, six never), at 192 channels to 0.2 less 1.2 (of eight rounds a fifth).
+// Narrow towers are ahead of one launch per convolution at every size they take (10 x 128, us: 64 boards 234 / 311, 889 578 / 790,
+// 2368 1279 / 1737; 10 x 64 1.36 to 1.65 times).  Wide ones come in whole rounds of four boards per pair, of which the last may
+// be nearly empty, and lose more to that the more rounds precede it.  20 x 256, tower / launches: 593 boards 1955 / 1966, 888
+// 2264 / 2572; 889 2745 / 2674, 920 2780 / 2806, 1184 3130 / 3290; 1185 3606 / 3440, 1340 3829 / 3783, 1420 3939 / 3949, 1480
+// 3996 / 4085; 1481 4489 / 4248, 1776 4946 / 4836, 2368 6544 / 6380.  20 x 192: 1185 2484 / 2486, 1777 3656 / 3646, 2072
+// 3951 / 4101; 2073 4283 / 4217, 2140 4339 / 4398, 2368 4572 / 4664.  So with `full` whole rounds before it the last round has to
+// be filled to 0.7 full - 2 (a tenth of a fourth round, four fifths of a fifth, a sixth never), at 192 channels to
+// 0.2 full - 1.2 (a fifth of an eighth).
 bool gemm_tc_tower_pays(int channels, int boards, int sm_count) {
   const int row_blocks = (boards + 1) / 2;
   if (row_blocks > tower_row_blocks(channels, sm_count)) return false;

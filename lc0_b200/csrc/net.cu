@@ -1314,9 +1314,7 @@ struct Net : NetBase {
   // forward().
   void build_towers() {
     if constexpr (sizeof(T) == 2) {
-      // Measured (evaluations per second, tower / per-layer launches): 10 blocks of 128 filters 176 100 / 161 400 at
-      // batch 64 and 670 800 / 589 000 at batch 256; 20 blocks of 256 filters, whose tower kernel works on CTA pairs,
-      // 68 300 / 59 400 at batch 64, 219 000 / 205 300 at 256, 304 000 / 300 000 at 2048.
+      // Towers of more than 128 filters work on CTA pairs; at which batches either form runs: gemm_tc_tower_pays.
       if (!tower || res.empty() || C > 256) { tower = false; return; }
       for (const auto& r : res)
         if (!r.se) { tower = false; return; }
