@@ -1284,17 +1284,24 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       load_col_regs<kMode>(p, cr_nb, lane, cr);
     }
     auto row_of = [&](int t) { return (tile_of(t) / n_tiles) * (2 * BM) + (int)rank * BM + quarter * 32 + lane; };
+    // The general form on four groups reads them where it needs them: a tile ahead they are eight registers more of 96, and what
+    // that spilled cost products without statistics 4 to 9 % (65536x4096x256 with a scale 221 us, 241 ahead) and those with everything
+    // 11 % (65536x1024x576, LayerNorms of A and of the residual, statistics: 146, 162 ahead).
+    constexpr bool kAhead = kMode != kAny || kGroups == 2;
     RowStats row_stats;
-    fetch_row_stats<kMode>(p, row_of(pair), row_stats);
+    if constexpr (kAhead) fetch_row_stats<kMode>(p, row_of(pair), row_stats);
     for (int t = pair; t < tiles; t += pairs, ++tile_it) {
       const uint32_t acc = tile_it & 1, aph = (tile_it >> 1) & 1;
       const int m = row_of(t), n0 = col_of(t), width = width_of(t);
       RowCtx rc;
-      use_row_stats<kMode>(p, row_stats, rc);
-      if (t + pairs < tiles) fetch_row_stats<kMode>(p, row_of(t + pairs), row_stats);
+      if constexpr (kAhead) {
+        use_row_stats<kMode>(p, row_stats, rc);
+        if (t + pairs < tiles) fetch_row_stats<kMode>(p, row_of(t + pairs), row_stats);
+      }
       if (!mbar_wait(smem_u32(&tfull_bar[acc]), aph, abort_flag, 4)) break;
       tcgen05_fence_after();
       const uint32_t trow = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
+      if constexpr (!kAhead) load_row_ctx(p, m, rc);
       const float* se_row = nullptr;
       if constexpr (kMode == kConv) {
         if (p.se_k > 0) {  // this CTA's 128 rows are two boards with all their channels
@@ -1784,7 +1791,6 @@ cudaError_t launch_pair_mode(const GemmParams& g, int* status, int sm_count, cud
 // (one kernel that asked for everything at run time: 87, 48.6, 37.5, 41.5; 42, 50.6, 22.9, 25.8; 24.8, 104).
 // Residual in no compiled form (operator interface), 9 to 16 k-blocks, two groups / four, faster issue:
 //   with Mish                                  65536x1024x576 170 / 152   x768 185 / 164   x1024 200 / 178   65536x512x1024 120 / 113
-//   LayerNorm of A, residual, statistics       65536x1024x576 156 / 134   x768 166 / 153   x1024 185 / 167   65536x512x1024 112 / 108
 //   residual alone                             65536x1024x576 142 / 127   x768 150 / 137   x1024 162 / 163   65536x512x1024 103 / 104
 // Statistics without a residual are as fast or faster on two (65536x1024x1024 153 / 155, 65536x512x1024 98 / 102).
 template <typename T>
