@@ -923,7 +923,11 @@ cudaError_t launch_se(const T* x, const float* conv_bias, const T* skip, const f
     const size_t tile = (size_t)64 * C * sizeof(T), rest = (size_t)(3 * se_k * C + 2048 + 6 * C + 2 * se_k) * sizeof(float);
     const int stage_skip = rest + 2 * tile <= kMaxSmem;
     const size_t smem = rest + (stage_skip ? 2 : 1) * tile;
-    if (smem <= kMaxSmem) {
+    // Of 512 channels an SM holds one block of this kernel and two of se_vec_kernel: where the skip input is not staged either, more
+    // than a round of them (148 SMs) is behind.  16 bits, 12 hidden units, four blocks of 512 filters, us, se_vec_kernel / this one: 64
+    // boards 346 / 332, 148 490 / 481, 200 726 / 759, 512 1490 / 1555, 1000 2740 / 2881.  256 channels stay ahead (fp32, 32
+    // units, 1 to 2 % of the network at every size).
+    if (smem <= kMaxSmem && (stage_skip || C <= 256 || n <= 148)) {
       const auto kernel = se_staged_kernel<T, (sizeof(T) == 2)>;
       if (smem > 48 * 1024) {
         cudaError_t e = raise_smem_limit<&se_staged_kernel<T, (sizeof(T) == 2)>>((int)kMaxSmem);

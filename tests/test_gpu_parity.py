@@ -222,6 +222,21 @@ def test_squeeze_excitation_after_the_convolution(filters, se):
     _assert_fp32_scalar(out["q"], want["q"])
 
 
+def test_squeeze_excitation_of_512_filters_on_both_sides_of_a_round():
+    """Up to 148 boards with the matrices in shared memory, beyond them without: the same bits."""
+    net = mknet.make_net("cfg2", blocks=2, filters=512, se=12)
+    _, pos, n, g = load_compact("cfg4_2layer_b1024")
+    masks, values = np.array(pos["masks"][:160]), np.array(pos["values"][:160])
+    nw = network.Network(net, "precision=fp16,max_batch=160")
+    whole = nw.evaluate(masks, values)
+    for batch in (148, 149):
+        out = nw.evaluate(masks[:batch], values[:batch])
+        for k in ("policy", "q", "d", "m"):
+            np.testing.assert_array_equal(out[k], whole[k][:batch])
+    assert nw.device_status() == 0
+    nw.close()
+
+
 def _mini(kind, width):
     if kind == "attention":  # heads of depth `width`
         return mknet.make_net("cfg3_mini", emb=256, heads=256 // width, layers=8)
