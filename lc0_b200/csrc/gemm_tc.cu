@@ -1789,10 +1789,15 @@ cudaError_t launch_pair_mode(const GemmParams& g, int* status, int sm_count, cud
 //   residual, statistics   16384x1024x1024 39 / 41 / 36   16384x1024x1536 48 / 54 / 49   32768x256x256 24 / 22 / 22   32768x256x512 27 / 25 / 25
 //   neither                8192x4096x256 19.5 / 21.7 / 19.6   32768x4096x256 84 / 95 / 87
 // (one kernel that asked for everything at run time: 87, 48.6, 37.5, 41.5; 42, 50.6, 22.9, 25.8; 24.8, 104).
-// Residual in no compiled form (operator interface), 9 to 16 k-blocks, two groups / four, faster issue:
-//   with Mish                                  65536x1024x576 170 / 152   x768 185 / 164   x1024 200 / 178   65536x512x1024 120 / 113
-//   residual alone                             65536x1024x576 142 / 127   x768 150 / 137   x1024 162 / 163   65536x512x1024 103 / 104
-// Statistics without a residual are as fast or faster on two (65536x1024x1024 153 / 155, 65536x512x1024 98 / 102).
+// Residual or statistics in no compiled form (operator interface), four groups with the slower issue (what they had before the
+// epilogues were compiled per form) / with the faster one:
+//   residual, both LayerNorms, statistics   8192x1024x576 22.1 / 23.6   65536x1536x576 158 / 169   x704 up to 7 % slower, x768 6 %
+//   residual alone or with an activation    8192x1536x576 25.5 / 27.5   16384x512: x640 4 %, x768 1 to 2 %
+//   all these forms from 14 k-blocks on     0.92 to 1.00 of the slower issue's time on the mean of the sizes, at worst 1.05
+// and beyond 8 k-blocks two groups / four, faster issue: with Mish 65536x1024x576 170 / 152, x1024 200 / 178; residual alone
+// 65536x1024x768 150 / 137, x1024 162 / 163.
+//   statistics without a residual, four groups, slower issue / two: 65536x1536x520 1 / 1.07 to 1.11, x576 1 / 1.05, x640 1 / 0.98 to
+//   1.02, x1024 1 / 0.85 to 0.93
 template <typename T>
 cudaError_t launch_pair(const GemmParams& g, int* status, int sm_count, cudaStream_t s) {
   const bool few = g.K <= 8 * BK && g.conv_cin == 0 && g.se_k == 0;
@@ -1808,7 +1813,8 @@ cudaError_t launch_pair(const GemmParams& g, int* status, int sm_count, cudaStre
     case kConv:
       return launch_pair_mode<T, 2, true, kConv>(g, status, sm_count, s);
     default:
-      if (few) return launch_pair_mode<T, 4, false, kAny>(g, status, sm_count, s);
+      if (few || (g.conv_cin == 0 && g.K <= (g.res ? 12 : g.out_stats ? 9 : 8) * BK))
+        return launch_pair_mode<T, 4, false, kAny>(g, status, sm_count, s);
       return g.res && g.conv_cin == 0 && g.K <= 16 * BK ? launch_pair_mode<T, 4, true, kAny>(g, status, sm_count, s)
                                                         : launch_pair_mode<T, 2, true, kAny>(g, status, sm_count, s);
   }

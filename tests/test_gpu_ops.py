@@ -491,10 +491,11 @@ def test_second_output_of_the_pair_kernel_with_folded_input(lib, whole_tiles):
 
 @pytest.mark.parametrize("prec", [1, 2])
 @pytest.mark.parametrize("form", ["res act", "stats act", "norm res", "norm res stats"])
-@pytest.mark.parametrize("M,N,K", [(8192, 1024, 512), (8200, 1000, 520), (8200, 1000, 1024), (8192, 1024, 1032)])
+@pytest.mark.parametrize("M,N,K", [(8192, 1024, 512), (8200, 1000, 520), (8192, 1024, 576), (8200, 1000, 584), (8200, 1000, 768),
+                                   (8192, 1024, 776), (8200, 1000, 1024), (8192, 1024, 1032)])
 def test_forms_of_the_pair_kernel_that_no_layer_has(lib, prec, form, M, N, K):
     """Residual or statistics beside an activation or a folded LayerNorm of A: both sides of the lines between two and four
-    groups of epilogue warps (8 and 16 k-blocks), ragged rows, columns and k-blocks."""
+    groups of epilogue warps and the forms of issue (8, 9, 12 and 16 k-blocks), ragged rows, columns and k-blocks."""
     dt = DT[prec]
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
