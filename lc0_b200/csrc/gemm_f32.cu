@@ -11,17 +11,18 @@
 // The tensor core adds to its accumulator with truncation, which over a long K range would cost more digits than an FMA chain
 // has to lose.  So the sums of order 1 stay in tensor memory for 32 k only and are then added, rounded, in registers.  The small
 // orders stay there for the whole range: 20 truncations per 64 k, each below 2^-23 of a sum that is below 2^-6.9 of sum |a||w|,
-// i.e. at most 2^-25.6 of sum |a||w| per 64 k where all terms have one sign.  A row's sum is taken in the same order at every
-// number of rows and grid.
+// i.e. at most 2^-25.6 of sum |a||w| per 64 k where all terms have one sign.  A long K over few columns is summed in two to eight
+// pieces (f32_pieces), each with its small orders, by a CTA of a cluster each or in turn.  A row's sum is taken in the same order at
+// every number of rows and grid.
 // Error against sums in 64 bits (relative 2-norm), this kernel / FMA kernel (convolutions: the FMA kernel on the gathered taps), of
 // operands as the networks have them (weights of both signs):
 //   normal operands    1024x1024x256 0.68e-7 / 1.5e-7   1024x3072x1024 0.95e-7 / 2.9e-7   512x1024x1536 1.1e-7 / 2.5e-7
-//                      128x512x4096 1.7e-7 / 2.9e-7   convolutions 112 -> 128 0.94e-7 / 1.5e-7   256 -> 256 1.2e-7 / 2.2e-7
+//                      128x512x4096 1.0e-7 / 3.0e-7   convolutions 112 -> 128 0.82e-7 / 1.5e-7   256 -> 256 0.89e-7 / 2.2e-7
 //   non-negative A     the same within 5 %
 // Where one sign or one term prevails the FMA kernel can be the better one: both operands non-negative, 1024x3072x1024
-// 0.81e-7 / 1.3e-7, 512x1024x1536 0.80e-7 / 0.77e-7, 128x512x4096 1.3e-7 / 0.80e-7, convolution 256 -> 256 0.99e-7 / 0.68e-7;
+// 0.81e-7 / 1.3e-7, 512x1024x1536 0.80e-7 / 0.77e-7, 128x512x4096 0.63e-7 / 0.79e-7, convolution 256 -> 256 0.61e-7 / 0.68e-7;
 // operands over eight decades 0.1e-7 .. 1.3e-7 / 0.1e-7 .. 1.2e-7; every operand 1 + 2^-8 - 2^-17 + 2^-23 (the most that can be
-// left out), 4096 k 5.3e-7 / 0.6e-7.
+// left out), 1536 k in one piece 1.4e-7 / 1.0e-7.
 // With 64 k per rounded sum 1024x3072x1024 had 1.04e-7.
 //
 // The FMA pipe has 74 TFLOP/s and gave half of them; six MMAs for one leave 277 at the measured bf16 rate.  What paces a
@@ -63,20 +64,28 @@ struct F32Params {
   int conv_cin;   // convolution: A is [M][cin] on 8x8 boards, W [9][N][cin]
   int cblocks;    // ... k-blocks per tap
   int k_blocks;
+  int pieces;     // of K, each summed by itself; see f32_pieces
   int vec_c;      // C may be written, skip and bias read in 16-byte pieces
   int* status;
 };
+
+// What a CTA does with the pieces of K: there is one; it takes them in turn; a CTA of a cluster takes each.
+enum F32Pieces { kOnePiece, kInTurn, kCluster };
 
 template <int BN> struct F32Tile {
   static constexpr int kRaw = 128 * 64 * 4, kW = 3 * BN * 128;  // bytes of a k-block: two boxes of 32 fp32 columns, pieces of W
   static constexpr int kStage = kRaw + kW;
   static constexpr int kStages = BN == 64 ? 3 : 4;
   static constexpr int kOut = 128 * (BN + 4) * 4;  // the tile's sums, in place of the ring
+  // sums of the pieces so far: of 32 columns in registers; 64 would not leave enough of those and have room behind the ring
+  static constexpr bool kOutBehind = BN > 32;
   static constexpr int kBytes = kStages * kStage + 1024 /*alignment*/ + 256 /*barriers*/;
+  static constexpr int bytes(F32Pieces mode) { return kBytes + (mode == kInTurn && kOutBehind ? kOut : 0); }
   static_assert(kStages * kStage >= kOut, "the sums take the place of the ring");
-  // tensor memory: two buffers for the order-1 sums of either half of a k-block, the small orders (BN columns each), stages of A's
-  // pieces (for either half of the k-block 3 x 16 columns)
-  static constexpr int kXCol = 4 * BN, kACol = 5 * BN, kCols = 512;
+  // tensor memory: two buffers for the order-1 sums of either half of a k-block, one or two for the small orders (BN columns each),
+  // stages of A's pieces (for either half of the k-block 3 x 16 columns)
+  static constexpr int kXBufs = BN == 32 ? 2 : 1;
+  static constexpr int kXCol = 4 * BN, kACol = (4 + kXBufs) * BN, kCols = 512;
   static_assert(kACol + kAStages * 96 <= kCols, "tensor memory");
 };
 
@@ -118,6 +127,17 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const float* __restr
   out[2 * count + i] = __ushort_as_bfloat16((unsigned short)u3);
 }
 
+__device__ __forceinline__ float4 add_rn(const float4 a, const float4 b) {
+  return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+}
+// The four numbers at `q`'s place in the shared memory of CTA `rank` of the cluster.
+__device__ __forceinline__ float4 load_peer(const float* q, int rank) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(mapa(smem_u32(q), (uint32_t)rank)) : "memory");
+  return v;
+}
+
 // Row m, column n of the product from the fp32 operands, by a whole warp.
 template <bool kConv>
 __device__ __forceinline__ float warp_dot(const F32Params& p, int m, int n) {
@@ -137,7 +157,7 @@ __device__ __forceinline__ float warp_dot(const F32Params& p, int m, int n) {
   return warp_sum(v);
 }
 
-template <int BN, bool kConv>
+template <int BN, bool kConv, F32Pieces kMode>
 __global__ void __launch_bounds__(kF32Threads, 1)
 gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const F32Params p) {
   using L = F32Tile<BN>;
@@ -150,13 +170,19 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   uint64_t* aempty_bar = afull_bar + AS;                                   // [AS] ... and read by the MMAs
   uint64_t* hfull_bar = aempty_bar + AS;                                   // [2] order-1 sums complete
   uint64_t* hempty_bar = hfull_bar + 2;                                    // [2] ... and read by eight warps
-  uint64_t* xfull_bar = hempty_bar + 2;                                    // every MMA done
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xfull_bar + 1);
+  uint64_t* xfull_bar = hempty_bar + 2;                                    // [kXBufs] every MMA of a piece of K done
+  uint64_t* xempty_bar = xfull_bar + L::kXBufs;                            // [kXBufs] its small orders read by eight warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xempty_bar + L::kXBufs);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
-  const int n0 = (int)blockIdx.x * BN, m0 = (int)blockIdx.y * 128;
-  const int kbn = p.k_blocks;
+  const int ks = kMode == kCluster ? p.pieces : 1, rank = kMode == kCluster ? (int)blockIdx.x % ks : 0;
+  const int n0 = (int)blockIdx.x / ks * BN, m0 = (int)blockIdx.y * 128;
+  // this CTA's k-blocks [kb0, kb0 + kbn) and where its q-th piece of them ends
+  const int kb0 = kMode == kCluster ? rank * p.k_blocks / ks : 0;
+  const int kbn = kMode == kCluster ? (rank + 1) * p.k_blocks / ks - kb0 : p.k_blocks;
+  const int nq = kMode == kInTurn ? p.pieces : 1;
+  auto piece_end = [&](int q) { return kMode == kInTurn ? (q + 1) * kbn / nq : kbn; };
 
   if (tid == 256) {
     tma_prefetch_map(&tmap_w);
@@ -173,7 +199,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       mbar_init(smem_u32(&hfull_bar[i]), 1);
       mbar_init(smem_u32(&hempty_bar[i]), 8);
     }
-    mbar_init(smem_u32(xfull_bar), 1);
+    for (int i = 0; i < L::kXBufs; ++i) {
+      mbar_init(smem_u32(&xfull_bar[i]), 1);
+      mbar_init(smem_u32(&xempty_bar[i]), 8);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -189,6 +218,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   // after the allocation: the next kernel's CTAs must not take the tensor memory that this one still waits for
   grid_launch_dependents();
   const uint32_t tmem = *tmem_slot;
+  float* out = reinterpret_cast<float*>(kMode == kInTurn && L::kOutBehind ? smem + S * L::kStage + 256 : smem);
 
   if (warp < 8) {
     // ---------------- A: fp32 rows -> pieces ----------------
@@ -227,10 +257,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       auto load_w = [&](int i, int s) {
         const uint32_t fb = smem_u32(&full_bar[s]), dst = smem_u32(smem + s * L::kStage) + L::kRaw;
         mbar_expect_tx(fb, L::kStage);
-        int row = n0, x = i * 64, plane = p.N;
+        int row = n0, x = (kb0 + i) * 64, plane = p.N;
         if constexpr (kConv) {
-          const int tap = i / p.cblocks;
-          x = (i - tap * p.cblocks) * 64;
+          const int tap = (kb0 + i) / p.cblocks;
+          x = (kb0 + i - tap * p.cblocks) * 64;
           row += tap * p.N;
           plane = 9 * p.N;
         }
@@ -250,12 +280,12 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         }
         const uint32_t fb = smem_u32(&full_bar[s]), dst = smem_u32(smem + s * L::kStage);
         if constexpr (kConv) {
-          const int tap = i / p.cblocks, x = (i - tap * p.cblocks) * 64;
+          const int tap = (kb0 + i) / p.cblocks, x = (kb0 + i - tap * p.cblocks) * 64;
 #pragma unroll
           for (int h = 0; h < 2; ++h) tma_load_4d(dst + h * 16384, &tmap_a, x + 32 * h, tap % 3 - 1, tap / 3 - 1, m0 >> 6, fb);
         } else {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * 16384, &tmap_a, i * 64 + 32 * h, m0, fb);
+          for (int h = 0; h < 2; ++h) tma_load_2d(dst + h * 16384, &tmap_a, (kb0 + i) * 64 + 32 * h, m0, fb);
         }
         if (++s == S) { s = 0; ph ^= 1; }
       }
@@ -266,33 +296,38 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     if (elect_one()) {
       constexpr uint32_t one = make_idesc<__nv_bfloat16, BN>();
       bool good = true;
-      int s = 0;
-      for (int i = 0; i < kbn; ++i) {
-        // A's pieces are in place; the warps that wrote them have seen the weights land too
-        if (!mbar_wait(smem_u32(&afull_bar[i & 1]), (i >> 1) & 1, abort_flag, 5)) { good = false; break; }
-        if (i > 1 && !mbar_wait(smem_u32(&hempty_bar[i & 1]), ((i >> 1) & 1) ^ 1, abort_flag, 6)) { good = false; break; }
-        tcgen05_fence_after();
-        const int a = i & 1;
-        const uint32_t sw = smem_u32(smem + s * L::kStage) + L::kRaw, a1 = tmem + L::kACol + a * 96;
-        const uint32_t h = tmem + a * 2 * BN, x = tmem + L::kXCol;
-        const uint64_t w1 = make_smem_desc(sw), w2 = make_smem_desc(sw + BN * 128), w3 = make_smem_desc(sw + 2 * BN * 128);
+      int s = 0, i = 0;
+      for (int q = 0; q < nq && good; ++q) {
+        const int first = i, end = piece_end(q), xb = q % L::kXBufs;
+        // the small orders of the piece that had this buffer have been read
+        if (q >= L::kXBufs && !mbar_wait(smem_u32(&xempty_bar[xb]), (q / L::kXBufs - 1) & 1, abort_flag, 9)) { good = false; break; }
+        for (; i < end; ++i) {
+          // A's pieces are in place; the warps that wrote them have seen the weights land too
+          if (!mbar_wait(smem_u32(&afull_bar[i & 1]), (i >> 1) & 1, abort_flag, 5)) { good = false; break; }
+          if (i > 1 && !mbar_wait(smem_u32(&hempty_bar[i & 1]), ((i >> 1) & 1) ^ 1, abort_flag, 6)) { good = false; break; }
+          tcgen05_fence_after();
+          const int a = i & 1;
+          const uint32_t sw = smem_u32(smem + s * L::kStage) + L::kRaw, a1 = tmem + L::kACol + a * 96;
+          const uint32_t h = tmem + a * 2 * BN, x = tmem + L::kXCol + xb * BN;
+          const uint64_t w1 = make_smem_desc(sw), w2 = make_smem_desc(sw + BN * 128), w3 = make_smem_desc(sw + 2 * BN * 128);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) mma_ts(h + (k >> 1) * BN, a1 + (k >> 1) * 48 + 8 * (k & 1), w1 + 2 * k, one, (k & 1) ? 1u : 0u);
-        tcgen05_commit(smem_u32(&hfull_bar[a]));
+          for (int k = 0; k < 4; ++k) mma_ts(h + (k >> 1) * BN, a1 + (k >> 1) * 48 + 8 * (k & 1), w1 + 2 * k, one, (k & 1) ? 1u : 0u);
+          tcgen05_commit(smem_u32(&hfull_bar[a]));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t ak = a1 + (k >> 1) * 48 + 8 * (k & 1);
-          mma_ts(x, ak, w3 + 2 * k, one, (i > 0 || k > 0) ? 1u : 0u);
-          mma_ts(x, ak + 16, w2 + 2 * k, one, 1u);
-          mma_ts(x, ak + 32, w1 + 2 * k, one, 1u);
-          mma_ts(x, ak, w2 + 2 * k, one, 1u);
-          mma_ts(x, ak + 16, w1 + 2 * k, one, 1u);
+          for (int k = 0; k < 4; ++k) {
+            const uint32_t ak = a1 + (k >> 1) * 48 + 8 * (k & 1);
+            mma_ts(x, ak, w3 + 2 * k, one, (i > first || k > 0) ? 1u : 0u);
+            mma_ts(x, ak + 16, w2 + 2 * k, one, 1u);
+            mma_ts(x, ak + 32, w1 + 2 * k, one, 1u);
+            mma_ts(x, ak, w2 + 2 * k, one, 1u);
+            mma_ts(x, ak + 16, w1 + 2 * k, one, 1u);
+          }
+          tcgen05_commit(smem_u32(&aempty_bar[a]));
+          tcgen05_commit(smem_u32(&empty_bar[s]));
+          if (++s == S) s = 0;
         }
-        tcgen05_commit(smem_u32(&aempty_bar[a]));
-        tcgen05_commit(smem_u32(&empty_bar[s]));
-        if (++s == S) s = 0;
+        if (good) tcgen05_commit(smem_u32(&xfull_bar[xb]));
       }
-      if (good) tcgen05_commit(smem_u32(xfull_bar));
     }
     __syncwarp();
   } else {
@@ -301,56 +336,99 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     constexpr int kCols = BN / 2;
     const int quarter = warp & 3, half = (warp - 10) >> 2;
     const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + half * kCols;
-    float acc[kCols];
-#pragma unroll
-    for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
+    constexpr bool kKeep = kMode == kInTurn && !L::kOutBehind;
+    float acc[kCols], tot[kKeep ? kCols : 1];
+    float* row = out + (quarter * 32 + lane) * (BN + 4) + half * kCols;
     bool good = true;
-    for (int i = 0; i < kbn; ++i) {
-      const int b = i & 1;
-      if (!mbar_wait(smem_u32(&hfull_bar[b]), (i >> 1) & 1, abort_flag, 7)) { good = false; break; }
+    for (int q = 0, i = 0; q < nq && good; ++q) {
+      const int end = piece_end(q), xb = q % L::kXBufs;
+#pragma unroll
+      for (int j = 0; j < kCols; ++j) acc[j] = 0.f;
+      for (; i < end; ++i) {
+        const int b = i & 1;
+        if (!mbar_wait(smem_u32(&hfull_bar[b]), (i >> 1) & 1, abort_flag, 7)) { good = false; break; }
+        tcgen05_fence_after();
+#pragma unroll
+        for (int c = 0; c < kCols; c += 16) {
+          uint32_t r0[16], r1[16];
+          tmem_ld16(ta + 2 * b * BN + c, r0);
+          tmem_ld16(ta + (2 * b + 1) * BN + c, r1);
+          tmem_ld_wait();
+          if (c + 16 >= kCols) {  // the last columns are in registers: the k-block after the next may overwrite them
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&hempty_bar[b]));
+          }
+#pragma unroll
+          for (int k = 0; k < 16; ++k)
+            acc[c + k] = __fadd_rn(acc[c + k], __fadd_rn(__uint_as_float(r0[k]), __uint_as_float(r1[k])));
+        }
+      }
+      if (good) good = mbar_wait(smem_u32(&xfull_bar[xb]), (q / L::kXBufs) & 1, abort_flag, 8);
       tcgen05_fence_after();
+      // the piece's sums, the small orders last
 #pragma unroll
       for (int c = 0; c < kCols; c += 16) {
-        uint32_t r0[16], r1[16];
-        tmem_ld16(ta + 2 * b * BN + c, r0);
-        tmem_ld16(ta + (2 * b + 1) * BN + c, r1);
+        uint32_t x[16];
+        tmem_ld16(ta + L::kXCol + xb * BN + c, x);
         tmem_ld_wait();
-        if (c + 16 >= kCols) {  // the last columns are in registers: the k-block after the next may overwrite them
+        if (kMode == kInTurn && c + 16 >= kCols) {
           tcgen05_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&hempty_bar[b]));
+          if (lane == 0) mbar_arrive(smem_u32(&xempty_bar[xb]));
         }
 #pragma unroll
-        for (int k = 0; k < 16; ++k)
-          acc[c + k] = __fadd_rn(acc[c + k], __fadd_rn(__uint_as_float(r0[k]), __uint_as_float(r1[k])));
+        for (int j = 0; j < 16; j += 4) {
+          float4 v = make_float4(__fadd_rn(acc[c + j], __uint_as_float(x[j])), __fadd_rn(acc[c + j + 1], __uint_as_float(x[j + 1])),
+                                 __fadd_rn(acc[c + j + 2], __uint_as_float(x[j + 2])), __fadd_rn(acc[c + j + 3], __uint_as_float(x[j + 3])));
+          if constexpr (kKeep) {
+            if (q > 0) v = add_rn(make_float4(tot[c + j], tot[c + j + 1], tot[c + j + 2], tot[c + j + 3]), v);
+            tot[c + j] = v.x; tot[c + j + 1] = v.y; tot[c + j + 2] = v.z; tot[c + j + 3] = v.w;
+          } else {
+            if (kMode == kInTurn && q > 0) v = add_rn(*reinterpret_cast<const float4*>(row + c + j), v);
+            *reinterpret_cast<float4*>(row + c + j) = v;  // where the ring was, which is free after the only piece, or behind it
+          }
+        }
       }
     }
-    if (good) good = mbar_wait(smem_u32(xfull_bar), 0, abort_flag, 8);
-    tcgen05_fence_after();
-    // the ring is free: the sums go through it, together with the small orders
-    float* out = reinterpret_cast<float*>(smem);
-    float* row = out + (quarter * 32 + lane) * (BN + 4) + half * kCols;
+    if constexpr (kKeep) {
 #pragma unroll
-    for (int c = 0; c < kCols; c += 16) {
-      uint32_t x[16];
-      tmem_ld16(ta + L::kXCol + c, x);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 16; j += 4)
-        *reinterpret_cast<float4*>(row + c + j) =
-            make_float4(__fadd_rn(acc[c + j], __uint_as_float(x[j])), __fadd_rn(acc[c + j + 1], __uint_as_float(x[j + 1])),
-                        __fadd_rn(acc[c + j + 2], __uint_as_float(x[j + 2])), __fadd_rn(acc[c + j + 3], __uint_as_float(x[j + 3])));
+      for (int c = 0; c < kCols; c += 4) *reinterpret_cast<float4*>(row + c) = make_float4(tot[c], tot[c + 1], tot[c + 2], tot[c + 3]);
     }
     tcgen05_fence_before();
-    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if constexpr (kMode != kCluster) asm volatile("bar.sync 1, 256;" ::: "memory");
+  }
+  auto free_tmem = [&] {
+    if (warp == 9) {
+      tcgen05_fence_after();
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)L::kCols) : "memory");
+    }
+    __syncwarp();
+  };
+  if constexpr (kMode == kCluster) {
+    // The sums of the others' pieces.  Tensor memory is given back ahead of the wait for them: an SM of theirs may be held by a
+    // cluster of another network's kernel that waits for this one's.
+    __syncwarp();
+    tcgen05_fence_before();
+    __syncthreads();
+    free_tmem();
+    cluster_sync_all();
+  }
+
+  if (warp >= 10) {
     grid_dependency_wait();  // the residual input
     const int t = tid - 320;
 #pragma unroll 1
-    for (int e = t * 4; e < 128 * BN; e += 1024) {
+    for (int e = t * 4 + rank * 1024; e < 128 * BN; e += 1024 * ks) {  // the CTAs of a cluster take turns
       const int r = e / BN, c = e % BN, m = m0 + r, n = n0 + c;
-      const float4 q = *reinterpret_cast<const float4*>(out + r * (BN + 4) + c);
-      float v[4] = {q.x, q.y, q.z, q.w};
       const bool in = m < p.M && n < p.N;
+      const float* mine = out + r * (BN + 4) + c;
+      float4 q = *reinterpret_cast<const float4*>(mine);
+      if (kMode == kCluster && in) {
+        q = load_peer(mine, 0);
+        for (int j = 1; j < ks; ++j) q = add_rn(q, load_peer(mine, j));
+      }
+      float v[4] = {q.x, q.y, q.z, q.w};
       bool again = false;
 #pragma unroll
       for (int j = 0; j < 4; ++j) again |= in && n + j < p.N && !(fabsf(v[j]) <= 3.402823466e38f);
@@ -396,11 +474,13 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       }
     }
   }
-  tcgen05_fence_before();
-  __syncthreads();
-  if (warp == 9) {
-    tcgen05_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)L::kCols) : "memory");
+  __syncwarp();
+  if constexpr (kMode == kCluster) {
+    cluster_sync_all();  // the others have read this CTA's sums
+  } else {
+    tcgen05_fence_before();
+    __syncthreads();
+    free_tmem();
   }
   if (*abort_flag) {
     // Give copies that may still be in flight time to land before the CTA's shared memory is released.
@@ -409,36 +489,66 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   }
 }
 
-template <int BN, bool kConv>
+template <int BN, bool kConv, F32Pieces kMode>
 cudaError_t launch_f32_bn(const F32Params& p, const void* planes, cudaStream_t s) {
   using L = F32Tile<BN>;
-  auto kernel = gemm_f32_kernel<BN, kConv>;
-  static std::atomic<unsigned long long> attr_mask{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  cudaError_t e = raise_smem_limit<&gemm_f32_kernel<BN, kConv, kMode>>(L::bytes(kMode));
   if (e != cudaSuccess) return e;
-  if (!(attr_mask.load() >> (dev & 63) & 1ull)) {
-    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes)) != cudaSuccess) return e;
-    attr_mask.fetch_or(1ull << (dev & 63));
-  }
   CUtensorMap ma, mw;
   if ((e = gemm_f32_map(p.A, p.lda, p.M, kConv ? p.conv_cin : p.K, kConv, &ma)) != cudaSuccess) return e;
   const int rows = 3 * (kConv ? 9 : 1) * p.N, cols = kConv ? p.conv_cin : p.K;
   if ((e = gemm_tensor_map(planes, cols, rows, cols, BN, TypeTag<__nv_bfloat16>::prec, &mw)) != cudaSuccess) return e;
-  return launch_dependent(kernel, dim3(ceil_div(p.N, BN), ceil_div(p.M, 128)), dim3(kF32Threads), L::kBytes, s, ma, mw, p);
+  const int ks = kMode == kCluster ? p.pieces : 1;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(ceil_div(p.N, BN) * ks, ceil_div(p.M, 128));
+  lc.blockDim = dim3(kF32Threads);
+  lc.dynamicSmemBytes = L::bytes(kMode);
+  lc.stream = s;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (kMode == kCluster) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = ks;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  if (t_dependent_launch) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  lc.attrs = attr;
+  lc.numAttrs = na;
+  return cudaLaunchKernelEx(&lc, gemm_f32_kernel<BN, kConv, kMode>, ma, mw, p);
 }
+
+// Pieces that K is summed in, from N and K alone, so that a row's sum is the same in every batch: one to about nine k-blocks where the
+// columns are so few that the tiles of a small batch leave most SMs idle.  fp32 networks, us, FMA kernel / one piece / pieces: 20 x 256
+// residual 1 board 1131 / 1282 / 616, 3 1156 / 1332 / 631, 8 1674 / 1340 / 664; 10 x 128 4 boards 405 / 418 / 308; three blocks of
+// 512 filters 1 board 467 / 664 / 370.  Taken in turn they cost a few per cent where the tiles fill the GPU (20 x 256, 64
+// boards 7485 / 1724 / 1774; 10 x 128 1315 / 458 / 468).
+int f32_pieces(int N, int k_blocks) {
+  return N > 512 || k_blocks < 18 ? 1 : k_blocks < 36 ? 2 : k_blocks < 72 ? 4 : 8;
+}
+
 
 // Tile width: rounds of tiles (one per SM) times a tile's time, its k-blocks and its ends in ns.  Measured at 32 / 64 columns, us:
 // 64x1024x1024 13.0 / 16.3, 1024x1024x1024 28.0 / 19.6, 1024x1024x1536 37.1 / 25.4, 1024x3072x1024 82 / 56, 512x4096x256 27.8 / 19.8,
 // convolution of 64 boards 16.3 / 20.7, of 512 111 / 82.
 template <bool kConv>
-cudaError_t launch_f32(const F32Params& p, const void* planes, int sm_count, cudaStream_t s) {
+cudaError_t launch_f32(F32Params& p, const void* planes, int sm_count, cudaStream_t s) {
   const long long m_tiles = ceil_div(p.M, 128);
   auto cost = [&](int bn, int block, int ends) {
     return ceil_div(m_tiles * ceil_div(p.N, bn), sm_count) * ((long long)p.k_blocks * block + ends);
   };
-  if (cost(32, 525, 4800) < cost(64, 700, 7000)) return launch_f32_bn<32, kConv>(p, planes, s);
-  return launch_f32_bn<64, kConv>(p, planes, s);
+  p.pieces = f32_pieces(p.N, p.k_blocks);
+  const bool narrow = cost(32, 525, 4800) < cost(64, 700, 7000);
+  if (p.pieces == 1)
+    return narrow ? launch_f32_bn<32, kConv, kOnePiece>(p, planes, s) : launch_f32_bn<64, kConv, kOnePiece>(p, planes, s);
+  // clusters while the tiles of 32 columns times the pieces are one round (an eighth of the SMs may not form whole clusters)
+  if (m_tiles * ceil_div(p.N, 32) * p.pieces <= sm_count - sm_count / 8) return launch_f32_bn<32, kConv, kCluster>(p, planes, s);
+  return narrow ? launch_f32_bn<32, kConv, kInTurn>(p, planes, s) : launch_f32_bn<64, kConv, kInTurn>(p, planes, s);
 }
 
 bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }

@@ -154,6 +154,31 @@ def test_fp32_tensor_core_products(lib, conv, shape):
         assert torch.equal(_f32_op(lib, A[:rows], W, b, None, conv), whole[:rows])
 
 
+@pytest.mark.parametrize("conv,N,K", [(0, 512, 1088), (0, 512, 1152), (0, 520, 1152), (0, 33, 2240), (0, 96, 2304), (0, 64, 4544), (0, 250, 4608),
+                                      (1, 128, 64), (1, 96, 112), (1, 128, 128), (1, 256, 256), (1, 40, 448), (1, 512, 512), (1, 520, 512)])
+def test_fp32_tensor_core_products_in_pieces_of_k(lib, conv, N, K):
+    """Both sides of the lines where K is summed in two, four and eight pieces (18, 36 and 72 k-blocks, 512 columns): a CTA of a cluster
+    for each piece on few rows, in turn on tiles of 32 and of 64 columns beyond; the same bits everywhere."""
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    A = torch.randn(64 * 150, K, device="cuda", generator=g)
+    W = torch.randn(*((9, N, K) if conv else (N, K)), device="cuda", generator=g) * K ** -0.5
+    b, skip = torch.randn(N, device="cuda", generator=g), torch.randn(A.shape[0], N, device="cuda", generator=g)
+    plain = _f32_op(lib, A, W, None, None, conv)
+    want, size = _f32_want(A[:640], W, conv)
+    # as in test_fp32_tensor_core_products: a piece's two additions more are at most what its shorter chains save
+    blocks = (9 if conv else 1) * ((K + 63) // 64)
+    assert ((plain[:640].double() - want).abs() <= (4 + 2 * blocks + 1) * 2.0 ** -24 * size).all()
+    whole = _f32_op(lib, A, W, b, skip, conv, oracle.ACT_RELU, 0.5)
+    ref = torch.add(skip, torch.relu(plain + b), alpha=0.5)
+    assert ((whole - ref).abs() <= 2.0 ** -22 * (ref.abs() + skip.abs())).all()  # the epilogue alone, contracted or not
+    for rows in (64, 128, 192, 256, 640, 1600, 4096):
+        assert torch.equal(_f32_op(lib, A[:rows], W, None, None, conv), plain[:rows])
+        assert torch.equal(_f32_op(lib, A[:rows], W, b, skip[:rows], conv, oracle.ACT_RELU, 0.5), whole[:rows])
+    A[3, 5], A[70, 1] = float("inf"), float("nan")  # computed again by FMAs, also from the sums of a cluster
+    few, many = _f32_op(lib, A[:128], W, b, None, conv), _f32_op(lib, A, W, b, None, conv)[:128]
+    assert torch.equal(few.nan_to_num(7e4, 8e4, 9e4), many.nan_to_num(7e4, 8e4, 9e4)) and not torch.isfinite(few[3]).any()
+
+
 def _taps(A):
     """The rows of A that a 3x3 convolution reads, side by side: [M][9 * K]."""
     x = torch.nn.functional.pad(A.view(-1, 8, 8, A.shape[1]), (0, 0, 1, 1, 1, 1))
